@@ -14,12 +14,12 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT_DIR, "libcxg.so")
-SOURCES = ["cxg_api.cu", "cxg_kernels.cu", "cxg_pattern.cu", "cxg_v2.cu", "cxg_solve.cu", "cxg_batch.cu", "cxg_recover.cu",
+SOURCES = ["cxg_api.cu", "cxg_kernels.cu", "cxg_pattern.cu", "cxg_v2.cu", "cxg_fp64.cu", "cxg_gather.cu", "cxg_solve.cu", "cxg_batch.cu", "cxg_recover.cu",
            "cxg_refpattern.cu", "cxg_mpc.cu", "cxg_sparse_solve.cu", "cxg_film.cu"]
 # Per-file flags: the reference-pattern mask evaluates K_e in the reference's own FP64
 # operation order, so it must not contract multiply-adds.
 EXTRA_FLAGS = {"cxg_refpattern.cu": ["-fmad=false"]}
-HEADERS = ["cxg_internal.cuh", "cxg_elements.hpp", "cxg_plan.hpp", os.path.join("..", "..", "include", "cxg.h")]
+HEADERS = ["cxg_internal.cuh", "cxg_element.cuh", "cxg_elements.hpp", "cxg_plan.hpp", os.path.join("..", "..", "include", "cxg.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -347,7 +347,8 @@ V2Args v2_args(cxg_plan* p, const double* f_ext, bool accumulate) {
   v.inc_ptr = p->pat.inc_ptr;
   v.inc_code = p->pat.inc_code;
   v.f_ext = f_ext;
-  v.max_adj = p->pat.max_adj;
+  v.npe = nodes_of(p->type);
+  v.nbp = blocks_padded(v.npe);
   v.accumulate = accumulate ? 1 : 0;
   v.e_begin = 0;
   v.e_end = p->n_elems;
@@ -370,15 +371,12 @@ ElemArgs base_args(cxg_plan* p) {
   a.poisson = p->poisson;
   a.elem_mat = p->elem_mat;
   a.mats = p->mats;
-  a.node_base = p->pat.node_base;
-  a.node_rowlen = p->pat.node_rowlen;
+  a.node = p->pat.node;
   a.node_mask = p->pat.node_mask;
-  a.node_eq0 = p->pat.node_eq0;
   a.prescribed = p->prescribed;
-  a.slot = p->pat.slot;
-  a.adj_len = p->pat.adj_len;
-  a.bnd_ptr = p->pat.bnd_ptr;
+  a.pairs = p->pat.pairs;
   a.bnd_node = p->pat.bnd_node;
+  a.bnd_col = p->pat.bnd_col;
   a.n_gauss = p->n_gauss;
   a.status = p->status;
   a.th_temp = p->th_temp;
@@ -611,8 +609,8 @@ int cxg_plan_destroy(cxg_plan* p) {
   thermal::release(p);
   cudaFree(p->film_mem);
   void* bufs[] = {p->coords, p->conn, p->young, p->poisson, p->elem_mat, p->mats, p->dof_eq, p->prescribed,
-                  p->pat.row_ptr, p->pat.col_idx, p->pat.node_base, p->pat.node_rowlen, p->pat.node_mask,
-                  p->pat.node_eq0, p->pat.slot, p->pat.adj_len, p->pat.bnd_ptr, p->pat.bnd_node, p->pat.inc_ptr, p->pat.inc_code, p->state[0], p->state[1],
+                  p->pat.row_ptr, p->pat.col_idx, p->pat.node, p->pat.node_mask, p->pat.pairs,
+                  p->pat.bnd_node, p->pat.bnd_col, p->pat.inc_ptr, p->pat.inc_code, p->state[0], p->state[1],
                   p->status, p->edata, p->fdata};
   for (void* b : bufs) cudaFree(b);
   for (auto& row : p->sched)

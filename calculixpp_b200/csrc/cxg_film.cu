@@ -21,10 +21,8 @@ namespace cxg {
 
 namespace {
 
-__host__ __device__ constexpr int upper_block(int n, int a, int b) { return a * n - a * (a - 1) / 2 + (b - a); }
-
 __global__ void film_elem_kernel(ElemArgs A, int type, FilmArgs F, double* edata) {
-  const int n = nodes_of(type), NB = n * (n + 1) / 2;
+  const int n = nodes_of(type), nbp = blocks_padded(n);
   constexpr double kTri[3][3] = {{1.0 / 6.0, 1.0 / 6.0, 1.0 / 6.0},
                                  {2.0 / 3.0, 1.0 / 6.0, 1.0 / 6.0},
                                  {1.0 / 6.0, 2.0 / 3.0, 1.0 / 6.0}};
@@ -33,7 +31,7 @@ __global__ void film_elem_kernel(ElemArgs A, int type, FilmArgs F, double* edata
   for (int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; g < F.n_felem;
        g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t e = F.felem[g];
-    double* blocks = edata + e * (static_cast<int64_t>(NB) * 10);
+    double* blocks = edata + e * (static_cast<int64_t>(nbp) * 9);
     for (int32_t k = F.fptr[g]; k < F.fptr[g + 1]; ++k) {
       const int32_t f = F.flist[k];
       int fn[8], nf = 0;
@@ -72,7 +70,7 @@ __global__ void film_elem_kernel(ElemArgs A, int type, FilmArgs F, double* edata
         for (int j = 0; j < nf; ++j) {
           const int a = fn[i], b = fn[j];
           if (a > b) continue;  // the stored upper block (a, b) carries the pair once
-          double* blk = blocks + upper_block(n, a, b) * 10;
+          double* blk = blocks + blk_index(n, a, b) * 9;
           const double v = h * M[i][j];
           blk[0] += v;
           blk[4] += v;

@@ -1,0 +1,359 @@
+// P2, the row gather: every CSR value written exactly once, no atomics, no shared memory.
+//
+// One warp per node a. The plan lists the element blocks that contribute to a's node pairs
+// (a, b), pair by pair and in element order, in records of 11 (NodeRec, PairRec). Three
+// groups of nine lanes each walk a third of that list; a lane carries one entry of the 3x3
+// block. A contribution is one coalesced 72-byte (FP32: 36-byte) read and one add in a
+// register, and where a pair ends the group writes its block, three runs of three values
+// that the next pairs of the same rows continue. The three runs are padded to the same
+// number of records, so a round is straight-line code: 11 block reads in flight per lane,
+// the next record fetched meanwhile.
+//
+// What bounds it: the element blocks come in from HBM once and the values go out once;
+// in between the L1 serves every block twice (rows of a and of b).
+//
+// Mixed precision (DIAG) forms the diagonal block as minus the FP64 sum of the row's
+// other entries (per group, then the three groups in order; the element pass stores the
+// blocks (a, a) as zeros), so rigid translations stay in the null space to FP64 accuracy. Interior nodes (every neighbour fully free) write
+// full-width rows; at the others the list of neighbours gives each pair's compressed
+// column, and prescribed columns go to the rhs (-K_fc u_c, src/fem/assembly.cpp:95-96).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "cxg_internal.cuh"
+
+namespace cxg {
+
+namespace {
+
+constexpr unsigned kAll = 0xffffffffu;
+
+__device__ __forceinline__ NodeRec load_node(const NodeRec* p) {
+  union {
+    int4 q[3];
+    NodeRec r;
+  } u;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) u.q[i] = __ldg(reinterpret_cast<const int4*>(p) + i);
+  return u.r;
+}
+
+__device__ __forceinline__ PairRec load_pairs(const PairRec* p) {
+  union {
+    int4 q[3];
+    PairRec r;
+  } u;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) u.q[i] = __ldg(reinterpret_cast<const int4*>(p) + i);
+  return u.r;
+}
+
+// Index of a stored block in the element buffer. With windows the buffer is a ring of
+// `ring` elements; every element of a window lies in [ring_base, ring_base + 2 ring), so
+// one conditional subtraction gives the slot.
+template <bool WIN>
+__device__ __forceinline__ int64_t block_slot(uint32_t block, int64_t ring_blocks, int64_t base_blocks) {
+  if constexpr (WIN) {
+    const int64_t d = static_cast<int64_t>(block) - base_blocks;
+    return d < ring_blocks ? d : d - ring_blocks;
+  }
+  return block;
+}
+
+// Where a pair ends: write the entry, start the next pair three columns on. Predicated
+// rather than branched: some group ends a pair at most steps.
+template <bool SUM>
+__device__ __forceinline__ void end_pair(unsigned last, double*& o, double& v, double& sum) {
+  if constexpr (SUM)
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.u32 p, %3, 0;\n@p st.global.f64 [%0], %1;\n@p add.f64 %2, %2, %1;\n"
+        "@p mov.f64 %1, 0d0000000000000000;\n@p add.s64 %0, %0, 24;\n}"
+        : "+l"(o), "+d"(v), "+d"(sum)
+        : "r"(last)
+        : "memory");
+  else
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.global.f64 [%0], %1;\n"
+        "@p mov.f64 %1, 0d0000000000000000;\n@p add.s64 %0, %0, 24;\n}"
+        : "+l"(o), "+d"(v)
+        : "r"(last)
+        : "memory");
+}
+
+template <typename R, int KIND, bool WIN>
+__device__ __forceinline__ void gather_nodes(const ElemArgs& A, const V2Args& V, unsigned bid, unsigned nblk) {
+  constexpr bool DIAG = KIND == GATHER_DIAG;
+  constexpr int UN = kPairRec;
+  const int lane = threadIdx.x & 31;
+  const int64_t gwarp = static_cast<int64_t>(bid) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t nwarps = static_cast<int64_t>(nblk) * (blockDim.x >> 5);
+  // lanes 27 .. 31 follow the third group without writing
+  const int q = min(lane / 9, 2), k = lane < 27 ? lane - 9 * q : 0, ki = k / 3, kj = k - 3 * ki;
+  const R* ed = reinterpret_cast<const R*>(V.edata) + k;
+  const int64_t ring_blocks = V.ring * V.nbp, base_blocks = V.ring_base * V.nbp;
+  const int64_t n_begin = WIN ? V.n_begin : 0, n_end = WIN ? V.n_end : A.n_nodes;
+  for (int64_t idx = n_begin + gwarp; idx < n_end; idx += nwarps) {
+    const int64_t a = WIN ? static_cast<int64_t>(V.node_order[idx]) : n_end - 1 - idx;
+    const NodeRec nd = load_node(A.node + a);
+    const int K = nd.npair, L = nd.len_mask & 0xfffffff, ma = nd.len_mask >> 28, self = nd.diag;
+    const bool full = L == 3 * K, plain = full && !V.accumulate;
+    double* const rows = A.vals + nd.base;
+    // what prescribed columns move to the rhs: of row ki (own pair and later ones), of
+    // row kj (earlier ones)
+    double rd = 0.0, rt = 0.0;
+    // the lane's entry of the block of pair p, wherever it goes
+    auto put = [&](int p, double v) {
+      const int i = p < self ? kj : ki, j = p < self ? ki : kj;
+      if (full) {
+        double* o = rows + i * L + 3 * p + j;
+        *o = V.accumulate ? *o + v : v;
+        return;
+      }
+      if (!((ma >> i) & 1)) return;
+      const uint32_t at = static_cast<uint32_t>(__ldg(A.bnd_col + nd.bnd0 + p));
+      const int mb = at >> 28;
+      if ((mb >> j) & 1) {
+        double* o = rows + static_cast<int64_t>(__popc(ma & ((1 << i) - 1))) * L + (at & 0xfffffff) +
+                    __popc(mb & ((1 << j) - 1));
+        *o = V.accumulate ? *o + v : v;
+      } else {
+        const double c = v * A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p)) + j];
+        if (p < self)
+          rt -= c;
+        else
+          rd -= c;
+      }
+    };
+    if (ma) {
+      int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
+      const PairRec* list = A.pairs + nd.list0 + q;
+      PairRec rec;
+      if (nd.rounds) rec = load_pairs(list);
+      // the off-diagonal blocks' sums (DIAG): entry (ki, kj) of the blocks from the own
+      // pair on, entry (kj, ki) of those before it
+      double own = 0.0, before = 0.0;
+      double v = 0.0;
+      // before the own pair a lane writes entry (kj, ki), from there on (ki, kj)
+      double* o = rows + 3 * p + (p < self ? kj * L + ki : ki * L + kj);
+      const int64_t turn = static_cast<int64_t>(ki - kj) * (L - 1);
+      for (uint32_t r = 0; r < nd.rounds; ++r) {
+        R x[UN];
+#pragma unroll
+        for (int i = 0; i < UN; ++i) {
+          x[i] = __ldg(ed + 9 * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks));
+        }
+        const bool turns = rec.flags >> 31;
+        const unsigned ends = lane < 27 ? rec.flags : 0u;
+        list += 3;
+        if (r + 1 < nd.rounds) rec = load_pairs(list);
+        if (plain && !turns) {
+#pragma unroll
+          for (int i = 0; i < UN; ++i) {
+            v += static_cast<double>(x[i]);
+            end_pair<DIAG>(ends & (1u << i), o, v, own);
+          }
+        } else if (plain) {
+#pragma unroll
+          for (int i = 0; i < UN; ++i) {
+            v += static_cast<double>(x[i]);
+            end_pair<DIAG>(ends & (1u << i), o, v, own);
+            if (ends & (0x10000u << i)) {
+              o += turn;
+              if (DIAG) before = own;
+              own = DIAG ? 0.0 : own;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < UN; ++i) {
+            v += static_cast<double>(x[i]);
+            if (ends & (1u << i)) {
+              if (!DIAG || p != self) put(p, v);
+              own += v;
+              v = 0.0;
+              ++p;
+              if (DIAG && (ends & (0x10000u << i))) {
+                before = own;
+                own = 0.0;
+              }
+            }
+          }
+        }
+      }
+      if constexpr (DIAG) {
+        // a run that ends before the own pair holds earlier pairs only
+        if ((q == 0 ? nd.pair1 : q == 1 ? nd.pair2 : K) <= self) {
+          before = own;
+          own = 0.0;
+        }
+        __syncwarp();  // orders the block below after the loop's write of the same place
+        const double t = own + __shfl_sync(kAll, before, min(9 * (lane / 9) + 3 * kj + ki, 31));
+        const double t1 = __shfl_sync(kAll, t, (lane + 9) & 31), t2 = __shfl_sync(kAll, t, (lane + 18) & 31);
+        if (lane < 9 && K > 0) put(self, -((t + t1) + t2));
+      }
+      if (A.rhs) {
+        double v = 0.0;
+        if (!full) {  // (full rows have no prescribed column)
+          rd += __shfl_down_sync(kAll, rd, 9) + __shfl_down_sync(kAll, rd, 18);
+          rt += __shfl_down_sync(kAll, rt, 9) + __shfl_down_sync(kAll, rt, 18);
+          rd += __shfl_down_sync(kAll, rd, 1) + __shfl_down_sync(kAll, rd, 2);  // lane 3 i: row i
+          rt += __shfl_down_sync(kAll, rt, 3) + __shfl_down_sync(kAll, rt, 6);  // lane i: row i
+          v = rd + __shfl_sync(kAll, rt, lane / 3);
+        }
+        if (lane == 0 || lane == 3 || lane == 6) {
+          const int r = lane / 3;
+          if ((ma >> r) & 1) {
+            const int64_t eq = nd.eq0 + __popc(ma & ((1 << r) - 1));
+            const double prev = V.accumulate ? A.rhs[eq] : (V.f_ext ? V.f_ext[3 * a + r] : 0.0);
+            A.rhs[eq] = prev + v;
+          }
+        }
+      }
+    }
+  }
+}
+
+template <typename R, int KIND, bool WIN>
+__global__ void __launch_bounds__(256, 3) gather_kernel(ElemArgs A, V2Args V) {
+  gather_nodes<R, KIND, WIN>(A, V, blockIdx.x, gridDim.x);
+}
+
+// Internal force of every node: one thread per component, the element forces in element
+// order. Beside the row gather the three dependent loads of this sum cost every node
+// their latency; here they overlap across threads.
+template <bool WIN>
+__global__ void __launch_bounds__(256) force_kernel(ElemArgs A, V2Args V) {
+  const int64_t first = 3 * (WIN ? V.n_begin : 0), last = 3 * (WIN ? V.n_end : A.n_nodes);
+  for (int64_t t = first + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < last;
+       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t a = WIN ? static_cast<int64_t>(V.node_order[t / 3]) : t / 3;
+    const int d = static_cast<int>(t % 3);
+    const int64_t i1 = V.inc_ptr[a + 1];
+    double f = 0.0;
+#pragma unroll 4
+    for (int64_t i = V.inc_ptr[a]; i < i1; ++i) {
+      int64_t s = __ldg(V.inc_code + i);
+      if constexpr (WIN) {
+        s -= V.ring_base * V.npe;
+        if (s >= V.ring * V.npe) s -= V.ring * V.npe;
+      }
+      f += __ldg(V.fdata + 3 * s + d);
+    }
+    A.f_int[3 * a + d] = (V.accumulate ? A.f_int[3 * a + d] : 0.0) + f;
+  }
+}
+
+int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+cudaError_t launch_forces(const ElemArgs& a, const V2Args& v, cudaStream_t s) {
+  const int64_t count = 3 * (v.n_end - v.n_begin);
+  if (!a.f_int || count <= 0) return cudaSuccess;
+  const int64_t grid = std::min<int64_t>((count + 255) / 256, 8 * static_cast<int64_t>(sm_count()));
+  (v.node_order ? force_kernel<true> : force_kernel<false>)<<<static_cast<unsigned>(grid), 256, 0, s>>>(a, v);
+  return cudaGetLastError();
+}
+
+template <typename R, int KIND>
+cudaError_t launch_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, cudaStream_t s) {
+  auto kern = v.node_order ? gather_kernel<R, KIND, true> : gather_kernel<R, KIND, false>;
+  const int warps = cfg.p2_warps > 0 ? std::min(cfg.p2_warps, 8) : 8;
+  const int64_t count = v.n_end - v.n_begin;
+  if (count <= 0) return cudaSuccess;
+  int per_sm = 0;
+  const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, 0);
+  if (err != cudaSuccess) return err;
+  if (cfg.p2_blocks_per_sm > 0) per_sm = std::min(per_sm, cfg.p2_blocks_per_sm);
+  const int64_t grid = std::min<int64_t>((count + warps - 1) / warps, static_cast<int64_t>(std::max(per_sm, 1)) * sm_count());
+  kern<<<static_cast<unsigned>(grid), warps * 32, 0, s>>>(a, v);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_gather(int kind, bool tangent, const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg,
+                          cudaStream_t s) {
+  cudaError_t e;
+  switch (kind) {
+    case GATHER_FULL: e = launch_t<double, GATHER_FULL>(a, v, cfg, s); break;
+    case GATHER_DIAG: e = launch_t<float, GATHER_DIAG>(a, v, cfg, s); break;
+    default: return cudaErrorInvalidValue;
+  }
+  return e == cudaSuccess && tangent ? launch_forces(a, v, s) : e;
+}
+
+// ---- one gather for a batch of element-type groups ------------------------------------
+namespace {
+
+struct GatherSlot {
+  ElemArgs a;
+  V2Args v;
+  int64_t blk0;
+};
+struct GatherPass {
+  GatherSlot s[kMaxBatchSlots];
+  int32_t n;
+};
+static_assert(sizeof(GatherPass) <= 4096, "batch pass arguments exceed the kernel parameter space");
+
+// Slot k owns blocks [blk0_k, blk0_{k+1}) of the grid; the arguments are read in place
+// from the parameter space.
+template <typename R, int KIND>
+__global__ void __launch_bounds__(256) gather_batch_kernel(const __grid_constant__ GatherPass P) {
+  int k = 0;
+  while (k + 1 < P.n && static_cast<int64_t>(blockIdx.x) >= P.s[k + 1].blk0) ++k;
+  const GatherSlot& S = P.s[k];
+  const int64_t end = k + 1 < P.n ? P.s[k + 1].blk0 : static_cast<int64_t>(gridDim.x);
+  const unsigned bid = blockIdx.x - static_cast<unsigned>(S.blk0), nblk = static_cast<unsigned>(end - S.blk0);
+  gather_nodes<R, KIND, false>(S.a, S.v, bid, nblk);
+}
+
+template <typename R, int KIND>
+cudaError_t launch_batch_t(const BatchSlotIn* in, int n, cudaStream_t s) {
+  auto kern = gather_batch_kernel<R, KIND>;
+  GatherPass P{};
+  int warps = 8;
+  for (int k = 0; k < n; ++k)
+    if (in[k].cfg.p2_warps > 0) warps = std::min(warps, in[k].cfg.p2_warps);
+  int per_sm = 0;
+  const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, 0);
+  if (err != cudaSuccess) return err;
+  if (per_sm < 1) return cudaErrorInvalidConfiguration;
+  int64_t need[kMaxBatchSlots], grid[kMaxBatchSlots];
+  double w[kMaxBatchSlots];
+  for (int k = 0; k < n; ++k) {
+    need[k] = std::max<int64_t>(1, (in[k].v.n_end - in[k].v.n_begin + warps - 1) / warps);
+    w[k] = in[k].p2_weight;
+  }
+  share_blocks(w, need, n, static_cast<int64_t>(per_sm) * sm_count(), grid);
+  int64_t blk = 0;
+  for (int k = 0; k < n; ++k) {
+    P.s[k].a = in[k].a;
+    P.s[k].v = in[k].v;
+    P.s[k].blk0 = blk;
+    blk += grid[k];
+  }
+  P.n = n;
+  kern<<<static_cast<unsigned>(blk), warps * 32, 0, s>>>(P);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_gather_batch(int kind, bool tangent, const BatchSlotIn* in, int n, cudaStream_t s) {
+  if (tangent)
+    for (int k = 0; k < n; ++k) {
+      const cudaError_t e = launch_forces(in[k].a, in[k].v, s);
+      if (e != cudaSuccess) return e;
+    }
+  if (kind == GATHER_DIAG) return launch_batch_t<float, GATHER_DIAG>(in, n, s);
+  if (kind == GATHER_FULL) return launch_batch_t<double, GATHER_FULL>(in, n, s);
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace cxg

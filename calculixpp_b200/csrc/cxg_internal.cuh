@@ -55,6 +55,49 @@ constexpr int kNTotal = nn_offset(C3D15) + nn_size(C3D15);
 extern __constant__ double c_N[kNTotal];
 extern __constant__ double c_w[8][kMaxGauss];
 
+// What the row gather needs of one node, fetched with three 16-byte loads. Its pairs
+// (neighbours, itself included, ascending) are cut into three runs of near-equal numbers
+// of contributions, starting at pairs 0, pair1 and pair2; run q's contributions are the
+// entries of the records list0 + 3 r + q, r < rounds (PairRec). Blocks of pairs with a
+// smaller node are read as stored and written transposed (see blk_index).
+struct __align__(16) NodeRec {
+  int64_t base;      // CSR offset of the node's first free row
+  uint32_t len_mask; // length of each of the node's rows | free components << 28
+  int32_t eq0;       // first free equation (or -1)
+  uint32_t list0;
+  uint32_t rounds;
+  uint32_t bnd0;     // first of the node's entries in bnd_node / bnd_col
+  uint16_t npair;
+  uint16_t diag;     // the node's own position among its pairs
+  uint16_t pair1, pair2;
+  uint32_t pad[3];
+};
+static_assert(sizeof(NodeRec) == 48, "NodeRec is three 16-byte loads");
+
+// Up to 11 contributions of element blocks to consecutive pairs of a node, in pair order
+// and element order within a pair: block[i] is e * blocks_padded(n) + blk_index(n, min,
+// max) of the pair's local nodes; bit i of flags: the last contribution of its pair; bit
+// 16 + i: and the next pair is the node with itself (bit 31: some run of this round has
+// that). Unused entries, after the last flagged one, repeat a block of the node.
+constexpr int kPairRec = 11;
+struct __align__(16) PairRec {
+  uint32_t flags;
+  uint32_t block[kPairRec];
+};
+static_assert(sizeof(PairRec) == 48, "PairRec is three 16-byte loads");
+
+// 3x3 blocks of an element in the element buffer: one per local node pair (a, b), a <= b,
+// 9 consecutive values at 9 * blk_index. The stored block is that of the two nodes in
+// ascending mesh order (K_ba where node b precedes node a), so all elements that share a
+// pair store it the same way round. An element's block count is padded so that every
+// element starts 16-byte aligned in both precisions, which bulk copies need (8-byte
+// aligned in FP32 for the families of 4 and 6 nodes, which copy with plain stores).
+__host__ __device__ constexpr int blk_index(int n, int a, int b) { return a * n - a * (a - 1) / 2 + (b - a); }
+__host__ __device__ constexpr int blocks_padded(int n) {
+  const int nb = n * (n + 1) / 2;
+  return n < 8 ? (nb + 1) / 2 * 2 : (nb + 3) / 4 * 4;
+}
+
 // Everything an element-integration launch reads or writes. Pointers are device
 // pointers; optional ones may be null.
 struct ElemArgs {
@@ -68,16 +111,13 @@ struct ElemArgs {
   const double* poisson;    // [E]
   const int32_t* elem_mat;  // [E] or null -> material 0
   const J2Mat* mats;        // [n_mats]
-  // DOF map / CSR addressing (scatter mode)
-  const int64_t* node_base;   // [N] CSR offset of the node's first free row
-  const int32_t* node_rowlen; // [N] length of each of the node's rows
+  // DOF map / CSR addressing (row gather), see PatternOut
+  const NodeRec* node;        // [N]
   const uint8_t* node_mask;   // [N] bit i: component i free
-  const int32_t* node_eq0;    // [N] first free equation of the node (or -1)
   const double* prescribed;   // [3N]
-  const uint16_t* slot;       // [E*n*n] position of node b in node a's adjacency list
-  const uint16_t* adj_len;    // [N] adjacency list length (row gather)
-  const int64_t* bnd_ptr;     // [N+1] adjacency of the compressed-row nodes
+  const PairRec* pairs;
   const int32_t* bnd_node;
+  const int32_t* bnd_col;
   // state (tangent mode), SoA [13][G]
   const double* state_c;
   double* state_t;
@@ -112,8 +152,7 @@ struct V2Args {
   const int64_t* inc_ptr;   // node -> incident elements
   const int32_t* inc_code;
   const double* f_ext;      // [3N] load vector for the rhs, or null
-  int64_t max_adj;          // longest adjacency list of any node
-  int64_t row_stride;       // set by the launcher: doubles per row-buffer copy
+  int npe, nbp;             // nodes and (padded) blocks per element
   int accumulate;           // add into vals / rhs / f_int instead of overwriting
   // The window of one element-pass + row-gather pair: the element pass integrates
   // elements [e_begin, e_end), the row gather the nodes node_order[n_begin..n_end)
@@ -155,6 +194,15 @@ struct BatchSlotIn {
   LaunchCfg cfg;
   double p1_weight = 1.0, p2_weight = 1.0;
 };
+// Blocks of a persistent grid of `total` blocks shared out in proportion to the slots'
+// weights, at least one and at most `need` per slot.
+void share_blocks(const double* weight, const int64_t* need, int n, int64_t total, int64_t* grid);
+// Row gather (cxg_gather.cu). GATHER_FULL: FP64 blocks, every entry summed; GATHER_DIAG:
+// FP32 blocks, the diagonal block from the row's other entries.
+enum GatherKind : int { GATHER_FULL = 0, GATHER_DIAG = 1 };
+cudaError_t launch_gather(int kind, bool tangent, const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg,
+                          cudaStream_t s);
+cudaError_t launch_gather_batch(int kind, bool tangent, const BatchSlotIn* slots, int n_slots, cudaStream_t s);
 cudaError_t launch_v2_batch(int mode, int precision, const BatchSlotIn* slots, int n_slots, int passes,
                             cudaStream_t s);
 // Tiles the batch kernels take (2x2; 2x4 in the mixed-precision linear pass).
@@ -262,22 +310,16 @@ struct PatternOut {
   int64_t nnz = 0;
   int64_t* row_ptr = nullptr;   // [n_free+1]
   int32_t* col_idx = nullptr;   // [nnz]
-  int64_t* node_base = nullptr;
-  int32_t* node_rowlen = nullptr;
-  uint8_t* node_mask = nullptr;
-  int32_t* node_eq0 = nullptr;
-  uint16_t* slot = nullptr;     // [E*n*n] position of node b in node a's adjacency list
-  // node adjacency (neighbours of a node, itself included, ascending): the list length
-  // of every node, and the list itself for the nodes with a neighbour that is not fully
-  // free (bnd_node[bnd_ptr[a] .. bnd_ptr[a+1]); empty for the others)
-  uint16_t* adj_len = nullptr;  // [N]
-  int64_t* bnd_ptr = nullptr;   // [N+1]
+  NodeRec* node = nullptr;      // [N]
+  uint8_t* node_mask = nullptr; // [N]
+  PairRec* pairs = nullptr;     // contributions of the element blocks, see NodeRec
+  // neighbour, and compressed column | free components << 28, of every pair of the nodes
+  // with a neighbour that is not fully free (NodeRec::bnd0)
   int32_t* bnd_node = nullptr;
+  int32_t* bnd_col = nullptr;
   // node -> incident elements, ascending element order: codes e*n + local node index
   int64_t* inc_ptr = nullptr;   // [N+1]
   int32_t* inc_code = nullptr;  // [E*n]
-  int64_t max_row = 0;          // max over nodes of (free rows) x (row length)
-  int64_t max_adj = 0;          // max over nodes of the adjacency list length
   int64_t device_bytes = 0;
 };
 // Returns a cxg_status code; on error *msg is set.

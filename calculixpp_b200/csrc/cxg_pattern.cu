@@ -12,15 +12,16 @@
 //   3. node_base(a) = exclusive scan of (free rows of a) * rowlen(a); row_ptr and
 //      col_idx follow. This relies on the reference's free numbering being ascending
 //      in g = 3*node + comp (constraint_transform.cpp:78-82), which is validated;
-//   4. the slot map stores, per element and ordered node pair (a, b), the position of b
-//      in a's adjacency list (uint16), so the row gather adds block (a, b) into a's
-//      rows with no search; the gather keeps the list length of every node (adj_len)
-//      and, for the nodes with a neighbour that is not fully free (their rows are
-//      compressed), the neighbours themselves (bnd_ptr, bnd_node).
+//   4. the sort carries with every key the element block it comes from, so the sorted
+//      values are, pair by pair and in element order, the blocks that the row gather sums;
+//      they are packed into the records it reads (NodeRec, PairRec); the nodes with a
+//      neighbour that is not fully free (their rows are compressed) also keep the
+//      neighbours and their columns (bnd_node, bnd_col).
 // The pattern is topological: an entry whose every element contribution is exactly
 // zero is kept (the reference skips exact-zero contributions, assembly.cpp:90).
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
+#include <thrust/iterator/counting_iterator.h>
 
 #include <algorithm>
 #include <cstdio>
@@ -79,14 +80,17 @@ __global__ void node_info_kernel(const int32_t* dof_eq, int64_t n_nodes, uint8_t
 }
 
 __global__ void pair_keys_kernel(const int32_t* conn, int64_t n_elems, int npe, uint64_t N,
-                                 uint64_t* keys) {
+                                 uint64_t* keys, uint32_t* codes) {
   const int64_t total = n_elems * npe * npe;
+  const int nbp = blocks_padded(npe);
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t e = i / (npe * npe);
     const int r = static_cast<int>(i % (npe * npe));
     const int a = r / npe, b = r % npe;
     keys[i] = static_cast<uint64_t>(conn[e * npe + a]) * N + static_cast<uint64_t>(conn[e * npe + b]);
+    const int blk = a <= b ? blk_index(npe, a, b) : blk_index(npe, b, a);
+    codes[i] = static_cast<uint32_t>(e * nbp + blk);
   }
 }
 
@@ -107,18 +111,80 @@ __global__ void node_ptr_kernel(const uint64_t* uniq, int64_t M, int64_t n_nodes
   }
 }
 
-__global__ void rowlen_kernel(const uint64_t* uniq, const int64_t* node_ptr, int64_t n_nodes,
-                              uint64_t N, const uint8_t* mask, int32_t* rowlen, int32_t* adj_off,
-                              int64_t* node_nnz) {
+__global__ void rowlen_kernel(const uint64_t* uniq, const uint32_t* start, const int64_t* node_ptr, int64_t n_nodes,
+                              uint64_t N, const uint8_t* mask, int32_t* rowlen, int32_t* adj_off, int64_t* node_nnz,
+                              int64_t* bnd_len, int64_t* n_rec, NodeRec* node, int* overflow) {
   for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n_nodes;
        a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t t0 = node_ptr[a], t1 = node_ptr[a + 1], k = t1 - t0;
+    NodeRec r{};
     int32_t run = 0;
-    for (int64_t t = node_ptr[a]; t < node_ptr[a + 1]; ++t) {
+    int64_t cut[2] = {t1, t1};
+    const uint64_t c0 = k > 0 ? start[t0] : 0, span = k > 0 ? start[t1] - c0 : 0;
+    for (int64_t t = t0; t < t1; ++t) {
+      const int64_t b = static_cast<int64_t>(uniq[t] % N);
+      if (b == a) r.diag = static_cast<uint16_t>(t - t0);
       adj_off[t] = run;
-      run += __popc(mask[uniq[t] % N]);
+      run += __popc(mask[b]);
+      // the cuts: the pair starts nearest to one and two thirds of the contributions
+      for (int g = 0; g < 2; ++g) {
+        const int64_t to = static_cast<int64_t>((g + 1) * span), s0 = 3 * static_cast<int64_t>(start[t] - c0),
+                      s1 = 3 * static_cast<int64_t>(start[t + 1] - c0);
+        if (cut[g] == t1 && s1 > to) cut[g] = to - s0 <= s1 - to ? t : t + 1;
+      }
     }
+    uint32_t longest = 0;
+    const int64_t at[4] = {t0, cut[0], cut[1], t1};
+    for (int g = 0; g < 3; ++g) longest = max(longest, k > 0 ? start[at[g + 1]] - start[at[g]] : 0u);
+    r.rounds = (longest + kPairRec - 1) / kPairRec;
+    r.npair = static_cast<uint16_t>(k);
+    r.pair1 = static_cast<uint16_t>(cut[0] - t0);
+    r.pair2 = static_cast<uint16_t>(cut[1] - t0);
     rowlen[a] = run;
     node_nnz[a] = static_cast<int64_t>(__popc(mask[a])) * run;
+    if (k > 65535) atomicExch(overflow, 1);  // list positions are uint16
+    bnd_len[a] = run == 3 * k ? 0 : k;
+    n_rec[a] = 3 * static_cast<int64_t>(r.rounds);
+    node[a] = r;
+  }
+}
+
+// The contribution records of every node, one warp per node, a lane per record. A
+// contribution is the last of its pair when the next one starts another.
+__global__ void pair_rec_kernel(const NodeRec* node, const uint32_t* start, const int64_t* node_ptr,
+                                const uint32_t* codes, const uint64_t* keys, int64_t total, int64_t n_nodes,
+                                PairRec* pairs) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+  for (int64_t a = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; a < n_nodes; a += nw) {
+    const NodeRec nd = node[a];
+    const int64_t t0 = node_ptr[a], t1 = node_ptr[a + 1];
+    for (uint32_t i = lane; i < 3 * nd.rounds; i += 32) {
+      const int g = i % 3;
+      const uint32_t lo = start[g == 0 ? t0 : t0 + (g == 1 ? nd.pair1 : nd.pair2)];
+      const uint32_t hi = start[g == 2 ? t1 : t0 + (g == 0 ? nd.pair1 : nd.pair2)];
+      PairRec r;
+      // the round of the own pair's predecessor, in whichever run that is
+      const uint32_t own = start[t0 + nd.diag];
+      const int64_t cut[4] = {t0, t0 + nd.pair1, t0 + nd.pair2, t1};
+      bool turn = false;
+      for (int h = 0; h < 3; ++h)
+        turn = turn || (own > start[cut[h]] && own < start[cut[h + 1]] &&
+                        (own - 1 - start[cut[h]]) / kPairRec == i / 3);
+      r.flags = turn ? 0x80000000u : 0u;
+      for (int j = 0; j < kPairRec; ++j) {
+        const uint32_t c = lo + i / 3 * kPairRec + j;
+        if (c < hi) {
+          r.block[j] = codes[c];
+          if (c + 1 == total || keys[c] != keys[c + 1]) r.flags |= 1u << j;
+          if (c + 1 == own && c + 1 < hi) r.flags |= 0x10000u << j;
+          // (a run that begins with the own pair has no such entry)
+        } else {
+          r.block[j] = codes[hi > lo ? hi - 1 : start[t0]];
+        }
+      }
+      pairs[nd.list0 + i] = r;
+    }
   }
 }
 
@@ -136,8 +202,7 @@ __global__ void col_idx_kernel(const uint64_t* uniq, int64_t M, uint64_t N, cons
                                const int32_t* adj_off, int32_t* col_idx) {
   for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < M;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t a = static_cast<int64_t>(uniq[t] / N);
-    const int64_t b = static_cast<int64_t>(uniq[t] % N);
+    const int64_t a = static_cast<int64_t>(uniq[t] / N), b = static_cast<int64_t>(uniq[t] % N);
     const int nfa = __popc(mask[a]);
     const int nfb = __popc(mask[b]);
     for (int r = 0; r < nfa; ++r) {
@@ -147,50 +212,34 @@ __global__ void col_idx_kernel(const uint64_t* uniq, int64_t M, uint64_t N, cons
   }
 }
 
-__global__ void slot_kernel(const int32_t* conn, int64_t n_elems, int npe, uint64_t N,
-                            const uint64_t* uniq, const int64_t* node_ptr, uint16_t* slot, int* overflow) {
-  const int64_t total = n_elems * npe * npe;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t e = i / (npe * npe);
-    const int r = static_cast<int>(i % (npe * npe));
-    const int64_t na = conn[e * npe + r / npe];
-    const uint64_t key = static_cast<uint64_t>(na) * N + static_cast<uint64_t>(conn[e * npe + r % npe]);
-    int64_t lo = node_ptr[na], hi = node_ptr[na + 1];
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (uniq[mid] < key)
-        lo = mid + 1;
-      else
-        hi = mid;
-    }
-    const int64_t pos = lo - node_ptr[na];
-    if (pos > 65534) atomicExch(overflow, 1);  // list lengths are uint16
-    slot[i] = static_cast<uint16_t>(pos);
-  }
-}
-
-// adjacency list length per node (uint16, and int64 for the max reduction), and the
-// list length again for the nodes whose rows are compressed (row length != 3 x list
-// length), 0 for the others
-__global__ void adj_len_kernel(const int64_t* node_ptr, const int32_t* rowlen, int64_t n_nodes, uint16_t* adj_len,
-                               int64_t* len64, int64_t* bnd_len) {
+// the rest of the node records
+__global__ void node_rec_kernel(const int64_t* node_base, const int32_t* rowlen,
+                                const int32_t* eq0, const uint8_t* mask, const int64_t* bnd_ptr,
+                                const int64_t* rec_ptr, int64_t n_nodes, NodeRec* node) {
   for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n_nodes;
        a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t k = node_ptr[a + 1] - node_ptr[a];
-    adj_len[a] = static_cast<uint16_t>(k);
-    len64[a] = k;
-    bnd_len[a] = rowlen[a] == 3 * k ? 0 : k;
+    NodeRec r = node[a];
+    r.base = node_base[a];
+    r.len_mask = static_cast<uint32_t>(rowlen[a]) | static_cast<uint32_t>(mask[a]) << 28;
+    r.eq0 = eq0[a];
+    r.bnd0 = static_cast<uint32_t>(bnd_ptr[a]);
+    r.list0 = static_cast<uint32_t>(rec_ptr[a]);
+    node[a] = r;
   }
 }
 
-// neighbours of the compressed-row nodes, in list order
+// neighbours and compressed columns of the compressed-row nodes, in list order
 __global__ void bnd_node_kernel(const uint64_t* uniq, int64_t M, uint64_t N, const int64_t* node_ptr,
-                                const int64_t* bnd_ptr, int32_t* bnd_node) {
+                                const int64_t* bnd_ptr, const int64_t* bnd_len, const int32_t* adj_off,
+                                const uint8_t* mask, int32_t* bnd_node, int32_t* bnd_col) {
   for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < M;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t a = static_cast<int64_t>(uniq[t] / N);
-    if (bnd_ptr[a + 1] > bnd_ptr[a]) bnd_node[bnd_ptr[a] + (t - node_ptr[a])] = static_cast<int32_t>(uniq[t] % N);
+    const int64_t a = static_cast<int64_t>(uniq[t] / N), b = static_cast<int64_t>(uniq[t] % N);
+    if (bnd_len[a] > 0) {
+      const int64_t o = bnd_ptr[a] + (t - node_ptr[a]);
+      bnd_node[o] = static_cast<int32_t>(b);
+      bnd_col[o] = adj_off[t] | static_cast<int32_t>(mask[b]) << 28;
+    }
   }
 }
 
@@ -258,6 +307,17 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
   int64_t* d_node_ptr = nullptr;
   int32_t* d_adj_off = nullptr;
   int64_t* d_node_nnz = nullptr;
+  int64_t* d_node_base = nullptr;
+  int64_t* d_bnd_len = nullptr;
+  int64_t* d_bnd_ptr = nullptr;
+  int32_t* d_rowlen = nullptr;
+  int32_t* d_eq0 = nullptr;
+  uint32_t* d_codes = nullptr;
+  uint32_t* d_codes2 = nullptr;
+  uint32_t* d_start = nullptr;
+  int64_t* d_n_rec = nullptr;
+  int64_t* d_rec_ptr = nullptr;
+  uint64_t* sorted = nullptr;
   int h_flag = 0;
   int64_t M = 0;
   uint64_t* uniq = nullptr;
@@ -326,124 +386,108 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
   d_scan = nullptr;
 
   CXG_TRY(dalloc(&out->node_mask, n_nodes, &out->device_bytes));
-  CXG_TRY(dalloc(&out->node_eq0, n_nodes, &out->device_bytes));
-  CXG_TRY(dalloc(&out->node_rowlen, n_nodes, &out->device_bytes));
-  CXG_TRY(dalloc(&out->node_base, n_nodes, &out->device_bytes));
-  node_info_kernel<<<grid_for(n_nodes), 256, 0, s>>>(d_dof_eq, n_nodes, out->node_mask, out->node_eq0);
+  CXG_TRY(dalloc(&out->node, n_nodes, &out->device_bytes));
+  CXG_TRY(dalloc(&d_eq0, n_nodes, &scratch));
+  CXG_TRY(dalloc(&d_rowlen, n_nodes, &scratch));
+  CXG_TRY(dalloc(&d_node_base, n_nodes, &scratch));
+  node_info_kernel<<<grid_for(n_nodes), 256, 0, s>>>(d_dof_eq, n_nodes, out->node_mask, d_eq0);
   CXG_TRY(cudaGetLastError());
 
-  // node adjacency by sort + unique of the element node-pair keys
+  // node adjacency and its element blocks: stable sort of (node-pair key, block code),
+  // then one key and its first position per pair
   CXG_TRY(dalloc(&d_keys, P, &scratch));
   CXG_TRY(dalloc(&d_keys2, P, &scratch));
-  pair_keys_kernel<<<grid_for(P), 256, 0, s>>>(d_conn, n_elems, npe, N, d_keys);
+  CXG_TRY(dalloc(&d_codes, P + 1, &scratch));
+  CXG_TRY(dalloc(&d_codes2, P + 1, &scratch));
+  pair_keys_kernel<<<grid_for(P), 256, 0, s>>>(d_conn, n_elems, npe, N, d_keys, d_codes);
   CXG_TRY(cudaGetLastError());
   {
     cub::DoubleBuffer<uint64_t> db(d_keys, d_keys2);
+    cub::DoubleBuffer<uint32_t> dc(d_codes, d_codes2);
     temp_bytes = 0;
-    CXG_TRY(cub::DeviceRadixSort::SortKeys(nullptr, temp_bytes, db, static_cast<int>(P), 0, end_bit, s));
+    CXG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, db, dc, static_cast<int>(P), 0, end_bit, s));
     CXG_TRY(cudaMalloc(&d_temp, temp_bytes));
-    CXG_TRY(cub::DeviceRadixSort::SortKeys(d_temp, temp_bytes, db, static_cast<int>(P), 0, end_bit, s));
+    CXG_TRY(cub::DeviceRadixSort::SortPairs(d_temp, temp_bytes, db, dc, static_cast<int>(P), 0, end_bit, s));
+    CXG_TRY(cudaStreamSynchronize(s));
     cudaFree(d_temp);
     d_temp = nullptr;
-    uint64_t* sorted = db.Current();
+    d_codes = dc.Current();
+    d_codes2 = dc.Alternate();
+    d_start = d_codes2;
+    sorted = db.Current();
     uint64_t* other = db.Alternate();
     CXG_TRY(cudaMalloc(&d_M, sizeof(int64_t)));
+    CXG_TRY(cudaMemsetAsync(d_M, 0, sizeof(int64_t), s));
+    const thrust::counting_iterator<uint32_t> at(0u);
     temp_bytes = 0;
-    CXG_TRY(cub::DeviceSelect::Unique(nullptr, temp_bytes, sorted, other, d_M, static_cast<int>(P), s));
+    CXG_TRY(cub::DeviceSelect::UniqueByKey(nullptr, temp_bytes, sorted, at, other, d_start, d_M, static_cast<int>(P), s));
     CXG_TRY(cudaMalloc(&d_temp, temp_bytes));
-    CXG_TRY(cub::DeviceSelect::Unique(d_temp, temp_bytes, sorted, other, d_M, static_cast<int>(P), s));
+    CXG_TRY(cub::DeviceSelect::UniqueByKey(d_temp, temp_bytes, sorted, at, other, d_start, d_M, static_cast<int>(P), s));
     CXG_TRY(cudaMemcpyAsync(&M, d_M, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     CXG_TRY(cudaStreamSynchronize(s));
     cudaFree(d_temp);
     d_temp = nullptr;
     uniq = other;
+    const uint32_t total = static_cast<uint32_t>(P);
+    CXG_TRY(cudaMemcpyAsync(d_start + M, &total, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   }
 
   CXG_TRY(dalloc(&d_node_ptr, n_nodes + 1, &scratch));
   CXG_TRY(dalloc(&d_adj_off, M, &scratch));
   CXG_TRY(dalloc(&d_node_nnz, n_nodes, &scratch));
+  CXG_TRY(dalloc(&d_bnd_len, n_nodes, &scratch));
+  CXG_TRY(dalloc(&d_bnd_ptr, n_nodes, &scratch));
+  CXG_TRY(dalloc(&d_n_rec, n_nodes, &scratch));
+  CXG_TRY(dalloc(&d_rec_ptr, n_nodes, &scratch));
   node_ptr_kernel<<<grid_for(n_nodes + 1), 256, 0, s>>>(uniq, M, n_nodes, N, d_node_ptr);
   CXG_TRY(cudaGetLastError());
-  rowlen_kernel<<<grid_for(n_nodes), 256, 0, s>>>(uniq, d_node_ptr, n_nodes, N, out->node_mask,
-                                                  out->node_rowlen, d_adj_off, d_node_nnz);
+  CXG_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), s));
+  rowlen_kernel<<<grid_for(n_nodes), 256, 0, s>>>(uniq, d_start, d_node_ptr, n_nodes, N, out->node_mask, d_rowlen,
+                                                  d_adj_off, d_node_nnz, d_bnd_len, d_n_rec, out->node, d_flag);
   CXG_TRY(cudaGetLastError());
   temp_bytes = 0;
-  CXG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, d_node_nnz, out->node_base, static_cast<int>(n_nodes), s));
+  CXG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, d_node_nnz, d_node_base, static_cast<int>(n_nodes), s));
   CXG_TRY(cudaMalloc(&d_temp, temp_bytes));
-  CXG_TRY(cub::DeviceScan::ExclusiveSum(d_temp, temp_bytes, d_node_nnz, out->node_base, static_cast<int>(n_nodes), s));
+  CXG_TRY(cub::DeviceScan::ExclusiveSum(d_temp, temp_bytes, d_node_nnz, d_node_base, static_cast<int>(n_nodes), s));
+  CXG_TRY(cub::DeviceScan::ExclusiveSum(d_temp, temp_bytes, d_bnd_len, d_bnd_ptr, static_cast<int>(n_nodes), s));
+  CXG_TRY(cub::DeviceScan::ExclusiveSum(d_temp, temp_bytes, d_n_rec, d_rec_ptr, static_cast<int>(n_nodes), s));
   {
-    int64_t last_base = 0, last_nnz = 0;
-    if (n_nodes > 0) {
-      CXG_TRY(cudaMemcpyAsync(&last_base, out->node_base + n_nodes - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-      CXG_TRY(cudaMemcpyAsync(&last_nnz, d_node_nnz + n_nodes - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    }
+    int64_t last[6] = {0, 0, 0, 0, 0, 0};
+    const int64_t* src[6] = {d_node_base, d_node_nnz, d_bnd_ptr, d_bnd_len, d_rec_ptr, d_n_rec};
+    for (int i = 0; i < 6; ++i)
+      CXG_TRY(cudaMemcpyAsync(&last[i], src[i] + n_nodes - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    CXG_TRY(cudaMemcpyAsync(&h_flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
     CXG_TRY(cudaStreamSynchronize(s));
-    out->nnz = last_base + last_nnz;
+    if (h_flag) {
+      *msg = "a node has more than 65535 neighbours; not supported";
+      rc = 5;
+      goto done;
+    }
+    out->nnz = last[0] + last[1];
+    CXG_TRY(dalloc(&out->bnd_node, static_cast<size_t>(last[2] + last[3]), &out->device_bytes));
+    CXG_TRY(dalloc(&out->bnd_col, static_cast<size_t>(last[2] + last[3]), &out->device_bytes));
+    CXG_TRY(dalloc(&out->pairs, static_cast<size_t>(last[4] + last[5]), &out->device_bytes));
   }
+  cudaFree(d_temp);
+  d_temp = nullptr;
 
   CXG_TRY(dalloc(&out->row_ptr, static_cast<size_t>(n_free) + 1, &out->device_bytes));
   CXG_TRY(dalloc(&out->col_idx, static_cast<size_t>(out->nnz), &out->device_bytes));
-  CXG_TRY(dalloc(&out->slot, static_cast<size_t>(P), &out->device_bytes));
-  row_ptr_kernel<<<grid_for(n_nodes), 256, 0, s>>>(n_nodes, out->node_mask, out->node_eq0, out->node_base,
-                                                   out->node_rowlen, out->row_ptr);
+  row_ptr_kernel<<<grid_for(n_nodes), 256, 0, s>>>(n_nodes, out->node_mask, d_eq0, d_node_base, d_rowlen, out->row_ptr);
   CXG_TRY(cudaGetLastError());
   CXG_TRY(cudaMemcpyAsync(out->row_ptr + n_free, &out->nnz, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-  col_idx_kernel<<<grid_for(M), 256, 0, s>>>(uniq, M, N, out->node_mask, out->node_eq0, out->node_base,
-                                             out->node_rowlen, d_adj_off, out->col_idx);
+  col_idx_kernel<<<grid_for(M), 256, 0, s>>>(uniq, M, N, out->node_mask, d_eq0, d_node_base, d_rowlen, d_adj_off,
+                                             out->col_idx);
   CXG_TRY(cudaGetLastError());
-  CXG_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), s));
-  slot_kernel<<<grid_for(P), 256, 0, s>>>(d_conn, n_elems, npe, N, uniq, d_node_ptr, out->slot, d_flag);
+  bnd_node_kernel<<<grid_for(M), 256, 0, s>>>(uniq, M, N, d_node_ptr, d_bnd_ptr, d_bnd_len, d_adj_off, out->node_mask, out->bnd_node,
+                                              out->bnd_col);
   CXG_TRY(cudaGetLastError());
-  CXG_TRY(cudaMemcpyAsync(&h_flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-  CXG_TRY(cudaStreamSynchronize(s));
-  if (h_flag) {
-    *msg = "a node has more than 65535 neighbours; not supported";
-    rc = 5;
-    goto done;
-  }
-
-  // largest per-node row block (free rows x row length) and adjacency list (they size
-  // the gather's buffers); list lengths, and the neighbours of the compressed-row nodes
-  {
-    int64_t* d_max = nullptr;
-    int64_t* d_bnd_len = nullptr;
-    CXG_TRY(cudaMalloc(&d_max, 2 * sizeof(int64_t)));
-    CXG_TRY(cudaMalloc(&d_bnd_len, sizeof(int64_t) * static_cast<size_t>(std::max<int64_t>(n_nodes, 1))));
-    temp_bytes = 0;
-    CXG_TRY(cub::DeviceReduce::Max(nullptr, temp_bytes, d_node_nnz, d_max, static_cast<int>(n_nodes), s));
-    size_t scan_bytes = 0;
-    CXG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_bnd_len, d_bnd_len, static_cast<int>(n_nodes) + 1, s));
-    temp_bytes = std::max(temp_bytes, scan_bytes);
-    CXG_TRY(cudaMalloc(&d_temp, temp_bytes));
-    CXG_TRY(cub::DeviceReduce::Max(d_temp, temp_bytes, d_node_nnz, d_max, static_cast<int>(n_nodes), s));
-    CXG_TRY(dalloc(&out->adj_len, n_nodes, &out->device_bytes));
-    CXG_TRY(dalloc(&out->bnd_ptr, n_nodes + 1, &out->device_bytes));
-    adj_len_kernel<<<grid_for(n_nodes), 256, 0, s>>>(d_node_ptr, out->node_rowlen, n_nodes, out->adj_len, d_node_nnz,
-                                                     d_bnd_len);
-    CXG_TRY(cudaGetLastError());
-    CXG_TRY(cub::DeviceReduce::Max(d_temp, temp_bytes, d_node_nnz, d_max + 1, static_cast<int>(n_nodes), s));
-    CXG_TRY(cudaMemsetAsync(out->bnd_ptr + n_nodes, 0, sizeof(int64_t), s));
-    CXG_TRY(cub::DeviceScan::ExclusiveSum(d_temp, temp_bytes, d_bnd_len, out->bnd_ptr, static_cast<int>(n_nodes), s));
-    int64_t hm[2] = {0, 0}, last[2] = {0, 0};
-    CXG_TRY(cudaMemcpyAsync(hm, d_max, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    if (n_nodes > 0) {
-      CXG_TRY(cudaMemcpyAsync(&last[0], out->bnd_ptr + n_nodes - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-      CXG_TRY(cudaMemcpyAsync(&last[1], d_bnd_len + n_nodes - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    }
-    CXG_TRY(cudaStreamSynchronize(s));
-    const int64_t n_bnd = last[0] + last[1];
-    CXG_TRY(cudaMemcpyAsync(out->bnd_ptr + n_nodes, &n_bnd, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    CXG_TRY(dalloc(&out->bnd_node, n_bnd, &out->device_bytes));
-    bnd_node_kernel<<<grid_for(M), 256, 0, s>>>(uniq, M, N, d_node_ptr, out->bnd_ptr, out->bnd_node);
-    CXG_TRY(cudaGetLastError());
-    CXG_TRY(cudaStreamSynchronize(s));
-    out->max_row = n_nodes > 0 ? hm[0] : 0;
-    out->max_adj = n_nodes > 0 ? hm[1] : 0;
-    cudaFree(d_max);
-    cudaFree(d_bnd_len);
-    cudaFree(d_temp);
-    d_temp = nullptr;
-  }
+  node_rec_kernel<<<grid_for(n_nodes), 256, 0, s>>>(d_node_base, d_rowlen, d_eq0, out->node_mask, d_bnd_ptr,
+                                                    d_rec_ptr, n_nodes, out->node);
+  CXG_TRY(cudaGetLastError());
+  pair_rec_kernel<<<grid_for(32 * n_nodes), 256, 0, s>>>(out->node, d_start, d_node_ptr, d_codes, sorted, P, n_nodes,
+                                                         out->pairs);
+  CXG_TRY(cudaGetLastError());
 
   // node -> element incidence: stable sort of (node, e*n + local) by node
   {
@@ -482,6 +526,15 @@ done:
   cudaFree(d_node_ptr);
   cudaFree(d_adj_off);
   cudaFree(d_node_nnz);
+  cudaFree(d_node_base);
+  cudaFree(d_bnd_len);
+  cudaFree(d_bnd_ptr);
+  cudaFree(d_rowlen);
+  cudaFree(d_eq0);
+  cudaFree(d_codes);
+  cudaFree(d_codes2);
+  cudaFree(d_n_rec);
+  cudaFree(d_rec_ptr);
   return rc;
 }
 

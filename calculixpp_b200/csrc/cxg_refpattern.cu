@@ -231,7 +231,7 @@ struct RefWarp {
 
 template <int ET>
 __global__ void __launch_bounds__(kRefWarps * 32) refmask_kernel(ElemArgs A, double* out) {
-  constexpr int n = nodes_of(ET), nq = gauss_of(ET), NB = n * (n + 1) / 2, BS = 10;
+  constexpr int n = nodes_of(ET), nq = gauss_of(ET), NB = n * (n + 1) / 2;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   RefWarp<ET>& W = reinterpret_cast<RefWarp<ET>*>(smem)[warp];
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(kRefWarps * 32) refmask_kernel(ElemArgs A, dou
       }
     }
     __syncwarp();
-    double* dst = out + e * (NB * BS);
+    double* dst = out + e * (blocks_padded(n) * 9);
     for (int t = lane; t < NB * 9; t += 32) {
       const int blk = t / 9, q9 = t % 9;
       int ka = 0, r = blk;
@@ -315,7 +315,9 @@ __global__ void __launch_bounds__(kRefWarps * 32) refmask_kernel(ElemArgs A, dou
         if (da == db)
           for (int al = 0; al < 4; ++al) K += W.kappa * W.gamma[al][na] * W.gamma[al][nb];
       }
-      dst[blk * BS + q9] = K != 0.0 ? 1.0 : 0.0;
+      // blocks are stored in mesh order of their nodes (blk_index)
+      const bool swap = A.conn[e * n + ka] > A.conn[e * n + kb];
+      dst[blk * 9 + (swap ? 3 * (q9 % 3) + q9 / 3 : q9)] = K != 0.0 ? 1.0 : 0.0;
     }
     __syncwarp();
   }

@@ -12,28 +12,20 @@
 // stored N of the Gauss point). The upper blocks (a <= b) go to a per-element
 // buffer, FP32 in mixed precision, FP64 otherwise; the internal force goes beside them.
 //
-// P2 (row gather): one warp per node. It walks the node's incident elements in
-// element order, adds their block rows into the node's CSR rows held in shared memory
-// (plain read-modify-write: within one element every target is distinct), moves
-// prescribed columns into the rhs (-K_fc u_c, src/fem/assembly.cpp:95-96), adds the
-// load vector, and stores its rows once with coalesced writes. In mixed precision the
-// diagonal block of each element row is formed here in FP64 as minus the sum of that
-// row's off-diagonal FP32 blocks, so rigid translations stay in the null space exactly.
+// P2 (row gather, cxg_gather.cu): one warp per node sums, pair by pair, the element
+// blocks of each of the node's CSR entries.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
 
-#include "cxg_internal.cuh"
+#include "cxg_element.cuh"
 
 namespace cxg {
 
 namespace {
 
-constexpr int kT1 = 128;          // P1 threads per block
-constexpr int kW1 = kT1 / 32;
-constexpr double kSqrt3_2v2 = 1.224744871391589;
 
 struct TileList {
   int count;
@@ -77,142 +69,6 @@ struct Geo {
   static constexpr int NT = tiles.count;
   static constexpr int EPW = NT >= 32 ? 1 : 32 / NT;
 };
-
-__host__ __device__ constexpr int blk_index(int n, int a, int b) { return a * n - a * (a - 1) / 2 + (b - a); }
-
-// Stored 3x3 blocks are padded to 16 bytes (10 doubles, 12 floats) so that they move
-// with 128-bit accesses.
-template <typename R>
-__host__ __device__ constexpr int blk_stride() { return sizeof(R) == 8 ? 10 : 12; }
-
-// Slot of element e in the element buffer, a ring of `ring` elements (the whole mesh when
-// the assembly runs as one window; ring_base 0): e mod ring. Every element a window's
-// passes touch lies in [ring_base, ring_base + 2 ring), so one conditional subtraction
-// gives the slot, with no division in the inner loops.
-__device__ __forceinline__ int64_t ring_slot(int64_t e, const V2Args& V) {
-  const int64_t d = e - V.ring_base;
-  return d < V.ring ? d : d - V.ring;
-}
-
-template <typename R>
-__device__ __forceinline__ void store_block(R* dst, const R (&v)[9]) {
-  if constexpr (sizeof(R) == 8) {
-    double2* d = reinterpret_cast<double2*>(dst);
-    d[0] = make_double2(v[0], v[1]);
-    d[1] = make_double2(v[2], v[3]);
-    d[2] = make_double2(v[4], v[5]);
-    d[3] = make_double2(v[6], v[7]);
-    d[4] = make_double2(v[8], 0.0);
-  } else {
-    float4* d = reinterpret_cast<float4*>(dst);
-    d[0] = make_float4(v[0], v[1], v[2], v[3]);
-    d[1] = make_float4(v[4], v[5], v[6], v[7]);
-    d[2] = make_float4(v[8], 0.f, 0.f, 0.f);
-  }
-}
-
-template <typename R>
-__device__ __forceinline__ void load_block(const R* src, R (&v)[9]) {
-  if constexpr (sizeof(R) == 8) {
-    const double2* d = reinterpret_cast<const double2*>(src);
-    const double2 a = __ldg(d), b = __ldg(d + 1), c = __ldg(d + 2), e = __ldg(d + 3), f = __ldg(d + 4);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = e.x; v[7] = e.y; v[8] = f.x;
-  } else {
-    const float4* d = reinterpret_cast<const float4*>(src);
-    const float4 a = __ldg(d), b = __ldg(d + 1), c = __ldg(d + 2);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w; v[8] = c.x;
-  }
-}
-
-__device__ __forceinline__ void hardening2(const J2Mat& M, double ep, double& sy, double& h) {
-  const int n = M.n;
-  if (n == 1 || ep <= M.ep[0]) {
-    sy = M.sy[0];
-    h = 0.0;
-    return;
-  }
-  if (ep >= M.ep[n - 1]) {
-    sy = M.sy[n - 1];
-    h = 0.0;
-    return;
-  }
-  for (int i = 0; i + 1 < n; ++i) {
-    if (ep >= M.ep[i] && ep <= M.ep[i + 1]) {
-      h = (M.sy[i + 1] - M.sy[i]) / (M.ep[i + 1] - M.ep[i]);
-      sy = M.sy[i] + h * (ep - M.ep[i]);
-      return;
-    }
-  }
-  sy = M.sy[n - 1];
-  h = 0.0;
-}
-
-// J2 radial return + consistent tangent (restating src/fem/plasticity.cpp:90-236), FP64.
-// Returns true on the plastic branch; lam_s/mu_s/c: tangent parameters, nv: direction.
-__device__ bool j2_point(const J2Mat& M, double lam, double mu_el, double mu, const double* eps, const double* cs,
-                         double* ts, double* sig, double& lam_t, double& mu_t, double& c_t, double* nv,
-                         double& mu_hg) {
-  const double lam2mu = lam + 2.0 * mu_el;
-  double el[6];
-  for (int i = 0; i < 6; ++i) el[i] = eps[i] - cs[i];
-  double st[6];
-  st[0] = lam2mu * el[0] + lam * el[1] + lam * el[2];
-  st[1] = lam * el[0] + lam2mu * el[1] + lam * el[2];
-  st[2] = lam * el[0] + lam * el[1] + lam2mu * el[2];
-  st[3] = mu_el * el[3];
-  st[4] = mu_el * el[4];
-  st[5] = mu_el * el[5];
-  const double p = (st[0] + st[1] + st[2]) / 3.0;
-  const double s_tr[6] = {st[0] - p, st[1] - p, st[2] - p, st[3], st[4], st[5]};
-  double xi[6];
-  for (int i = 0; i < 6; ++i) xi[i] = s_tr[i] - cs[7 + i];
-  const double xi_norm = sqrt(xi[0] * xi[0] + xi[1] * xi[1] + xi[2] * xi[2] +
-                              2.0 * (xi[3] * xi[3] + xi[4] * xi[4] + xi[5] * xi[5]));
-  const double q_tr = kSqrt3_2v2 * xi_norm;
-  double sy0 = 0.0, h0 = 0.0;
-  if (M.plastic) hardening2(M, cs[6], sy0, h0);
-  if (!M.plastic || q_tr - sy0 <= 0.0 || xi_norm == 0.0) {
-    for (int i = 0; i < 6; ++i) sig[i] = st[i];
-    for (int i = 0; i < kStateDoubles; ++i) ts[i] = cs[i];
-    lam_t = lam;
-    mu_t = mu_el;
-    c_t = 0.0;
-    mu_hg = mu_el;
-    return 0;
-  }
-  const double ep0 = cs[6];
-  double dgamma = 0.0;
-  for (int it = 0; it < 50; ++it) {
-    double sy, h_iso;
-    hardening2(M, ep0 + dgamma, sy, h_iso);
-    const double g = q_tr - 3.0 * mu * dgamma - M.h_kin * dgamma - sy;
-    const double dg = -(3.0 * mu + M.h_kin + h_iso);
-    const double step = -g / dg;
-    dgamma += step;
-    if (dgamma < 0.0) dgamma = 0.0;
-    if (fabs(step) <= 1e-14 * (1.0 + fabs(dgamma))) break;
-  }
-  for (int i = 0; i < 6; ++i) nv[i] = xi[i] / xi_norm;
-  const double dev_scale = 2.0 * mu * dgamma * kSqrt3_2v2;
-  const double alpha_scale = (2.0 / 3.0) * M.h_kin * dgamma * kSqrt3_2v2;
-  const double dep_scale = dgamma * kSqrt3_2v2;
-  for (int i = 0; i < 6; ++i) {
-    sig[i] = (s_tr[i] - dev_scale * nv[i]) + (i < 3 ? p : 0.0);
-    ts[i] = cs[i] + dep_scale * nv[i] * (i < 3 ? 1.0 : 2.0);
-    ts[7 + i] = cs[7 + i] + alpha_scale * nv[i];
-  }
-  ts[6] = ep0 + dgamma;
-  double sy, h_iso;
-  hardening2(M, ep0 + dgamma, sy, h_iso);
-  const double theta = 1.0 - (2.0 * mu * dgamma * kSqrt3_2v2) / xi_norm;
-  const double denom = 1.0 + (h_iso + M.h_kin) / (3.0 * mu);
-  const double theta_bar = 1.0 / denom - (1.0 - theta);
-  lam_t = lam + (2.0 / 3.0) * (1.0 - theta) * mu;
-  mu_t = mu_el - (1.0 - theta) * mu;
-  c_t = 2.0 * mu * theta_bar;
-  mu_hg = mu_t - c_t * nv[3] * nv[3];
-  return true;
-}
 
 // Band around the yield surface, as a fraction of the current yield stress, inside which
 // the mixed-precision path decides and returns in FP64.
@@ -315,24 +171,6 @@ __device__ __forceinline__ int j2_point_mixed(const J2Mat& M, double lam, double
   return 1;
 }
 
-__constant__ double c_hg2[4][8] = {
-    {1, 1, -1, -1, -1, -1, 1, 1},
-    {1, -1, -1, 1, -1, 1, 1, -1},
-    {1, -1, 1, -1, 1, -1, 1, -1},
-    {-1, 1, -1, 1, 1, -1, 1, -1},
-};
-
-template <typename R>
-struct Vec4;
-template <>
-struct Vec4<float> {
-  using T = float4;
-};
-template <>
-struct Vec4<double> {
-  using T = double4;
-};
-
 // Shared-memory layout of per-(element, Gauss point) node vectors: node k lives in
 // slot(k) = k/2 for even k and npad/2 + k/2 for odd k, so the row nodes 2r + i of the
 // lanes' tiles occupy consecutive slots. FP32 vectors are float4 per slot; FP64 vectors
@@ -387,9 +225,16 @@ struct P1Smem {
   using G = Geo<ET, TILE>;
   static constexpr int n = G::n, nq = G::nq, npad = G::npad, EPW = G::EPW;
   static constexpr bool T = MODE == MODE_TANGENT;
-  static constexpr int kVec = EPW * nq * VecIdx<R, npad>::kBlock;
+  // Staged blocks: the finished blocks of a warp's elements are put together in shared
+  // memory, unpadded, and leave as one bulk copy per element. With one tile per lane
+  // (ALIAS) they take the place of the gradient vectors, which are dead by then.
+  static constexpr int kElem = blocks_padded(n) * 9;  // values of one element
+  static constexpr bool ALIAS = EPW * G::NT <= 32;
+  static constexpr int kGrad = EPW * nq * VecIdx<R, npad>::kBlock;
+  static constexpr int kVec = ALIAS && EPW * kElem > kGrad ? EPW * kElem : kGrad;
   static constexpr int HG = ET == C3D8R ? EPW : 1;  // hourglass data (C3D8R only)
-  R g[kVec];                                      // node vectors, see VecIdx
+  alignas(16) R g[kVec];                          // node vectors, see VecIdx
+  alignas(16) R stg[ALIAS ? 4 : EPW * kElem];
   R nvq[T ? EPW * nq * 8 : 4];  // return direction N (Voigt, 6 used) per plastic Gauss point
   R s[EPW][nq];
   R dp[T ? EPW : 1][T ? nq : 1][4];
@@ -403,6 +248,7 @@ struct P1Smem {
   double vol[HG];
   double mu_hg[HG];
   int plastic[EPW];
+  int id[EPW][n];  // mesh nodes
 };
 
 template <int ET, int MODE, typename R, int TILE>
@@ -484,6 +330,7 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
       const int node = conn_next[p];
       if (node >= 0) {
         const int ei = t / n, k = t % n;
+        W.id[ei][k] = node;
         for (int d = 0; d < 3; ++d) {
           W.x[ei][3 * k + d] = A.coords[3 * static_cast<int64_t>(node) + d];
           if (TAN) W.u[ei][3 * k + d] = A.u[3 * static_cast<int64_t>(node) + d];
@@ -491,6 +338,7 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
       }
     }
     load_conn(e0 + nwarps * EPW);
+    if (lane == 0) bulk_wait_read();  // the staged blocks of the last elements have left
     if (lane < EPW) {
       const int64_t e = e0 + lane;
       const double E = e < e_end ? A.young[e] : 1.0, nu = e < e_end ? A.poisson[e] : 0.0;
@@ -516,22 +364,13 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
           J[i][2] = fma(xk, d2, J[i][2]);
         }
       }
-      const double c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
-      const double c01 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
-      const double c02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-      const double det = J[0][0] * c00 + J[0][1] * c01 + J[0][2] * c02;
+      double it[3][3];
+      const double det = invert(J, it);
       if (!(det > 0.0)) {
         atomicCAS(&A.status->code, 0, 4);
         atomicMin(&A.status->bad_elem, static_cast<unsigned long long>(e));
       }
-      const double inv = 1.0 / det;
-      const double it[3][3] = {
-          {c00 * inv, c01 * inv, c02 * inv},
-          {(J[0][2] * J[2][1] - J[0][1] * J[2][2]) * inv, (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * inv,
-           (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * inv},
-          {(J[0][1] * J[1][2] - J[0][2] * J[1][1]) * inv, (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * inv,
-           (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * inv}};
-      const double sq = det * sw[q];
+      const double sq = mul(det, sw[q]);
       W.s[ei][q] = static_cast<R>(sq);
       if constexpr (ET == C3D8R) W.vol[ei] = sq;
       double H[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
@@ -539,7 +378,7 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
         const double d0 = sdN[(3 * k) * nq + q], d1 = sdN[(3 * k + 1) * nq + q], d2 = sdN[(3 * k + 2) * nq + q];
         double gk[3];
         for (int i = 0; i < 3; ++i) {
-          gk[i] = it[i][0] * d0 + it[i][1] * d1 + it[i][2] * d2;
+          gk[i] = fma(it[i][0], d0, fma(it[i][1], d1, mul(it[i][2], d2)));
           if constexpr (ET == C3D8R) W.gc[ei][i * n + k] = gk[i];
         }
         st3<R, npad>(W.g, ei * nq + q, node_slot(k, npad), gk[0], gk[1], gk[2]);
@@ -578,7 +417,7 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
 #pragma unroll
           for (int c = 7; c < kStateDoubles; ++c) A.state_t[c * A.n_gauss + gidx] = ts[c];
         }
-        for (int c = 0; c < 6; ++c) W.sig[ei][q][c] = sq * sig[c];
+        for (int c = 0; c < 6; ++c) W.sig[ei][q][c] = mul(sq, sig[c]);
         W.dp[ei][q][0] = static_cast<R>(sq * lt);
         W.dp[ei][q][1] = static_cast<R>(sq * mt);
         W.dp[ei][q][2] = static_cast<R>(sq * ct);
@@ -599,31 +438,79 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
         const int ei = t / 4, al = t % 4;
         double gx[3] = {0, 0, 0};
         for (int j = 0; j < 8; ++j)
-          for (int d = 0; d < 3; ++d) gx[d] += c_hg2[al][j] * W.x[ei][3 * j + d];
+          for (int d = 0; d < 3; ++d) gx[d] = fma(c_hg2[al][j], W.x[ei][3 * j + d], gx[d]);
         for (int j = 0; j < 8; ++j) {
           double corr = 0.0;
-          for (int d = 0; d < 3; ++d) corr += gx[d] * W.gc[ei][d * n + j];
+          for (int d = 0; d < 3; ++d) corr = fma(gx[d], W.gc[ei][d * n + j], corr);
           W.gam[ei][al * 8 + j] = c_hg2[al][j] - corr;
         }
       }
       if (lane < EPW) {
         double b2 = 0.0;
-        for (int t = 0; t < 3 * n; ++t) b2 += W.gc[lane][t] * W.gc[lane][t];
+        for (int t = 0; t < 3 * n; ++t) b2 = fma(W.gc[lane][t], W.gc[lane][t], b2);
         W.kappa[lane] = 0.05 * (TAN ? W.mu_hg[lane] : W.mu_j2[lane]) * W.vol[lane] * b2;
       }
       __syncwarp();
     }
+    // ---- internal force per element (material-point mode) --------------------
+    if (TAN) {
+      for (int t = lane; t < EPW * n; t += 32) {
+        const int ei = t / n, a = t % n;
+        const int64_t e = e0 + ei;
+        if (e >= e_end) continue;
+        double f[3] = {0, 0, 0};
+        for (int q = 0; q < nq; ++q) {
+          const double* S = W.sig[ei][q];
+          R rx, ry, rz;
+          ld3<R, npad>(W.g, ei * nq + q, node_slot(a, npad), rx, ry, rz);
+          const double gx = rx, gy = ry, gz = rz;
+          add_force(f, S, gx, gy, gz);
+        }
+        if constexpr (ET == C3D8R) {
+          for (int al = 0; al < 4; ++al) {
+            double gu[3] = {0, 0, 0};
+            for (int j = 0; j < 8; ++j)
+              for (int d = 0; d < 3; ++d) gu[d] = fma(W.gam[ei][al * 8 + j], W.u[ei][3 * j + d], gu[d]);
+            const double ka = mul(W.kappa[ei], W.gam[ei][al * 8 + a]);
+            for (int d = 0; d < 3; ++d) f[d] = fma(ka, gu[d], f[d]);
+          }
+        }
+        for (int d = 0; d < 3; ++d) V.fdata[ring_slot(e, V) * (3 * n) + 3 * a + d] = f[d];
+      }
+    }
     // ---- phase C: TR x TC node-pair tiles ---------------------------------------------
-    // Staged stores (FP64 linear mode, one tile per lane, the element's blocks fit the
-    // gradient area): once every tile is done the gradient vectors are dead, so the lanes
-    // put their blocks there unpadded and the warp writes the padded element buffer with
-    // consecutive 16-byte stores, instead of every lane writing its own 80-byte blocks
-    // across the element's buffer (about one cache line per lane and store instruction).
-    // Measured on C3D20 64^3: FP64 6.25 -> 6.10 ms per assembly; in FP32 the staging
-    // raised the 2x4 tile's registers from 126 to 168 and lost, so FP32 stores directly.
-    constexpr bool STAGE =
-        MODE == MODE_LINEAR && sizeof(R) == 8 && EPW * NT <= 32 && EPW * NB * 9 <= WS::kVec;
+    // Blocks are staged in shared memory and leave as bulk copies: a lane that writes its
+    // own blocks to the element's buffer touches about one cache line per lane and store
+    // instruction, and the gather would read the padding that aligns such stores.
+    R* stg = WS::ALIAS ? W.g : W.stg;
     R acc[TR][TC][9];
+    auto stage_tile = [&](int task) {
+      const int ei = task / NT, ti = task % NT, a0 = TR * s_tr[ti], b0 = TC * s_tc[ti];
+#pragma unroll
+      for (int i = 0; i < TR; ++i)
+#pragma unroll
+        for (int j = 0; j < TC; ++j) {
+          const int a = a0 + i, b = b0 + j;
+          if (a < n && b < n && a <= b) {
+            R h = R(0);
+            if constexpr (ET == C3D8R) {
+              double hd = 0.0;
+              for (int al = 0; al < 4; ++al) hd = fma(W.gam[ei][al * 8 + a], W.gam[ei][al * 8 + b], hd);
+              h = static_cast<R>(hd * W.kappa[ei]);
+            }
+            // FP32 diagonal blocks are not used: the gather forms them (GATHER_DIAG)
+            const bool drop = sizeof(R) == 4 && a == b;
+            R* d = stg + ei * WS::kElem + blk_index(n, a, b) * 9;
+            // in mesh order of the two nodes: transposed when b precedes a
+            const int na = W.id[ei][a], nb = W.id[ei][b], sx = na > nb ? 1 : 3, sy = 4 - sx;
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+#pragma unroll
+              for (int y = 0; y < 3; ++y)
+                d[x * sx + y * sy] = drop ? R(0) : acc[i][j][3 * x + y] + (x == y ? h : R(0));
+          }
+        }
+    };
     for (int task = lane; task < EPW * NT; task += 32) {
       const int ei = task / NT, ti = task % NT;
       const int64_t e = e0 + ei;
@@ -724,398 +611,38 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
             }
           }
         }
-        if constexpr (!STAGE) {
-          R* out = reinterpret_cast<R*>(V.edata) + ring_slot(e, V) * (NB * blk_stride<R>());
-#pragma unroll
-          for (int i = 0; i < TR; ++i)
-#pragma unroll
-            for (int j = 0; j < TC; ++j) {
-              const int a = a0 + i, b = b0 + j;
-              if (a < n && b < n && a <= b) {
-                R h = R(0);
-                if constexpr (ET == C3D8R) {
-                  double hd = 0.0;
-                  for (int al = 0; al < 4; ++al) hd += W.gam[ei][al * 8 + a] * W.gam[ei][al * 8 + b];
-                  h = static_cast<R>(hd * W.kappa[ei]);
-                }
-                R bv[9];
-#pragma unroll
-                for (int k = 0; k < 9; ++k) bv[k] = acc[i][j][k] + ((k % 4 == 0) ? h : R(0));
-                store_block<R>(out + blk_index(n, a, b) * blk_stride<R>(), bv);
-              }
-            }
-        }
+        if constexpr (!WS::ALIAS) stage_tile(task);
       }
     }
-    if constexpr (STAGE) {
-      static_assert(ET != C3D8R, "staged stores carry no hourglass term");
-      constexpr int BS = blk_stride<R>(), PER = 16 / static_cast<int>(sizeof(R)), CPB = BS / PER;
+    if constexpr (WS::ALIAS) {
       __syncwarp();  // every lane is done reading the gradient vectors
-      R* stg = W.g;  // EPW x NB blocks of 9 values
-      if (lane < EPW * NT) {
-        const int ei = lane / NT, ti = lane % NT;
-        if (e0 + ei < e_end) {
-          const int a0 = TR * s_tr[ti], b0 = TC * s_tc[ti];
-#pragma unroll
-          for (int i = 0; i < TR; ++i)
-#pragma unroll
-            for (int j = 0; j < TC; ++j) {
-              const int a = a0 + i, b = b0 + j;
-              if (a < n && b < n && a <= b) {
-                R* d = stg + (ei * NB + blk_index(n, a, b)) * 9;
-#pragma unroll
-                for (int k = 0; k < 9; ++k) d[k] = acc[i][j][k];
-              }
-            }
-        }
-      }
+      if (lane < EPW * NT && e0 + lane / NT < e_end) stage_tile(lane);
+    }
+    if constexpr (WS::kElem * sizeof(R) % 16 != 0) {
       __syncwarp();
       for (int ei = 0; ei < EPW && e0 + ei < e_end; ++ei) {
-        R* out = reinterpret_cast<R*>(V.edata) + ring_slot(e0 + ei, V) * (NB * BS);
-        const R* sb = stg + ei * NB * 9;
-        for (int pc = lane; pc < NB * CPB; pc += 32) {
-          const int k = pc / CPB, part = pc % CPB;
-          R v[4];
-#pragma unroll
-          for (int t = 0; t < PER; ++t) {
-            const int j = part * PER + t;
-            v[t] = j < 9 ? sb[k * 9 + j] : R(0);
-          }
-          if constexpr (sizeof(R) == 4) {
-            *reinterpret_cast<float4*>(out + k * BS + part * PER) = make_float4(v[0], v[1], v[2], v[3]);
-          } else {
-            *reinterpret_cast<double2*>(out + k * BS + part * PER) = make_double2(v[0], v[1]);
-          }
-        }
+        float2* out = reinterpret_cast<float2*>(reinterpret_cast<R*>(V.edata) + ring_slot(e0 + ei, V) * WS::kElem);
+        const float2* sb = reinterpret_cast<const float2*>(stg + ei * WS::kElem);
+        for (int t = lane; t < WS::kElem / 2; t += 32) out[t] = sb[t];
       }
-      __syncwarp();  // the next elements' Gauss-point phase rewrites the gradient area
+    } else {
+      fence_async_shared();
+      __syncwarp();
     }
-    // ---- phase D: internal force per element (material-point mode) --------------------
-    if (TAN) {
-      for (int t = lane; t < EPW * n; t += 32) {
-        const int ei = t / n, a = t % n;
-        const int64_t e = e0 + ei;
-        if (e >= e_end) continue;
-        double f[3] = {0, 0, 0};
-        for (int q = 0; q < nq; ++q) {
-          const double* S = W.sig[ei][q];
-          R rx, ry, rz;
-          ld3<R, npad>(W.g, ei * nq + q, node_slot(a, npad), rx, ry, rz);
-          const double gx = rx, gy = ry, gz = rz;
-          f[0] += S[0] * gx + S[3] * gy + S[4] * gz;
-          f[1] += S[3] * gx + S[1] * gy + S[5] * gz;
-          f[2] += S[4] * gx + S[5] * gy + S[2] * gz;
-        }
-        if constexpr (ET == C3D8R) {
-          for (int al = 0; al < 4; ++al) {
-            double gu[3] = {0, 0, 0};
-            for (int j = 0; j < 8; ++j)
-              for (int d = 0; d < 3; ++d) gu[d] += W.gam[ei][al * 8 + j] * W.u[ei][3 * j + d];
-            const double ka = W.kappa[ei] * W.gam[ei][al * 8 + a];
-            for (int d = 0; d < 3; ++d) f[d] += ka * gu[d];
-          }
-        }
-        for (int d = 0; d < 3; ++d) V.fdata[ring_slot(e, V) * (3 * n) + 3 * a + d] = f[d];
-      }
+    if (WS::kElem * sizeof(R) % 16 == 0 && lane == 0) {
+      for (int ei = 0; ei < EPW && e0 + ei < e_end; ++ei)
+        bulk_store(reinterpret_cast<R*>(V.edata) + ring_slot(e0 + ei, V) * WS::kElem, stg + ei * WS::kElem,
+                   WS::kElem * sizeof(R));
+      bulk_commit();
     }
     __syncwarp();
   }
+  if (lane == 0) bulk_wait();
 }
 
 template <int ET, int MODE, typename R, int TILE, bool J2F32>
 __global__ void __launch_bounds__(kT1, (p1_min_blocks<ET, MODE, R, TILE>())) p1_kernel(ElemArgs A, V2Args V) {
   p1_body<ET, MODE, R, TILE, J2F32>(A, V, blockIdx.x, gridDim.x);
-}
-
-// ---- P2: row gather ------------------------------------------------------------------
-// One warp per node a. The node's three rows are staged in shared memory at full width:
-// row i holds 3 entries for each node of a's adjacency list (position s, from the
-// element slot map), every component, free or not. Lanes form EG groups of GS lanes
-// (GS = 16 for elements of at most 16 nodes, else 32); lane lb of group s handles column node lb of incident element
-// k + s, so EG elements are applied per pass, each group into its own copy of the rows
-// (within one element every target is distinct: plain adds, no atomics). The inner
-// loop is one block fetch and 9 adds per lane. Every group copy is zeroed and read once
-// per node, which for the short rows of the <= 8-node families costs more shared-memory
-// traffic than the idle lanes of two 16-lane groups (measured on the C3D8 tangent
-// gather, two groups against four: FP64 10 %, mixed 12 % faster). The epilogue
-// reads every staged entry as the sum of the group copies in group order, and
-//  - in mixed precision forms the diagonal block of node a as minus the FP64 sum of
-//    all off-diagonal FP32 blocks in its rows (27 lanes: 9 entries x 3 phases, added in
-//    a fixed order), so rigid translations stay in the null space of K to FP64 accuracy;
-//  - stores the free rows: interior nodes (every neighbour fully free) as staged, with
-//    coalesced writes; the others lane by neighbour, at the compressed columns a warp
-//    scan of the neighbours' free-component counts gives, moving the prescribed
-//    columns into the rhs (-K_fc u_c, src/fem/assembly.cpp:95-96).
-// The node's incident-element codes come in with one coalesced load per 32 elements and
-// are handed out by shuffles.
-template <int ET, bool DIAGFIX>
-struct P2Geo {
-  static constexpr int n = nodes_of(ET);
-  static constexpr int GS = n <= 16 ? 16 : 32;
-  static constexpr int EG = 32 / GS;
-  // lanes n .. n + 2 of a group are idle in the block loop and gather the three
-  // components of the element forces (all families but C3D15, whose 16-lane groups
-  // leave one lane, and whose diagonal-block lane takes them)
-  static constexpr bool FIDLE = n + 3 <= GS;
-};
-
-template <typename R>
-struct P2Pass {
-  double v[9];
-  int64_t e;
-  int la, slotv;
-  bool active;
-};
-
-template <int ET, typename R, bool WIN>
-__device__ __forceinline__ void p2_fetch(const ElemArgs& A, const V2Args& V, const R* ed, int code, bool active,
-                                         int lb, P2Pass<R>& p) {
-  constexpr int n = nodes_of(ET), NB = n * (n + 1) / 2;
-  p.active = active;
-  p.e = code / n;
-  p.la = code % n;
-  if (active) {
-    p.slotv = __ldg(A.slot + (p.e * n + p.la) * n + lb);
-    const bool tr = lb < p.la;
-    R raw[9];
-    load_block<R>(ed + (WIN ? ring_slot(p.e, V) : p.e) * (NB * blk_stride<R>()) +
-                      (tr ? blk_index(n, lb, p.la) : blk_index(n, p.la, lb)) * blk_stride<R>(),
-                  raw);
-#pragma unroll
-    for (int q = 0; q < 9; ++q) p.v[q] = static_cast<double>(tr ? raw[3 * (q % 3) + q / 3] : raw[q]);
-  } else {
-    p.slotv = 0;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) p.v[q] = 0.0;
-  }
-}
-
-template <int ET, bool TAN, typename R, bool DIAGFIX, bool WIN>
-__device__ __forceinline__ void p2_body(const ElemArgs& A, const V2Args& V, unsigned bid, unsigned nblk) {
-  constexpr int n = nodes_of(ET);
-  constexpr int GS = P2Geo<ET, DIAGFIX>::GS, EG = P2Geo<ET, DIAGFIX>::EG;
-  constexpr unsigned kAll = 0xffffffffu;
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int stride = static_cast<int>(V.row_stride);  // doubles of one row-buffer copy
-  double* buf = reinterpret_cast<double*>(smem) + warp * (EG * stride);
-  const int64_t gwarp = static_cast<int64_t>(bid) * (blockDim.x >> 5) + warp;
-  const int64_t nwarps = static_cast<int64_t>(nblk) * (blockDim.x >> 5);
-  const R* ed = reinterpret_cast<const R*>(V.edata);
-  const int sub = lane / GS, lb = lane % GS;
-  const bool lane_ok = lb < n;
-  double* mine = buf + sub * stride;
-  // nodes [V.n_begin, V.n_end) of this window's node list (node_order, WIN), or of the mesh
-  const int64_t n_begin = WIN ? V.n_begin : 0, n_end = WIN ? V.n_end : A.n_nodes;
-  // per-node scalars, all loaded at the node's start
-  struct NodeInfo {
-    int64_t a, i0, i1, base;
-    int ma, L, K;
-  };
-  auto node_info = [&](int64_t idx) {
-    NodeInfo t;
-    t.a = WIN ? static_cast<int64_t>(V.node_order[idx]) : idx;
-    t.ma = A.node_mask[t.a];
-    t.K = A.adj_len[t.a];
-    t.i0 = V.inc_ptr[t.a];
-    t.i1 = V.inc_ptr[t.a + 1];
-    t.base = A.node_base[t.a];
-    t.L = static_cast<int>(A.node_rowlen[t.a]);
-    return t;
-  };
-  for (int64_t idx = n_begin + gwarp; idx < n_end; idx += nwarps) {
-    const NodeInfo cur_node = node_info(idx);
-    const int64_t a = cur_node.a;
-    const int ma = cur_node.ma;
-    const int K = cur_node.K;  // neighbours, a itself included
-    const int W = 3 * K;                               // full-width row length
-    const int total = 3 * W;
-    const int64_t i0 = cur_node.i0, i1 = cur_node.i1;
-    const int L = cur_node.L;
-    // every copy starts 16-byte aligned (stride is even) and holds at least total + 1
-    // doubles when total is odd
-    for (int g = 0; g < EG; ++g)
-      for (int t = lane; 2 * t < total; t += 32)
-        reinterpret_cast<double2*>(buf + g * stride)[t] = make_double2(0.0, 0.0);
-    __syncwarp();
-    constexpr bool FIDLE = P2Geo<ET, DIAGFIX>::FIDLE;
-    // a's internal force: component lb - n on lanes lb = n .. n + 2 (FIDLE), else all
-    // three on the lane of each element's diagonal block
-    double fs[FIDLE ? 1 : 3] = {};
-    int slot_aa = 0;  // position of node a in its own adjacency list (DIAGFIX)
-    for (int64_t c0 = i0; c0 < i1; c0 += 32) {
-      const int cnt = static_cast<int>(i1 - c0 < 32 ? i1 - c0 : 32);
-      const int code_l = lane < cnt ? __ldg(V.inc_code + c0 + lane) : 0;
-      for (int k = 0; k < cnt; k += EG) {
-        P2Pass<R> cur;
-        p2_fetch<ET, R, WIN>(A, V, ed, __shfl_sync(kAll, code_l, (k + sub) & 31), lane_ok && k + sub < cnt, lb, cur);
-        if (cur.active && (!DIAGFIX || lb != cur.la)) {
-          double* c = mine + 3 * cur.slotv;
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            c[i * W] += cur.v[3 * i];
-            c[i * W + 1] += cur.v[3 * i + 1];
-            c[i * W + 2] += cur.v[3 * i + 2];
-          }
-        }
-        if constexpr (TAN && FIDLE) {
-          if (lb >= n && lb < n + 3 && k + sub < cnt)
-            fs[0] += __ldg(V.fdata + (WIN ? ring_slot(cur.e, V) : cur.e) * (3 * n) + 3 * cur.la + (lb - n));
-        } else if constexpr (TAN) {
-          if (cur.active && lb == cur.la)
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-              fs[d] += __ldg(V.fdata + (WIN ? ring_slot(cur.e, V) : cur.e) * (3 * n) + 3 * cur.la + d);
-        }
-        if (DIAGFIX && cur.active && lb == cur.la) slot_aa = cur.slotv;
-        __syncwarp();
-      }
-    }
-    // staged entry t: the group copies summed in group order
-    auto staged = [&](int t) {
-      double v = buf[t];
-#pragma unroll
-      for (int g = 1; g < EG; ++g) v += buf[g * stride + t];
-      return v;
-    };
-    if (DIAGFIX) {
-      // diagonal block of node a: minus the FP64 sum of every off-diagonal block in its
-      // rows. Lane 9 p + q (p < 3) sums entry q of the blocks of neighbours p, p + 3,
-      // ... in neighbour order; lane q then adds the three phases in phase order.
-      slot_aa = static_cast<int>(__reduce_max_sync(kAll, static_cast<unsigned>(slot_aa)));
-      const int q = lane % 9, p = lane / 9, qi = q / 3, qj = q - 3 * qi;
-      double d = 0.0;
-      if (p < 3)
-        for (int s = p; s < K; s += 3)
-          if (s != slot_aa) d += staged(qi * W + 3 * s + qj);
-      const double d1 = __shfl_sync(kAll, d, (lane + 9) & 31), d2 = __shfl_sync(kAll, d, (lane + 18) & 31);
-      if (lane < 9 && i1 > i0) buf[qi * W + 3 * slot_aa + qj] = -((d + d1) + d2);
-      __syncwarp();
-    }
-    // Interior nodes (every neighbour fully free, L == W) store the staged rows as they
-    // are, coalesced. At the others each lane takes a neighbour: a warp scan of the
-    // neighbours' free-component counts gives its first compressed column, its free
-    // columns are stored there and its prescribed columns go to the rhs.
-    double rr[3] = {0.0, 0.0, 0.0};
-    double* orow0 = A.vals + cur_node.base;
-    if (L == W) {
-      double* orow = orow0;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        if (!((ma >> i) & 1)) continue;
-        for (int c = lane; c < L; c += 32) {
-          const double v = staged(i * W + c);
-          orow[c] = V.accumulate ? orow[c] + v : v;
-        }
-        orow += L;
-      }
-    } else {
-      const int32_t* nbr = A.bnd_node + A.bnd_ptr[a];
-      int carry = 0;
-      for (int s0 = 0; s0 < K; s0 += 32) {
-        const int s = s0 + lane;
-        const bool ok = s < K;
-        const int b = ok ? __ldg(nbr + s) : 0;
-        const int mb = ok ? static_cast<int>(A.node_mask[b]) : 0;
-        const int pc = __popc(mb);
-        int incl = pc;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-          const int y = __shfl_up_sync(kAll, incl, off);
-          if (lane >= off) incl += y;
-        }
-        const int c = carry + incl - pc;
-        carry += __shfl_sync(kAll, incl, 31);
-        if (ok) {
-#pragma unroll
-          for (int jj = 0; jj < 3; ++jj) {
-            if ((mb >> jj) & 1) {
-              const int col = c + __popc(mb & ((1 << jj) - 1));
-              int ri = 0;
-#pragma unroll
-              for (int i = 0; i < 3; ++i) {
-                if (!((ma >> i) & 1)) continue;
-                double* o = orow0 + static_cast<int64_t>(ri) * L + col;
-                const double v = staged(i * W + 3 * s + jj);
-                *o = V.accumulate ? *o + v : v;
-                ++ri;
-              }
-            } else {
-              const double pv = A.prescribed[3 * static_cast<int64_t>(b) + jj];
-              if (pv != 0.0) {
-#pragma unroll
-                for (int i = 0; i < 3; ++i) rr[i] -= staged(i * W + 3 * s + jj) * pv;
-              }
-            }
-          }
-        }
-      }
-    }
-    if (A.rhs) {
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        double v = rr[r];
-        // interior nodes have no prescribed columns: every lane's term is +0.0
-        if (L != W)
-          for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(kAll, v, off);
-        if (lane == 0 && ((ma >> r) & 1)) {
-          const int64_t eq = A.node_eq0[a] + __popc(ma & ((1 << r) - 1));
-          const double prev = V.accumulate ? A.rhs[eq] : (V.f_ext ? V.f_ext[3 * a + r] : 0.0);
-          A.rhs[eq] = prev + v;
-        }
-      }
-    }
-    if (TAN && A.f_int) {
-      if constexpr (FIDLE) {
-        // group partials (each in incidence order) added in group order
-        double v = fs[0];
-#pragma unroll
-        for (int g = 1; g < EG; ++g) v += __shfl_sync(kAll, fs[0], (lane + g * GS) & 31);
-        if (lane >= n && lane < n + 3) {
-          const int d = lane - n;
-          A.f_int[3 * a + d] = (V.accumulate ? A.f_int[3 * a + d] : 0.0) + v;
-        }
-      } else {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          double v = fs[d];
-          for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(kAll, v, off);
-          if (lane == 0) A.f_int[3 * a + d] = (V.accumulate ? A.f_int[3 * a + d] : 0.0) + v;
-        }
-      }
-    }
-    __syncwarp();
-  }
-}
-
-// Blocks of at most 8 warps, compiled without a register budget (48-72 registers).
-// WIN: the windowed schedule (node list and element ring); the one-window gather is
-// compiled without either, so it keeps the registers of a plain node loop.
-template <int ET, bool TAN, typename R, bool DIAGFIX, bool WIN>
-__global__ void p2_kernel(ElemArgs A, V2Args V) {
-  p2_body<ET, TAN, R, DIAGFIX, WIN>(A, V, blockIdx.x, gridDim.x);
-}
-
-// The gather of the <= 8-node families, compiled for 5 resident 8-warp blocks per SM
-// (<= 48 registers): their row buffers are small, so registers, not shared memory, bound
-// their resident warps, and the latency-bound gather runs faster with more of them.
-template <int ET, bool TAN, typename R, bool DIAGFIX, bool WIN>
-__global__ void __launch_bounds__(256, 5) p2_kernel_small(ElemArgs A, V2Args V) {
-  p2_body<ET, TAN, R, DIAGFIX, WIN>(A, V, blockIdx.x, gridDim.x);
-}
-
-int sm_count() {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
-// Persistent grid: blocks_per_sm (0 = as many as are resident) blocks on every SM,
-// capped by the work available.
-int64_t persistent_grid(int64_t need, int resident, int blocks_per_sm) {
-  const int per_sm = blocks_per_sm > 0 ? std::min(blocks_per_sm, std::max(resident, 1)) : std::max(resident, 1);
-  return std::max<int64_t>(1, std::min<int64_t>(need, static_cast<int64_t>(per_sm) * sm_count()));
 }
 
 template <int ET, int MODE, typename R, int TILE>
@@ -1140,45 +667,17 @@ cudaError_t launch_p1_tile(const ElemArgs& a, const V2Args& v, const LaunchCfg& 
   return cudaGetLastError();
 }
 
-// Tile shapes instantiated: 2x4 and 2x2 everywhere, 4x4 in the linear pass with FP32
-// accumulators.
-template <int ET, int MODE, typename R>
+// Tile shapes of the FP32 pass: 2x4, 2x2 and 4x4 in linear mode. The material-point pass
+// has 2x2 tiles whatever was asked (its tiles carry three accumulator terms: 2x4 measured
+// 1.6 times slower), and so has the FP64 pass its own (cxg_fp64.cu).
+template <int ET, int MODE>
 cudaError_t launch_p1_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, cudaStream_t s) {
-  if (cfg.tile == 1) return launch_p1_tile<ET, MODE, R, 1>(a, v, cfg, s);
-  if constexpr (MODE == MODE_LINEAR && sizeof(R) == 4) {
-    if (cfg.tile == 2) return launch_p1_tile<ET, MODE, R, 2>(a, v, cfg, s);
+  if (MODE == MODE_TANGENT || cfg.tile == 1) return launch_p1_tile<ET, MODE, float, 1>(a, v, cfg, s);
+  if constexpr (MODE == MODE_LINEAR) {
+    if (cfg.tile == 2) return launch_p1_tile<ET, MODE, float, 2>(a, v, cfg, s);
+    if (cfg.tile == 0) return launch_p1_tile<ET, MODE, float, 0>(a, v, cfg, s);
   }
-  if (cfg.tile != 0) return cudaErrorInvalidValue;
-  return launch_p1_tile<ET, MODE, R, 0>(a, v, cfg, s);
-}
-
-template <int ET, bool TAN, typename R, bool DF>
-cudaError_t launch_p2_t(const ElemArgs& a, V2Args v, const LaunchCfg& cfg, cudaStream_t s) {
-  auto kern = v.node_order ? p2_kernel<ET, TAN, R, DF, true> : p2_kernel<ET, TAN, R, DF, false>;
-  if constexpr (nodes_of(ET) <= 8)
-    kern = v.node_order ? p2_kernel_small<ET, TAN, R, DF, true> : p2_kernel_small<ET, TAN, R, DF, false>;
-  // warps per block: as many as fit in ~160 KB of row buffers, up to 8 (or the
-  // configured count when it fits). Per warp: EG full-width copies of three rows of
-  // 3 x max_adj doubles. (Shared memory beyond that comes out of the L1 cache the
-  // scattered block loads reuse.)
-  const int64_t stride = std::max<int64_t>(2, (9 * v.max_adj + 1) / 2 * 2);
-  const int64_t wbytes = P2Geo<ET, DF>::EG * stride * 8;
-  int warps = cfg.p2_warps > 0 ? std::min(cfg.p2_warps, 8) : 8;
-  while (warps > 1 && warps * wbytes > 160 * 1024) warps /= 2;
-  const size_t smem = static_cast<size_t>(warps) * wbytes;
-  if (smem > 220 * 1024) return cudaErrorInvalidConfiguration;
-  v.row_stride = stride;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (err != cudaSuccess) return err;
-  int per_sm = 0;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem);
-  if (err != cudaSuccess) return err;
-  const int64_t count = v.n_end - v.n_begin;
-  if (count <= 0) return cudaSuccess;
-  const int64_t need = (count + warps - 1) / warps;
-  const int64_t grid = persistent_grid(need, per_sm, cfg.p2_blocks_per_sm);
-  kern<<<static_cast<unsigned>(grid), warps * 32, smem, s>>>(a, v);
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 template <int ET>
@@ -1213,14 +712,14 @@ cudaError_t launch_v2_pair(int mode, int precision, const ElemArgs& a, const V2A
   cudaError_t err = cudaSuccess;
   if (mode == MODE_LINEAR) {
     if (c.passes & 1)
-      err = precision ? launch_p1_t<ET, MODE_LINEAR, float>(a, v, c, s) : launch_p1_t<ET, MODE_LINEAR, double>(a, v, c, s);
+      err = precision ? launch_p1_t<ET, MODE_LINEAR>(a, v, c, s) : launch_p1_fp64(ET, MODE_LINEAR, a, v, c, s);
     if (err != cudaSuccess || !(c.passes & 2)) return err;
-    return precision ? launch_p2_t<ET, false, float, true>(a, v, c, s) : launch_p2_t<ET, false, double, false>(a, v, c, s);
+    return launch_gather(precision ? GATHER_DIAG : GATHER_FULL, false, a, v, c, s);
   }
   if (c.passes & 1)
-    err = precision ? launch_p1_t<ET, MODE_TANGENT, float>(a, v, c, s) : launch_p1_t<ET, MODE_TANGENT, double>(a, v, c, s);
+    err = precision ? launch_p1_t<ET, MODE_TANGENT>(a, v, c, s) : launch_p1_fp64(ET, MODE_TANGENT, a, v, c, s);
   if (err != cudaSuccess || !(c.passes & 2)) return err;
-  return precision ? launch_p2_t<ET, true, float, true>(a, v, c, s) : launch_p2_t<ET, true, double, false>(a, v, c, s);
+  return launch_gather(precision ? GATHER_DIAG : GATHER_FULL, true, a, v, c, s);
 }
 
 // ---- scalar-block element pass (mass, geometric stiffness) ---------------------------
@@ -1302,7 +801,7 @@ __global__ void __launch_bounds__(kScalarWarps * 32) scalar_kernel(ElemArgs A, V
       }
     }
     __syncwarp();
-    double* out = reinterpret_cast<double*>(V.edata) + e * (NB * blk_stride<double>());
+    double* out = reinterpret_cast<double*>(V.edata) + e * (blocks_padded(n) * 9);
     for (int p = lane; p < NB; p += 32) {
       const int a = s_pa[p], b = s_pb[p];
       double val = 0.0;
@@ -1334,7 +833,8 @@ __global__ void __launch_bounds__(kScalarWarps * 32) scalar_kernel(ElemArgs A, V
         }
       }
       const double bv[9] = {val, 0.0, 0.0, 0.0, val, 0.0, 0.0, 0.0, val};
-      store_block<double>(out + p * blk_stride<double>(), bv);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) out[p * 9 + k] = bv[k];
     }
     __syncwarp();
   }
@@ -1370,14 +870,22 @@ cudaError_t launch_scalar_type(int kind, const ElemArgs& a, const V2Args& v, con
 
 }  // namespace
 
+void share_blocks(const double* weight, const int64_t* need, int n, int64_t total, int64_t* grid) {
+  double sum = 0.0;
+  for (int k = 0; k < n; ++k) sum += weight[k] > 0.0 ? weight[k] : 0.0;
+  for (int k = 0; k < n; ++k) {
+    const double f = sum > 0.0 ? std::max(weight[k], 0.0) / sum : 1.0 / n;
+    const int64_t g = static_cast<int64_t>(std::llround(f * static_cast<double>(total)));
+    grid[k] = std::max<int64_t>(1, std::min<int64_t>(need[k], g));
+  }
+}
+
 size_t v2_bytes_per_element(int t, int precision, bool tangent) {
   return v2_edata_bytes(t, 1, precision) + (tangent ? sizeof(double) * 3 * nodes_of(t) : 0);
 }
 
 size_t v2_edata_bytes(int t, int64_t n_elems, int precision) {
-  const int n = nodes_of(t);
-  return static_cast<size_t>(n_elems) * (n * (n + 1) / 2) *
-         (precision ? blk_stride<float>() * sizeof(float) : blk_stride<double>() * sizeof(double));
+  return static_cast<size_t>(n_elems) * blocks_padded(nodes_of(t)) * 9 * (precision ? sizeof(float) : sizeof(double));
 }
 
 cudaError_t launch_v2(int t, int mode, int precision, const ElemArgs& a, const V2Args& v, cudaStream_t s,
@@ -1396,41 +904,6 @@ cudaError_t launch_v2(int t, int mode, int precision, const ElemArgs& a, const V
 }
 
 // ---- one launch per pass for a batch of element-type groups ---------------------------
-// Slot k of a pass is one group (one element type, the concatenated models of that type)
-// and owns blocks [blk0_k, blk0_{k+1}) of the grid. A block reads its slot's arguments
-// in place from the kernel's parameter space (a copy in shared memory measured slower:
-// the bodies' shared-memory stores made every argument a reload) and runs the group's
-// element-pass or row-gather body with its index among the slot's blocks in place of
-// blockIdx. The bodies are the ones the
-// per-group kernels inline, so every value is the same bit for bit; the kernel holds
-// the largest register count of its bodies, which is what a group pays for sharing
-// the launch.
-struct BatchSlot {
-  ElemArgs a;
-  V2Args v;
-  int64_t blk0;
-  int32_t type, tile;
-};
-struct BatchPass {
-  BatchSlot s[kMaxBatchSlots];
-  int32_t n;
-};
-static_assert(sizeof(BatchPass) <= 4096, "batch pass arguments exceed the kernel parameter space");
-
-// Slot of this block (block-uniform).
-__device__ __forceinline__ int slot_of(const BatchPass& P) {
-  int k = 0;
-  while (k + 1 < P.n && static_cast<int64_t>(blockIdx.x) >= P.s[k + 1].blk0) ++k;
-  return k;
-}
-
-// This block's index among its slot's blocks, and their count.
-__device__ __forceinline__ void slot_blocks(const BatchPass& P, int k, unsigned& bid, unsigned& nblk) {
-  const int64_t end = k + 1 < P.n ? P.s[k + 1].blk0 : static_cast<int64_t>(gridDim.x);
-  bid = blockIdx.x - static_cast<unsigned>(P.s[k].blk0);
-  nblk = static_cast<unsigned>(end - P.s[k].blk0);
-}
-
 template <int ET, int MODE, typename R, int TILE, bool J2F32>
 __device__ __forceinline__ void p1_slot(const ElemArgs& A, const V2Args& V, unsigned bid, unsigned nblk) {
   p1_body<ET, MODE, R, TILE, J2F32>(A, V, bid, nblk);
@@ -1457,10 +930,9 @@ __device__ __forceinline__ void p1_slot_tile(int tile, const ElemArgs& A, const 
 template <int MODE, typename R, bool J2F32>
 __global__ void __launch_bounds__(kT1, 3) p1_batch_kernel(const __grid_constant__ BatchPass P) {
   // the slot's arguments are read in place from the (read-only) parameter space
-  const int k = slot_of(P);
-  const BatchSlot& S = P.s[k];
   unsigned bid, nblk;
-  slot_blocks(P, k, bid, nblk);
+  const int k = slot_blocks(P, bid, nblk);
+  const BatchSlot& S = P.s[k];
   switch (S.type) {
     case C3D4: p1_slot_tile<C3D4, MODE, R, J2F32>(S.tile, S.a, S.v, bid, nblk); break;
     case C3D10: p1_slot_tile<C3D10, MODE, R, J2F32>(S.tile, S.a, S.v, bid, nblk); break;
@@ -1474,35 +946,6 @@ __global__ void __launch_bounds__(kT1, 3) p1_batch_kernel(const __grid_constant_
   }
 }
 
-template <int ET, bool TAN, typename R, bool DF>
-__device__ __forceinline__ void p2_slot(const ElemArgs& A, const V2Args& V, unsigned bid, unsigned nblk) {
-  p2_body<ET, TAN, R, DF, false>(A, V, bid, nblk);
-}
-
-template <bool TAN, typename R, bool DF>
-__global__ void p2_batch_kernel(const __grid_constant__ BatchPass P) {
-  const int k = slot_of(P);
-  const BatchSlot& S = P.s[k];
-  unsigned bid, nblk;
-  slot_blocks(P, k, bid, nblk);
-  switch (S.type) {
-    case C3D4: p2_slot<C3D4, TAN, R, DF>(S.a, S.v, bid, nblk); break;
-    case C3D10: p2_slot<C3D10, TAN, R, DF>(S.a, S.v, bid, nblk); break;
-    case C3D8: p2_slot<C3D8, TAN, R, DF>(S.a, S.v, bid, nblk); break;
-    case C3D8R: p2_slot<C3D8R, TAN, R, DF>(S.a, S.v, bid, nblk); break;
-    case C3D20: p2_slot<C3D20, TAN, R, DF>(S.a, S.v, bid, nblk); break;
-    case C3D20R: p2_slot<C3D20R, TAN, R, DF>(S.a, S.v, bid, nblk); break;
-    case C3D6: p2_slot<C3D6, TAN, R, DF>(S.a, S.v, bid, nblk); break;
-    case C3D15: p2_slot<C3D15, TAN, R, DF>(S.a, S.v, bid, nblk); break;
-    default: break;
-  }
-}
-
-// Per-(family, tile) figures the launcher needs at run time.
-struct P1Shape {
-  size_t smem = 0;
-  int epw = 1;
-};
 template <int ET, int MODE, typename R, int TILE>
 P1Shape p1_shape_of() {
   return {p1_smem_bytes<ET, MODE, R, TILE>(), Geo<ET, TILE>::EPW};
@@ -1527,31 +970,21 @@ P1Shape p1_shape(int t, int tile) {
     default: return p1_shape_tile<C3D15, MODE, R>(tile);
   }
 }
-// Row-buffer copies per warp of the row gather (P2Geo::EG): two 16-lane groups for the
-// families of at most 16 nodes, one 32-lane group above.
-int p2_groups_of(int t) { return nodes_of(t) <= 16 ? 2 : 1; }
-
-// Blocks of a persistent grid of `total` blocks shared out in proportion to the
-// slots' weights, at least one and at most `need` per slot.
-void share_blocks(const double* weight, const int64_t* need, int n, int64_t total, int64_t* grid) {
-  double sum = 0.0;
-  for (int k = 0; k < n; ++k) sum += weight[k] > 0.0 ? weight[k] : 0.0;
-  for (int k = 0; k < n; ++k) {
-    const double f = sum > 0.0 ? std::max(weight[k], 0.0) / sum : 1.0 / n;
-    const int64_t g = static_cast<int64_t>(std::llround(f * static_cast<double>(total)));
-    grid[k] = std::max<int64_t>(1, std::min<int64_t>(need[k], g));
-  }
-}
-
-template <int MODE, typename R, bool J2F32>
-cudaError_t launch_p1_batch(const BatchSlotIn* in, int n, cudaStream_t s) {
-  auto kern = p1_batch_kernel<MODE, R, J2F32>;
+// Element pass of the whole batch: the kernel and the per-family figures of the mode and
+// precision (FP64 blocks: cxg_fp64.cu).
+cudaError_t launch_p1_batch(int mode, int precision, bool j2f32, const BatchSlotIn* in, int n, cudaStream_t s) {
+  const void* kern = !precision             ? p1_fp64_batch(mode)
+                     : mode == MODE_LINEAR ? reinterpret_cast<const void*>(p1_batch_kernel<MODE_LINEAR, float, false>)
+                     : j2f32               ? reinterpret_cast<const void*>(p1_batch_kernel<MODE_TANGENT, float, true>)
+                                           : reinterpret_cast<const void*>(p1_batch_kernel<MODE_TANGENT, float, false>);
   BatchPass P{};
   size_t smem = 0;
   int64_t need[kMaxBatchSlots], grid[kMaxBatchSlots];
   double w[kMaxBatchSlots];
   for (int k = 0; k < n; ++k) {
-    const P1Shape sh = p1_shape<MODE, R>(in[k].type, in[k].cfg.tile);
+    const P1Shape sh = !precision            ? p1_fp64_shape(in[k].type, mode)
+                       : mode == MODE_LINEAR ? p1_shape<MODE_LINEAR, float>(in[k].type, in[k].cfg.tile)
+                                             : p1_shape<MODE_TANGENT, float>(in[k].type, in[k].cfg.tile);
     smem = std::max(smem, sh.smem);
     const int64_t count = in[k].v.e_end - in[k].v.e_begin;
     need[k] = std::max<int64_t>(1, (count + kW1 * sh.epw - 1) / (kW1 * sh.epw));
@@ -1575,54 +1008,8 @@ cudaError_t launch_p1_batch(const BatchSlotIn* in, int n, cudaStream_t s) {
     blk += grid[k];
   }
   P.n = n;
-  kern<<<static_cast<unsigned>(blk), kT1, smem, s>>>(P);
-  return cudaGetLastError();
-}
-
-template <bool TAN, typename R, bool DF>
-cudaError_t launch_p2_batch(const BatchSlotIn* in, int n, cudaStream_t s) {
-  auto kern = p2_batch_kernel<TAN, R, DF>;
-  BatchPass P{};
-  // one block shape for every slot: the most warps every slot's row buffers allow in
-  // ~160 KB, at most 8 (or the smallest configured count)
-  int warps = 8;
-  int64_t wbytes_max = 0;
-  for (int k = 0; k < n; ++k) {
-    const int64_t stride = std::max<int64_t>(2, (9 * in[k].v.max_adj + 1) / 2 * 2);
-    const int64_t wbytes = p2_groups_of(in[k].type) * stride * 8;
-    wbytes_max = std::max(wbytes_max, wbytes);
-    if (in[k].cfg.p2_warps > 0) warps = std::min(warps, in[k].cfg.p2_warps);
-  }
-  while (warps > 1 && warps * wbytes_max > 160 * 1024) warps /= 2;
-  const size_t smem = static_cast<size_t>(warps) * wbytes_max;
-  if (smem > 220 * 1024) return cudaErrorInvalidConfiguration;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (err != cudaSuccess) return err;
-  int per_sm = 0;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem);
-  if (err != cudaSuccess) return err;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  int64_t need[kMaxBatchSlots], grid[kMaxBatchSlots];
-  double w[kMaxBatchSlots];
-  for (int k = 0; k < n; ++k) {
-    const int64_t count = in[k].v.n_end - in[k].v.n_begin;
-    need[k] = std::max<int64_t>(1, (count + warps - 1) / warps);
-    w[k] = in[k].p2_weight;
-  }
-  share_blocks(w, need, n, static_cast<int64_t>(per_sm) * sm_count(), grid);
-  int64_t blk = 0;
-  for (int k = 0; k < n; ++k) {
-    P.s[k].a = in[k].a;
-    P.s[k].v = in[k].v;
-    P.s[k].v.row_stride = std::max<int64_t>(2, (9 * in[k].v.max_adj + 1) / 2 * 2);
-    P.s[k].blk0 = blk;
-    P.s[k].type = in[k].type;
-    P.s[k].tile = in[k].cfg.tile;
-    blk += grid[k];
-  }
-  P.n = n;
-  kern<<<static_cast<unsigned>(blk), warps * 32, smem, s>>>(P);
-  return cudaGetLastError();
+  void* args[] = {&P};
+  return cudaLaunchKernel(kern, dim3(static_cast<unsigned>(blk)), dim3(kT1), args, smem, s);
 }
 
 cudaError_t launch_v2_batch(int mode, int precision, const BatchSlotIn* in, int n, int passes, cudaStream_t s) {
@@ -1638,22 +1025,10 @@ cudaError_t launch_v2_batch(int mode, int precision, const BatchSlotIn* in, int 
   }
   cudaError_t err = cudaSuccess;
   if (passes & 1) {
-    if (mode == MODE_LINEAR)
-      err = precision ? launch_p1_batch<MODE_LINEAR, float, false>(in, n, s)
-                      : launch_p1_batch<MODE_LINEAR, double, false>(in, n, s);
-    else if (precision)
-      err = j2f32 ? launch_p1_batch<MODE_TANGENT, float, true>(in, n, s)
-                  : launch_p1_batch<MODE_TANGENT, float, false>(in, n, s);
-    else
-      err = launch_p1_batch<MODE_TANGENT, double, false>(in, n, s);
+    err = launch_p1_batch(mode, precision, j2f32, in, n, s);
     if (err != cudaSuccess) return err;
   }
-  if (passes & 2) {
-    if (mode == MODE_LINEAR)
-      err = precision ? launch_p2_batch<false, float, true>(in, n, s) : launch_p2_batch<false, double, false>(in, n, s);
-    else
-      err = precision ? launch_p2_batch<true, float, true>(in, n, s) : launch_p2_batch<true, double, false>(in, n, s);
-  }
+  if (passes & 2) return launch_gather_batch(precision ? GATHER_DIAG : GATHER_FULL, mode == MODE_TANGENT, in, n, s);
   return err;
 }
 
