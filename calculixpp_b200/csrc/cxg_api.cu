@@ -954,8 +954,22 @@ int cxg_assemble_tangent(cxg_plan* p, const double* u, double* vals, double* f_i
 
 namespace {
 
-// The scalar-block operators (mass, geometric stiffness) on the FP64 element buffer
-// and the FP64 row gather; the rhs side effect of prescribed columns is discarded, as
+// The element buffer of the scalar operators: one FP64 value per element node pair.
+int ensure_scalar(cxg_plan* p) {
+  const size_t need = sizeof(double) * static_cast<size_t>(p->n_elems) * blocks_padded(nodes_of(p->type));
+  if (p->edata_bytes >= need) return CXG_OK;
+  cudaFree(p->edata);
+  p->edata = nullptr;
+  p->device_bytes -= static_cast<int64_t>(p->edata_bytes);
+  p->edata_bytes = 0;
+  CHECK_CUDA(cudaMalloc(&p->edata, std::max<size_t>(need, 16)), "element buffer");
+  p->edata_bytes = need;
+  p->device_bytes += static_cast<int64_t>(need);
+  return CXG_OK;
+}
+
+// The scalar operators (mass, geometric stiffness): one value per element pair and the
+// scalar row gather; the rhs side effect of prescribed columns is discarded, as
 // in the reference (src/fem/assembly.cpp:286-288, 320-322).
 int assemble_scalar(cxg_plan* p, int kind, const double* input, size_t input_bytes, double* vals, void* stream) {
   if (int rc0 = reject_refpat(p)) return rc0;
@@ -966,16 +980,7 @@ int assemble_scalar(cxg_plan* p, int kind, const double* input, size_t input_byt
   int rc = staged(p, 0, vals, vb, false, s, &dv);
   if (!rc && input) rc = staged(p, 5, input, input_bytes, true, s, &din);
   if (rc) return rc;
-  const size_t need = v2_edata_bytes(p->type, p->n_elems, CXG_FP64);
-  if (p->edata_bytes < need) {
-    cudaFree(p->edata);
-    p->edata = nullptr;
-    p->device_bytes -= static_cast<int64_t>(p->edata_bytes);
-    p->edata_bytes = 0;
-    CHECK_CUDA(cudaMalloc(&p->edata, std::max<size_t>(need, 16)), "element buffer");
-    p->edata_bytes = need;
-    p->device_bytes += static_cast<int64_t>(need);
-  }
+  if ((rc = ensure_scalar(p))) return rc;
   ElemArgs a = base_args(p);
   a.vals = static_cast<double*>(dv);
   a.rhs = nullptr;
@@ -983,9 +988,7 @@ int assemble_scalar(cxg_plan* p, int kind, const double* input, size_t input_byt
   const double* d = static_cast<const double*>(din);
   CHECK_CUDA(launch_scalar_pass(p->type, kind, a, v, kind == 3 ? nullptr : d, kind == 3 ? d : nullptr, s),
              "element pass");
-  LaunchCfg gather_only;
-  gather_only.passes = 2;
-  CHECK_CUDA(launch_v2(p->type, MODE_LINEAR, CXG_FP64, a, v, s, gather_only), "row gather");
+  CHECK_CUDA(launch_gather(GATHER_SCALAR, false, a, v, LaunchCfg{}, s), "row gather");
   if ((rc = copy_out(vals, dv, vb, s))) return rc;
   if (dv != vals) CHECK_CUDA(cudaStreamSynchronize(s), "synchronize");
   return CXG_OK;
@@ -1142,29 +1145,24 @@ int cxg_assemble_conduction(cxg_plan* p, const double* conductivity, const doubl
   if (!rc) rc = staged(p, 1, rhs, rb, false, s, &dr);
   if (!rc) rc = staged(p, 5, conductivity, sizeof(double) * static_cast<size_t>(p->n_elems), true, s, &dk);
   if (rc) return rc;
-  if (flux || p->films.n_films > 0) {
-    // nodal flux (and film loads) into component 0 of a 3N load vector (plan staging slot 2)
-    if (p->stage_bytes[2] < 24 * N) {
+  if (p->films.n_films > 0 || (flux && !on_device(flux))) {
+    // nodal flux and film loads in a buffer of the plan (staging slot 2)
+    if (p->stage_bytes[2] < 8 * N) {
       cudaFree(p->stage[2]);
       p->stage[2] = nullptr;
       p->stage_bytes[2] = 0;
-      CHECK_CUDA(cudaMalloc(&p->stage[2], 24 * N), "flux staging");
-      p->stage_bytes[2] = 24 * N;
+      CHECK_CUDA(cudaMalloc(&p->stage[2], 8 * N), "flux staging");
+      p->stage_bytes[2] = 8 * N;
     }
     df = p->stage[2];
-    CHECK_CUDA(cudaMemsetAsync(df, 0, 24 * N, s), "flux staging");
-    if (flux) CHECK_CUDA(cudaMemcpy2DAsync(df, 24, flux, 8, 8, N, cudaMemcpyDefault, s), "flux upload");
+    if (flux)
+      CHECK_CUDA(cudaMemcpyAsync(df, flux, 8 * N, cudaMemcpyDefault, s), "flux upload");
+    else
+      CHECK_CUDA(cudaMemsetAsync(df, 0, 8 * N, s), "flux staging");
+  } else {
+    df = const_cast<double*>(flux);
   }
-  const size_t need = v2_edata_bytes(p->type, p->n_elems, CXG_FP64);
-  if (p->edata_bytes < need) {
-    cudaFree(p->edata);
-    p->edata = nullptr;
-    p->device_bytes -= static_cast<int64_t>(p->edata_bytes);
-    p->edata_bytes = 0;
-    CHECK_CUDA(cudaMalloc(&p->edata, std::max<size_t>(need, 16)), "element buffer");
-    p->edata_bytes = need;
-    p->device_bytes += static_cast<int64_t>(need);
-  }
+  if ((rc = ensure_scalar(p))) return rc;
   ElemArgs a = base_args(p);
   a.vals = static_cast<double*>(dv);
   a.rhs = static_cast<double*>(dr);
@@ -1173,9 +1171,7 @@ int cxg_assemble_conduction(cxg_plan* p, const double* conductivity, const doubl
   if (p->films.n_films > 0)
     CHECK_CUDA(launch_films(p->type, a, p->films, static_cast<double*>(p->edata), static_cast<double*>(df), s),
                "film faces");
-  LaunchCfg gather_only;
-  gather_only.passes = 2;
-  CHECK_CUDA(launch_v2(p->type, MODE_LINEAR, CXG_FP64, a, v, s, gather_only), "row gather");
+  CHECK_CUDA(launch_gather(GATHER_ONE_DOF, false, a, v, LaunchCfg{}, s), "row gather");
   if ((rc = copy_out(vals, dv, vb, s))) return rc;
   if ((rc = copy_out(rhs, dr, rb, s))) return rc;
   if (dv != vals || (rhs && dr != rhs)) CHECK_CUDA(cudaStreamSynchronize(s), "synchronize");

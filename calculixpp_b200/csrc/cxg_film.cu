@@ -4,10 +4,10 @@
 // Film pass: one thread per element that carries films, its films in film order. For
 // each film face it evaluates M_ij = int N_i N_j dA and L_i = int N_i dA with the face
 // rule (3-point triangle, 2x2 quad; dA = |t_xi x t_eta| w), adds h M_ij to the element's
-// FP64 block of nodes (fn_i, fn_j) that the conduction element pass wrote (so the row
+// value of nodes (fn_i, fn_j) that the conduction element pass wrote (so the row
 // gather scatters the film matrix with the element's, prescribed columns included), and
 // writes h T_sink L_i per face node. Load pass: one thread per node that lies on a film
-// face sums those loads in film order into component 0 of the load vector the gather
+// face sums those loads in film order into the nodal load vector the gather
 // adds to the rhs. No atomics: results do not depend on scheduling.
 #include <cuda_runtime.h>
 
@@ -31,7 +31,7 @@ __global__ void film_elem_kernel(ElemArgs A, int type, FilmArgs F, double* edata
   for (int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; g < F.n_felem;
        g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t e = F.felem[g];
-    double* blocks = edata + e * (static_cast<int64_t>(nbp) * 9);
+    double* blocks = edata + e * static_cast<int64_t>(nbp);
     for (int32_t k = F.fptr[g]; k < F.fptr[g + 1]; ++k) {
       const int32_t f = F.flist[k];
       int fn[8], nf = 0;
@@ -70,11 +70,7 @@ __global__ void film_elem_kernel(ElemArgs A, int type, FilmArgs F, double* edata
         for (int j = 0; j < nf; ++j) {
           const int a = fn[i], b = fn[j];
           if (a > b) continue;  // the stored upper block (a, b) carries the pair once
-          double* blk = blocks + blk_index(n, a, b) * 9;
-          const double v = h * M[i][j];
-          blk[0] += v;
-          blk[4] += v;
-          blk[8] += v;
+          blocks[blk_index(n, a, b)] += h * M[i][j];
         }
         F.load[static_cast<int64_t>(f) * 8 + i] = hs * L[i];
       }
@@ -82,12 +78,12 @@ __global__ void film_elem_kernel(ElemArgs A, int type, FilmArgs F, double* edata
   }
 }
 
-__global__ void film_load_kernel(FilmArgs F, double* f_ext3) {
+__global__ void film_load_kernel(FilmArgs F, double* f_ext) {
   for (int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; g < F.n_fnode;
        g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     double s = 0.0;
     for (int32_t k = F.fnptr[g]; k < F.fnptr[g + 1]; ++k) s += F.load[F.fnlist[k]];
-    f_ext3[3 * F.fnode[g]] += s;
+    f_ext[F.fnode[g]] += s;
   }
 }
 
@@ -97,7 +93,7 @@ unsigned film_grid(int64_t n) {
 
 }  // namespace
 
-cudaError_t launch_films(int type, const ElemArgs& a, const FilmArgs& f, double* edata, double* f_ext3,
+cudaError_t launch_films(int type, const ElemArgs& a, const FilmArgs& f, double* edata, double* f_ext,
                          cudaStream_t s) {
   if (f.n_felem > 0) {
     film_elem_kernel<<<film_grid(f.n_felem), 128, 0, s>>>(a, type, f, edata);
@@ -105,7 +101,7 @@ cudaError_t launch_films(int type, const ElemArgs& a, const FilmArgs& f, double*
     if (e != cudaSuccess) return e;
   }
   if (f.n_fnode > 0) {
-    film_load_kernel<<<film_grid(f.n_fnode), 128, 0, s>>>(f, f_ext3);
+    film_load_kernel<<<film_grid(f.n_fnode), 128, 0, s>>>(f, f_ext);
     return cudaGetLastError();
   }
   return cudaSuccess;

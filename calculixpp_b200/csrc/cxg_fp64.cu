@@ -446,7 +446,215 @@ __global__ void __launch_bounds__(kT1, 2) p1_fp64_batch_kernel(const __grid_cons
   }
 }
 
+// ---- scalar operators ------------------------------------------------------------------
+// Mass, geometric stiffness and conduction give every node pair one value (times I): m_ab
+// = sum_q rho detJ w N_a N_b (element_mass, src/fem/element.cpp:786-812), its row sums on
+// the diagonal for the lumped mass (element.cpp:814-831), k_ab = sum_q detJ w g_a .
+// sigma_q . g_b (element_geometric_stiffness + accumulate_kgeo, element.cpp:482-508,
+// 833-854), k_ab = sum_q k detJ w g_a . g_b (element_conduction, element.cpp:745-765).
+// The same tasks and operands as above, one accumulator per tile pair: the three
+// components are three more products. A lane's two values go straight to the element's
+// packed row (8 bytes a pair; the 3x3 blocks this replaced were nine values, eight of them
+// zeros or copies, written and read back: C3D15 conduction of 85,050 elements 399 + 720 us
+// for pass and gather).
+enum ScalarKind : int { MASS = 1, LUMPED = 2, GEOMETRIC = 3, CONDUCTION = 4 };
+
+template <int ET, int KIND>
+struct SSmem {
+  using G = DGeo<ET>;
+  static constexpr bool GRAD = KIND >= GEOMETRIC, GEO = KIND == GEOMETRIC;
+  double g[GRAD ? G::EPB * G::ES : 1];
+  double s[G::EPB][G::NQP];                        // detJ w, times rho or k
+  double sig[GEO ? G::EPB : 1][6][GEO ? G::NQP : 1];  // stress of the points
+  double x[G::EPB][3 * G::n];
+};
+
+// Per block: natural derivatives and weights, and for the masses the shape functions, one
+// row of NQP values per node (rows and points padded with zeros).
+template <int ET, int KIND>
+constexpr int scalar_table() {
+  using G = DGeo<ET>;
+  return (G::n * 3 + 1) * G::nq + (KIND <= LUMPED ? G::NTL * 8 * G::NQP : 0);
+}
+template <int ET, int KIND>
+constexpr size_t scalar_smem_bytes() {
+  return (sizeof(double) * scalar_table<ET, KIND>() + 15) / 16 * 16 + kW1 * ((sizeof(SSmem<ET, KIND>) + 15) / 16 * 16);
+}
+
+template <int ET, int KIND>
+__global__ void __launch_bounds__(kT1, 4) scalar_kernel(ElemArgs A, V2Args V, const double* density,
+                                                        const double* gp_stress) {
+  using G = DGeo<ET>;
+  using WS = SSmem<ET, KIND>;
+  constexpr int n = G::n, nq = G::nq, EPB = G::EPB, QS = G::QS, P = G::P, ES = G::ES, KS = G::KS, NQP = G::NQP;
+  constexpr int NB = n * (n + 1) / 2;
+  constexpr bool GRAD = WS::GRAD, GEO = WS::GEO;
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* sdN = reinterpret_cast<double*>(smem);  // [n][3][nq]
+  double* sw = sdN + n * 3 * nq;
+  double* sN = sw + nq;  // [node][NQP]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  WS& W = *reinterpret_cast<WS*>(smem + (sizeof(double) * scalar_table<ET, KIND>() + 15) / 16 * 16 +
+                                 warp * ((sizeof(WS) + 15) / 16 * 16));
+  for (int i = threadIdx.x; i < n * 3 * nq; i += blockDim.x) sdN[i] = c_dN[dn_offset(ET) + i];
+  for (int i = threadIdx.x; i < nq; i += blockDim.x) sw[i] = c_w[ET][i];
+  if constexpr (!GRAD)
+    for (int i = threadIdx.x; i < G::NTL * 8 * NQP; i += blockDim.x) {
+      const int k = i / NQP, q = i % NQP;
+      sN[i] = k < n && q < nq ? c_N[nn_offset(ET) + k * nq + q] : 0.0;
+    }
+  if (GRAD)
+    for (int t = lane; t < EPB * ES; t += 32) W.g[t] = 0.0;
+  for (int t = lane; t < EPB * NQP; t += 32) W.s[t / NQP][t % NQP] = 0.0;
+  if (GEO)
+    for (int t = lane; t < EPB * 6 * NQP; t += 32) W.sig[t / (6 * NQP)][t / NQP % 6][t % NQP] = 0.0;
+  __syncthreads();
+  const int64_t gwarp = static_cast<int64_t>(blockIdx.x) * kW1 + warp;
+  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kW1;
+  for (int64_t e0 = gwarp * EPB; e0 < A.n_elems; e0 += nwarps * EPB) {
+    for (int t = lane; t < EPB * n; t += 32) {
+      if (e0 + t / n >= A.n_elems) break;
+      const int64_t node = A.conn[e0 * n + t];
+      for (int d = 0; d < 3; ++d) W.x[t / n][3 * (t % n) + d] = A.coords[3 * node + d];
+    }
+    __syncwarp();
+    for (int t = lane; t < EPB * nq; t += 32) {
+      const int ei = t / nq, q = t % nq;
+      const int64_t e = e0 + ei;
+      if (e >= A.n_elems) continue;
+      double J[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+      for (int k = 0; k < n; ++k) {
+        const double d0 = sdN[(3 * k) * nq + q], d1 = sdN[(3 * k + 1) * nq + q], d2 = sdN[(3 * k + 2) * nq + q];
+        for (int i = 0; i < 3; ++i) {
+          const double xk = W.x[ei][3 * k + i];
+          J[i][0] = fma(xk, d0, J[i][0]);
+          J[i][1] = fma(xk, d1, J[i][1]);
+          J[i][2] = fma(xk, d2, J[i][2]);
+        }
+      }
+      double it[3][3];
+      const double det = invert(J, it);
+      if (!(det > 0.0)) {
+        atomicCAS(&A.status->code, 0, 4);
+        atomicMin(&A.status->bad_elem, static_cast<unsigned long long>(e));
+      }
+      W.s[ei][q] = GEO ? det * sw[q] : density[e] * det * sw[q];
+      if constexpr (GRAD) {
+        double* gq = W.g + ei * ES;
+        for (int k = 0; k < n; ++k) {
+          const double d0 = sdN[(3 * k) * nq + q], d1 = sdN[(3 * k + 1) * nq + q], d2 = sdN[(3 * k + 2) * nq + q];
+          for (int i = 0; i < 3; ++i)
+            gq[i * P + k * QS + (q ^ G::turn(k))] = fma(it[i][0], d0, fma(it[i][1], d1, mul(it[i][2], d2)));
+        }
+      }
+      if constexpr (GEO)
+        for (int c = 0; c < 6; ++c) W.sig[ei][c][q] = gp_stress ? gp_stress[(e * nq + q) * 6 + c] : 0.0;
+    }
+    __syncwarp();
+    const int row = lane >> 2, col = lane & 3, turn = G::turn(row);
+#pragma unroll 1
+    for (int ei = 0; ei < EPB && e0 + ei < A.n_elems; ++ei) {
+      double* out = reinterpret_cast<double*>(V.edata) + (e0 + ei) * blocks_padded(n);
+      if constexpr (KIND == LUMPED) {
+        // row sums sum_b sum_q s N_a N_b on the diagonal, zeros elsewhere
+        for (int t = lane; t < NB; t += 32) out[t] = 0.0;
+        __syncwarp();
+        for (int a = lane; a < n; a += 32) {
+          double m = 0.0;
+          for (int b = 0; b < n; ++b) {
+            double v = 0.0;
+            for (int q = 0; q < nq; ++q) v += W.s[ei][q] * sN[a * NQP + q] * sN[b * NQP + q];
+            m += v;
+          }
+          out[blk_index(n, a, a)] = m;
+        }
+        continue;
+      }
+#pragma unroll 1
+      for (int ta = 0; ta < G::NTL; ++ta)
+#pragma unroll 1
+        for (int tb = ta; tb < G::NTL; ++tb) {
+          double acc[3][2] = {};  // one sum per component, so that the products overlap
+          const double* gA = (GRAD ? W.g + ei * ES : sN) + (8 * ta + row) * QS + col;
+          const double* gB = (GRAD ? W.g + ei * ES : sN) + (8 * tb + row) * QS + col;
+#pragma unroll
+          for (int ks = 0; ks < KS; ++ks) {
+            const double s = W.s[ei][4 * ks + col];
+            if constexpr (!GRAD) {
+              dmma(acc[ks % 3], s * gA[4 * ks], gB[4 * ks]);
+            } else {
+              double a[3];
+#pragma unroll
+              for (int x = 0; x < 3; ++x) a[x] = s * gA[x * P + ((4 * ks) ^ turn)];
+              if constexpr (GEO) {
+                const int q = 4 * ks + col;
+                const double s0 = W.sig[ei][0][q], s1 = W.sig[ei][1][q], s2 = W.sig[ei][2][q], s3 = W.sig[ei][3][q],
+                             s4 = W.sig[ei][4][q], s5 = W.sig[ei][5][q], a0 = a[0], a1 = a[1], a2 = a[2];
+                a[0] = s0 * a0 + s3 * a1 + s4 * a2;
+                a[1] = s3 * a0 + s1 * a1 + s5 * a2;
+                a[2] = s4 * a0 + s5 * a1 + s2 * a2;
+              }
+#pragma unroll
+              for (int x = 0; x < 3; ++x) dmma(acc[x], a[x], gB[x * P + ((4 * ks) ^ turn)]);
+            }
+          }
+          const int a = 8 * ta + row;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int b = 8 * tb + 2 * col + h;
+            if (a < n && b < n && a <= b) out[blk_index(n, a, b)] = (acc[0][h] + acc[1][h]) + acc[2][h];
+          }
+        }
+    }
+    __syncwarp();
+  }
+}
+
+template <int ET, int KIND>
+cudaError_t launch_scalar_t(const ElemArgs& a, const V2Args& v, const double* density, const double* gp_stress,
+                            cudaStream_t s) {
+  if (a.n_elems == 0) return cudaSuccess;
+  auto kern = scalar_kernel<ET, KIND>;
+  constexpr size_t smem = scalar_smem_bytes<ET, KIND>();
+  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (err != cudaSuccess) return err;
+  int per_sm = 0;
+  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kT1, smem);
+  if (err != cudaSuccess) return err;
+  constexpr int per_block = kW1 * DGeo<ET>::EPB;
+  const int64_t grid = persistent_grid((a.n_elems + per_block - 1) / per_block, per_sm, 0);
+  kern<<<static_cast<unsigned>(grid), kT1, smem, s>>>(a, v, density, gp_stress);
+  return cudaGetLastError();
+}
+
+template <int ET>
+cudaError_t launch_scalar_type(int kind, const ElemArgs& a, const V2Args& v, const double* density,
+                               const double* gp_stress, cudaStream_t s) {
+  switch (kind) {
+    case MASS: return launch_scalar_t<ET, MASS>(a, v, density, gp_stress, s);
+    case LUMPED: return launch_scalar_t<ET, LUMPED>(a, v, density, gp_stress, s);
+    case GEOMETRIC: return launch_scalar_t<ET, GEOMETRIC>(a, v, density, gp_stress, s);
+    case CONDUCTION: return launch_scalar_t<ET, CONDUCTION>(a, v, density, gp_stress, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_scalar_pass(int t, int kind, const ElemArgs& a, const V2Args& v, const double* density,
+                               const double* gp_stress, cudaStream_t s) {
+  switch (t) {
+    case C3D4: return launch_scalar_type<C3D4>(kind, a, v, density, gp_stress, s);
+    case C3D10: return launch_scalar_type<C3D10>(kind, a, v, density, gp_stress, s);
+    case C3D8: return launch_scalar_type<C3D8>(kind, a, v, density, gp_stress, s);
+    case C3D8R: return launch_scalar_type<C3D8R>(kind, a, v, density, gp_stress, s);
+    case C3D20: return launch_scalar_type<C3D20>(kind, a, v, density, gp_stress, s);
+    case C3D20R: return launch_scalar_type<C3D20R>(kind, a, v, density, gp_stress, s);
+    case C3D6: return launch_scalar_type<C3D6>(kind, a, v, density, gp_stress, s);
+    case C3D15: return launch_scalar_type<C3D15>(kind, a, v, density, gp_stress, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
 
 cudaError_t launch_p1_fp64(int t, int mode, const ElemArgs& a, const V2Args& v, const LaunchCfg& c, cudaStream_t s) {
   const bool tan = mode == MODE_TANGENT;

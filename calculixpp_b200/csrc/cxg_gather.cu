@@ -83,14 +83,15 @@ __device__ __forceinline__ void end_pair(unsigned last, double*& o, double& v, d
 
 template <typename R, int KIND, bool WIN>
 __device__ __forceinline__ void gather_nodes(const ElemArgs& A, const V2Args& V, unsigned bid, unsigned nblk) {
-  constexpr bool DIAG = KIND == GATHER_DIAG;
+  constexpr bool DIAG = KIND == GATHER_DIAG, SCALAR = KIND == GATHER_SCALAR;
   constexpr int UN = kPairRec;
   const int lane = threadIdx.x & 31;
   const int64_t gwarp = static_cast<int64_t>(bid) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t nwarps = static_cast<int64_t>(nblk) * (blockDim.x >> 5);
   // lanes 27 .. 31 follow the third group without writing
   const int q = min(lane / 9, 2), k = lane < 27 ? lane - 9 * q : 0, ki = k / 3, kj = k - 3 * ki;
-  const R* ed = reinterpret_cast<const R*>(V.edata) + k;
+  const R* ed = reinterpret_cast<const R*>(V.edata) + (SCALAR ? 0 : k);
+  const bool mine = !SCALAR || ki == kj;  // the other entries of a multiple of I are zero
   const int64_t ring_blocks = V.ring * V.nbp, base_blocks = V.ring_base * V.nbp;
   const int64_t n_begin = WIN ? V.n_begin : 0, n_end = WIN ? V.n_end : A.n_nodes;
   for (int64_t idx = n_begin + gwarp; idx < n_end; idx += nwarps) {
@@ -141,7 +142,8 @@ __device__ __forceinline__ void gather_nodes(const ElemArgs& A, const V2Args& V,
         R x[UN];
 #pragma unroll
         for (int i = 0; i < UN; ++i) {
-          x[i] = __ldg(ed + 9 * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks));
+          x[i] = R(0);
+          if (mine) x[i] = __ldg(ed + (SCALAR ? 1 : 9) * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks));
         }
         const bool turns = rec.flags >> 31;
         const unsigned ends = lane < 27 ? rec.flags : 0u;
@@ -214,9 +216,61 @@ __device__ __forceinline__ void gather_nodes(const ElemArgs& A, const V2Args& V,
   }
 }
 
+// One temperature per node: a lane walks one of the three runs of a node, ten nodes to a
+// warp, one value per contribution and per pair.
+__device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& V) {
+  constexpr int UN = kPairRec;
+  const int lane = threadIdx.x & 31, j = lane / 3, q = lane - 3 * j;
+  const int64_t gwarp = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+  const double* ed = reinterpret_cast<const double*>(V.edata);
+  for (int64_t a0 = 10 * gwarp; a0 < A.n_nodes; a0 += 10 * nwarps) {
+    const int64_t a = a0 + j;
+    const bool on = lane < 30 && a < A.n_nodes;
+    NodeRec nd{};
+    if (on) nd = load_node(A.node + a);
+    const bool free = (nd.len_mask >> 28) & 1, full = (nd.len_mask & 0xfffffff) == nd.npair;
+    double rr = 0.0;
+    if (free) {
+      int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
+      const PairRec* list = A.pairs + nd.list0 + q;
+      double* o = A.vals + nd.base;
+      double v = 0.0;
+      for (uint32_t r = 0; r < nd.rounds; ++r, list += 3) {
+        const PairRec rec = load_pairs(list);
+        double x[UN];
+#pragma unroll
+        for (int i = 0; i < UN; ++i) x[i] = __ldg(ed + rec.block[i]);
+#pragma unroll
+        for (int i = 0; i < UN; ++i) {
+          v += x[i];
+          if (rec.flags & (1u << i)) {
+            if (full) {
+              o[p] = v;
+            } else {
+              const uint32_t at = static_cast<uint32_t>(__ldg(A.bnd_col + nd.bnd0 + p));
+              if (at >> 28)
+                o[at & 0xfffffff] = v;
+              else
+                rr -= v * A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p))];
+            }
+            v = 0.0;
+            ++p;
+          }
+        }
+      }
+    }
+    const double r1 = __shfl_down_sync(kAll, rr, 1), r2 = __shfl_down_sync(kAll, rr, 2);
+    if (A.rhs && free && q == 0) A.rhs[nd.eq0] = (V.f_ext ? V.f_ext[a] : 0.0) + ((rr + r1) + r2);
+  }
+}
+
 template <typename R, int KIND, bool WIN>
 __global__ void __launch_bounds__(256, 3) gather_kernel(ElemArgs A, V2Args V) {
-  gather_nodes<R, KIND, WIN>(A, V, blockIdx.x, gridDim.x);
+  if constexpr (KIND == GATHER_ONE_DOF)
+    gather_one_dof(A, V);
+  else
+    gather_nodes<R, KIND, WIN>(A, V, blockIdx.x, gridDim.x);
 }
 
 // Internal force of every node: one thread per component, the element forces in element
@@ -261,7 +315,10 @@ cudaError_t launch_forces(const ElemArgs& a, const V2Args& v, cudaStream_t s) {
 
 template <typename R, int KIND>
 cudaError_t launch_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, cudaStream_t s) {
-  auto kern = v.node_order ? gather_kernel<R, KIND, true> : gather_kernel<R, KIND, false>;
+  auto kern = gather_kernel<R, KIND, false>;
+  if constexpr (KIND == GATHER_FULL || KIND == GATHER_DIAG) {
+    if (v.node_order) kern = gather_kernel<R, KIND, true>;
+  }
   const int warps = cfg.p2_warps > 0 ? std::min(cfg.p2_warps, 8) : 8;
   const int64_t count = v.n_end - v.n_begin;
   if (count <= 0) return cudaSuccess;
@@ -269,7 +326,8 @@ cudaError_t launch_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, c
   const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, 0);
   if (err != cudaSuccess) return err;
   if (cfg.p2_blocks_per_sm > 0) per_sm = std::min(per_sm, cfg.p2_blocks_per_sm);
-  const int64_t grid = std::min<int64_t>((count + warps - 1) / warps, static_cast<int64_t>(std::max(per_sm, 1)) * sm_count());
+  const int64_t block_nodes = static_cast<int64_t>(warps) * (KIND == GATHER_ONE_DOF ? 10 : 1);
+  const int64_t grid = std::min<int64_t>((count + block_nodes - 1) / block_nodes, static_cast<int64_t>(std::max(per_sm, 1)) * sm_count());
   kern<<<static_cast<unsigned>(grid), warps * 32, 0, s>>>(a, v);
   return cudaGetLastError();
 }
@@ -282,6 +340,8 @@ cudaError_t launch_gather(int kind, bool tangent, const ElemArgs& a, const V2Arg
   switch (kind) {
     case GATHER_FULL: e = launch_t<double, GATHER_FULL>(a, v, cfg, s); break;
     case GATHER_DIAG: e = launch_t<float, GATHER_DIAG>(a, v, cfg, s); break;
+    case GATHER_SCALAR: e = launch_t<double, GATHER_SCALAR>(a, v, cfg, s); break;
+    case GATHER_ONE_DOF: e = launch_t<double, GATHER_ONE_DOF>(a, v, cfg, s); break;
     default: return cudaErrorInvalidValue;
   }
   return e == cudaSuccess && tangent ? launch_forces(a, v, s) : e;

@@ -198,8 +198,10 @@ struct BatchSlotIn {
 // weights, at least one and at most `need` per slot.
 void share_blocks(const double* weight, const int64_t* need, int n, int64_t total, int64_t* grid);
 // Row gather (cxg_gather.cu). GATHER_FULL: FP64 blocks, every entry summed; GATHER_DIAG:
-// FP32 blocks, the diagonal block from the row's other entries.
-enum GatherKind : int { GATHER_FULL = 0, GATHER_DIAG = 1 };
+// FP32 blocks, the diagonal block from the row's other entries; GATHER_SCALAR: one FP64
+// value per pair, standing for its multiple of I; GATHER_ONE_DOF: the same on a
+// temperature plan, whose nodes have component 0 only (f_ext is then one value per node).
+enum GatherKind : int { GATHER_FULL = 0, GATHER_DIAG = 1, GATHER_SCALAR = 2, GATHER_ONE_DOF = 3 };
 cudaError_t launch_gather(int kind, bool tangent, const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg,
                           cudaStream_t s);
 cudaError_t launch_gather_batch(int kind, bool tangent, const BatchSlotIn* slots, int n_slots, cudaStream_t s);
@@ -212,8 +214,8 @@ size_t v2_edata_bytes(int elem_type, int64_t n_elems, int precision);
 size_t v2_bytes_per_element(int elem_type, int precision, bool tangent);
 // Element pass of the scalar-block operators (every 3x3 block is a scalar times I):
 // kind 1 consistent mass rho N_a N_b, 2 lumped mass (row sums on the diagonal), 3
-// geometric stiffness g_a . sigma . g_b, 4 conduction k g_a . g_b. Writes FP64 blocks
-// for the FP64 row gather. density[E] is rho (kinds 1, 2) or k (kind 4), gp_stress[6 G]
+// geometric stiffness g_a . sigma . g_b, 4 conduction k g_a . g_b. Writes one FP64 value
+// per element pair, at e * blocks_padded(n) + blk_index. density[E] is rho (kinds 1, 2) or k (kind 4), gp_stress[6 G]
 // (kind 3).
 cudaError_t launch_scalar_pass(int elem_type, int kind, const ElemArgs& a, const V2Args& v, const double* density,
                                const double* gp_stress, cudaStream_t s);
@@ -287,7 +289,7 @@ struct FilmArgs {
   const int32_t* fnlist = nullptr;
   double* load = nullptr;
 };
-cudaError_t launch_films(int elem_type, const ElemArgs& a, const FilmArgs& f, double* edata, double* f_ext3,
+cudaError_t launch_films(int elem_type, const ElemArgs& a, const FilmArgs& f, double* edata, double* f_ext,
                          cudaStream_t s);
 cudaError_t launch_adjoint(int elem_type, const ElemArgs& a, double* dc_dE, double* dc_dX,
                            cudaStream_t s);
