@@ -211,6 +211,43 @@ namespace api {
 // History components an assembly must carry (see cxg_plan::back_stress_zero).
 int state_comps(const cxg_plan* p) { return (p->back_stress_zero && !p->kinematic) ? 7 : kStateDoubles; }
 
+WorkLease::WorkLease(cxg_plan* p, size_t bytes, cudaStream_t s) : p_(p), s_(s) {
+  bytes = std::max<size_t>(bytes, 16);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if ((error = cudaStreamIsCapturing(s, &cap)) != cudaSuccess) return;
+  if (cap != cudaStreamCaptureStatusNone) {
+    error = cudaMallocAsync(reinterpret_cast<void**>(&ptr), bytes, s);
+    return;
+  }
+  lock_ = std::unique_lock<std::mutex>(p->work_mu);
+  if (!p->work_done) error = cudaEventCreateWithFlags(&p->work_done, cudaEventDisableTiming);
+  if (error == cudaSuccess && p->work_bytes < bytes) {
+    cudaFree(p->work);  // waits for its last use
+    p->device_bytes -= static_cast<int64_t>(p->work_bytes);
+    p->work = nullptr;
+    p->work_bytes = 0;
+    error = cudaMalloc(reinterpret_cast<void**>(&p->work), bytes);
+    if (error == cudaSuccess) {
+      p->work_bytes = bytes;
+      p->device_bytes += static_cast<int64_t>(bytes);
+      p->work_stream = s;
+    }
+  } else if (error == cudaSuccess && s != p->work_stream) {
+    error = cudaStreamWaitEvent(s, p->work_done, 0);
+  }
+  if (error == cudaSuccess) ptr = p->work;
+}
+
+WorkLease::~WorkLease() {
+  if (!lock_.owns_lock()) {
+    if (ptr) cudaFreeAsync(ptr, s_);
+    return;
+  }
+  if (!ptr) return;
+  cudaEventRecord(p_->work_done, s_);
+  p_->work_stream = s_;
+}
+
 int ensure_state(cxg_plan* p, cudaStream_t s) {
   if (p->state[0]) return CXG_OK;
   const size_t bytes = sizeof(double) * kStateDoubles * static_cast<size_t>(std::max<int64_t>(p->n_gauss, 1));
@@ -456,45 +493,64 @@ int cxg_plan_create(const cxg_mesh_desc* m, const cxg_dofmap_desc* d, int32_t pr
     cudaError_t _e = (expr);                 \
     if (_e != cudaSuccess) return fail(cuda_err(_e, where)); \
   } while (0)
-  TRYC(alloc_copy(&p->coords, m->coords, 3 * static_cast<size_t>(m->n_nodes), s, &p->device_bytes), "coords");
-  TRYC(alloc_copy(&p->conn, m->conn, static_cast<size_t>(m->n_elems) * npe, s, &p->device_bytes), "conn");
-  TRYC(alloc_copy(&p->dof_eq, d->dof_eq, 3 * static_cast<size_t>(m->n_nodes), s, &p->device_bytes), "dof_eq");
-  TRYC(alloc_copy(&p->prescribed, d->prescribed, 3 * static_cast<size_t>(m->n_nodes), s, &p->device_bytes),
-       "prescribed");
-  TRYC(alloc_copy(&p->mats, mats.data(), mats.size(), s, &p->device_bytes), "materials");
-  if (m->elem_mat)
-    TRYC(alloc_copy(&p->elem_mat, m->elem_mat, static_cast<size_t>(m->n_elems), s, &p->device_bytes), "elem_mat");
-  TRYC(alloc_copy(&p->young, m->young, static_cast<size_t>(m->n_elems), s, &p->device_bytes), "young");
-  TRYC(alloc_copy(&p->poisson, m->poisson, static_cast<size_t>(m->n_elems), s, &p->device_bytes), "poisson");
+  // Every copy of the mesh in one device block, 256-byte aligned parts: the allocations and
+  // frees, each with its own synchronisation, were most of a small plan's making.
+  const size_t N = static_cast<size_t>(m->n_nodes), E = static_cast<size_t>(m->n_elems);
+  std::vector<double> props(2 * static_cast<size_t>(m->n_materials));
+  for (int32_t i = 0; i < m->n_materials; ++i) {
+    props[static_cast<size_t>(i)] = m->materials[i].E;
+    props[static_cast<size_t>(m->n_materials + i)] = m->materials[i].nu;
+  }
+  size_t total = 0;
+  auto place = [&](size_t bytes) {
+    const size_t at = total;
+    total += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+    return at;
+  };
+  const size_t at_coords = place(24 * N), at_conn = place(4 * E * static_cast<size_t>(npe)), at_dof = place(12 * N),
+               at_pre = place(24 * N), at_mats = place(sizeof(J2Mat) * mats.size()),
+               at_em = place(m->elem_mat ? 4 * E : 0), at_young = place(8 * E), at_poisson = place(8 * E),
+               at_props = place(8 * props.size()), at_status = place(sizeof(DevStatus)), at_bad = place(sizeof(int));
+  TRYC(cudaMalloc(&p->mem, total), "plan");
+  p->device_bytes += static_cast<int64_t>(total);
+  char* mem = static_cast<char*>(p->mem);
+  p->coords = reinterpret_cast<double*>(mem + at_coords);
+  p->conn = reinterpret_cast<int32_t*>(mem + at_conn);
+  p->dof_eq = reinterpret_cast<int32_t*>(mem + at_dof);
+  p->prescribed = reinterpret_cast<double*>(mem + at_pre);
+  p->mats = reinterpret_cast<J2Mat*>(mem + at_mats);
+  p->elem_mat = m->elem_mat ? reinterpret_cast<int32_t*>(mem + at_em) : nullptr;
+  p->young = reinterpret_cast<double*>(mem + at_young);
+  p->poisson = reinterpret_cast<double*>(mem + at_poisson);
+  p->status = reinterpret_cast<DevStatus*>(mem + at_status);
+  int* dbad = reinterpret_cast<int*>(mem + at_bad);
+  double* dprops = reinterpret_cast<double*>(mem + at_props);
+  auto copy = [&](void* dst, const void* src, size_t bytes) {
+    return src && bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, s) : cudaSuccess;
+  };
+  TRYC(copy(p->coords, m->coords, 24 * N), "coords");
+  TRYC(copy(p->conn, m->conn, 4 * E * static_cast<size_t>(npe)), "conn");
+  TRYC(copy(p->dof_eq, d->dof_eq, 12 * N), "dof_eq");
+  TRYC(copy(p->prescribed, d->prescribed, 24 * N), "prescribed");
+  TRYC(copy(p->mats, mats.data(), sizeof(J2Mat) * mats.size()), "materials");
+  TRYC(copy(p->elem_mat, m->elem_mat, 4 * E), "elem_mat");
+  TRYC(copy(p->young, m->young, 8 * E), "young");
+  TRYC(copy(p->poisson, m->poisson, 8 * E), "poisson");
+  TRYC(copy(dprops, props.data(), 8 * props.size()), "material properties");
   {
-    std::vector<double> E(static_cast<size_t>(m->n_materials)), nu(E.size());
-    for (int32_t i = 0; i < m->n_materials; ++i) {
-      E[static_cast<size_t>(i)] = m->materials[i].E;
-      nu[static_cast<size_t>(i)] = m->materials[i].nu;
-    }
-    double *dE = nullptr, *dnu = nullptr;
-    int* dbad = nullptr;
-    int64_t dummy = 0;
-    TRYC(alloc_copy(&dE, E.data(), E.size(), s, &dummy), "material E");
-    TRYC(alloc_copy(&dnu, nu.data(), nu.size(), s, &dummy), "material nu");
-    TRYC(cudaMalloc(&dbad, sizeof(int)), "flag");
+    const DevStatus z{0, 0, ~0ull};
+    TRYC(cudaMemcpyAsync(p->status, &z, sizeof z, cudaMemcpyHostToDevice, s), "status");
     TRYC(cudaMemsetAsync(dbad, 0, sizeof(int), s), "flag");
     const unsigned grid = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((m->n_elems + 255) / 256, 4096)));
-    fill_props_kernel<<<grid, 256, 0, s>>>(p->elem_mat, dE, dnu, m->n_materials, m->n_elems,
+    fill_props_kernel<<<grid, 256, 0, s>>>(p->elem_mat, dprops, dprops + m->n_materials, m->n_materials, m->n_elems,
                                            m->young ? nullptr : p->young, m->poisson ? nullptr : p->poisson, dbad);
     TRYC(cudaGetLastError(), "material properties");
-    int bad = 0;
-    TRYC(cudaMemcpyAsync(&bad, dbad, sizeof(int), cudaMemcpyDeviceToHost, s), "flag");
-    TRYC(cudaStreamSynchronize(s), "material properties");
-    cudaFree(dE);
-    cudaFree(dnu);
-    cudaFree(dbad);
-    if (bad) return fail(set_err(CXG_ERR_INVALID_ARGUMENT, "elem_mat index outside [0, n_materials)"));
-  }
-  TRYC(cudaMalloc(&p->status, sizeof(DevStatus)), "status");
-  {
-    DevStatus z{0, 0, ~0ull};
-    TRYC(cudaMemcpyAsync(p->status, &z, sizeof z, cudaMemcpyHostToDevice, s), "status");
+    if (m->elem_mat) {
+      int bad = 0;
+      TRYC(cudaMemcpyAsync(&bad, dbad, sizeof(int), cudaMemcpyDeviceToHost, s), "flag");
+      TRYC(cudaStreamSynchronize(s), "material properties");
+      if (bad) return fail(set_err(CXG_ERR_INVALID_ARGUMENT, "elem_mat index outside [0, n_materials)"));
+    }
   }
   const char* msg = nullptr;
   rc = build_pattern(m->elem_type, m->n_nodes, m->n_elems, p->conn, p->dof_eq, d->n_free, &p->pat, &msg, s);
@@ -608,10 +664,7 @@ int cxg_plan_destroy(cxg_plan* p) {
   if (p->last_stream) cudaStreamSynchronize(p->last_stream);
   thermal::release(p);
   cudaFree(p->film_mem);
-  void* bufs[] = {p->coords, p->conn, p->young, p->poisson, p->elem_mat, p->mats, p->dof_eq, p->prescribed,
-                  p->pat.row_ptr, p->pat.col_idx, p->pat.node, p->pat.node_mask, p->pat.pairs,
-                  p->pat.bnd_node, p->pat.bnd_col, p->pat.inc_ptr, p->pat.inc_code, p->state[0], p->state[1],
-                  p->status, p->edata, p->fdata};
+  void* bufs[] = {p->mem, p->pat.mem[0], p->pat.mem[1], p->state[0], p->state[1], p->edata, p->fdata};
   for (void* b : bufs) cudaFree(b);
   for (auto& row : p->sched)
     for (WinSched& w : row) cudaFree(w.node_order);
@@ -628,6 +681,8 @@ int cxg_plan_destroy(cxg_plan* p) {
                   static_cast<void*>(mp.kc_x)})
     cudaFree(b);
   for (void* b : p->stage) cudaFree(b);
+  cudaFree(p->work);
+  if (p->work_done) cudaEventDestroy(p->work_done);
   delete p;
   return CXG_OK;
 }
@@ -795,14 +850,12 @@ __global__ void add_into_kernel(int64_t n, double* a, const double* b) {
 // thermal_strain_load_vector of the plan into out[3N] (device)
 int load_device(cxg_plan* p, double* out, cudaStream_t s) {
   const int n = nodes_of(p->type);
-  double* felem = nullptr;
-  CHECK_CUDA(cudaMallocAsync(&felem, sizeof(double) * std::max<size_t>(static_cast<size_t>(p->n_elems) * 3 * n, 1), s),
-             "thermal load scratch");
+  WorkLease work(p, sizeof(double) * static_cast<size_t>(p->n_elems) * 3 * n, s);
+  CHECK_CUDA(work.error, "thermal load scratch");
   ElemArgs a = base_args(p);
   a.u = nullptr;
-  const cudaError_t err = launch_recover(p->type, a, p->pat.inc_ptr, p->pat.inc_code, nullptr, nullptr, felem, nullptr,
+  const cudaError_t err = launch_recover(p->type, a, p->pat.inc_ptr, p->pat.inc_code, nullptr, nullptr, work.ptr, nullptr,
                                          nullptr, nullptr, out, true, s);
-  cudaFreeAsync(felem, s);
   CHECK_CUDA(err, "thermal load kernels");
   return CXG_OK;
 }
@@ -1217,17 +1270,16 @@ int cxg_recover_fields(cxg_plan* p, const double* u, const double* f_ext, double
   if (!rc) rc = staged(p, 5, reaction, ub, false, s, &drf);
   if (rc) return rc;
   const int n = nodes_of(p->type);
-  double* scratch = nullptr;
   const int sets = p->type == C3D10 ? n : 1;  // value sets per element, see cxg_recover.cu
   const size_t scratch_doubles = static_cast<size_t>(p->n_elems) * (12 * sets + 3 * n);
-  CHECK_CUDA(cudaMallocAsync(&scratch, sizeof(double) * std::max<size_t>(scratch_doubles, 1), s), "recovery scratch");
+  WorkLease work(p, sizeof(double) * scratch_doubles, s);
+  CHECK_CUDA(work.error, "recovery scratch");
   ElemArgs a = base_args(p);
   a.u = static_cast<const double*>(du);
-  const cudaError_t err = launch_recover(p->type, a, p->pat.inc_ptr, p->pat.inc_code, nullptr, scratch,
-                                         scratch + 12 * static_cast<size_t>(sets) * static_cast<size_t>(p->n_elems),
+  const cudaError_t err = launch_recover(p->type, a, p->pat.inc_ptr, p->pat.inc_code, nullptr, work.ptr,
+                                         work.ptr + 12 * static_cast<size_t>(sets) * static_cast<size_t>(p->n_elems),
                                          static_cast<const double*>(df), static_cast<double*>(dst),
                                          static_cast<double*>(dss), static_cast<double*>(drf), false, s);
-  cudaFreeAsync(scratch, s);
   CHECK_CUDA(err, "recovery kernels");
   if ((rc = copy_out(strain, dst, sb, s))) return rc;
   if ((rc = copy_out(stress, dss, sb, s))) return rc;
@@ -1464,10 +1516,13 @@ int cxg_adjoint_compliance(cxg_plan* p, const double* u, double* dc_dE, double* 
   if (!rc) rc = staged(p, 1, dc_dE, eb, false, s, &dE);
   if (!rc) rc = staged(p, 4, dc_dX, ub, false, s, &dX);
   if (rc) return rc;
-  if (dX) CHECK_CUDA(cudaMemsetAsync(dX, 0, ub, s), "zero dc_dX");
+  WorkLease work(p, dX ? sizeof(double) * static_cast<size_t>(p->n_elems) * 3 * nodes_of(p->type) : 0, s);
+  CHECK_CUDA(work.error, "adjoint scratch");
   ElemArgs a = base_args(p);
   a.u = static_cast<const double*>(du);
-  CHECK_CUDA(launch_adjoint(p->type, a, static_cast<double*>(dE), static_cast<double*>(dX), s), "adjoint kernel");
+  const cudaError_t err = launch_adjoint(p->type, a, p->pat.inc_ptr, p->pat.inc_code, work.ptr, static_cast<double*>(dE),
+                                         static_cast<double*>(dX), s);
+  CHECK_CUDA(err, "adjoint kernels");
   if ((rc = copy_out(dc_dE, dE, eb, s))) return rc;
   if ((rc = copy_out(dc_dX, dX, ub, s))) return rc;
   if ((dc_dE && dE != dc_dE) || (dc_dX && dX != dc_dX)) CHECK_CUDA(cudaStreamSynchronize(s), "sync");

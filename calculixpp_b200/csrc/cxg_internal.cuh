@@ -70,7 +70,7 @@ struct __align__(16) NodeRec {
   uint16_t npair;
   uint16_t diag;     // the node's own position among its pairs
   uint16_t pair1, pair2;
-  uint32_t pad[3];
+  uint32_t pad[3];   // (the pattern builder's cuts while it works)
 };
 static_assert(sizeof(NodeRec) == 48, "NodeRec is three 16-byte loads");
 
@@ -291,8 +291,9 @@ struct FilmArgs {
 };
 cudaError_t launch_films(int elem_type, const ElemArgs& a, const FilmArgs& f, double* edata, double* f_ext,
                          cudaStream_t s);
-cudaError_t launch_adjoint(int elem_type, const ElemArgs& a, double* dc_dE, double* dc_dX,
-                           cudaStream_t s);
+// Compliance adjoint (cxg_recover.cu); felem[3nE]: scratch for dc_dX (null without it).
+cudaError_t launch_adjoint(int elem_type, const ElemArgs& a, const int64_t* inc_ptr, const int32_t* inc_code,
+                           double* felem, double* dc_dE, double* dc_dX, cudaStream_t s);
 cudaError_t launch_spmv(int32_t nrows, const int64_t* rp, const int32_t* ci, const double* v, const double* x,
                         double* y, cudaStream_t s);
 // Jacobi-preconditioned CG on CSR; work holds 5*n + 2056 doubles.
@@ -309,6 +310,7 @@ cudaError_t ensure_tables();
 
 // Pattern construction (cxg_pattern.cu).
 struct PatternOut {
+  void* mem[2] = {nullptr, nullptr};  // the device blocks that hold all of these
   int64_t nnz = 0;
   int64_t* row_ptr = nullptr;   // [n_free+1]
   int32_t* col_idx = nullptr;   // [nnz]

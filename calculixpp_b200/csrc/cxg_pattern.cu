@@ -2,26 +2,27 @@
 //
 // The reference accumulates (row, col) keys into an unordered_map element by element
 // (src/fem/assembly.cpp:76-100) and flushes unordered COO triplets (211-221). Here the
-// pattern is built once per mesh and DOF map, in canonical sorted CSR form:
-//   1. every element emits the n^2 node-pair keys a*N + b; a device radix sort and
-//      unique give the node adjacency graph, sorted by (a, b);
-//   2. each node a gets its free-component mask; all rows of a share one column
-//      structure (the free components of a's neighbours, ascending), so per node
-//      rowlen(a) = sum over neighbours of their free-component count and the offset
-//      of neighbour b inside a's rows is the running sum before b;
-//   3. node_base(a) = exclusive scan of (free rows of a) * rowlen(a); row_ptr and
-//      col_idx follow. This relies on the reference's free numbering being ascending
-//      in g = 3*node + comp (constraint_transform.cpp:78-82), which is validated;
-//   4. the sort carries with every key the element block it comes from, so the sorted
-//      values are, pair by pair and in element order, the blocks that the row gather sums;
-//      they are packed into the records it reads (NodeRec, PairRec); the nodes with a
-//      neighbour that is not fully free (their rows are compressed) also keep the
-//      neighbours and their columns (bnd_node, bnd_col).
+// pattern is built once per mesh and DOF map, in canonical sorted CSR form, node by node:
+//   1. the node -> element incidence comes from one stable sort of the connectivity;
+//   2. one warp per node gathers the nodes of its incident elements (its candidates, in
+//      element order), and orders them by (node, position) in shared memory, each
+//      candidate's place being the number of smaller ones: equal nodes are then one
+//      neighbour of the node and its contributions in element order;
+//   3. a first sweep counts: neighbours, the row length (all rows of a node share one
+//      column structure, the free components of its neighbours, ascending), the cuts of
+//      the contribution list; scans over the nodes give every node its place in the CSR
+//      arrays and in the record lists. This relies on the reference's free numbering being
+//      ascending in g = 3*node + comp (constraint_transform.cpp:78-82), which is validated;
+//   4. a second sweep orders the candidates again and writes row_ptr, col_idx, the
+//      records that the row gather reads (NodeRec, PairRec) and, for the nodes with a
+//      neighbour that is not fully free (their rows are compressed), the neighbours and
+//      their columns (bnd_node, bnd_col).
+// A global sort of all element node pairs would carry 24 bytes of scratch per pair through
+// six passes, and its allocations alone took longer than both sweeps together.
 // The pattern is topological: an entry whose every element contribution is exactly
 // zero is kept (the reference skips exact-zero contributions, assembly.cpp:90).
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
-#include <thrust/iterator/counting_iterator.h>
 
 #include <algorithm>
 #include <cstdio>
@@ -31,38 +32,26 @@
 namespace cxg {
 namespace {
 
-__global__ void check_conn_kernel(const int32_t* conn, int64_t total, int64_t n_nodes, int* flag,
-                                  unsigned long long* bad, int npe) {
+struct BuildFlags {
+  int bad_conn, bad_numbering, too_many, pad;
+  unsigned long long bad_elem;
+};
+
+__global__ void check_conn_kernel(const int32_t* conn, int64_t total, int64_t n_nodes, int npe, int32_t* codes,
+                                  BuildFlags* f) {
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int32_t v = conn[i];
+    codes[i] = static_cast<int32_t>(i);
     if (v < 0 || v >= n_nodes) {
-      atomicExch(flag, 1);
-      atomicMin(bad, static_cast<unsigned long long>(i / npe));
+      atomicExch(&f->bad_conn, 1);
+      atomicMin(&f->bad_elem, static_cast<unsigned long long>(i / npe));
     }
   }
 }
 
-__global__ void free_flags_kernel(const int32_t* dof_eq, int64_t ndof, int32_t* flags) {
-  for (int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; g < ndof;
-       g += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    flags[g] = dof_eq[g] >= 0 ? 1 : 0;
-}
-
-__global__ void check_numbering_kernel(const int32_t* dof_eq, const int32_t* scan, int64_t ndof,
-                                       int* flag) {
-  for (int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; g < ndof;
-       g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int32_t eq = dof_eq[g];
-    if (eq >= 0 && eq != scan[g]) atomicExch(flag, 1);
-    if (eq < -1) atomicExch(flag, 1);
-  }
-}
-
-// Free-component mask of every element node, so the row gather needs no connectivity
-// lookup before it knows which columns of a block exist.
-__global__ void node_info_kernel(const int32_t* dof_eq, int64_t n_nodes, uint8_t* mask,
-                                 int32_t* eq0) {
+// Free-component mask and first equation of every node, and the free count scanned below.
+__global__ void node_info_kernel(const int32_t* dof_eq, int64_t n_nodes, uint8_t* mask, int32_t* eq0, int32_t* free) {
   for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n_nodes;
        a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     int m = 0;
@@ -76,177 +65,22 @@ __global__ void node_info_kernel(const int32_t* dof_eq, int64_t n_nodes, uint8_t
     }
     mask[a] = static_cast<uint8_t>(m);
     eq0[a] = first;
+    free[a] = __popc(m);
   }
 }
 
-__global__ void pair_keys_kernel(const int32_t* conn, int64_t n_elems, int npe, uint64_t N,
-                                 uint64_t* keys, uint32_t* codes) {
-  const int64_t total = n_elems * npe * npe;
-  const int nbp = blocks_padded(npe);
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t e = i / (npe * npe);
-    const int r = static_cast<int>(i % (npe * npe));
-    const int a = r / npe, b = r % npe;
-    keys[i] = static_cast<uint64_t>(conn[e * npe + a]) * N + static_cast<uint64_t>(conn[e * npe + b]);
-    const int blk = a <= b ? blk_index(npe, a, b) : blk_index(npe, b, a);
-    codes[i] = static_cast<uint32_t>(e * nbp + blk);
-  }
-}
-
-__global__ void node_ptr_kernel(const uint64_t* uniq, int64_t M, int64_t n_nodes, uint64_t N,
-                                int64_t* node_ptr) {
-  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a <= n_nodes;
-       a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const uint64_t key = static_cast<uint64_t>(a) * N;
-    int64_t lo = 0, hi = M;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (uniq[mid] < key)
-        lo = mid + 1;
-      else
-        hi = mid;
-    }
-    node_ptr[a] = lo;
-  }
-}
-
-__global__ void rowlen_kernel(const uint64_t* uniq, const uint32_t* start, const int64_t* node_ptr, int64_t n_nodes,
-                              uint64_t N, const uint8_t* mask, int32_t* rowlen, int32_t* adj_off, int64_t* node_nnz,
-                              int64_t* bnd_len, int64_t* n_rec, NodeRec* node, int* overflow) {
+__global__ void check_numbering_kernel(const int32_t* dof_eq, const int32_t* scan, const uint8_t* mask, int64_t n_nodes,
+                                       int32_t n_free, BuildFlags* f) {
   for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n_nodes;
        a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t t0 = node_ptr[a], t1 = node_ptr[a + 1], k = t1 - t0;
-    NodeRec r{};
-    int32_t run = 0;
-    int64_t cut[2] = {t1, t1};
-    const uint64_t c0 = k > 0 ? start[t0] : 0, span = k > 0 ? start[t1] - c0 : 0;
-    for (int64_t t = t0; t < t1; ++t) {
-      const int64_t b = static_cast<int64_t>(uniq[t] % N);
-      if (b == a) r.diag = static_cast<uint16_t>(t - t0);
-      adj_off[t] = run;
-      run += __popc(mask[b]);
-      // the cuts: the pair starts nearest to one and two thirds of the contributions
-      for (int g = 0; g < 2; ++g) {
-        const int64_t to = static_cast<int64_t>((g + 1) * span), s0 = 3 * static_cast<int64_t>(start[t] - c0),
-                      s1 = 3 * static_cast<int64_t>(start[t + 1] - c0);
-        if (cut[g] == t1 && s1 > to) cut[g] = to - s0 <= s1 - to ? t : t + 1;
-      }
+    int32_t next = scan[a];
+    for (int d = 0; d < 3; ++d) {
+      const int32_t eq = dof_eq[3 * a + d];
+      if (eq < -1 || (eq >= 0 && eq != next)) atomicExch(&f->bad_numbering, 1);
+      next += eq >= 0;
     }
-    uint32_t longest = 0;
-    const int64_t at[4] = {t0, cut[0], cut[1], t1};
-    for (int g = 0; g < 3; ++g) longest = max(longest, k > 0 ? start[at[g + 1]] - start[at[g]] : 0u);
-    r.rounds = (longest + kPairRec - 1) / kPairRec;
-    r.npair = static_cast<uint16_t>(k);
-    r.pair1 = static_cast<uint16_t>(cut[0] - t0);
-    r.pair2 = static_cast<uint16_t>(cut[1] - t0);
-    rowlen[a] = run;
-    node_nnz[a] = static_cast<int64_t>(__popc(mask[a])) * run;
-    if (k > 65535) atomicExch(overflow, 1);  // list positions are uint16
-    bnd_len[a] = run == 3 * k ? 0 : k;
-    n_rec[a] = 3 * static_cast<int64_t>(r.rounds);
-    node[a] = r;
+    if (a == n_nodes - 1 && next != n_free) atomicExch(&f->bad_numbering, 1);
   }
-}
-
-// The contribution records of every node, one warp per node, a lane per record. A
-// contribution is the last of its pair when the next one starts another.
-__global__ void pair_rec_kernel(const NodeRec* node, const uint32_t* start, const int64_t* node_ptr,
-                                const uint32_t* codes, const uint64_t* keys, int64_t total, int64_t n_nodes,
-                                PairRec* pairs) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nw = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t a = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; a < n_nodes; a += nw) {
-    const NodeRec nd = node[a];
-    const int64_t t0 = node_ptr[a], t1 = node_ptr[a + 1];
-    for (uint32_t i = lane; i < 3 * nd.rounds; i += 32) {
-      const int g = i % 3;
-      const uint32_t lo = start[g == 0 ? t0 : t0 + (g == 1 ? nd.pair1 : nd.pair2)];
-      const uint32_t hi = start[g == 2 ? t1 : t0 + (g == 0 ? nd.pair1 : nd.pair2)];
-      PairRec r;
-      // the round of the own pair's predecessor, in whichever run that is
-      const uint32_t own = start[t0 + nd.diag];
-      const int64_t cut[4] = {t0, t0 + nd.pair1, t0 + nd.pair2, t1};
-      bool turn = false;
-      for (int h = 0; h < 3; ++h)
-        turn = turn || (own > start[cut[h]] && own < start[cut[h + 1]] &&
-                        (own - 1 - start[cut[h]]) / kPairRec == i / 3);
-      r.flags = turn ? 0x80000000u : 0u;
-      for (int j = 0; j < kPairRec; ++j) {
-        const uint32_t c = lo + i / 3 * kPairRec + j;
-        if (c < hi) {
-          r.block[j] = codes[c];
-          if (c + 1 == total || keys[c] != keys[c + 1]) r.flags |= 1u << j;
-          if (c + 1 == own && c + 1 < hi) r.flags |= 0x10000u << j;
-          // (a run that begins with the own pair has no such entry)
-        } else {
-          r.block[j] = codes[hi > lo ? hi - 1 : start[t0]];
-        }
-      }
-      pairs[nd.list0 + i] = r;
-    }
-  }
-}
-
-__global__ void row_ptr_kernel(int64_t n_nodes, const uint8_t* mask, const int32_t* eq0,
-                               const int64_t* node_base, const int32_t* rowlen, int64_t* row_ptr) {
-  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n_nodes;
-       a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int nf = __popc(mask[a]);
-    for (int r = 0; r < nf; ++r) row_ptr[eq0[a] + r] = node_base[a] + static_cast<int64_t>(r) * rowlen[a];
-  }
-}
-
-__global__ void col_idx_kernel(const uint64_t* uniq, int64_t M, uint64_t N, const uint8_t* mask,
-                               const int32_t* eq0, const int64_t* node_base, const int32_t* rowlen,
-                               const int32_t* adj_off, int32_t* col_idx) {
-  for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < M;
-       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t a = static_cast<int64_t>(uniq[t] / N), b = static_cast<int64_t>(uniq[t] % N);
-    const int nfa = __popc(mask[a]);
-    const int nfb = __popc(mask[b]);
-    for (int r = 0; r < nfa; ++r) {
-      const int64_t pos = node_base[a] + static_cast<int64_t>(r) * rowlen[a] + adj_off[t];
-      for (int j = 0; j < nfb; ++j) col_idx[pos + j] = eq0[b] + j;
-    }
-  }
-}
-
-// the rest of the node records
-__global__ void node_rec_kernel(const int64_t* node_base, const int32_t* rowlen,
-                                const int32_t* eq0, const uint8_t* mask, const int64_t* bnd_ptr,
-                                const int64_t* rec_ptr, int64_t n_nodes, NodeRec* node) {
-  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n_nodes;
-       a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    NodeRec r = node[a];
-    r.base = node_base[a];
-    r.len_mask = static_cast<uint32_t>(rowlen[a]) | static_cast<uint32_t>(mask[a]) << 28;
-    r.eq0 = eq0[a];
-    r.bnd0 = static_cast<uint32_t>(bnd_ptr[a]);
-    r.list0 = static_cast<uint32_t>(rec_ptr[a]);
-    node[a] = r;
-  }
-}
-
-// neighbours and compressed columns of the compressed-row nodes, in list order
-__global__ void bnd_node_kernel(const uint64_t* uniq, int64_t M, uint64_t N, const int64_t* node_ptr,
-                                const int64_t* bnd_ptr, const int64_t* bnd_len, const int32_t* adj_off,
-                                const uint8_t* mask, int32_t* bnd_node, int32_t* bnd_col) {
-  for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < M;
-       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t a = static_cast<int64_t>(uniq[t] / N), b = static_cast<int64_t>(uniq[t] % N);
-    if (bnd_len[a] > 0) {
-      const int64_t o = bnd_ptr[a] + (t - node_ptr[a]);
-      bnd_node[o] = static_cast<int32_t>(b);
-      bnd_col[o] = adj_off[t] | static_cast<int32_t>(mask[b]) << 28;
-    }
-  }
-}
-
-__global__ void iota_kernel(int32_t* v, int64_t n) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    v[i] = static_cast<int32_t>(i);
 }
 
 __global__ void inc_ptr_kernel(const int32_t* sorted_nodes, int64_t m, int64_t n_nodes, int64_t* ptr) {
@@ -264,14 +98,229 @@ __global__ void inc_ptr_kernel(const int32_t* sorted_nodes, int64_t m, int64_t n
   }
 }
 
+__global__ void max_inc_kernel(const int64_t* inc_ptr, int64_t n_nodes, int* out) {
+  int m = 0;
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n_nodes;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    m = max(m, static_cast<int>(inc_ptr[a + 1] - inc_ptr[a]));
+  m = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(m));
+  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(out, m);
+}
+
+constexpr int kWarps = 4;
+
+// What both sweeps know of a node: its candidates in order (ord[r]: candidate position,
+// nb[r]: its node), in this warp's part of `store` (2 * cap values, shared or global).
+// Candidate c is local node c % n of the c / n-th incident element.
+struct Sweep {
+  const int32_t* conn;
+  const int64_t* inc_ptr;
+  const int32_t* inc_code;
+  int npe, nbp;
+};
+
+// Orders the candidates of node a; returns their number. raw: scratch for their nodes.
+__device__ int order_candidates(const Sweep& S, int64_t a, int32_t* raw, int32_t* nb, int32_t* ord) {
+  const int lane = threadIdx.x & 31;
+  const int64_t i0 = S.inc_ptr[a];
+  const int n = S.npe, cnt = static_cast<int>(S.inc_ptr[a + 1] - i0) * n;
+  for (int c = lane; c < cnt; c += 32) raw[c] = S.conn[static_cast<int64_t>(S.inc_code[i0 + c / n] / n) * n + c % n];
+  __syncwarp();
+  for (int c0 = 0; c0 < cnt; c0 += 32) {
+    const int c = c0 + lane;
+    const int32_t v = c < cnt ? raw[c] : 0;
+    int rank = 0;
+    for (int t = 0; t < cnt; ++t) {
+      const int32_t w = raw[t];
+      rank += w < v || (w == v && t < c);
+    }
+    if (c < cnt) {
+      nb[rank] = v;
+      ord[rank] = c;
+    }
+  }
+  __syncwarp();
+  return cnt;
+}
+
+// Neighbours before and contribution runs: calls at(r, p, first) for every candidate rank
+// r on its lane, p its neighbour's position and first whether it opens that neighbour.
+template <class F>
+__device__ void each_candidate(const int32_t* nb, int cnt, F at) {
+  const int lane = threadIdx.x & 31;
+  int before = 0;
+  for (int r0 = 0; r0 < cnt; r0 += 32) {
+    const int r = r0 + lane;
+    const bool first = r < cnt && (r == 0 || nb[r] != nb[r - 1]);
+    const unsigned w = __ballot_sync(0xffffffffu, first);
+    const int p = before + __popc(w & ((2u << lane) - 1)) - 1;
+    at(r, p, first);
+    before += __popc(w);
+  }
+}
+
+// First sweep: counts, row length, cuts.
+__global__ void __launch_bounds__(kWarps * 32) count_kernel(Sweep S, int64_t n_nodes, const uint8_t* mask, int cap,
+                                                            int32_t* big, NodeRec* node, int64_t* node_nnz,
+                                                            int64_t* bnd_len, int64_t* n_rec, BuildFlags* f) {
+  extern __shared__ int32_t sh[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t gw = static_cast<int64_t>(blockIdx.x) * kWarps + warp, nw = static_cast<int64_t>(gridDim.x) * kWarps;
+  int32_t* raw = big ? big + gw * 3 * cap : sh + warp * 3 * cap;
+  int32_t *nb = raw + cap, *ord = nb + cap;
+  for (int64_t a = gw; a < n_nodes; a += nw) {
+    const int cnt = order_candidates(S, a, raw, nb, ord);
+    int len = 0, K = 0, self = 0;
+    // the neighbour starts nearest to one and two thirds of the contributions
+    int cut[2] = {cnt, cnt}, pos[2] = {0, 0}, err[2] = {3 * cnt + 1, 3 * cnt + 1};
+    each_candidate(nb, cnt, [&](int r, int p, bool first) {
+      if (r >= cnt) return;
+      if (first) {
+        len += __popc(mask[nb[r]]);
+        if (nb[r] == a) self = p;
+        for (int g = 0; g < 2; ++g) {
+          const int d = abs(3 * r - (g + 1) * cnt);
+          if (d < err[g]) {
+            err[g] = d;
+            cut[g] = r;
+            pos[g] = p;
+          }
+        }
+      }
+      K = max(K, p + 1);
+    });
+    len = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(len));
+    K = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(K));
+    self = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(self));
+    for (int g = 0; g < 2; ++g) {
+      // (the end of the list is a cut too, for nodes with one or two neighbours)
+      const unsigned e = __reduce_min_sync(0xffffffffu, static_cast<unsigned>(err[g]));
+      const unsigned win = __ballot_sync(0xffffffffu, static_cast<unsigned>(err[g]) == e && cut[g] < cnt);
+      const int src = win ? __ffs(win) - 1 : 0;
+      const bool end = static_cast<unsigned>(3 * cnt - (g + 1) * cnt) < e || !win;
+      const int c = __shfl_sync(0xffffffffu, cut[g], src), q = __shfl_sync(0xffffffffu, pos[g], src);
+      cut[g] = end ? cnt : c;
+      pos[g] = end ? K : q;
+    }
+    if (lane == 0) {
+      const int longest = max(cut[0], max(cut[1] - cut[0], cnt - cut[1]));
+      NodeRec r{};
+      r.len_mask = static_cast<uint32_t>(len);
+      r.rounds = static_cast<uint32_t>((longest + kPairRec - 1) / kPairRec);
+      r.npair = static_cast<uint16_t>(K);
+      r.diag = static_cast<uint16_t>(self);
+      r.pair1 = static_cast<uint16_t>(pos[0]);
+      r.pair2 = static_cast<uint16_t>(pos[1]);
+      r.pad[0] = static_cast<uint32_t>(cut[0]);
+      r.pad[1] = static_cast<uint32_t>(cut[1]);
+      if (K > 65535) atomicExch(&f->too_many, 1);  // list positions are uint16
+      node[a] = r;
+      node_nnz[a] = static_cast<int64_t>(__popc(mask[a])) * len;
+      bnd_len[a] = len == 3 * K ? 0 : K;
+      n_rec[a] = 3 * static_cast<int64_t>(r.rounds);
+    }
+    __syncwarp();
+  }
+}
+
+// Second sweep: the CSR rows, the records and the lists of the compressed-row nodes.
+__global__ void __launch_bounds__(kWarps * 32) write_kernel(Sweep S, int64_t n_nodes, const uint8_t* mask,
+                                                            const int32_t* eq0, const int64_t* node_base,
+                                                            const int64_t* bnd_ptr, const int64_t* rec_ptr, int cap,
+                                                            int32_t* big, NodeRec* node, int64_t* row_ptr,
+                                                            int32_t* col_idx, PairRec* pairs, int32_t* bnd_node,
+                                                            int32_t* bnd_col) {
+  extern __shared__ int32_t sh[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t gw = static_cast<int64_t>(blockIdx.x) * kWarps + warp, nw = static_cast<int64_t>(gridDim.x) * kWarps;
+  int32_t* raw = big ? big + gw * 3 * cap : sh + warp * 3 * cap;
+  int32_t *nb = raw + cap, *ord = nb + cap;
+  for (int64_t a = gw; a < n_nodes; a += nw) {
+    const int cnt = order_candidates(S, a, raw, nb, ord);
+    NodeRec nd = node[a];
+    const int cut1 = static_cast<int>(nd.pad[0]), cut2 = static_cast<int>(nd.pad[1]);
+    const int L = static_cast<int>(nd.len_mask), ma = mask[a], nfa = __popc(ma), K = nd.npair;
+    nd.base = node_base[a];
+    nd.list0 = static_cast<uint32_t>(rec_ptr[a]);
+    nd.bnd0 = static_cast<uint32_t>(bnd_ptr[a]);
+    nd.eq0 = eq0[a];
+    nd.len_mask = static_cast<uint32_t>(L) | static_cast<uint32_t>(ma) << 28;
+    nd.pad[0] = nd.pad[1] = 0;
+    __syncwarp();
+    if (lane == 0) node[a] = nd;
+    if (lane < nfa) row_ptr[nd.eq0 + lane] = nd.base + static_cast<int64_t>(lane) * L;
+    // columns: the free components of the neighbours in order
+    int run = 0, own = -1;  // free components of the neighbours before this chunk; rank of the own pair
+    each_candidate(nb, cnt, [&](int r, int p, bool first) {
+      const int b = first ? nb[r] : 0;
+      const int mb = first ? mask[b] : 0, pc = __popc(mb);
+      int incl = pc;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += y;
+      }
+      const int col = run + incl - pc;
+      run += __shfl_sync(0xffffffffu, incl, 31);
+      if (!first) return;
+      if (b == a) own = r;
+      const int32_t e = eq0[b];
+      for (int i = 0; i < nfa; ++i)
+        for (int j = 0; j < pc; ++j) col_idx[nd.base + static_cast<int64_t>(i) * L + col + j] = e + j;
+      if (L != 3 * K) {
+        bnd_node[nd.bnd0 + p] = b;
+        bnd_col[nd.bnd0 + p] = col | mb << 28;
+      }
+    });
+    own = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(own + 1)) - 1;
+    // records: run g holds ranks [lo, hi), record r of it 11 of them
+    const int from[4] = {0, cut1, cut2, cnt};
+    int turn = -1;  // round in which the pair before the own one ends (not at a run's start)
+    for (int g = 0; g < 3; ++g)
+      if (own > from[g] && own < from[g + 1]) turn = (own - 1 - from[g]) / kPairRec;
+    const int64_t i0 = S.inc_ptr[a];
+    const int n = S.npe;
+    auto block = [&](int r) {
+      const int c = ord[r], code = S.inc_code[i0 + c / n], la = code % n, lb = c % n;
+      return static_cast<uint32_t>((code / n) * S.nbp + (la <= lb ? blk_index(n, la, lb) : blk_index(n, lb, la)));
+    };
+    for (int i = lane; i < 3 * static_cast<int>(nd.rounds); i += 32) {
+      const int g = i % 3, lo = g == 0 ? 0 : g == 1 ? cut1 : cut2, hi = g == 0 ? cut1 : g == 1 ? cut2 : cnt;
+      PairRec rec;
+      rec.flags = i / 3 == turn ? 0x80000000u : 0u;
+      for (int j = 0; j < kPairRec; ++j) {
+        const int r = lo + i / 3 * kPairRec + j;
+        if (r < hi) {
+          rec.block[j] = block(r);
+          if (r + 1 == cnt || nb[r] != nb[r + 1]) rec.flags |= 1u << j;
+          if (r + 1 == own && r + 1 < hi) rec.flags |= 0x10000u << j;
+        } else {
+          rec.block[j] = block(hi > lo ? hi - 1 : 0);
+        }
+      }
+      pairs[nd.list0 + i] = rec;
+    }
+    __syncwarp();
+  }
+}
+
 unsigned grid_for(int64_t n, int threads = 256) {
   return static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((n + threads - 1) / threads, 65536)));
 }
 
+// Parts of one device block, each 256-byte aligned.
+struct Parts {
+  size_t bytes = 0;
+  template <typename T>
+  size_t add(size_t count) {
+    const size_t at = bytes;
+    bytes += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+    return at;
+  }
+};
 template <typename T>
-cudaError_t dalloc(T** p, size_t count, int64_t* bytes) {
-  *bytes += static_cast<int64_t>(count * sizeof(T));
-  return cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T));
+T* part(void* base, size_t at) {
+  return reinterpret_cast<T*>(static_cast<char*>(base) + at);
 }
 
 }  // namespace
@@ -290,40 +339,8 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
                   const int32_t* d_dof_eq, int32_t n_free, PatternOut* out, const char** msg,
                   cudaStream_t s) {
   const int npe = nodes_of(elem_type);
-  const uint64_t N = static_cast<uint64_t>(n_nodes);
-  const int64_t ndof = 3 * n_nodes;
-  const int64_t P = n_elems * npe * npe;
+  const int64_t P = n_elems * npe * npe, m = n_elems * npe;
   int rc = 0;
-  int64_t scratch = 0;
-  int* d_flag = nullptr;
-  unsigned long long* d_bad = nullptr;
-  int32_t* d_flags = nullptr;
-  int32_t* d_scan = nullptr;
-  uint64_t* d_keys = nullptr;
-  uint64_t* d_keys2 = nullptr;
-  void* d_temp = nullptr;
-  size_t temp_bytes = 0;
-  int64_t* d_M = nullptr;
-  int64_t* d_node_ptr = nullptr;
-  int32_t* d_adj_off = nullptr;
-  int64_t* d_node_nnz = nullptr;
-  int64_t* d_node_base = nullptr;
-  int64_t* d_bnd_len = nullptr;
-  int64_t* d_bnd_ptr = nullptr;
-  int32_t* d_rowlen = nullptr;
-  int32_t* d_eq0 = nullptr;
-  uint32_t* d_codes = nullptr;
-  uint32_t* d_codes2 = nullptr;
-  uint32_t* d_start = nullptr;
-  int64_t* d_n_rec = nullptr;
-  int64_t* d_rec_ptr = nullptr;
-  uint64_t* sorted = nullptr;
-  int h_flag = 0;
-  int64_t M = 0;
-  uint64_t* uniq = nullptr;
-  unsigned long long h_bad = 0;
-  int end_bit = 1;
-
   if (P >= (static_cast<int64_t>(1) << 31)) {
     *msg = "mesh too large for one plan (n_elems * nodes^2 >= 2^31); split it into partitions";
     return 5;
@@ -332,209 +349,147 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
     *msg = "node count exceeds int32 indexing";
     return 5;
   }
-  while (end_bit < 64 && (N * N) >> end_bit) ++end_bit;
+  const int in = static_cast<int>(n_nodes), im = static_cast<int>(m);
+  int node_bits = 1;
+  while (node_bits < 31 && (n_nodes >> node_bits) != 0) ++node_bits;
 
-  CXG_TRY(cudaMalloc(&d_flag, sizeof(int)));
-  CXG_TRY(cudaMalloc(&d_bad, sizeof(unsigned long long)));
-  CXG_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), s));
-  CXG_TRY(cudaMemsetAsync(d_bad, 0xff, sizeof(unsigned long long), s));
-
-  // connectivity range check
-  check_conn_kernel<<<grid_for(n_elems * npe), 256, 0, s>>>(d_conn, n_elems * npe, n_nodes, d_flag, d_bad, npe);
-  CXG_TRY(cudaGetLastError());
-  CXG_TRY(cudaMemcpyAsync(&h_flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-  CXG_TRY(cudaMemcpyAsync(&h_bad, d_bad, sizeof(h_bad), cudaMemcpyDeviceToHost, s));
-  CXG_TRY(cudaStreamSynchronize(s));
-  if (h_flag) {
-    static thread_local char buf[160];
-    snprintf(buf, sizeof buf, "element references unknown node (element index %llu)", h_bad);
-    *msg = buf;
-    rc = 6;
-    goto done;
+  // What stays with the plan and has a known size, and the build's scratch: one block each.
+  void* scratch = nullptr;
+  void* big = nullptr;
+  Parts keep, tmp;
+  const size_t k_mask = keep.add<uint8_t>(n_nodes), k_node = keep.add<NodeRec>(n_nodes),
+               k_row = keep.add<int64_t>(static_cast<size_t>(n_free) + 1), k_inc = keep.add<int64_t>(n_nodes + 1),
+               k_code = keep.add<int32_t>(m);
+  size_t sort_bytes = 0, scan32 = 0, scan64 = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, static_cast<const int32_t*>(nullptr),
+                                  static_cast<int32_t*>(nullptr), static_cast<const int32_t*>(nullptr),
+                                  static_cast<int32_t*>(nullptr), im, 0, node_bits, s);
+  cub::DeviceScan::ExclusiveSum(nullptr, scan32, static_cast<int32_t*>(nullptr), static_cast<int32_t*>(nullptr), in, s);
+  cub::DeviceScan::ExclusiveSum(nullptr, scan64, static_cast<int64_t*>(nullptr), static_cast<int64_t*>(nullptr), in, s);
+  const size_t cub_bytes = std::max(sort_bytes, std::max(scan32, scan64));
+  const size_t t_flags = tmp.add<BuildFlags>(1), t_max = tmp.add<int>(1), t_cub = tmp.add<char>(cub_bytes),
+               t_eq0 = tmp.add<int32_t>(n_nodes), t_free = tmp.add<int32_t>(n_nodes), t_scan = tmp.add<int32_t>(n_nodes),
+               t_sorted = tmp.add<int32_t>(m), t_codes = tmp.add<int32_t>(m);
+  size_t t_len[3], t_off[3];  // node_nnz, bnd_len, n_rec and their scans
+  for (int i = 0; i < 3; ++i) {
+    t_len[i] = tmp.add<int64_t>(n_nodes);
+    t_off[i] = tmp.add<int64_t>(n_nodes);
   }
-
-  // free numbering must be ascending in g (SPC-only constraint transform)
-  CXG_TRY(cudaMalloc(&d_flags, sizeof(int32_t) * std::max<int64_t>(ndof, 1)));
-  CXG_TRY(cudaMalloc(&d_scan, sizeof(int32_t) * std::max<int64_t>(ndof, 1)));
-  free_flags_kernel<<<grid_for(ndof), 256, 0, s>>>(d_dof_eq, ndof, d_flags);
-  CXG_TRY(cudaGetLastError());
-  CXG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, d_flags, d_scan, static_cast<int>(ndof), s));
-  CXG_TRY(cudaMalloc(&d_temp, temp_bytes));
-  CXG_TRY(cub::DeviceScan::ExclusiveSum(d_temp, temp_bytes, d_flags, d_scan, static_cast<int>(ndof), s));
-  check_numbering_kernel<<<grid_for(ndof), 256, 0, s>>>(d_dof_eq, d_scan, ndof, d_flag);
-  CXG_TRY(cudaGetLastError());
+  BuildFlags hf{};
+  int max_inc = 0, cap = 0;
+  int64_t last[3] = {0, 0, 0}, len[3] = {0, 0, 0};
+  Sweep S{};
+  unsigned sweep_grid = 0;
+  size_t sweep_smem = 0;
   {
-    int32_t last_scan = 0, last_flag = 0;
-    if (ndof > 0) {
-      CXG_TRY(cudaMemcpyAsync(&last_scan, d_scan + ndof - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-      CXG_TRY(cudaMemcpyAsync(&last_flag, d_flags + ndof - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    }
-    CXG_TRY(cudaMemcpyAsync(&h_flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CXG_TRY(cudaMalloc(&out->mem[0], keep.bytes));
+    out->device_bytes += static_cast<int64_t>(keep.bytes);
+    CXG_TRY(cudaMalloc(&scratch, tmp.bytes));
+    out->node_mask = part<uint8_t>(out->mem[0], k_mask);
+    out->node = part<NodeRec>(out->mem[0], k_node);
+    out->row_ptr = part<int64_t>(out->mem[0], k_row);
+    out->inc_ptr = part<int64_t>(out->mem[0], k_inc);
+    out->inc_code = part<int32_t>(out->mem[0], k_code);
+    BuildFlags* f = part<BuildFlags>(scratch, t_flags);
+    int* d_max = part<int>(scratch, t_max);
+    hf.bad_elem = ~0ull;
+    CXG_TRY(cudaMemcpyAsync(f, &hf, sizeof hf, cudaMemcpyHostToDevice, s));
+    CXG_TRY(cudaMemsetAsync(d_max, 0, sizeof(int), s));
+    int32_t* eq0 = part<int32_t>(scratch, t_eq0);
+    int32_t* codes = part<int32_t>(scratch, t_codes);
+    int32_t* sorted = part<int32_t>(scratch, t_sorted);
+    check_conn_kernel<<<grid_for(m), 256, 0, s>>>(d_conn, m, n_nodes, npe, codes, f);
+    node_info_kernel<<<grid_for(n_nodes), 256, 0, s>>>(d_dof_eq, n_nodes, out->node_mask, eq0,
+                                                       part<int32_t>(scratch, t_free));
+    CXG_TRY(cudaGetLastError());
+    size_t cb = cub_bytes;
+    CXG_TRY(cub::DeviceScan::ExclusiveSum(part<char>(scratch, t_cub), cb, part<int32_t>(scratch, t_free),
+                                          part<int32_t>(scratch, t_scan), in, s));
+    check_numbering_kernel<<<grid_for(n_nodes), 256, 0, s>>>(d_dof_eq, part<int32_t>(scratch, t_scan), out->node_mask,
+                                                             n_nodes, n_free, f);
+    // node -> element incidence: stable sort of (node, e*n + local) by node. Nodes outside
+    // the mesh (an error, reported below) sort by their low bits and are not followed.
+    CXG_TRY(cub::DeviceRadixSort::SortPairs(part<char>(scratch, t_cub), cb, d_conn, sorted, codes, out->inc_code, im, 0,
+                                            node_bits, s));
+    CXG_TRY(cudaMemcpyAsync(&hf, f, sizeof hf, cudaMemcpyDeviceToHost, s));
+    inc_ptr_kernel<<<grid_for(n_nodes + 1), 256, 0, s>>>(sorted, m, n_nodes, out->inc_ptr);
+    max_inc_kernel<<<grid_for(n_nodes), 256, 0, s>>>(out->inc_ptr, n_nodes, d_max);
+    CXG_TRY(cudaGetLastError());
+    CXG_TRY(cudaMemcpyAsync(&max_inc, d_max, sizeof(int), cudaMemcpyDeviceToHost, s));
     CXG_TRY(cudaStreamSynchronize(s));
-    if (h_flag || last_scan + last_flag != n_free) {
+    if (hf.bad_conn) {
+      static thread_local char buf[160];
+      snprintf(buf, sizeof buf, "element references unknown node (element index %llu)", hf.bad_elem);
+      *msg = buf;
+      rc = 6;
+      goto done;
+    }
+    if (hf.bad_numbering) {
       *msg = "dof_eq must number the free DOFs 0..n_free-1 in increasing global DOF order "
              "(SPC-only constraint transform)";
       rc = 5;
       goto done;
     }
-  }
-  cudaFree(d_temp);
-  d_temp = nullptr;
-  cudaFree(d_flags);
-  d_flags = nullptr;
-  cudaFree(d_scan);
-  d_scan = nullptr;
-
-  CXG_TRY(dalloc(&out->node_mask, n_nodes, &out->device_bytes));
-  CXG_TRY(dalloc(&out->node, n_nodes, &out->device_bytes));
-  CXG_TRY(dalloc(&d_eq0, n_nodes, &scratch));
-  CXG_TRY(dalloc(&d_rowlen, n_nodes, &scratch));
-  CXG_TRY(dalloc(&d_node_base, n_nodes, &scratch));
-  node_info_kernel<<<grid_for(n_nodes), 256, 0, s>>>(d_dof_eq, n_nodes, out->node_mask, d_eq0);
-  CXG_TRY(cudaGetLastError());
-
-  // node adjacency and its element blocks: stable sort of (node-pair key, block code),
-  // then one key and its first position per pair
-  CXG_TRY(dalloc(&d_keys, P, &scratch));
-  CXG_TRY(dalloc(&d_keys2, P, &scratch));
-  CXG_TRY(dalloc(&d_codes, P + 1, &scratch));
-  CXG_TRY(dalloc(&d_codes2, P + 1, &scratch));
-  pair_keys_kernel<<<grid_for(P), 256, 0, s>>>(d_conn, n_elems, npe, N, d_keys, d_codes);
-  CXG_TRY(cudaGetLastError());
-  {
-    cub::DoubleBuffer<uint64_t> db(d_keys, d_keys2);
-    cub::DoubleBuffer<uint32_t> dc(d_codes, d_codes2);
-    temp_bytes = 0;
-    CXG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, db, dc, static_cast<int>(P), 0, end_bit, s));
-    CXG_TRY(cudaMalloc(&d_temp, temp_bytes));
-    CXG_TRY(cub::DeviceRadixSort::SortPairs(d_temp, temp_bytes, db, dc, static_cast<int>(P), 0, end_bit, s));
+    // The sweeps' candidate lists: shared memory up to 2048 per warp (96 KB a block), one
+    // slice of global memory per warp beyond.
+    cap = std::max(1, max_inc * npe);
+    sweep_smem = sizeof(int32_t) * kWarps * 3 * static_cast<size_t>(cap);
+    sweep_grid = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((n_nodes + kWarps - 1) / kWarps, 65536)));
+    if (cap > 2048) {
+      sweep_grid = std::min(sweep_grid, 256u);
+      sweep_smem = 0;
+      CXG_TRY(cudaMalloc(&big, sizeof(int32_t) * 3 * static_cast<size_t>(cap) * kWarps * sweep_grid));
+    } else {
+      CXG_TRY(cudaFuncSetAttribute(count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sweep_smem)));
+      CXG_TRY(cudaFuncSetAttribute(write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sweep_smem)));
+    }
+    S = Sweep{d_conn, out->inc_ptr, out->inc_code, npe, blocks_padded(npe)};
+    int64_t *lens[3], *offs[3];
+    for (int i = 0; i < 3; ++i) {
+      lens[i] = part<int64_t>(scratch, t_len[i]);
+      offs[i] = part<int64_t>(scratch, t_off[i]);
+    }
+    count_kernel<<<sweep_grid, kWarps * 32, sweep_smem, s>>>(S, n_nodes, out->node_mask, cap, static_cast<int32_t*>(big),
+                                                             out->node, lens[0], lens[1], lens[2], f);
+    CXG_TRY(cudaGetLastError());
+    for (int i = 0; i < 3; ++i) {
+      cb = cub_bytes;
+      CXG_TRY(cub::DeviceScan::ExclusiveSum(part<char>(scratch, t_cub), cb, lens[i], offs[i], in, s));
+      if (n_nodes > 0) {
+        CXG_TRY(cudaMemcpyAsync(&last[i], offs[i] + n_nodes - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        CXG_TRY(cudaMemcpyAsync(&len[i], lens[i] + n_nodes - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+      }
+    }
+    CXG_TRY(cudaMemcpyAsync(&hf, f, sizeof hf, cudaMemcpyDeviceToHost, s));
     CXG_TRY(cudaStreamSynchronize(s));
-    cudaFree(d_temp);
-    d_temp = nullptr;
-    d_codes = dc.Current();
-    d_codes2 = dc.Alternate();
-    d_start = d_codes2;
-    sorted = db.Current();
-    uint64_t* other = db.Alternate();
-    CXG_TRY(cudaMalloc(&d_M, sizeof(int64_t)));
-    CXG_TRY(cudaMemsetAsync(d_M, 0, sizeof(int64_t), s));
-    const thrust::counting_iterator<uint32_t> at(0u);
-    temp_bytes = 0;
-    CXG_TRY(cub::DeviceSelect::UniqueByKey(nullptr, temp_bytes, sorted, at, other, d_start, d_M, static_cast<int>(P), s));
-    CXG_TRY(cudaMalloc(&d_temp, temp_bytes));
-    CXG_TRY(cub::DeviceSelect::UniqueByKey(d_temp, temp_bytes, sorted, at, other, d_start, d_M, static_cast<int>(P), s));
-    CXG_TRY(cudaMemcpyAsync(&M, d_M, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    CXG_TRY(cudaStreamSynchronize(s));
-    cudaFree(d_temp);
-    d_temp = nullptr;
-    uniq = other;
-    const uint32_t total = static_cast<uint32_t>(P);
-    CXG_TRY(cudaMemcpyAsync(d_start + M, &total, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  }
-
-  CXG_TRY(dalloc(&d_node_ptr, n_nodes + 1, &scratch));
-  CXG_TRY(dalloc(&d_adj_off, M, &scratch));
-  CXG_TRY(dalloc(&d_node_nnz, n_nodes, &scratch));
-  CXG_TRY(dalloc(&d_bnd_len, n_nodes, &scratch));
-  CXG_TRY(dalloc(&d_bnd_ptr, n_nodes, &scratch));
-  CXG_TRY(dalloc(&d_n_rec, n_nodes, &scratch));
-  CXG_TRY(dalloc(&d_rec_ptr, n_nodes, &scratch));
-  node_ptr_kernel<<<grid_for(n_nodes + 1), 256, 0, s>>>(uniq, M, n_nodes, N, d_node_ptr);
-  CXG_TRY(cudaGetLastError());
-  CXG_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), s));
-  rowlen_kernel<<<grid_for(n_nodes), 256, 0, s>>>(uniq, d_start, d_node_ptr, n_nodes, N, out->node_mask, d_rowlen,
-                                                  d_adj_off, d_node_nnz, d_bnd_len, d_n_rec, out->node, d_flag);
-  CXG_TRY(cudaGetLastError());
-  temp_bytes = 0;
-  CXG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, d_node_nnz, d_node_base, static_cast<int>(n_nodes), s));
-  CXG_TRY(cudaMalloc(&d_temp, temp_bytes));
-  CXG_TRY(cub::DeviceScan::ExclusiveSum(d_temp, temp_bytes, d_node_nnz, d_node_base, static_cast<int>(n_nodes), s));
-  CXG_TRY(cub::DeviceScan::ExclusiveSum(d_temp, temp_bytes, d_bnd_len, d_bnd_ptr, static_cast<int>(n_nodes), s));
-  CXG_TRY(cub::DeviceScan::ExclusiveSum(d_temp, temp_bytes, d_n_rec, d_rec_ptr, static_cast<int>(n_nodes), s));
-  {
-    int64_t last[6] = {0, 0, 0, 0, 0, 0};
-    const int64_t* src[6] = {d_node_base, d_node_nnz, d_bnd_ptr, d_bnd_len, d_rec_ptr, d_n_rec};
-    for (int i = 0; i < 6; ++i)
-      CXG_TRY(cudaMemcpyAsync(&last[i], src[i] + n_nodes - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    CXG_TRY(cudaMemcpyAsync(&h_flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CXG_TRY(cudaStreamSynchronize(s));
-    if (h_flag) {
+    if (hf.too_many) {
       *msg = "a node has more than 65535 neighbours; not supported";
       rc = 5;
       goto done;
     }
-    out->nnz = last[0] + last[1];
-    CXG_TRY(dalloc(&out->bnd_node, static_cast<size_t>(last[2] + last[3]), &out->device_bytes));
-    CXG_TRY(dalloc(&out->bnd_col, static_cast<size_t>(last[2] + last[3]), &out->device_bytes));
-    CXG_TRY(dalloc(&out->pairs, static_cast<size_t>(last[4] + last[5]), &out->device_bytes));
-  }
-  cudaFree(d_temp);
-  d_temp = nullptr;
-
-  CXG_TRY(dalloc(&out->row_ptr, static_cast<size_t>(n_free) + 1, &out->device_bytes));
-  CXG_TRY(dalloc(&out->col_idx, static_cast<size_t>(out->nnz), &out->device_bytes));
-  row_ptr_kernel<<<grid_for(n_nodes), 256, 0, s>>>(n_nodes, out->node_mask, d_eq0, d_node_base, d_rowlen, out->row_ptr);
-  CXG_TRY(cudaGetLastError());
-  CXG_TRY(cudaMemcpyAsync(out->row_ptr + n_free, &out->nnz, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-  col_idx_kernel<<<grid_for(M), 256, 0, s>>>(uniq, M, N, out->node_mask, d_eq0, d_node_base, d_rowlen, d_adj_off,
-                                             out->col_idx);
-  CXG_TRY(cudaGetLastError());
-  bnd_node_kernel<<<grid_for(M), 256, 0, s>>>(uniq, M, N, d_node_ptr, d_bnd_ptr, d_bnd_len, d_adj_off, out->node_mask, out->bnd_node,
-                                              out->bnd_col);
-  CXG_TRY(cudaGetLastError());
-  node_rec_kernel<<<grid_for(n_nodes), 256, 0, s>>>(d_node_base, d_rowlen, d_eq0, out->node_mask, d_bnd_ptr,
-                                                    d_rec_ptr, n_nodes, out->node);
-  CXG_TRY(cudaGetLastError());
-  pair_rec_kernel<<<grid_for(32 * n_nodes), 256, 0, s>>>(out->node, d_start, d_node_ptr, d_codes, sorted, P, n_nodes,
-                                                         out->pairs);
-  CXG_TRY(cudaGetLastError());
-
-  // node -> element incidence: stable sort of (node, e*n + local) by node
-  {
-    const int64_t m = n_elems * npe;
-    int32_t *d_codes = nullptr, *d_nodes_sorted = nullptr;
-    CXG_TRY(dalloc(&out->inc_ptr, n_nodes + 1, &out->device_bytes));
-    CXG_TRY(dalloc(&out->inc_code, m, &out->device_bytes));
-    CXG_TRY(cudaMalloc(&d_codes, sizeof(int32_t) * std::max<int64_t>(m, 1)));
-    CXG_TRY(cudaMalloc(&d_nodes_sorted, sizeof(int32_t) * std::max<int64_t>(m, 1)));
-    iota_kernel<<<grid_for(m), 256, 0, s>>>(d_codes, m);
-    CXG_TRY(cudaGetLastError());
-    int node_bits = 1;
-    while (node_bits < 31 && (n_nodes >> node_bits) != 0) ++node_bits;
-    temp_bytes = 0;
-    CXG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, d_conn, d_nodes_sorted, d_codes, out->inc_code,
-                                            static_cast<int>(m), 0, node_bits, s));
-    CXG_TRY(cudaMalloc(&d_temp, temp_bytes));
-    CXG_TRY(cub::DeviceRadixSort::SortPairs(d_temp, temp_bytes, d_conn, d_nodes_sorted, d_codes, out->inc_code,
-                                            static_cast<int>(m), 0, node_bits, s));
-    inc_ptr_kernel<<<grid_for(n_nodes + 1), 256, 0, s>>>(d_nodes_sorted, m, n_nodes, out->inc_ptr);
+    out->nnz = last[0] + len[0];
+    const size_t nbnd = static_cast<size_t>(last[1] + len[1]);
+    Parts rest;
+    const size_t r_col = rest.add<int32_t>(static_cast<size_t>(out->nnz)),
+                 r_pairs = rest.add<PairRec>(static_cast<size_t>(last[2] + len[2])), r_bn = rest.add<int32_t>(nbnd),
+                 r_bc = rest.add<int32_t>(nbnd);
+    CXG_TRY(cudaMalloc(&out->mem[1], rest.bytes));
+    out->device_bytes += static_cast<int64_t>(rest.bytes);
+    out->col_idx = part<int32_t>(out->mem[1], r_col);
+    out->pairs = part<PairRec>(out->mem[1], r_pairs);
+    out->bnd_node = part<int32_t>(out->mem[1], r_bn);
+    out->bnd_col = part<int32_t>(out->mem[1], r_bc);
+    CXG_TRY(cudaMemcpyAsync(out->row_ptr + n_free, &out->nnz, sizeof(int64_t), cudaMemcpyHostToDevice, s));
+    write_kernel<<<sweep_grid, kWarps * 32, sweep_smem, s>>>(S, n_nodes, out->node_mask, eq0, offs[0], offs[1], offs[2],
+                                                             cap, static_cast<int32_t*>(big), out->node, out->row_ptr,
+                                                             out->col_idx, out->pairs, out->bnd_node, out->bnd_col);
     CXG_TRY(cudaGetLastError());
     CXG_TRY(cudaStreamSynchronize(s));
-    cudaFree(d_codes);
-    cudaFree(d_nodes_sorted);
   }
 
 done:
-  cudaFree(d_temp);
-  cudaFree(d_flag);
-  cudaFree(d_bad);
-  cudaFree(d_flags);
-  cudaFree(d_scan);
-  cudaFree(d_keys);
-  cudaFree(d_keys2);
-  cudaFree(d_M);
-  cudaFree(d_node_ptr);
-  cudaFree(d_adj_off);
-  cudaFree(d_node_nnz);
-  cudaFree(d_node_base);
-  cudaFree(d_bnd_len);
-  cudaFree(d_bnd_ptr);
-  cudaFree(d_rowlen);
-  cudaFree(d_eq0);
-  cudaFree(d_codes);
-  cudaFree(d_codes2);
-  cudaFree(d_n_rec);
-  cudaFree(d_rec_ptr);
+  cudaFree(big);
+  cudaFree(scratch);
   return rc;
 }
 

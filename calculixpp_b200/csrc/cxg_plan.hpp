@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -66,6 +67,7 @@ struct cxg_plan {
   int device = 0;
   int64_t n_nodes = 0, n_elems = 0, n_gauss = 0;
   int32_t type = 0, n_free = 0, precision = 0;
+  void* mem = nullptr;  // the device block of the mesh copies below, up to status
   double* coords = nullptr;
   int32_t* conn = nullptr;
   double* young = nullptr;
@@ -112,6 +114,13 @@ struct cxg_plan {
   // *FILM faces of a temperature plan (cxg_thermal_plan_set_films); one device block
   cxg::FilmArgs films;
   void* film_mem = nullptr;
+  // WorkLease of the field operators (api::WorkLease): one buffer, grown on demand, and an
+  // event after its last use.
+  std::mutex work_mu;
+  double* work = nullptr;
+  size_t work_bytes = 0;
+  cudaEvent_t work_done = nullptr;
+  cudaStream_t work_stream = nullptr;
 };
 
 
@@ -136,6 +145,22 @@ void apply_windows(const cxg_plan* p, bool tangent, V2Args& v);
 int ensure_state(cxg_plan* p, cudaStream_t s);
 int state_comps(const cxg_plan* p);
 ElemArgs base_args(cxg_plan* p);
+// The plan's scratch for the launches of one call on stream s: held until the object goes
+// out of scope; a later call on another stream waits for this one's work. While s is being
+// captured the scratch is allocated and freed by the graph instead.
+class WorkLease {
+ public:
+  WorkLease(cxg_plan* p, size_t bytes, cudaStream_t s);
+  ~WorkLease();
+  WorkLease(const WorkLease&) = delete;
+  cudaError_t error = cudaSuccess;
+  double* ptr = nullptr;
+
+ private:
+  cxg_plan* p_;
+  cudaStream_t s_;
+  std::unique_lock<std::mutex> lock_;
+};
 
 }  // namespace api
 }  // namespace cxg
