@@ -175,6 +175,8 @@ const int64_t* active_row_ptr(const cxg_plan* p) {
 const int32_t* active_col_idx(const cxg_plan* p) {
   return p->mpc.on ? p->mpc.lists.col_idx : p->refpat.on ? p->refpat.col_idx : p->pat.col_idx;
 }
+// The node records of that pattern, where it is the plan's own.
+const NodeRec* active_nodes(const cxg_plan* p) { return p->mpc.on || p->refpat.on ? nullptr : p->pat.node; }
 int32_t active_n_free(const cxg_plan* p) { return p->mpc.on ? p->mpc.n_free : p->n_free; }
 
 // K_ff and rhs of a plan with multi-point constraints from its extended assembly
@@ -184,7 +186,7 @@ cudaError_t mpc_reduce(cxg_plan* p, double* vals, double* rhs, cudaStream_t s) {
   cudaError_t e = mpc_reduce_values(m.lists, m.vals_x, vals, s);
   if (e != cudaSuccess || !rhs) return e;
   if (m.c_x) {
-    e = launch_spmv(p->n_free, p->pat.row_ptr, p->pat.col_idx, m.vals_x, m.c_x, m.kc_x, s);
+    e = launch_spmv(p->n_free, p->pat.row_ptr, p->pat.col_idx, m.vals_x, m.c_x, m.kc_x, s, p->pat.node, p->n_nodes);
     if (e != cudaSuccess) return e;
   }
   return mpc_reduce_rhs(m.lists, m.rhs_x, m.c_x ? m.kc_x : nullptr, p->n_free, m.tmp_x, m.n_free, rhs, s);
@@ -1541,7 +1543,7 @@ int cxg_spmv(cxg_plan* p, const double* vals, const double* x, double* y, void* 
   if (!rc) rc = staged(p, 1, y, nb, false, s, &dy);
   if (rc) return rc;
   CHECK_CUDA(launch_spmv(active_n_free(p), active_row_ptr(p), active_col_idx(p), static_cast<const double*>(dv),
-                         static_cast<const double*>(dx), static_cast<double*>(dy), s), "spmv");
+                         static_cast<const double*>(dx), static_cast<double*>(dy), s, active_nodes(p), p->n_nodes), "spmv");
   if ((rc = copy_out(y, dy, nb, s))) return rc;
   if (dy != y) CHECK_CUDA(cudaStreamSynchronize(s), "sync");
   return CXG_OK;
@@ -1571,7 +1573,7 @@ int cxg_solve_cg(cxg_plan* p, const double* vals, const double* rhs, double* x, 
   double rel = 0.0;
   CHECK_CUDA(cg_solve(active_n_free(p), active_row_ptr(p), active_col_idx(p), static_cast<const double*>(dv),
                       static_cast<const double*>(db), static_cast<double*>(dx), rtol, max_iter,
-                      static_cast<double*>(p->stage[5]), &it, &rel, s), "cg");
+                      static_cast<double*>(p->stage[5]), &it, &rel, s, active_nodes(p), p->n_nodes), "cg");
   if ((rc = copy_out(x, dx, nb, s))) return rc;
   CHECK_CUDA(cudaStreamSynchronize(s), "sync");
   if (iterations) *iterations = it;

@@ -294,12 +294,14 @@ cudaError_t launch_films(int elem_type, const ElemArgs& a, const FilmArgs& f, do
 // Compliance adjoint (cxg_recover.cu); felem[3nE]: scratch for dc_dX (null without it).
 cudaError_t launch_adjoint(int elem_type, const ElemArgs& a, const int64_t* inc_ptr, const int32_t* inc_code,
                            double* felem, double* dc_dE, double* dc_dX, cudaStream_t s);
+// y = A x on CSR; node (null: any CSR matrix) for a matrix on a plan's own pattern.
 cudaError_t launch_spmv(int32_t nrows, const int64_t* rp, const int32_t* ci, const double* v, const double* x,
-                        double* y, cudaStream_t s);
-// Jacobi-preconditioned CG on CSR; work holds 5*n + 2056 doubles.
+                        double* y, cudaStream_t s, const NodeRec* node = nullptr, int64_t n_nodes = 0);
+// Jacobi-preconditioned CG on CSR; work holds 5*n + 2056 doubles; node as above.
 cudaError_t cg_solve(int32_t n, const int64_t* rp, const int32_t* ci, const double* v, const double* b, double* x,
-                     double rtol, int max_iter, double* work, int* iters_out, double* rel_out, cudaStream_t s);
-// The same CG loop with z = M^-1 r given by `precond` (launched on the loop's stream);
+                     double rtol, int max_iter, double* work, int* iters_out, double* rel_out, cudaStream_t s,
+                     const NodeRec* node = nullptr, int64_t n_nodes = 0);
+// CG with z = M^-1 r given by `precond` (launched on the loop's stream);
 // work holds 5*n + 2056 doubles, the fifth n-vector unused by the loop.
 using Preconditioner = std::function<cudaError_t(const double* r, double* z)>;
 cudaError_t pcg_solve(int32_t n, const int64_t* rp, const int32_t* ci, const double* v, const double* b, double* x,
