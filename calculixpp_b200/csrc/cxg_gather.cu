@@ -28,6 +28,13 @@ namespace cxg {
 namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
+// Warps per block unless the caller asks for others, one node each: blocks are handed out
+// as they finish, so nodes of one and of eight incident elements, full and compressed rows
+// even out (a grid of resident blocks striding over the nodes: C3D20 64^3 mixed 2885 us,
+// this way 2218; blocks of 8 warps 2330).
+constexpr int kWarps = 4;
+// (Registers: 64 a thread where the blocks are FP32, 80 where they are FP64: 64 spill there
+// and lose, C3D8 128^3 2908 -> 3239 us; with FP32 they win, C3D20 64^3 2190 -> 2007 us.)
 
 __device__ __forceinline__ NodeRec load_node(const NodeRec* p) {
   union {
@@ -82,134 +89,132 @@ __device__ __forceinline__ void end_pair(unsigned last, double*& o, double& v, d
 }
 
 template <typename R, int KIND, bool WIN>
-__device__ __forceinline__ void gather_nodes(const ElemArgs& A, const V2Args& V, unsigned bid, unsigned nblk) {
+__device__ __forceinline__ void gather_node(const ElemArgs& A, const V2Args& V, unsigned bid) {
   constexpr bool DIAG = KIND == GATHER_DIAG, SCALAR = KIND == GATHER_SCALAR;
   constexpr int UN = kPairRec;
   const int lane = threadIdx.x & 31;
-  const int64_t gwarp = static_cast<int64_t>(bid) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int64_t nwarps = static_cast<int64_t>(nblk) * (blockDim.x >> 5);
+  const int64_t n_begin = WIN ? V.n_begin : 0, n_end = WIN ? V.n_end : A.n_nodes;
+  const int64_t idx = n_begin + static_cast<int64_t>(bid) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (idx >= n_end) return;
   // lanes 27 .. 31 follow the third group without writing
   const int q = min(lane / 9, 2), k = lane < 27 ? lane - 9 * q : 0, ki = k / 3, kj = k - 3 * ki;
   const R* ed = reinterpret_cast<const R*>(V.edata) + (SCALAR ? 0 : k);
   const bool mine = !SCALAR || ki == kj;  // the other entries of a multiple of I are zero
   const int64_t ring_blocks = V.ring * V.nbp, base_blocks = V.ring_base * V.nbp;
-  const int64_t n_begin = WIN ? V.n_begin : 0, n_end = WIN ? V.n_end : A.n_nodes;
-  for (int64_t idx = n_begin + gwarp; idx < n_end; idx += nwarps) {
-    const int64_t a = WIN ? static_cast<int64_t>(V.node_order[idx]) : n_end - 1 - idx;
-    const NodeRec nd = load_node(A.node + a);
-    const int K = nd.npair, L = nd.len_mask & 0xfffffff, ma = nd.len_mask >> 28, self = nd.diag;
-    const bool full = L == 3 * K, plain = full && !V.accumulate;
-    double* const rows = A.vals + nd.base;
-    // what prescribed columns move to the rhs: of row ki (own pair and later ones), of
-    // row kj (earlier ones)
-    double rd = 0.0, rt = 0.0;
-    // the lane's entry of the block of pair p, wherever it goes
-    auto put = [&](int p, double v) {
-      const int i = p < self ? kj : ki, j = p < self ? ki : kj;
-      if (full) {
-        double* o = rows + i * L + 3 * p + j;
-        *o = V.accumulate ? *o + v : v;
-        return;
+  const int64_t a = WIN ? static_cast<int64_t>(V.node_order[idx]) : n_end - 1 - idx;
+  const NodeRec nd = load_node(A.node + a);
+  const int K = nd.npair, L = nd.len_mask & 0xfffffff, ma = nd.len_mask >> 28, self = nd.diag;
+  const bool full = L == 3 * K, plain = full && !V.accumulate;
+  double* const rows = A.vals + nd.base;
+  // what prescribed columns move to the rhs: of row ki (own pair and later ones), of
+  // row kj (earlier ones)
+  double rd = 0.0, rt = 0.0;
+  // the lane's entry of the block of pair p, wherever it goes
+  auto put = [&](int p, double v) {
+    const int i = p < self ? kj : ki, j = p < self ? ki : kj;
+    if (full) {
+      double* o = rows + i * L + 3 * p + j;
+      *o = V.accumulate ? *o + v : v;
+      return;
+    }
+    if (!((ma >> i) & 1)) return;
+    const uint32_t at = static_cast<uint32_t>(__ldg(A.bnd_col + nd.bnd0 + p));
+    const int mb = at >> 28;
+    if ((mb >> j) & 1) {
+      double* o = rows + static_cast<int64_t>(__popc(ma & ((1 << i) - 1))) * L + (at & 0xfffffff) +
+                  __popc(mb & ((1 << j) - 1));
+      *o = V.accumulate ? *o + v : v;
+    } else {
+      const double c = v * A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p)) + j];
+      if (p < self)
+        rt -= c;
+      else
+        rd -= c;
+    }
+  };
+  if (ma) {
+    int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
+    const PairRec* list = A.pairs + nd.list0 + q;
+    PairRec rec;
+    if (nd.rounds) rec = load_pairs(list);
+    // the off-diagonal blocks' sums (DIAG): entry (ki, kj) of the blocks from the own
+    // pair on, entry (kj, ki) of those before it
+    double own = 0.0, before = 0.0;
+    double v = 0.0;
+    // before the own pair a lane writes entry (kj, ki), from there on (ki, kj)
+    double* o = rows + 3 * p + (p < self ? kj * L + ki : ki * L + kj);
+    const int64_t turn = static_cast<int64_t>(ki - kj) * (L - 1);
+    for (uint32_t r = 0; r < nd.rounds; ++r) {
+      R x[UN];
+#pragma unroll
+      for (int i = 0; i < UN; ++i) {
+        x[i] = R(0);
+        if (mine) x[i] = __ldg(ed + (SCALAR ? 1 : 9) * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks));
       }
-      if (!((ma >> i) & 1)) return;
-      const uint32_t at = static_cast<uint32_t>(__ldg(A.bnd_col + nd.bnd0 + p));
-      const int mb = at >> 28;
-      if ((mb >> j) & 1) {
-        double* o = rows + static_cast<int64_t>(__popc(ma & ((1 << i) - 1))) * L + (at & 0xfffffff) +
-                    __popc(mb & ((1 << j) - 1));
-        *o = V.accumulate ? *o + v : v;
-      } else {
-        const double c = v * A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p)) + j];
-        if (p < self)
-          rt -= c;
-        else
-          rd -= c;
-      }
-    };
-    if (ma) {
-      int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
-      const PairRec* list = A.pairs + nd.list0 + q;
-      PairRec rec;
-      if (nd.rounds) rec = load_pairs(list);
-      // the off-diagonal blocks' sums (DIAG): entry (ki, kj) of the blocks from the own
-      // pair on, entry (kj, ki) of those before it
-      double own = 0.0, before = 0.0;
-      double v = 0.0;
-      // before the own pair a lane writes entry (kj, ki), from there on (ki, kj)
-      double* o = rows + 3 * p + (p < self ? kj * L + ki : ki * L + kj);
-      const int64_t turn = static_cast<int64_t>(ki - kj) * (L - 1);
-      for (uint32_t r = 0; r < nd.rounds; ++r) {
-        R x[UN];
+      const bool turns = rec.flags >> 31;
+      const unsigned ends = lane < 27 ? rec.flags : 0u;
+      list += 3;
+      if (r + 1 < nd.rounds) rec = load_pairs(list);
+      if (plain && !turns) {
 #pragma unroll
         for (int i = 0; i < UN; ++i) {
-          x[i] = R(0);
-          if (mine) x[i] = __ldg(ed + (SCALAR ? 1 : 9) * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks));
+          v += static_cast<double>(x[i]);
+          end_pair<DIAG>(ends & (1u << i), o, v, own);
         }
-        const bool turns = rec.flags >> 31;
-        const unsigned ends = lane < 27 ? rec.flags : 0u;
-        list += 3;
-        if (r + 1 < nd.rounds) rec = load_pairs(list);
-        if (plain && !turns) {
+      } else if (plain) {
 #pragma unroll
-          for (int i = 0; i < UN; ++i) {
-            v += static_cast<double>(x[i]);
-            end_pair<DIAG>(ends & (1u << i), o, v, own);
+        for (int i = 0; i < UN; ++i) {
+          v += static_cast<double>(x[i]);
+          end_pair<DIAG>(ends & (1u << i), o, v, own);
+          if (ends & (0x10000u << i)) {
+            o += turn;
+            if (DIAG) before = own;
+            own = DIAG ? 0.0 : own;
           }
-        } else if (plain) {
+        }
+      } else {
 #pragma unroll
-          for (int i = 0; i < UN; ++i) {
-            v += static_cast<double>(x[i]);
-            end_pair<DIAG>(ends & (1u << i), o, v, own);
-            if (ends & (0x10000u << i)) {
-              o += turn;
-              if (DIAG) before = own;
-              own = DIAG ? 0.0 : own;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < UN; ++i) {
-            v += static_cast<double>(x[i]);
-            if (ends & (1u << i)) {
-              if (!DIAG || p != self) put(p, v);
-              own += v;
-              v = 0.0;
-              ++p;
-              if (DIAG && (ends & (0x10000u << i))) {
-                before = own;
-                own = 0.0;
-              }
+        for (int i = 0; i < UN; ++i) {
+          v += static_cast<double>(x[i]);
+          if (ends & (1u << i)) {
+            if (!DIAG || p != self) put(p, v);
+            own += v;
+            v = 0.0;
+            ++p;
+            if (DIAG && (ends & (0x10000u << i))) {
+              before = own;
+              own = 0.0;
             }
           }
         }
       }
-      if constexpr (DIAG) {
-        // a run that ends before the own pair holds earlier pairs only
-        if ((q == 0 ? nd.pair1 : q == 1 ? nd.pair2 : K) <= self) {
-          before = own;
-          own = 0.0;
-        }
-        __syncwarp();  // orders the block below after the loop's write of the same place
-        const double t = own + __shfl_sync(kAll, before, min(9 * (lane / 9) + 3 * kj + ki, 31));
-        const double t1 = __shfl_sync(kAll, t, (lane + 9) & 31), t2 = __shfl_sync(kAll, t, (lane + 18) & 31);
-        if (lane < 9 && K > 0) put(self, -((t + t1) + t2));
+    }
+    if constexpr (DIAG) {
+      // a run that ends before the own pair holds earlier pairs only
+      if ((q == 0 ? nd.pair1 : q == 1 ? nd.pair2 : K) <= self) {
+        before = own;
+        own = 0.0;
       }
-      if (A.rhs) {
-        double v = 0.0;
-        if (!full) {  // (full rows have no prescribed column)
-          rd += __shfl_down_sync(kAll, rd, 9) + __shfl_down_sync(kAll, rd, 18);
-          rt += __shfl_down_sync(kAll, rt, 9) + __shfl_down_sync(kAll, rt, 18);
-          rd += __shfl_down_sync(kAll, rd, 1) + __shfl_down_sync(kAll, rd, 2);  // lane 3 i: row i
-          rt += __shfl_down_sync(kAll, rt, 3) + __shfl_down_sync(kAll, rt, 6);  // lane i: row i
-          v = rd + __shfl_sync(kAll, rt, lane / 3);
-        }
-        if (lane == 0 || lane == 3 || lane == 6) {
-          const int r = lane / 3;
-          if ((ma >> r) & 1) {
-            const int64_t eq = nd.eq0 + __popc(ma & ((1 << r) - 1));
-            const double prev = V.accumulate ? A.rhs[eq] : (V.f_ext ? V.f_ext[3 * a + r] : 0.0);
-            A.rhs[eq] = prev + v;
-          }
+      __syncwarp();  // orders the block below after the loop's write of the same place
+      const double t = own + __shfl_sync(kAll, before, min(9 * (lane / 9) + 3 * kj + ki, 31));
+      const double t1 = __shfl_sync(kAll, t, (lane + 9) & 31), t2 = __shfl_sync(kAll, t, (lane + 18) & 31);
+      if (lane < 9 && K > 0) put(self, -((t + t1) + t2));
+    }
+    if (A.rhs) {
+      double v = 0.0;
+      if (!full) {  // (full rows have no prescribed column)
+        rd += __shfl_down_sync(kAll, rd, 9) + __shfl_down_sync(kAll, rd, 18);
+        rt += __shfl_down_sync(kAll, rt, 9) + __shfl_down_sync(kAll, rt, 18);
+        rd += __shfl_down_sync(kAll, rd, 1) + __shfl_down_sync(kAll, rd, 2);  // lane 3 i: row i
+        rt += __shfl_down_sync(kAll, rt, 3) + __shfl_down_sync(kAll, rt, 6);  // lane i: row i
+        v = rd + __shfl_sync(kAll, rt, lane / 3);
+      }
+      if (lane == 0 || lane == 3 || lane == 6) {
+        const int r = lane / 3;
+        if ((ma >> r) & 1) {
+          const int64_t eq = nd.eq0 + __popc(ma & ((1 << r) - 1));
+          const double prev = V.accumulate ? A.rhs[eq] : (V.f_ext ? V.f_ext[3 * a + r] : 0.0);
+          A.rhs[eq] = prev + v;
         }
       }
     }
@@ -221,56 +226,52 @@ __device__ __forceinline__ void gather_nodes(const ElemArgs& A, const V2Args& V,
 __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& V) {
   constexpr int UN = kPairRec;
   const int lane = threadIdx.x & 31, j = lane / 3, q = lane - 3 * j;
-  const int64_t gwarp = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
   const double* ed = reinterpret_cast<const double*>(V.edata);
-  for (int64_t a0 = 10 * gwarp; a0 < A.n_nodes; a0 += 10 * nwarps) {
-    const int64_t a = a0 + j;
-    const bool on = lane < 30 && a < A.n_nodes;
-    NodeRec nd{};
-    if (on) nd = load_node(A.node + a);
-    const bool free = (nd.len_mask >> 28) & 1, full = (nd.len_mask & 0xfffffff) == nd.npair;
-    double rr = 0.0;
-    if (free) {
-      int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
-      const PairRec* list = A.pairs + nd.list0 + q;
-      double* o = A.vals + nd.base;
-      double v = 0.0;
-      for (uint32_t r = 0; r < nd.rounds; ++r, list += 3) {
-        const PairRec rec = load_pairs(list);
-        double x[UN];
+  const int64_t a = 10 * (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) + j;
+  const bool on = lane < 30 && a < A.n_nodes;
+  NodeRec nd{};
+  if (on) nd = load_node(A.node + a);
+  const bool free = (nd.len_mask >> 28) & 1, full = (nd.len_mask & 0xfffffff) == nd.npair;
+  double rr = 0.0;
+  if (free) {
+    int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
+    const PairRec* list = A.pairs + nd.list0 + q;
+    double* o = A.vals + nd.base;
+    double v = 0.0;
+    for (uint32_t r = 0; r < nd.rounds; ++r, list += 3) {
+      const PairRec rec = load_pairs(list);
+      double x[UN];
 #pragma unroll
-        for (int i = 0; i < UN; ++i) x[i] = __ldg(ed + rec.block[i]);
+      for (int i = 0; i < UN; ++i) x[i] = __ldg(ed + rec.block[i]);
 #pragma unroll
-        for (int i = 0; i < UN; ++i) {
-          v += x[i];
-          if (rec.flags & (1u << i)) {
-            if (full) {
-              o[p] = v;
-            } else {
-              const uint32_t at = static_cast<uint32_t>(__ldg(A.bnd_col + nd.bnd0 + p));
-              if (at >> 28)
-                o[at & 0xfffffff] = v;
-              else
-                rr -= v * A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p))];
-            }
-            v = 0.0;
-            ++p;
+      for (int i = 0; i < UN; ++i) {
+        v += x[i];
+        if (rec.flags & (1u << i)) {
+          if (full) {
+            o[p] = v;
+          } else {
+            const uint32_t at = static_cast<uint32_t>(__ldg(A.bnd_col + nd.bnd0 + p));
+            if (at >> 28)
+              o[at & 0xfffffff] = v;
+            else
+              rr -= v * A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p))];
           }
+          v = 0.0;
+          ++p;
         }
       }
     }
-    const double r1 = __shfl_down_sync(kAll, rr, 1), r2 = __shfl_down_sync(kAll, rr, 2);
-    if (A.rhs && free && q == 0) A.rhs[nd.eq0] = (V.f_ext ? V.f_ext[a] : 0.0) + ((rr + r1) + r2);
   }
+  const double r1 = __shfl_down_sync(kAll, rr, 1), r2 = __shfl_down_sync(kAll, rr, 2);
+  if (A.rhs && free && q == 0) A.rhs[nd.eq0] = (V.f_ext ? V.f_ext[a] : 0.0) + ((rr + r1) + r2);
 }
 
 template <typename R, int KIND, bool WIN>
-__global__ void __launch_bounds__(256, 3) gather_kernel(ElemArgs A, V2Args V) {
+__global__ void __launch_bounds__(256, KIND == GATHER_DIAG ? 4 : 3) gather_kernel(ElemArgs A, V2Args V) {
   if constexpr (KIND == GATHER_ONE_DOF)
     gather_one_dof(A, V);
   else
-    gather_nodes<R, KIND, WIN>(A, V, blockIdx.x, gridDim.x);
+    gather_node<R, KIND, WIN>(A, V, blockIdx.x);
 }
 
 // Internal force of every node: one thread per component, the element forces in element
@@ -298,17 +299,10 @@ __global__ void __launch_bounds__(256) force_kernel(ElemArgs A, V2Args V) {
   }
 }
 
-int sm_count() {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 cudaError_t launch_forces(const ElemArgs& a, const V2Args& v, cudaStream_t s) {
   const int64_t count = 3 * (v.n_end - v.n_begin);
   if (!a.f_int || count <= 0) return cudaSuccess;
-  const int64_t grid = std::min<int64_t>((count + 255) / 256, 8 * static_cast<int64_t>(sm_count()));
+  const int64_t grid = std::min<int64_t>((count + 255) / 256, 148 * 8);
   (v.node_order ? force_kernel<true> : force_kernel<false>)<<<static_cast<unsigned>(grid), 256, 0, s>>>(a, v);
   return cudaGetLastError();
 }
@@ -319,15 +313,11 @@ cudaError_t launch_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, c
   if constexpr (KIND == GATHER_FULL || KIND == GATHER_DIAG) {
     if (v.node_order) kern = gather_kernel<R, KIND, true>;
   }
-  const int warps = cfg.p2_warps > 0 ? std::min(cfg.p2_warps, 8) : 8;
+  const int warps = cfg.p2_warps > 0 ? std::min(cfg.p2_warps, 8) : kWarps;
   const int64_t count = v.n_end - v.n_begin;
   if (count <= 0) return cudaSuccess;
-  int per_sm = 0;
-  const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, 0);
-  if (err != cudaSuccess) return err;
-  if (cfg.p2_blocks_per_sm > 0) per_sm = std::min(per_sm, cfg.p2_blocks_per_sm);
   const int64_t block_nodes = static_cast<int64_t>(warps) * (KIND == GATHER_ONE_DOF ? 10 : 1);
-  const int64_t grid = std::min<int64_t>((count + block_nodes - 1) / block_nodes, static_cast<int64_t>(std::max(per_sm, 1)) * sm_count());
+  const int64_t grid = (count + block_nodes - 1) / block_nodes;
   kern<<<static_cast<unsigned>(grid), warps * 32, 0, s>>>(a, v);
   return cudaGetLastError();
 }
@@ -368,36 +358,25 @@ __global__ void __launch_bounds__(256) gather_batch_kernel(const __grid_constant
   int k = 0;
   while (k + 1 < P.n && static_cast<int64_t>(blockIdx.x) >= P.s[k + 1].blk0) ++k;
   const GatherSlot& S = P.s[k];
-  const int64_t end = k + 1 < P.n ? P.s[k + 1].blk0 : static_cast<int64_t>(gridDim.x);
-  const unsigned bid = blockIdx.x - static_cast<unsigned>(S.blk0), nblk = static_cast<unsigned>(end - S.blk0);
-  gather_nodes<R, KIND, false>(S.a, S.v, bid, nblk);
+  gather_node<R, KIND, false>(S.a, S.v, blockIdx.x - static_cast<unsigned>(S.blk0));
 }
 
 template <typename R, int KIND>
 cudaError_t launch_batch_t(const BatchSlotIn* in, int n, cudaStream_t s) {
   auto kern = gather_batch_kernel<R, KIND>;
   GatherPass P{};
-  int warps = 8;
+  int warps = 0;  // one block shape for every slot: the smallest that was asked for
   for (int k = 0; k < n; ++k)
-    if (in[k].cfg.p2_warps > 0) warps = std::min(warps, in[k].cfg.p2_warps);
-  int per_sm = 0;
-  const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, 0);
-  if (err != cudaSuccess) return err;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  int64_t need[kMaxBatchSlots], grid[kMaxBatchSlots];
-  double w[kMaxBatchSlots];
-  for (int k = 0; k < n; ++k) {
-    need[k] = std::max<int64_t>(1, (in[k].v.n_end - in[k].v.n_begin + warps - 1) / warps);
-    w[k] = in[k].p2_weight;
-  }
-  share_blocks(w, need, n, static_cast<int64_t>(per_sm) * sm_count(), grid);
+    if (in[k].cfg.p2_warps > 0) warps = warps ? std::min(warps, in[k].cfg.p2_warps) : in[k].cfg.p2_warps;
+  warps = warps ? std::min(warps, 8) : kWarps;
   int64_t blk = 0;
   for (int k = 0; k < n; ++k) {
     P.s[k].a = in[k].a;
     P.s[k].v = in[k].v;
     P.s[k].blk0 = blk;
-    blk += grid[k];
+    blk += (in[k].v.n_end - in[k].v.n_begin + warps - 1) / warps;
   }
+  if (blk <= 0) return cudaSuccess;
   P.n = n;
   kern<<<static_cast<unsigned>(blk), warps * 32, 0, s>>>(P);
   return cudaGetLastError();
