@@ -92,7 +92,25 @@ def _dev(a, dtype, device):
 
 
 def _stream():
-    return _vp(torch.cuda.current_stream().cuda_stream)
+    return _vp(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+
+
+class _on:
+    """The plan's device as the current one; nothing to do (and no context switch to pay
+    for on every call) where it is already."""
+
+    __slots__ = ("ctx",)
+
+    def __init__(self, device):
+        self.ctx = None if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+    def __enter__(self):
+        if self.ctx is not None:
+            self.ctx.__enter__()
+
+    def __exit__(self, *exc):
+        if self.ctx is not None:
+            self.ctx.__exit__(*exc)
 
 
 def _c_material(m: Material, keep: list):
@@ -125,17 +143,14 @@ class Plan:
         self.dof_eq, self.prescribed, self.n_free = dof_eq, prescribed, n_free
         keep = []
         mats = (_lib.CxgMaterial * len(model.materials))(*[_c_material(x, keep) for x in model.materials])
-        coords = _dev(m.coords, torch.float64, dev)
-        conn = _dev(m.conn.reshape(-1), torch.int32, dev)
-        young = _dev(m.young, torch.float64, dev) if m.young is not None else None
-        poisson = _dev(m.poisson, torch.float64, dev) if m.poisson is not None else None
-        elem_mat = _dev(model.elem_mat, torch.int32, dev) if model.elem_mat is not None else None
-        d_dof = _dev(dof_eq, torch.int32, dev)
-        d_pre = _dev(prescribed, torch.float64, dev)
-        desc = _lib.CxgMeshDesc(m.n_nodes, m.n_elems, m.etype, _ptr(coords), _ptr(conn), _ptr(young),
-                                _ptr(poisson), _ptr(elem_mat), len(model.materials),
-                                C.cast(mats, _vp))
-        dmap = _lib.CxgDofmapDesc(_ptr(d_dof), _ptr(d_pre), n_free)
+        # host arrays go to the library as they are (it copies them to the plan's memory)
+        arrays = {k: None if v is None else self._host(v, t, keep) for k, (v, t) in {
+            "coords": (m.coords, np.float64), "conn": (m.conn, np.int32), "young": (m.young, np.float64),
+            "poisson": (m.poisson, np.float64), "elem_mat": (model.elem_mat, np.int32), "dof": (dof_eq, np.int32),
+            "pre": (prescribed, np.float64)}.items()}
+        desc = _lib.CxgMeshDesc(m.n_nodes, m.n_elems, m.etype, arrays["coords"], arrays["conn"], arrays["young"],
+                                arrays["poisson"], arrays["elem_mat"], len(model.materials), C.cast(mats, _vp))
+        dmap = _lib.CxgDofmapDesc(arrays["dof"], arrays["pre"], n_free)
         handle = _vp()
         with torch.cuda.device(dev):
             torch.cuda.synchronize()
@@ -151,6 +166,16 @@ class Plan:
         rp, ci = _vp(), _vp()
         _lib.check(self.lib.cxg_plan_pattern_device(self.h, C.byref(rp), C.byref(ci)))
         self._pattern = None
+
+    def _host(self, a, dtype, keep):
+        """Address of `a` as a contiguous array of dtype (a host array, or a tensor on the GPU)."""
+        if isinstance(a, torch.Tensor):
+            a = _dev(a, torch.float64 if dtype is np.float64 else torch.int32, self.device)
+            keep.append(a)
+            return _ptr(a)
+        a = np.ascontiguousarray(a, dtype=dtype)
+        keep.append(a)
+        return _vp(a.ctypes.data)
 
     # -- lifetime ------------------------------------------------------------------
     def close(self):
@@ -303,7 +328,7 @@ class Plan:
         vals = torch.empty(self.nnz, dtype=torch.float64, device=dev) if vals is None else vals
         rhs = torch.empty(self.n_free, dtype=torch.float64, device=dev) if rhs is None else rhs
         fe = None if f_ext is None else _dev(f_ext, torch.float64, dev)
-        with torch.cuda.device(dev):
+        with _on(dev):
             _lib.check(self.lib.cxg_assemble_linear(self.h, _ptr(vals), _ptr(rhs), _ptr(fe), _stream()))
             if check:
                 self.check()
@@ -312,7 +337,7 @@ class Plan:
     def accumulate_linear(self, vals, rhs=None):
         """Add this plan's element contributions to vals (and rhs) in place; the element
         kernel alone, no zeroing and no load vector (cxg_assemble_linear_ex, CXG_ACCUMULATE)."""
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_assemble_linear_ex(self.h, _ptr(vals), _ptr(rhs), None, _lib.ACCUMULATE,
                                                        _stream()))
 
@@ -323,7 +348,7 @@ class Plan:
         rhs = torch.empty(self.n_free, dtype=torch.float64, device=dev) if rhs is None else rhs
         du = _dev(u, torch.float64, dev)
         fe = None if f_ext is None else _dev(f_ext, torch.float64, dev)
-        with torch.cuda.device(dev):
+        with _on(dev):
             _lib.check(self.lib.cxg_assemble_tangent(self.h, _ptr(du), _ptr(vals), _ptr(f_int), _ptr(rhs),
                                                      _ptr(fe), _stream()))
             if check:
@@ -335,7 +360,7 @@ class Plan:
         density per element."""
         vals = torch.empty(self.nnz, dtype=torch.float64, device=self.device) if vals is None else vals
         d = _dev(density, torch.float64, self.device)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_assemble_mass(self.h, _ptr(d), int(bool(lumped)), _ptr(vals), _stream()))
             if check:
                 self.check()
@@ -346,7 +371,7 @@ class Plan:
         src/fem/assembly.cpp:300-331); gp_stress (n_gauss, 6) Voigt per Gauss point."""
         vals = torch.empty(self.nnz, dtype=torch.float64, device=self.device) if vals is None else vals
         sg = None if gp_stress is None else _dev(gp_stress, torch.float64, self.device).reshape(-1)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_assemble_geometric(self.h, _ptr(sg), _ptr(vals), _stream()))
             if check:
                 self.check()
@@ -356,7 +381,7 @@ class Plan:
         """Gauss-point stress (n_gauss, 6) for the full displacement u (recover_gauss_stress,
         src/fem/stress.cpp:147-187)."""
         out = torch.empty(self.n_gauss * 6, dtype=torch.float64, device=self.device)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_recover_gauss_stress(self.h, _ptr(_dev(u, torch.float64, self.device)), _ptr(out),
                                                          _stream()))
             self.check()
@@ -370,7 +395,7 @@ class Plan:
         ss = torch.empty(6 * N, dtype=torch.float64, device=self.device)
         rf = torch.empty(3 * N, dtype=torch.float64, device=self.device)
         fe = None if f_ext is None else _dev(f_ext, torch.float64, self.device)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_recover_fields(self.h, _ptr(_dev(u, torch.float64, self.device)), _ptr(fe),
                                                    _ptr(st), _ptr(ss), _ptr(rf), _stream()))
             self.check()
@@ -379,23 +404,23 @@ class Plan:
     # -- material state -------------------------------------------------------------
     def state(self, committed=True):
         out = torch.empty(self.n_gauss * 13, dtype=torch.float64, device=self.device)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_state_get(self.h, _lib.COMMITTED if committed else _lib.TRIAL, _ptr(out)))
         return out.view(self.n_gauss, 13)
 
     def set_state(self, state, committed=True):
         s = _dev(state, torch.float64, self.device).reshape(-1)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_state_set(self.h, _lib.COMMITTED if committed else _lib.TRIAL, _ptr(s)))
 
     def commit(self):
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_state_commit(self.h, _stream()))
 
     # -- reduced-system products, solve and adjoint ------------------------------------------
     def spmv(self, vals, x):
         y = torch.empty(self.n_free, dtype=torch.float64, device=self.device)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_spmv(self.h, _ptr(vals), _ptr(_dev(x, torch.float64, self.device)), _ptr(y),
                                          _stream()))
         return y
@@ -405,7 +430,7 @@ class Plan:
         x = torch.zeros(self.n_free, dtype=torch.float64, device=self.device) if x is None else x
         it = C.c_int32()
         rel = C.c_double()
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_solve_cg(self.h, _ptr(vals), _ptr(_dev(rhs, torch.float64, self.device)), _ptr(x),
                                              float(rtol), int(max_iter), C.byref(it), C.byref(rel), _stream()))
         return x, int(it.value), float(rel.value)
@@ -425,7 +450,7 @@ class Plan:
         m = self.model.mesh
         dE = torch.empty(m.n_elems, dtype=torch.float64, device=self.device)
         dX = torch.empty(3 * m.n_nodes, dtype=torch.float64, device=self.device)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_adjoint_compliance(self.h, _ptr(_dev(u, torch.float64, self.device)), _ptr(dE),
                                                        _ptr(dX), _stream()))
             self.check()
@@ -462,7 +487,7 @@ class ThermalPlan(Plan):
         desc = _lib.CxgMeshDesc(mesh.n_nodes, mesh.n_elems, mesh.etype, _ptr(coords), _ptr(conn), None, None, None, 1,
                                 C.cast(mats, _vp))
         handle = _vp()
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_thermal_plan_create(C.byref(desc), _vp(deq.ctypes.data), _vp(pre.ctypes.data), nf,
                                                         C.byref(handle)))
         self.h = handle
@@ -483,7 +508,7 @@ class ThermalPlan(Plan):
         if not (e.size == f.size == hh.size == sk.size):
             raise ValueError("elem, face, h and sink must have one entry per film")
         ptr = lambda a: a.ctypes.data_as(C.c_void_p) if a.size else None
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check(self.lib.cxg_thermal_plan_set_films(self.h, e.size, ptr(e), ptr(f), ptr(hh), ptr(sk)))
 
     def assemble_conduction(self, conductivity, flux=None, vals=None, rhs=None, check=True):
@@ -493,7 +518,7 @@ class ThermalPlan(Plan):
         rhs = torch.empty(self.n_free, dtype=torch.float64, device=dev) if rhs is None else rhs
         k = _dev(conductivity, torch.float64, dev)
         q = None if flux is None else _dev(flux, torch.float64, dev)
-        with torch.cuda.device(dev):
+        with _on(dev):
             _lib.check(self.lib.cxg_assemble_conduction(self.h, _ptr(k), _ptr(q), _ptr(vals), _ptr(rhs), _stream()))
             if check:
                 self.check()

@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT_DIR, "libcxg.so")
-SOURCES = ["cxg_api.cu", "cxg_kernels.cu", "cxg_pattern.cu", "cxg_v2.cu", "cxg_fp64.cu", "cxg_gather.cu", "cxg_solve.cu", "cxg_batch.cu", "cxg_recover.cu",
+SOURCES = ["cxg_api.cu", "cxg_kernels.cu", "cxg_pattern.cu", "cxg_pool.cu", "cxg_launch.cu", "cxg_v2.cu", "cxg_fp64.cu", "cxg_gather.cu", "cxg_solve.cu", "cxg_batch.cu", "cxg_recover.cu",
            "cxg_refpattern.cu", "cxg_mpc.cu", "cxg_sparse_solve.cu", "cxg_film.cu"]
 # Per-file flags: the reference-pattern mask evaluates K_e in the reference's own FP64
 # operation order, so it must not contract multiply-adds.

@@ -224,11 +224,14 @@ WorkLease::WorkLease(cxg_plan* p, size_t bytes, cudaStream_t s) : p_(p), s_(s) {
   lock_ = std::unique_lock<std::mutex>(p->work_mu);
   if (!p->work_done) error = cudaEventCreateWithFlags(&p->work_done, cudaEventDisableTiming);
   if (error == cudaSuccess && p->work_bytes < bytes) {
-    cudaFree(p->work);  // waits for its last use
+    if (p->work) {
+      cudaDeviceSynchronize();  // its last use
+      device_free(p->work);
+    }
     p->device_bytes -= static_cast<int64_t>(p->work_bytes);
     p->work = nullptr;
     p->work_bytes = 0;
-    error = cudaMalloc(reinterpret_cast<void**>(&p->work), bytes);
+    error = device_alloc(reinterpret_cast<void**>(&p->work), bytes);
     if (error == cudaSuccess) {
       p->work_bytes = bytes;
       p->device_bytes += static_cast<int64_t>(bytes);
@@ -348,21 +351,23 @@ int ensure_v2(cxg_plan* p, bool tangent) {
   }
   const size_t need = v2_edata_bytes(p->type, w.ring, p->precision);
   if (p->edata_bytes < need) {
-    cudaFree(p->edata);
+    if (p->edata) CHECK_CUDA(cudaDeviceSynchronize(), "synchronize");
+    device_free(p->edata);
     p->edata = nullptr;
     p->device_bytes -= static_cast<int64_t>(p->edata_bytes);
     p->edata_bytes = 0;
-    CHECK_CUDA(cudaMalloc(&p->edata, std::max<size_t>(need, 16)), "element buffer");
+    CHECK_CUDA(device_alloc(&p->edata, need), "element buffer");
     p->edata_bytes = need;
     p->device_bytes += static_cast<int64_t>(need);
   }
   const size_t fb = sizeof(double) * 3 * nodes_of(p->type) * static_cast<size_t>(w.ring);
   if (tangent && p->fdata_bytes < fb) {
-    cudaFree(p->fdata);
+    if (p->fdata) CHECK_CUDA(cudaDeviceSynchronize(), "synchronize");
+    device_free(p->fdata);
     p->fdata = nullptr;
     p->device_bytes -= static_cast<int64_t>(p->fdata_bytes);
     p->fdata_bytes = 0;
-    CHECK_CUDA(cudaMalloc(&p->fdata, fb), "force buffer");
+    CHECK_CUDA(device_alloc(reinterpret_cast<void**>(&p->fdata), fb), "force buffer");
     p->fdata_bytes = fb;
     p->device_bytes += static_cast<int64_t>(fb);
   }
@@ -476,6 +481,7 @@ int cxg_plan_create(const cxg_mesh_desc* m, const cxg_dofmap_desc* d, int32_t pr
   p->n_gauss = m->n_elems * gauss_of(m->elem_type);
   p->n_mats = m->n_materials;
   p->has_plastic = plastic;
+  p->cfg[CXG_MIXED].tile = default_tile(m->elem_type);
   for (const J2Mat& jm : mats) p->kinematic = p->kinematic || jm.h_kin != 0.0;
   const int npe = nodes_of(m->elem_type);
   cudaStream_t s = nullptr;
@@ -513,7 +519,7 @@ int cxg_plan_create(const cxg_mesh_desc* m, const cxg_dofmap_desc* d, int32_t pr
                at_pre = place(24 * N), at_mats = place(sizeof(J2Mat) * mats.size()),
                at_em = place(m->elem_mat ? 4 * E : 0), at_young = place(8 * E), at_poisson = place(8 * E),
                at_props = place(8 * props.size()), at_status = place(sizeof(DevStatus)), at_bad = place(sizeof(int));
-  TRYC(cudaMalloc(&p->mem, total), "plan");
+  TRYC(device_alloc(&p->mem, total), "plan");
   p->device_bytes += static_cast<int64_t>(total);
   char* mem = static_cast<char*>(p->mem);
   p->coords = reinterpret_cast<double*>(mem + at_coords);
@@ -666,8 +672,16 @@ int cxg_plan_destroy(cxg_plan* p) {
   if (p->last_stream) cudaStreamSynchronize(p->last_stream);
   thermal::release(p);
   cudaFree(p->film_mem);
-  void* bufs[] = {p->mem, p->pat.mem[0], p->pat.mem[1], p->state[0], p->state[1], p->edata, p->fdata};
-  for (void* b : bufs) cudaFree(b);
+  // (cudaFree would wait for all of the device's work; so does this, once)
+  cudaDeviceSynchronize();
+  int current = p->device;
+  cudaGetDevice(&current);
+  if (current != p->device) cudaSetDevice(p->device);
+  for (void* b : {p->mem, p->pat.mem[0], p->pat.mem[1], p->edata, static_cast<void*>(p->fdata), static_cast<void*>(p->work)})
+    device_free(b);
+  device_trim();
+  if (current != p->device) cudaSetDevice(current);
+  for (double* b : p->state) cudaFree(b);
   for (auto& row : p->sched)
     for (WinSched& w : row) cudaFree(w.node_order);
   for (void* b : {static_cast<void*>(p->refpat.row_ptr), static_cast<void*>(p->refpat.col_idx),
@@ -683,7 +697,6 @@ int cxg_plan_destroy(cxg_plan* p) {
                   static_cast<void*>(mp.kc_x)})
     cudaFree(b);
   for (void* b : p->stage) cudaFree(b);
-  cudaFree(p->work);
   if (p->work_done) cudaEventDestroy(p->work_done);
   delete p;
   return CXG_OK;
@@ -1013,11 +1026,12 @@ namespace {
 int ensure_scalar(cxg_plan* p) {
   const size_t need = sizeof(double) * static_cast<size_t>(p->n_elems) * blocks_padded(nodes_of(p->type));
   if (p->edata_bytes >= need) return CXG_OK;
-  cudaFree(p->edata);
+  if (p->edata) CHECK_CUDA(cudaDeviceSynchronize(), "synchronize");
+  device_free(p->edata);
   p->edata = nullptr;
   p->device_bytes -= static_cast<int64_t>(p->edata_bytes);
   p->edata_bytes = 0;
-  CHECK_CUDA(cudaMalloc(&p->edata, std::max<size_t>(need, 16)), "element buffer");
+  CHECK_CUDA(device_alloc(&p->edata, need), "element buffer");
   p->edata_bytes = need;
   p->device_bytes += static_cast<int64_t>(need);
   return CXG_OK;

@@ -166,18 +166,18 @@ __constant__ double c_hg2[4][8] = {
     {-1, 1, -1, 1, 1, -1, 1, -1},
 };
 
-int sm_count() {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 // Persistent grid: blocks_per_sm (0 = as many as are resident) blocks on every SM,
 // capped by the work available.
-int64_t persistent_grid(int64_t need, int resident, int blocks_per_sm) {
+int64_t persistent_grid(int64_t need, int resident, int sms, int blocks_per_sm) {
   const int per_sm = blocks_per_sm > 0 ? std::min(blocks_per_sm, std::max(resident, 1)) : std::max(resident, 1);
-  return std::max<int64_t>(1, std::min<int64_t>(need, static_cast<int64_t>(per_sm) * sm_count()));
+  return std::max<int64_t>(1, std::min<int64_t>(need, static_cast<int64_t>(per_sm) * sms));
+}
+
+// Launches an element pass on a persistent grid (see launch_kernel).
+cudaError_t launch_persistent(const void* kern, size_t smem, int64_t need, int blocks_per_sm, cudaStream_t s, void** args) {
+  int per_sm = 0, sms = 0;
+  const cudaError_t e = kernel_shape(kern, kT1, smem, &per_sm, &sms);
+  return e != cudaSuccess ? e : launch_kernel(kern, persistent_grid(need, per_sm, sms, blocks_per_sm), kT1, smem, s, args);
 }
 
 // Slot k of a pass is one group (one element type, the concatenated models of that type)

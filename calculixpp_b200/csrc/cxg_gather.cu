@@ -33,6 +33,8 @@ constexpr unsigned kAll = 0xffffffffu;
 // even out (a grid of resident blocks striding over the nodes: C3D20 64^3 mixed 2885 us,
 // this way 2218; blocks of 8 warps 2330).
 constexpr int kWarps = 4;
+// Grids that are resident at once on a B200 let the next kernel on the stream start early.
+constexpr unsigned kOneWave = 148 * 6;
 // (Registers: 64 a thread where the blocks are FP32, 80 where they are FP64: 64 spill there
 // and lose, C3D8 128^3 2908 -> 3239 us; with FP32 they win, C3D20 64^3 2190 -> 2007 us.)
 
@@ -105,6 +107,13 @@ __device__ __forceinline__ void gather_node(const ElemArgs& A, const V2Args& V, 
   const NodeRec nd = load_node(A.node + a);
   const int K = nd.npair, L = nd.len_mask & 0xfffffff, ma = nd.len_mask >> 28, self = nd.diag;
   const bool full = L == 3 * K, plain = full && !V.accumulate;
+  const PairRec* list = A.pairs + nd.list0 + q;
+  PairRec rec{};
+  if (ma && nd.rounds) rec = load_pairs(list);
+  // (the records are the plan's own; blocks and outputs are other kernels' too, and are
+  // read with plain loads, since the element pass may still be writing when this starts)
+  wait_for_kernel_before();
+  if (gridDim.x <= kOneWave) let_next_kernel_start();
   double* const rows = A.vals + nd.base;
   // what prescribed columns move to the rhs: of row ki (own pair and later ones), of
   // row kj (earlier ones)
@@ -134,9 +143,6 @@ __device__ __forceinline__ void gather_node(const ElemArgs& A, const V2Args& V, 
   };
   if (ma) {
     int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
-    const PairRec* list = A.pairs + nd.list0 + q;
-    PairRec rec;
-    if (nd.rounds) rec = load_pairs(list);
     // the off-diagonal blocks' sums (DIAG): entry (ki, kj) of the blocks from the own
     // pair on, entry (kj, ki) of those before it
     double own = 0.0, before = 0.0;
@@ -149,7 +155,7 @@ __device__ __forceinline__ void gather_node(const ElemArgs& A, const V2Args& V, 
 #pragma unroll
       for (int i = 0; i < UN; ++i) {
         x[i] = R(0);
-        if (mine) x[i] = __ldg(ed + (SCALAR ? 1 : 9) * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks));
+        if (mine) x[i] = ed[(SCALAR ? 1 : 9) * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks)];
       }
       const bool turns = rec.flags >> 31;
       const unsigned ends = lane < 27 ? rec.flags : 0u;
@@ -232,6 +238,8 @@ __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& 
   NodeRec nd{};
   if (on) nd = load_node(A.node + a);
   const bool free = (nd.len_mask >> 28) & 1, full = (nd.len_mask & 0xfffffff) == nd.npair;
+  wait_for_kernel_before();
+  if (gridDim.x <= kOneWave) let_next_kernel_start();
   double rr = 0.0;
   if (free) {
     int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
@@ -242,7 +250,7 @@ __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& 
       const PairRec rec = load_pairs(list);
       double x[UN];
 #pragma unroll
-      for (int i = 0; i < UN; ++i) x[i] = __ldg(ed + rec.block[i]);
+      for (int i = 0; i < UN; ++i) x[i] = ed[rec.block[i]];
 #pragma unroll
       for (int i = 0; i < UN; ++i) {
         v += x[i];
@@ -293,7 +301,7 @@ __global__ void __launch_bounds__(256) force_kernel(ElemArgs A, V2Args V) {
         s -= V.ring_base * V.npe;
         if (s >= V.ring * V.npe) s -= V.ring * V.npe;
       }
-      f += __ldg(V.fdata + 3 * s + d);
+      f += V.fdata[3 * s + d];
     }
     A.f_int[3 * a + d] = (V.accumulate ? A.f_int[3 * a + d] : 0.0) + f;
   }
@@ -318,8 +326,10 @@ cudaError_t launch_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, c
   if (count <= 0) return cudaSuccess;
   const int64_t block_nodes = static_cast<int64_t>(warps) * (KIND == GATHER_ONE_DOF ? 10 : 1);
   const int64_t grid = (count + block_nodes - 1) / block_nodes;
-  kern<<<static_cast<unsigned>(grid), warps * 32, 0, s>>>(a, v);
-  return cudaGetLastError();
+  ElemArgs A = a;
+  V2Args V = v;
+  void* args[] = {&A, &V};
+  return launch_kernel(reinterpret_cast<const void*>(kern), grid, warps * 32, 0, s, args);
 }
 
 }  // namespace
@@ -378,8 +388,8 @@ cudaError_t launch_batch_t(const BatchSlotIn* in, int n, cudaStream_t s) {
   }
   if (blk <= 0) return cudaSuccess;
   P.n = n;
-  kern<<<static_cast<unsigned>(blk), warps * 32, 0, s>>>(P);
-  return cudaGetLastError();
+  void* args[] = {&P};
+  return launch_kernel(reinterpret_cast<const void*>(kern), blk, warps * 32, 0, s, args);
 }
 
 }  // namespace

@@ -310,6 +310,25 @@ cudaError_t pcg_solve(int32_t n, const int64_t* rp, const int32_t* ci, const dou
 // Element tables (constant memory) are uploaded once per device.
 cudaError_t ensure_tables();
 
+// Resident blocks per SM of a kernel and the SM count of the current device, asked of the
+// runtime once per thread, kernel and shape (cxg_launch.cu); sets the kernel's shared memory.
+cudaError_t kernel_shape(const void* kern, int threads, size_t smem, int* per_sm, int* sms);
+// Launches kern. Unless s is being captured, it may start while the kernel before it on s
+// drains (programmatic stream serialisation): kernels launched this way wait_for_kernel_before()
+// ahead of anything an earlier kernel may have written, or may still read.
+cudaError_t launch_kernel(const void* kern, int64_t grid, int threads, size_t smem, cudaStream_t s, void** args);
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
+// Device memory of plans (cxg_pool.cu): from a pool of the current device that keeps up to
+// 512 MB of what is freed. device_free expects that no work on the block is pending, and
+// device_trim, after a group of frees, returns what is above that to the device.
+cudaError_t device_alloc(void** out, size_t bytes);
+void device_free(void* ptr);
+void device_trim();
+
 // Pattern construction (cxg_pattern.cu).
 struct PatternOut {
   void* mem[2] = {nullptr, nullptr};  // the device blocks that hold all of these

@@ -382,9 +382,9 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
   unsigned sweep_grid = 0;
   size_t sweep_smem = 0;
   {
-    CXG_TRY(cudaMalloc(&out->mem[0], keep.bytes));
+    CXG_TRY(device_alloc(&out->mem[0], keep.bytes));
     out->device_bytes += static_cast<int64_t>(keep.bytes);
-    CXG_TRY(cudaMalloc(&scratch, tmp.bytes));
+    CXG_TRY(device_alloc(&scratch, tmp.bytes));
     out->node_mask = part<uint8_t>(out->mem[0], k_mask);
     out->node = part<NodeRec>(out->mem[0], k_node);
     out->row_ptr = part<int64_t>(out->mem[0], k_row);
@@ -438,7 +438,7 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
     if (cap > 2048) {
       sweep_grid = std::min(sweep_grid, 256u);
       sweep_smem = 0;
-      CXG_TRY(cudaMalloc(&big, sizeof(int32_t) * 3 * static_cast<size_t>(cap) * kWarps * sweep_grid));
+      CXG_TRY(device_alloc(&big, sizeof(int32_t) * 3 * static_cast<size_t>(cap) * kWarps * sweep_grid));
     } else {
       CXG_TRY(cudaFuncSetAttribute(count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sweep_smem)));
       CXG_TRY(cudaFuncSetAttribute(write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sweep_smem)));
@@ -473,7 +473,7 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
     const size_t r_col = rest.add<int32_t>(static_cast<size_t>(out->nnz)),
                  r_pairs = rest.add<PairRec>(static_cast<size_t>(last[2] + len[2])), r_bn = rest.add<int32_t>(nbnd),
                  r_bc = rest.add<int32_t>(nbnd);
-    CXG_TRY(cudaMalloc(&out->mem[1], rest.bytes));
+    CXG_TRY(device_alloc(&out->mem[1], rest.bytes));
     out->device_bytes += static_cast<int64_t>(rest.bytes);
     out->col_idx = part<int32_t>(out->mem[1], r_col);
     out->pairs = part<PairRec>(out->mem[1], r_pairs);
@@ -488,8 +488,9 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
   }
 
 done:
-  cudaFree(big);
-  cudaFree(scratch);
+  cudaStreamSynchronize(s);  // (an error may have left work on the scratch)
+  device_free(big);
+  device_free(scratch);
   return rc;
 }
 

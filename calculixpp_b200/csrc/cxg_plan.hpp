@@ -57,6 +57,22 @@ struct MpcPlan {
 };
 }  // namespace cxg
 
+// Node-pair tile of the mixed-precision linear element pass when none is asked for, by what
+// measured fastest on a B200 (us, tiles 2x4 / 2x2 / 4x4): C3D15 65,536 elements 205 / 188 /
+// 150, C3D10 82,944 117 / 90 / 103, C3D20R 46,656 178 / 164 / 179, C3D8 262,144 212 / 196 /
+// 236, C3D6 221,184 112 / 107 / 123; C3D20 46,656 289 / 343 / 325, C3D8R 211 / 223 / 291 and
+// C3D4 59 / 67 / 66 keep 2x4.
+inline int default_tile(int type) {
+  switch (type) {
+    case cxg::C3D15: return 2;
+    case cxg::C3D10:
+    case cxg::C3D20R:
+    case cxg::C3D8:
+    case cxg::C3D6: return 1;
+    default: return 0;
+  }
+}
+
 inline cxg::LaunchCfg tangent_default() {
   cxg::LaunchCfg c;
   c.tile = 1;

@@ -289,13 +289,11 @@ cudaError_t launch_elem(const ElemArgs& a, double* gp_stress, double* emean, dou
   auto kern = field_elem_kernel<ET, KIND>;
   constexpr size_t smem = field_smem_bytes<ET, KIND>();
   static_assert(smem <= 227 * 1024, "field pass shared memory");
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (err != cudaSuccess) return err;
-  int per_sm = 0;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kT1, smem);
+  int per_sm = 0, sms = 0;
+  const cudaError_t err = kernel_shape(reinterpret_cast<const void*>(kern), kT1, smem, &per_sm, &sms);
   if (err != cudaSuccess) return err;
   constexpr int per_block = kW1 * FieldSmem<ET, KIND>::EPB;
-  const int64_t grid = persistent_grid((a.n_elems + per_block - 1) / per_block, per_sm, 0);
+  const int64_t grid = persistent_grid((a.n_elems + per_block - 1) / per_block, per_sm, sms, 0);
   kern<<<static_cast<unsigned>(grid), kT1, smem, s>>>(a, gp_stress, emean, felem, dc_dE);
   return cudaGetLastError();
 }
@@ -306,7 +304,7 @@ cudaError_t launch_nodes(const ElemArgs& a, const int64_t* inc_ptr, const int32_
                          cudaStream_t s) {
   const int first = emean && (strain || stress) ? 0 : 12;
   const int64_t count = (15 - first) * a.n_nodes;
-  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((count + 255) / 256, 8 * static_cast<int64_t>(sm_count())));
+  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((count + 255) / 256, 148 * 8));
   field_node_kernel<ET><<<static_cast<unsigned>(grid), 256, 0, s>>>(a, inc_ptr, inc_code, emean, felem, f_ext, strain,
                                                                    stress, reaction, first);
   return cudaGetLastError();
