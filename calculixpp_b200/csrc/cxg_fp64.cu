@@ -32,6 +32,16 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
+// The transposed 8x8 result: v holds entries (row, 2 col), (row, 2 col + 1) of it on lane
+// (row, col), and then those of its transpose. 2x2 parts first, then the parts themselves.
+__device__ __forceinline__ void transposed(const double (&v)[2], double (&t)[2], int row, int col) {
+  const bool odd = row & 1;
+  const double got = __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[1], 4);
+  const int src = (2 * col + (row & 1)) * 4 + (row >> 1);
+  t[0] = __shfl_sync(0xffffffffu, odd ? got : v[0], src);
+  t[1] = __shfl_sync(0xffffffffu, odd ? v[1] : got, src);
+}
+
 template <int ET>
 struct DGeo {
   static constexpr int n = nodes_of(ET), nq = gauss_of(ET);
@@ -53,7 +63,10 @@ struct DGeo {
   static constexpr int kElem = blocks_padded(n) * 9;
   // Staged blocks: one element, leaving as one bulk copy, or one tile pair.
   static constexpr bool BULK = NTL == 1;
-  static constexpr int kStage = BULK ? kElem : 576;
+  static constexpr int kStage = BULK ? kElem : 578;
+  // (rows of 8 blocks, one value further from row 2 and two from row 6 on: a half warp's
+  // stores then lie in different banks; C3D20 536 -> 529 us)
+  static __host__ __device__ constexpr int stage_row(int r) { return r * 72 + (r + 2) / 4; }
 };
 
 template <int ET, bool TAN>
@@ -286,6 +299,17 @@ __device__ __forceinline__ void p1d_body(const ElemArgs& A, const V2Args& V, uns
           const double* gA = W.g + ei * ES + (8 * ta + row) * QS + col;
           const double* gB = W.g + ei * ES + (8 * tb + row) * QS + col;
           double L[3][3][2] = {};  // block entries (x, y) of pairs (a, b), (a, b + 1)
+          // A tile with itself: entry (y, x) of (a, b) is entry (x, y) of (b, a), so three of
+          // the nine products are transposes of others, 9 shuffles of doubles for 3 KS (an
+          // element with plastic points: 18 for 9 KS) products. C3D8 J2 128^3: 3258 -> 3087
+          // us; elastic elements of several tiles lost (C3D20 FP64 529 -> 539) and form all.
+          const bool self = G::NTL == 1, selfp = G::NTL == 1 || ta == tb;
+          auto mirror = [&](double (&m)[3][3][2]) {
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+#pragma unroll
+              for (int y = x + 1; y < 3; ++y) transposed(m[x][y], m[y][x], row, col);
+          };
           if (!pl) {
 #pragma unroll
             for (int ks = 0; ks < KS; ++ks) {
@@ -299,8 +323,10 @@ __device__ __forceinline__ void p1d_body(const ElemArgs& A, const V2Args& V, uns
 #pragma unroll
               for (int x = 0; x < 3; ++x)
 #pragma unroll
-                for (int y = 0; y < 3; ++y) dmma(L[x][y], a[x], b[y]);
+                for (int y = 0; y < 3; ++y)
+                  if (y >= x || !self) dmma(L[x][y], a[x], b[y]);
             }
+            if (self) mirror(L);
             const double lam = W.lam[ei], mu = W.mu[ei];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -333,10 +359,11 @@ __device__ __forceinline__ void p1d_body(const ElemArgs& A, const V2Args& V, uns
 #pragma unroll
               for (int x = 0; x < 3; ++x)
 #pragma unroll
-                for (int y = 0; y < 3; ++y) {
-                  dmma(L[x][y], sl * a[x], b[y]);
-                  dmma(M[x][y], sm * a[x], b[y]);
-                }
+                for (int y = 0; y < 3; ++y)
+                  if (y >= x || !selfp) {
+                    dmma(L[x][y], sl * a[x], b[y]);
+                    dmma(M[x][y], sm * a[x], b[y]);
+                  }
               // m = N g
               auto turned = [&](const double (&v)[3], double (&m)[3]) {
                 m[0] = fma(n0, v[0], fma(n3, v[1], mul(n4, v[2])));
@@ -349,7 +376,12 @@ __device__ __forceinline__ void p1d_body(const ElemArgs& A, const V2Args& V, uns
 #pragma unroll
               for (int x = 0; x < 3; ++x)
 #pragma unroll
-                for (int y = 0; y < 3; ++y) dmma(L[x][y], -sc * ma[x], mb[y]);
+                for (int y = 0; y < 3; ++y)
+                  if (y >= x || !selfp) dmma(L[x][y], -sc * ma[x], mb[y]);
+            }
+            if (selfp) {
+              mirror(L);
+              mirror(M);
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -374,7 +406,7 @@ __device__ __forceinline__ void p1d_body(const ElemArgs& A, const V2Args& V, uns
                 for (int x = 0; x < 3; ++x) L[x][x][h] = fma(hd, W.kappa[ei], L[x][x][h]);
               }
               const int sx = W.id[ei][a] > W.id[ei][b] ? 1 : 3, sy = 4 - sx;
-              double* d = W.stg + (G::BULK ? blk_index(n, a, b) : row * 8 + 2 * col + h) * 9;
+              double* d = W.stg + (G::BULK ? blk_index(n, a, b) * 9 : G::stage_row(row) + (2 * col + h) * 9);
 #pragma unroll
               for (int x = 0; x < 3; ++x)
 #pragma unroll
@@ -399,7 +431,7 @@ __device__ __forceinline__ void p1d_body(const ElemArgs& A, const V2Args& V, uns
 #pragma unroll
               for (int t = lane; t < 72; t += 32) {
                 const int b = 8 * tb + t / 9;
-                if (b < n && b >= ar) o[t] = W.stg[r * 72 + t];
+                if (b < n && b >= ar) o[t] = W.stg[G::stage_row(r) + t];
               }
             }
           }
