@@ -274,7 +274,7 @@ class Plan:
     def tune(self, step, tangent=False, reps=3):
         """Time `step()` (one assembly through this plan) with CUDA events for every tile
         and element-pass grid shape of the current precision, then for the row gather's
-        warps per block (8, 4, 2) at the kept element-pass shape, then for the
+        warps per block (4, 8, 2) at the kept element-pass shape, then for the
         element-buffer budget of the windowed assembly (one window, 40 % and 85 % of L2);
         keep the fastest and return it with its time in ms."""
 
@@ -304,7 +304,7 @@ class Plan:
                 ms = timed(tile, bps, 0)
                 if ms is not None and (best is None or ms < best[0]):
                     best = (ms, tile, bps, 0)
-        for warps in (4, 2):
+        for warps in (8, 2):
             ms = timed(best[1], best[2], warps)
             if ms is not None and ms < best[0]:
                 best = (ms, best[1], best[2], warps)
@@ -320,7 +320,7 @@ class Plan:
         self.set_ring_bytes(ring)
         self.set_launch_config(tangent, best[1], best[2], best[3])
         return {"tile": {0: "2x4", 1: "2x2", 2: "4x4"}[best[1]], "p1_blocks_per_sm": best[2],
-                "p2_warps": best[3] or 8, "ring_bytes": ring, "ms": ring_ms}
+                "p2_warps": best[3] or 4, "ring_bytes": ring, "ms": ring_ms}
 
     # -- assembly --------------------------------------------------------------------
     def assemble_linear(self, f_ext=None, vals=None, rhs=None, check=True):

@@ -235,9 +235,9 @@ WorkLease::WorkLease(cxg_plan* p, size_t bytes, cudaStream_t s) : p_(p), s_(s) {
     if (error == cudaSuccess) {
       p->work_bytes = bytes;
       p->device_bytes += static_cast<int64_t>(bytes);
-      p->work_stream = s;
     }
-  } else if (error == cudaSuccess && s != p->work_stream) {
+  } else if (error == cudaSuccess) {
+    // (also on the stream it was used on: another one may have been given that handle)
     error = cudaStreamWaitEvent(s, p->work_done, 0);
   }
   if (error == cudaSuccess) ptr = p->work;
@@ -250,7 +250,6 @@ WorkLease::~WorkLease() {
   }
   if (!ptr) return;
   cudaEventRecord(p_->work_done, s_);
-  p_->work_stream = s_;
 }
 
 int ensure_state(cxg_plan* p, cudaStream_t s) {

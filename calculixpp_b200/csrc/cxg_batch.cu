@@ -101,7 +101,7 @@ uint64_t cfg_hash(const cxg_batch* b) {
   for (const Group& g : b->groups)
     for (int pr = 0; pr < 2; ++pr) {
       const LaunchCfg& c = g.plan->cfg[pr];
-      for (int v : {c.tile, c.p1_blocks_per_sm, c.p2_warps, c.p2_blocks_per_sm}) h = (h ^ static_cast<uint64_t>(v + 7)) * 1099511628211ull;
+      for (int v : {c.tile, c.p1_blocks_per_sm, c.p2_warps}) h = (h ^ static_cast<uint64_t>(v + 7)) * 1099511628211ull;
       uint64_t w1 = 0, w2 = 0;
       std::memcpy(&w1, &g.fms1[pr], 8);
       std::memcpy(&w2, &g.fms2[pr], 8);
@@ -137,15 +137,11 @@ cudaError_t launch_group(cxg_batch* b, Group& g, double* vals, double* rhs, cons
   return launch_v2(p->type, MODE_LINEAR, b->precision, a, v, s, override_cfg ? *override_cfg : p->cfg[b->precision]);
 }
 
-// Pass-time estimates of a group when the tuner has not measured it: element pass ~
-// node pairs x (Gauss points + block stores), row gather ~ stored blocks.
+// Element-pass time of a group when the tuner has not measured it, in units that all groups
+// share: node pairs x (Gauss points + block stores).
 double p1_estimate(int t, int64_t ne) {
   const double n = nodes_of(t), nq = gauss_of(t);
   return static_cast<double>(ne) * n * n * (nq + 4.0);
-}
-double p2_estimate(int t, int64_t ne) {
-  const double n = nodes_of(t);
-  return static_cast<double>(ne) * n * (n + 1.0) / 2.0;
 }
 
 // Every group as one slot of the one-launch kernels. Linear mode when u is null, else
@@ -183,7 +179,6 @@ int fill_slots(cxg_batch* b, const double* u, double* vals, double* f_int, doubl
     in.cfg.tile = tan ? 1 : g.ftile[pr];
     in.cfg.p2_warps = b->fwarps[pr];
     in.p1_weight = tuned ? g.fms1[pr] : p1_estimate(g.type, p->n_elems);
-    in.p2_weight = tuned ? g.fms2[pr] : p2_estimate(g.type, p->n_elems);
     slots.push_back(in);
   }
   return CXG_OK;

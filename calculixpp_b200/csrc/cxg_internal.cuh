@@ -168,16 +168,14 @@ struct V2Args {
   const int64_t* win_e;
   const int64_t* win_n;
 };
-// Launch shape of the two passes. tile: element-pass node-pair tile (0 = 2x4, 1 = 2x2,
-// 2 = 4x4, the last in the linear pass with FP32 accumulators only);
-// *_blocks_per_sm: persistent grid per SM (0 = as many as are resident); p2_warps:
-// warps per row-gather block, at most 8 (0 = up to 8 as shared memory allows); passes: bit 0 the
-// element pass, bit 1 the row gather.
+// Launch shape of the two passes. tile: node-pair tile of the mixed-precision linear element
+// pass (0 = 2x4, 1 = 2x2, 2 = 4x4; the others have one shape); p1_blocks_per_sm: persistent
+// grid per SM of the element pass (0 = as many as are resident); p2_warps: warps per
+// row-gather block, at most 8 (0 = 4); passes: bit 0 the element pass, bit 1 the row gather.
 struct LaunchCfg {
   int tile = 0;
   int p1_blocks_per_sm = 0;
   int p2_warps = 0;
-  int p2_blocks_per_sm = 0;
   int passes = 3;
   // mixed-precision material-point pass: the J2 return in FP32 (j2_point_mixed) instead
   // of FP64
@@ -185,14 +183,14 @@ struct LaunchCfg {
 };
 // One element pass and one row gather for a whole batch of element-type groups: slot k
 // is group k's arguments (one window, mesh node order), its element type and launch
-// shape; the weights share the persistent grid of each pass between the slots.
+// shape; the weights share the element pass's persistent grid between the slots.
 constexpr int kMaxBatchSlots = 8;
 struct BatchSlotIn {
   ElemArgs a;
   V2Args v;
   int32_t type = 0;
   LaunchCfg cfg;
-  double p1_weight = 1.0, p2_weight = 1.0;
+  double p1_weight = 1.0;
 };
 // Blocks of a persistent grid of `total` blocks shared out in proportion to the slots'
 // weights, at least one and at most `need` per slot.

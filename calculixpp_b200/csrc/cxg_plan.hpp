@@ -136,7 +136,6 @@ struct cxg_plan {
   double* work = nullptr;
   size_t work_bytes = 0;
   cudaEvent_t work_done = nullptr;
-  cudaStream_t work_stream = nullptr;
 };
 
 

@@ -1,19 +1,22 @@
-// Assembly in two passes, with no atomics and every CSR value written exactly once.
+// The element pass in mixed precision, and the dispatch of both passes of an assembly:
+// P1 integrates the elements, P2 (the row gather, cxg_gather.cu) writes every CSR value
+// once, with no atomics. P1 in FP64 is in cxg_fp64.cu.
 //
-// P1 (element pass): each warp integrates EPW elements at once. Lanes first handle
-// (element, Gauss point) tasks: Jacobian, its inverse and the physical gradients in
-// FP64 (plus the J2 return in material-point mode, whose trial history is written
-// here, once per Gauss point). Then every lane owns a 2x4 tile of node pairs of one
-// element and accumulates the 8 corresponding 3x3 blocks of K_e in registers over the
-// Gauss points from float4/double4 gradient loads; elastic points use the Gram form
-// K_ab = lam G + mu (G^T + tr(G) I) with G = sum_q s_q g_a g_b^T, plastic elements the
-// full tangent sum_q s [lam* g_a g_b^T + mu* (g_b g_a^T + (g_a.g_b) I) - c m_a m_b^T]
-// (m = N g, N the return direction, formed in the tile loop from the gradients and the
-// stored N of the Gauss point). The upper blocks (a <= b) go to a per-element
-// buffer, FP32 in mixed precision, FP64 otherwise; the internal force goes beside them.
+// Each warp integrates EPW elements at once. Lanes first handle (element, Gauss point)
+// tasks: Jacobian, its inverse and the physical gradients in FP64 (plus the J2 return in
+// material-point mode, whose trial history is written here, once per Gauss point). Then
+// every lane owns a tile of node pairs of one element and accumulates their 3x3 blocks of
+// K_e in FP32 registers over the Gauss points from float4 gradient loads; elastic points
+// use the Gram form K_ab = lam G + mu (G^T + tr(G) I) with G = sum_q s_q g_a g_b^T,
+// plastic elements the full tangent sum_q s [lam* g_a g_b^T + mu* (g_b g_a^T +
+// (g_a.g_b) I) - c m_a m_b^T] (m = N g, N the return direction, formed in the tile loop
+// from the gradients and the stored N of the Gauss point). The upper blocks (a <= b) go to
+// a per-element buffer; the internal force goes beside them in FP64.
 //
-// P2 (row gather, cxg_gather.cu): one warp per node sums, pair by pair, the element
-// blocks of each of the node's CSR entries.
+// What bounds it: the shared-memory pipe (78 % busy on C3D20), since every tile reads the
+// Gauss points' gradients again. Staging the finished blocks and sending them as one bulk
+// copy per element took C3D20 64^3 from 1583 to 1525 us, and lets the gather read blocks
+// without padding. The rounding sequence of a block is the same for every tile shape.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,7 +28,6 @@
 namespace cxg {
 
 namespace {
-
 
 struct TileList {
   int count;
@@ -173,51 +175,34 @@ __device__ __forceinline__ int j2_point_mixed(const J2Mat& M, double lam, double
 
 // Shared-memory layout of per-(element, Gauss point) node vectors: node k lives in
 // slot(k) = k/2 for even k and npad/2 + k/2 for odd k, so the row nodes 2r + i of the
-// lanes' tiles occupy consecutive slots. FP32 vectors are float4 per slot; FP64 vectors
-// are split in two half planes of double2 (x,y | z,0) so consecutive slots are 16 bytes
-// apart. Either way one warp-wide vector load touches distinct banks. The plane block of
-// each (element, Gauss point) is followed by 16 bytes of padding: the blocks then start
-// 16 (mod 128) bytes apart, so the lanes of the Gauss-point phase, one block each,
-// store their vectors into 8 distinct 16-byte bank groups instead of one.
+// lanes' tiles occupy consecutive slots, float4 each: one warp-wide vector load touches
+// distinct banks. The plane block of each (element, Gauss point) is followed by 16 bytes of
+// padding: the blocks then start 16 (mod 128) bytes apart, so the lanes of the Gauss-point
+// phase, one block each, store their vectors into 8 distinct 16-byte bank groups.
 __host__ __device__ constexpr int node_slot(int k, int npad) { return (k & 1) ? npad / 2 + (k >> 1) : (k >> 1); }
 
 template <typename R, int NPAD>
 struct VecIdx {
+  static_assert(sizeof(R) == 4, "FP32 pass");
   // elements of one plane block (b = element*nq + q), padding included
-  static constexpr int kBlock = NPAD * 4 + (sizeof(R) == 4 ? 4 : 2);
+  static constexpr int kBlock = NPAD * 4 + 4;
   // flat index of component c of the vector in `slot` of plane block b
-  __device__ __forceinline__ static int at(int b, int slot, int c) {
-    if (sizeof(R) == 4) return b * kBlock + slot * 4 + c;
-    return b * kBlock + (c >> 1) * (NPAD * 2) + slot * 2 + (c & 1);
-  }
+  __device__ __forceinline__ static int at(int b, int slot, int c) { return b * kBlock + slot * 4 + c; }
 };
 
 // one vector store (x, y, z, 0) of a node vector
 template <typename R, int NPAD>
 __device__ __forceinline__ void st3(R* base, int b, int slot, double x, double y, double z) {
-  if constexpr (sizeof(R) == 4) {
-    *reinterpret_cast<float4*>(base + VecIdx<R, NPAD>::at(b, slot, 0)) =
-        make_float4(static_cast<float>(x), static_cast<float>(y), static_cast<float>(z), 0.f);
-  } else {
-    *reinterpret_cast<double2*>(base + VecIdx<R, NPAD>::at(b, slot, 0)) = make_double2(x, y);
-    *reinterpret_cast<double2*>(base + VecIdx<R, NPAD>::at(b, slot, 2)) = make_double2(z, 0.0);
-  }
+  *reinterpret_cast<float4*>(base + VecIdx<R, NPAD>::at(b, slot, 0)) =
+      make_float4(static_cast<float>(x), static_cast<float>(y), static_cast<float>(z), 0.f);
 }
 
 template <typename R, int NPAD>
 __device__ __forceinline__ void ld3(const R* base, int b, int slot, R& x, R& y, R& z) {
-  if (sizeof(R) == 4) {
-    const float4 v = *reinterpret_cast<const float4*>(base + VecIdx<R, NPAD>::at(b, slot, 0));
-    x = v.x;
-    y = v.y;
-    z = v.z;
-  } else {
-    const double2 v = *reinterpret_cast<const double2*>(base + VecIdx<R, NPAD>::at(b, slot, 0));
-    const double2 w = *reinterpret_cast<const double2*>(base + VecIdx<R, NPAD>::at(b, slot, 2));
-    x = v.x;
-    y = v.y;
-    z = w.x;
-  }
+  const float4 v = *reinterpret_cast<const float4*>(base + VecIdx<R, NPAD>::at(b, slot, 0));
+  x = v.x;
+  y = v.y;
+  z = v.z;
 }
 
 template <int ET, int MODE, typename R, int TILE>
@@ -260,17 +245,14 @@ constexpr size_t p1_smem_bytes() {
 
 // Resident blocks per SM the element pass asks the register allocator for: as many as
 // its shared memory allows, at most 3 (<= 170 registers per thread) for the tiles whose
-// accumulators fit that budget without spilling (2x2, and 2x4 in FP32), else 2 (no
-// limit below the 255-register ceiling). The mixed-precision material-point pass with
-// 2x2 tiles takes 4 (<= 128 registers): it spills 28 bytes per thread there and still
-// ran 10 % faster on the C3D8 J2 block, where the FP64 one lost 8 % to its spills.
+// accumulators fit that budget without spilling (2x2 and 2x4), else 2 (no limit below the
+// 255-register ceiling). The material-point pass takes 4 (<= 128 registers): it spills 28
+// bytes per thread there and still ran 10 % faster on the C3D8 J2 block.
 template <int ET, int MODE, typename R, int TILE>
 constexpr int p1_min_blocks() {
   constexpr size_t per_sm = 227 * 1024;
   constexpr int by_smem = static_cast<int>(per_sm / (p1_smem_bytes<ET, MODE, R, TILE>() + 1024));
-  constexpr int cap = (TILE == 1 && MODE == MODE_TANGENT && sizeof(R) == 4)   ? 4
-                      : (TILE == 1 || (TILE == 0 && sizeof(R) == 4)) ? 3
-                                                                     : 2;
+  constexpr int cap = MODE == MODE_TANGENT ? 4 : TILE <= 1 ? 3 : 2;
   return by_smem < 1 ? 1 : (by_smem > cap ? cap : by_smem);
 }
 
@@ -504,7 +486,7 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
               h = static_cast<R>(hd * W.kappa[ei]);
             }
             // FP32 diagonal blocks are not used: the gather forms them (GATHER_DIAG)
-            const bool drop = sizeof(R) == 4 && a == b;
+            const bool drop = a == b;
             R* d = stg + ei * WS::kElem + blk_index(n, a, b) * 9;
             // in mesh order of the two nodes: transposed when b precedes a
             const int na = W.id[ei][a], nb = W.id[ei][b], sx = na > nb ? 1 : 3, sy = 4 - sx;

@@ -167,11 +167,12 @@ CXG_API int cxg_plan_update_coords(cxg_plan* plan, const double* coords);
 /* Replace per-element Young's moduli [n_elems]. */
 CXG_API int cxg_plan_update_young(cxg_plan* plan, const double* young);
 /* Launch shape of the plan's two passes for the current precision; mode 0 = linear
- * assembly, 1 = material-point (tangent) assembly. tile: node-pair tile of the element
- * pass, 0 = 2x4 (default), 1 = 2x2, 2 = 4x4 (linear, mixed precision only);
- * p1_blocks_per_sm: persistent grid of the element pass (0 = all resident);
- * p2_warps: warps per row-gather block, 1 to 8 (0 = up to 8 as shared memory allows). Results
- * do not depend on the shape. */
+ * assembly, 1 = material-point (tangent) assembly. tile: node-pair tile of the
+ * mixed-precision linear element pass, 0 = 2x4, 1 = 2x2, 2 = 4x4 (linear, mixed precision
+ * only; the default follows the element family); the other passes have one shape, and take
+ * 0 and 1 without effect. p1_blocks_per_sm: persistent grid of the element pass (0 = all
+ * resident); p2_warps: warps per row-gather block, 1 to 8 (0 = 4). Results do not depend on
+ * the shape. */
 CXG_API int cxg_plan_set_launch_config(cxg_plan* plan, int32_t mode, int32_t tile, int32_t p1_blocks_per_sm,
                                        int32_t p2_warps);
 /* No counterpart in the reference. Mixed-precision material-point assembly: enable != 0
@@ -431,9 +432,9 @@ CXG_API int cxg_batch_set_precision(cxg_batch* batch, int32_t precision);
  * element pass and one row gather per element-type group, the groups as independent
  * branches of the graph form. CXG_BATCH_ONE_LAUNCH: one element pass and one row
  * gather for the whole batch (at most 8 groups, one window each), every group a slot
- * of the same persistent grid with a share of its blocks in proportion to the group's
- * pass time as cxg_batch_tune measures it (estimated from the element counts until
- * then). Its element pass takes 2x2 tiles, and 2x4 in mixed precision; the kernel
+ * of the element pass's persistent grid with a share of its blocks in proportion to the
+ * group's pass time as cxg_batch_tune measures it (estimated from the element counts until
+ * then). Its mixed-precision linear element pass takes 2x2 and 2x4 tiles; the kernel
  * holds the register count of its largest family. Results are the same bit for bit in
  * both modes. Applies to cxg_batch_assemble, cxg_batch_graph_launch,
  * cxg_batch_assemble_tangent and cxg_batch_tune; cxg_batch_group_config and
@@ -467,8 +468,8 @@ CXG_API int cxg_batch_commit(cxg_batch* batch, void* stream);
  * order, as cxg_state_get returns a plan's. */
 CXG_API int cxg_batch_get_state(const cxg_batch* batch, int32_t model, int32_t slot, double* out);
 /* Autotuner. For every group and the current precision it times each candidate launch
- * shape on the batch's own data with CUDA events: the element-pass node-pair tile
- * (2x4, 2x2 and, in mixed precision, 4x4), its persistent grid (blocks per SM) and
+ * shape on the batch's own data with CUDA events: the node-pair tile of the mixed-precision
+ * element pass (2x4, 2x2, 4x4), its persistent grid (blocks per SM) and
  * the row gather's warps per block. It keeps the fastest of each pass. vals and rhs
  * (device memory) serve as scratch and hold a complete assembly on return. Results are
  * looked up in and added to the JSON file cache_path (NULL: no cache), keyed by SM
