@@ -138,7 +138,9 @@ __device__ __forceinline__ void gather_node(const ElemArgs& A, const V2Args& V, 
                   __popc(mb & ((1 << j) - 1));
       *o = V.accumulate ? *o + v : v;
     } else {
-      const double c = v * A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p)) + j];
+      // (a zero value moves nothing, not even from an infinite entry, src/fem/assembly.cpp:95)
+      const double u = A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p)) + j];
+      const double c = u != 0.0 ? v * u : 0.0;
       if (p < self)
         rt -= c;
       else
@@ -263,10 +265,12 @@ __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& 
             o[p] = v;
           } else {
             const uint32_t at = static_cast<uint32_t>(__ldg(A.bnd_col + nd.bnd0 + p));
-            if (at >> 28)
+            if (at >> 28) {
               o[at & 0xfffffff] = v;
-            else
-              rr -= v * A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p))];
+            } else {
+              const double u = A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p))];
+              if (u != 0.0) rr -= v * u;
+            }
           }
           v = 0.0;
           ++p;
