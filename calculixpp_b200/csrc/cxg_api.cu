@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -1213,7 +1214,13 @@ int cxg_assemble_conduction(cxg_plan* p, const double* conductivity, const doubl
   if (!rc) rc = staged(p, 1, rhs, rb, false, s, &dr);
   if (!rc) rc = staged(p, 5, conductivity, sizeof(double) * static_cast<size_t>(p->n_elems), true, s, &dk);
   if (rc) return rc;
-  if (p->films.n_films > 0 || (flux && !on_device(flux))) {
+  // the gather reads the flux of one node while it writes the rhs of others
+  const auto apart = [](const void* x, size_t nx, const void* y, size_t ny) {
+    const auto a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y);
+    return a + nx <= b || b + ny <= a;
+  };
+  if (p->films.n_films > 0 ||
+      (flux && (!on_device(flux) || !apart(flux, 8 * N, dv, vb) || (dr && !apart(flux, 8 * N, dr, rb))))) {
     // nodal flux and film loads in a buffer of the plan (staging slot 2)
     if (p->stage_bytes[2] < 8 * N) {
       cudaFree(p->stage[2]);

@@ -2,7 +2,8 @@
 
 * a prescribed value of zero moves nothing to the rhs, whatever the stiffness entry
   (src/fem/assembly.cpp:95 skips it): one element with a modulus that is not a number leaves
-  the rhs exactly the load where all prescribed values are zero.
+  the rhs exactly the load where all prescribed values are zero;
+* a nodal flux and a rhs in the same memory.
 
 Bars: bit equality where both sides take the same steps, else 1e-12 relative Frobenius in
 FP64 (sums of at most a few hundred products whose error is cond(J) eps <= 2e2 x 1.1e-16)."""
@@ -39,3 +40,15 @@ def test_zero_prescribed_temperatures_move_nothing(cuda):
         vals, rhs = plan.assemble_conduction(k, q)
         assert not torch.isfinite(vals).all()
         assert np.array_equal(to_np(rhs), q[plan.t_dof_eq >= 0])
+
+
+def test_flux_in_the_memory_of_the_rhs(cuda):
+    mesh = box_model(mg.C3D8, 9, 8, 7).mesh
+    held = mg.face_nodes(mesh, 0, 0.0)
+    rng = np.random.default_rng(0)
+    k, flux = rng.uniform(10.0, 50.0, mesh.n_elems), rng.normal(size=mesh.n_nodes)
+    with ThermalPlan(mesh, held, rng.uniform(280.0, 320.0, held.size)) as plan:
+        vals, rhs = plan.assemble_conduction(k, flux)
+        both = torch.as_tensor(flux, device=cuda)
+        v, r = plan.assemble_conduction(k, both, rhs=both[:plan.n_free])
+        assert torch.equal(v, vals) and torch.equal(r, rhs)
