@@ -410,7 +410,15 @@ __device__ __forceinline__ void p1d_body(const ElemArgs& A, const V2Args& V, uns
                 for (int al = 0; al < 4; ++al) hd = fma(W.gam[ei][al * 8 + a], W.gam[ei][al * 8 + b], hd);
                 for (int x = 0; x < 3; ++x) L[x][x][h] = fma(hd, W.kappa[ei], L[x][x][h]);
               }
-              const int sx = W.id[ei][a] > W.id[ei][b] ? 1 : 3, sy = 4 - sx;
+              const int na = W.id[ei][a], nb = W.id[ei][b], sx = na > nb ? 1 : 3, sy = 4 - sx;
+              if (na == nb && a != b) {
+                // an element that names a node twice: the gather adds this block for (a, b) and
+                // for (b, a), K_ab + K_ab^T in all
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+#pragma unroll
+                  for (int y = x + 1; y < 3; ++y) L[x][y][h] = L[y][x][h] = 0.5 * (L[x][y][h] + L[y][x][h]);
+              }
               double* d = W.stg + (G::BULK ? blk_index(n, a, b) * 9 : G::stage_row(row) + (2 * col + h) * 9);
 #pragma unroll
               for (int x = 0; x < 3; ++x)

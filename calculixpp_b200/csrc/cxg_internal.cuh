@@ -89,7 +89,8 @@ static_assert(sizeof(PairRec) == 48, "PairRec is three 16-byte loads");
 // 3x3 blocks of an element in the element buffer: one per local node pair (a, b), a <= b,
 // 9 consecutive values at 9 * blk_index. The stored block is that of the two nodes in
 // ascending mesh order (K_ba where node b precedes node a), so all elements that share a
-// pair store it the same way round. An element's block count is padded so that every
+// pair store it the same way round; a node with itself, where an element names a node twice,
+// as the symmetric part, since (a, b) and (b, a) are the same pair then. An element's block count is padded so that every
 // element starts 16-byte aligned in both precisions, which bulk copies need (8-byte
 // aligned in FP32 for the families of 4 and 6 nodes, which copy with plain stores).
 __host__ __device__ constexpr int blk_index(int n, int a, int b) { return a * n - a * (a - 1) / 2 + (b - a); }

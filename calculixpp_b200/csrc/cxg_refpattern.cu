@@ -279,6 +279,7 @@ __global__ void __launch_bounds__(kRefWarps * 32) refmask_kernel(ElemArgs A, dou
     }
     __syncwarp();
     double* dst = out + e * (blocks_padded(n) * 9);
+    bool twice = false;  // some node of the element is named twice
     for (int t = lane; t < NB * 9; t += 32) {
       const int blk = t / 9, q9 = t % 9;
       int ka = 0, r = blk;
@@ -318,8 +319,24 @@ __global__ void __launch_bounds__(kRefWarps * 32) refmask_kernel(ElemArgs A, dou
       // blocks are stored in mesh order of their nodes (blk_index)
       const bool swap = A.conn[e * n + ka] > A.conn[e * n + kb];
       dst[blk * 9 + (swap ? 3 * (q9 % 3) + q9 / 3 : q9)] = K != 0.0 ? 1.0 : 0.0;
+      twice = twice || (ka != kb && A.conn[e * n + ka] == A.conn[e * n + kb]);
     }
     __syncwarp();
+    if (__any_sync(0xffffffffu, twice)) {
+      // the block of such a node with itself is gathered for (ka, kb) and, transposed, for (kb, ka)
+      for (int t = lane; t < NB * 3; t += 32) {
+        int ka = 0, r = t / 3;
+        while (r >= n - ka) {
+          r -= n - ka;
+          ++ka;
+        }
+        if (r == 0 || A.conn[e * n + ka] != A.conn[e * n + ka + r]) continue;
+        const int x = t % 3 == 2 ? 1 : 0, y = t % 3 == 0 ? 1 : 2;  // (0, 1), (0, 2), (1, 2)
+        double *up = dst + t / 3 * 9 + 3 * x + y, *low = dst + t / 3 * 9 + 3 * y + x;
+        *up = *low = *up + *low > 0.0 ? 1.0 : 0.0;
+      }
+      __syncwarp();
+    }
   }
 }
 

@@ -485,11 +485,11 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
               for (int al = 0; al < 4; ++al) hd = fma(W.gam[ei][al * 8 + a], W.gam[ei][al * 8 + b], hd);
               h = static_cast<R>(hd * W.kappa[ei]);
             }
-            // FP32 diagonal blocks are not used: the gather forms them (GATHER_DIAG)
-            const bool drop = a == b;
             R* d = stg + ei * WS::kElem + blk_index(n, a, b) * 9;
             // in mesh order of the two nodes: transposed when b precedes a
             const int na = W.id[ei][a], nb = W.id[ei][b], sx = na > nb ? 1 : 3, sy = 4 - sx;
+            // FP32 blocks of a mesh node with itself are not used: the gather forms them (GATHER_DIAG)
+            const bool drop = na == nb;
 #pragma unroll
             for (int x = 0; x < 3; ++x)
 #pragma unroll

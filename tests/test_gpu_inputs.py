@@ -3,17 +3,21 @@
 * a prescribed value of zero moves nothing to the rhs, whatever the stiffness entry
   (src/fem/assembly.cpp:95 skips it): one element with a modulus that is not a number leaves
   the rhs exactly the load where all prescribed values are zero;
-* a nodal flux and a rhs in the same memory.
+* a nodal flux and a rhs in the same memory;
+* elements that name a node two or three times: hexahedra collapsed to wedges, against the
+  oracle. In mixed precision 1e-5: FP32 blocks of about 2e2 x 6e-8.
 
 Bars: bit equality where both sides take the same steps, else 1e-12 relative Frobenius in
 FP64 (sums of at most a few hundred products whose error is cond(J) eps <= 2e2 x 1.1e-16)."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 import torch
 
-from calculixpp_b200 import Plan, ThermalPlan
+from calculixpp_b200 import Material, Model, Plan, ThermalPlan
 from calculixpp_b200 import meshgen as mg
-from tests.helpers import box_model, to_np
+from oracle.oracle import make_material
+from tests.helpers import ISO_TABLE, box_model, per_element_materials, rel_fro, to_np
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +56,52 @@ def test_flux_in_the_memory_of_the_rhs(cuda):
         both = torch.as_tensor(flux, device=cuda)
         v, r = plan.assemble_conduction(k, both, rhs=both[:plan.n_free])
         assert torch.equal(v, vals) and torch.equal(r, rhs)
+
+
+def collapsed(etype, jitter=0.05):
+    """Wedges written as hexahedra whose fourth edge has collapsed onto the third."""
+    quadratic = etype in (mg.C3D20, mg.C3D20R)
+    w = mg.box_mesh(mg.C3D15 if quadratic else mg.C3D6, 2, 2, 3, jitter=jitter, seed=1, straight_edges=True)
+    local = [0, 1, 2, 2, 3, 4, 5, 5] + ([6, 7, 2, 8, 9, 10, 5, 11, 12, 13, 14, 14] if quadratic else [])
+    m = mg.Mesh(w.coords, np.ascontiguousarray(w.conn[:, local]), etype)
+    m.young = np.random.default_rng(2).uniform(70e3, 210e3, m.n_elems)
+    m.poisson = np.full(m.n_elems, 0.3)
+    top = mg.face_nodes(m, 2, 1.0)
+    sn, sc, sv = mg.clamp_face_spc(m, 2, 0.0)
+    return Model(m, [Material(210000.0, 0.3)], None, (sn, sc, sv + 1e-3),
+                 (top, np.zeros(top.size, int), np.ones(top.size)))
+
+
+@pytest.mark.parametrize("precision,bar", [("fp64", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("jitter", [0.0, 0.05])
+@pytest.mark.parametrize("etype", [mg.C3D8, mg.C3D8R, mg.C3D20, mg.C3D20R])
+def test_elements_that_name_a_node_twice(cuda, port, etype, jitter, precision, bar):
+    model = collapsed(etype, jitter)
+    mats, em = per_element_materials(model)
+    dof_eq, pre, nf = model.dof_map()
+    f = model.external_load_vector()
+    rp, ci, v, rhs = port.assemble_linear(model.mesh, mats, em, dof_eq, pre, nf, f)
+    with Plan(model, precision) as plan:
+        vals, r = plan.assemble_linear(f)
+        A = sp.csr_matrix((to_np(vals), *(to_np(t) for t in reversed(plan.pattern()))), shape=(nf, nf))
+        O = sp.csr_matrix((v, ci, rp), shape=(nf, nf))
+        assert np.linalg.norm((A - O).data) <= bar * np.linalg.norm(v)
+        assert rel_fro(to_np(r), rhs) <= bar
+        plan.use_reference_pattern()
+        assert all(np.array_equal(to_np(a), b) for a, b in zip(plan.pattern(), (rp, ci)))
+
+
+def test_plastic_elements_that_name_a_node_twice(cuda, port):
+    model = collapsed(mg.C3D8)
+    model.mesh.young[:] = 210000.0
+    model.materials = [Material(210000.0, 0.3, ISO_TABLE)]
+    dof_eq, pre, nf = model.dof_map()
+    u = np.einsum("ij,nj->ni", np.random.default_rng(3).uniform(-0.01, 0.01, (3, 3)), model.mesh.coords).reshape(-1)
+    with Plan(model) as plan:
+        state = np.zeros((plan.n_gauss, 13))
+        mats = [make_material(210000.0, 0.3, ISO_TABLE, 0, 0.0)]
+        rp, ci, v, rhs, fi, _ = port.assemble_tangent(model.mesh, mats, None, dof_eq, pre, nf, u, state)
+        vals, f_int, r = plan.assemble_tangent(u)
+        assert (to_np(plan.state(committed=False))[:, 6] > 0).any()
+        assert rel_fro(to_np(vals), v) <= 1e-12
+        assert rel_fro(to_np(f_int), fi) <= 1e-12
