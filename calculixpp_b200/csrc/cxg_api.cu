@@ -12,6 +12,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <iterator>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -672,15 +673,8 @@ int cxg_plan_destroy(cxg_plan* p) {
   if (p->last_stream) cudaStreamSynchronize(p->last_stream);
   thermal::release(p);
   cudaFree(p->film_mem);
-  // (cudaFree would wait for all of the device's work; so does this, once)
-  cudaDeviceSynchronize();
-  int current = p->device;
-  cudaGetDevice(&current);
-  if (current != p->device) cudaSetDevice(p->device);
-  for (void* b : {p->mem, p->pat.mem[0], p->pat.mem[1], p->edata, static_cast<void*>(p->fdata), static_cast<void*>(p->work)})
-    device_free(b);
-  device_trim();
-  if (current != p->device) cudaSetDevice(current);
+  void* const pooled[] = {p->mem, p->pat.mem[0], p->pat.mem[1], p->edata, p->fdata, p->work};
+  device_free_all(p->device, pooled, static_cast<int>(std::size(pooled)));
   for (double* b : p->state) cudaFree(b);
   for (auto& row : p->sched)
     for (WinSched& w : row) cudaFree(w.node_order);

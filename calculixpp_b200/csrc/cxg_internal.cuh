@@ -322,11 +322,12 @@ __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepc
 #endif
 
 // Device memory of plans (cxg_pool.cu): from a pool of the current device that keeps up to
-// 512 MB of what is freed. device_free expects that no work on the block is pending, and
-// device_trim, after a group of frees, returns what is above that to the device.
+// 512 MB of what is freed. device_free expects that no work on the block is pending.
+// device_free_all waits for all work of `device` (as cudaFree would, once), whichever device
+// is current, frees its blocks and returns what is above the 512 MB to the device.
 cudaError_t device_alloc(void** out, size_t bytes);
 void device_free(void* ptr);
-void device_trim();
+void device_free_all(int device, void* const* blocks, int n);
 
 // Pattern construction (cxg_pattern.cu).
 struct PatternOut {

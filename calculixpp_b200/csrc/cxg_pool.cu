@@ -93,9 +93,15 @@ void device_free(void* ptr) {
   if (ptr && pool_of(&p) == cudaSuccess) cudaFreeAsync(ptr, p.stream);
 }
 
-void device_trim() {
+void device_free_all(int device, void* const* blocks, int n) {
+  int current = device;
+  cudaGetDevice(&current);
+  if (current != device) cudaSetDevice(device);
+  cudaDeviceSynchronize();
+  for (int i = 0; i < n; ++i) device_free(blocks[i]);
   Pool p;
   if (pool_of(&p) == cudaSuccess) cudaStreamSynchronize(p.stream);  // applies the pool's threshold
+  if (current != device) cudaSetDevice(current);
 }
 
 }  // namespace cxg

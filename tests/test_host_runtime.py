@@ -1,0 +1,56 @@
+"""The library's host-only runtime files against a stand-in for the CUDA runtime
+(tests/fake_cudart.cpp): which device is waited for before memory is freed. No GPU."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "calculixpp_b200", "csrc")
+MB = 1 << 20
+
+
+@pytest.fixture(scope="module")
+def built(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    include = next(p for p in (os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include"),) if os.path.isdir(p))
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-w", "-Wl,-Bsymbolic", "-I", include, "-x", "c++",
+                    os.path.join(HERE, "fake_cudart.cpp"), os.path.join(CSRC, "cxg_pool.cu"), "-o", out], check=True)
+    return out
+
+
+@pytest.fixture
+def fake(built, tmp_path):
+    """A copy of the library of its own: its pools and logs start empty."""
+    import shutil
+    lib = C.CDLL(shutil.copy(built, tmp_path / "libfake.so"))
+    lib.fake_log.restype = C.c_char_p
+    lib.t_alloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
+    lib.t_free.argtypes = [C.c_void_p]
+    lib.t_free_all.argtypes = [C.c_int, C.POINTER(C.c_void_p), C.c_int]
+    return lib
+
+
+def calls(lib):
+    got = lib.fake_log().decode().split()
+    lib.fake_clear()
+    return got
+
+
+def alloc(lib, nbytes):
+    p = C.c_void_p()
+    rc = lib.t_alloc(C.byref(p), nbytes)
+    return rc, p
+
+
+@pytest.mark.parametrize("current", [0, 1])
+def test_free_waits_for_the_device_of_the_blocks(fake, current):
+    fake.cudaSetDevice(1)
+    blocks = [alloc(fake, n * MB) for n in (10, 300)]
+    assert all(rc == 0 for rc, _ in blocks)
+    fake.cudaSetDevice(current)
+    calls(fake)
+    fake.t_free_all(1, (C.c_void_p * 3)(*[p for _, p in blocks], None), 3)
+    back = ["set@0"] if current == 0 else []
+    assert calls(fake) == (["set@1"] if back else []) + ["wait@1", "give@1", "free@1"] + back
