@@ -1214,7 +1214,7 @@ int cxg_assemble_conduction(cxg_plan* p, const double* conductivity, const doubl
     return a + nx <= b || b + ny <= a;
   };
   if (p->films.n_films > 0 ||
-      (flux && (!on_device(flux) || !apart(flux, 8 * N, dv, vb) || (dr && !apart(flux, 8 * N, dr, rb))))) {
+      (flux && (!kernel_reads(p->device, flux) || !apart(flux, 8 * N, dv, vb) || (dr && !apart(flux, 8 * N, dr, rb))))) {
     // nodal flux and film loads in a buffer of the plan (staging slot 2)
     if (p->stage_bytes[2] < 8 * N) {
       cudaFree(p->stage[2]);
@@ -1312,7 +1312,7 @@ int cxg_state_get(const cxg_plan* cp, int32_t slot, double* out) {
   int rc = ensure_state(p, nullptr);
   if (rc) return rc;
   CHECK_CUDA(cudaStreamSynchronize(p->last_stream), "synchronize");
-  if (on_device(out)) {
+  if (kernel_reads(p->device, out)) {
     // straight into the caller's buffer: allocating and freeing a copy of the history took
     // longer than reading it
     CHECK_CUDA(launch_state_transpose(p->state[slot], out, p->n_gauss, false, nullptr), "state read");
@@ -1334,7 +1334,7 @@ int cxg_state_set(cxg_plan* p, int32_t slot, const double* in) {
   int rc = ensure_state(p, nullptr);
   if (rc) return rc;
   CHECK_CUDA(cudaStreamSynchronize(p->last_stream), "synchronize");
-  if (on_device(in)) {
+  if (kernel_reads(p->device, in)) {
     CHECK_CUDA(launch_state_transpose(in, p->state[slot], p->n_gauss, true, nullptr), "state write");
     CHECK_CUDA(cudaDeviceSynchronize(), "state write");
     p->back_stress_zero = false;  // the caller may have set a back stress

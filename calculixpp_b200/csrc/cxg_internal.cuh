@@ -328,6 +328,9 @@ __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepc
 cudaError_t device_alloc(void** out, size_t bytes);
 void device_free(void* ptr);
 void device_free_all(int device, void* const* blocks, int n);
+// Whether a kernel on `device` can take the caller's doubles at ptr where they are: managed, or
+// in that device's own memory, and aligned. Anything else cudaMemcpy takes is copied first.
+bool kernel_reads(int device, const void* ptr);
 
 // Pattern construction (cxg_pattern.cu).
 struct PatternOut {

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <mutex>
 #include <unordered_set>
 
@@ -91,6 +92,16 @@ void device_free(void* ptr) {
   }
   Pool p;
   if (ptr && pool_of(&p) == cudaSuccess) cudaFreeAsync(ptr, p.stream);
+}
+
+bool kernel_reads(int device, const void* ptr) {
+  cudaPointerAttributes at;
+  if (!ptr || reinterpret_cast<uintptr_t>(ptr) % sizeof(double) != 0) return false;
+  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == device);
 }
 
 void device_free_all(int device, void* const* blocks, int n) {

@@ -13,6 +13,7 @@ namespace cxg {
 cudaError_t device_alloc(void** out, size_t bytes);
 void device_free(void* ptr);
 void device_free_all(int device, void* const* blocks, int n);
+bool kernel_reads(int device, const void* ptr);
 }  // namespace cxg
 
 namespace {
@@ -80,6 +81,14 @@ cudaError_t cudaFreeAsync(void* p, cudaStream_t s) {
   g_blocks.erase(p);
   return cudaSuccess;
 }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* at, const void* p) {
+  auto b = g_blocks.upper_bound(const_cast<void*>(p));
+  *at = {};
+  if (b == g_blocks.begin() || static_cast<const char*>(p) >= static_cast<char*>((--b)->first) + 16) return cudaErrorInvalidValue;
+  at->type = cudaMemoryTypeDevice;
+  at->device = b->second.device;
+  return cudaSuccess;
+}
 
 // ---- what the tests call
 const char* fake_log() { return g_log.c_str(); }
@@ -87,5 +96,6 @@ void fake_clear() { g_log.clear(); }
 int t_alloc(void** p, size_t n) { return cxg::device_alloc(p, n); }
 void t_free(void* p) { cxg::device_free(p); }
 void t_free_all(int device, void* const* p, int n) { cxg::device_free_all(device, p, n); }
+int t_kernel_reads(int device, const void* p) { return cxg::kernel_reads(device, p); }
 
 }  // extern "C"

@@ -4,6 +4,7 @@
   (src/fem/assembly.cpp:95 skips it): one element with a modulus that is not a number leaves
   the rhs exactly the load where all prescribed values are zero;
 * a nodal flux and a rhs in the same memory;
+* device buffers that start between two doubles, for the history and the nodal flux;
 * elements that name a node two or three times: hexahedra collapsed to wedges, against the
   oracle. In mixed precision 1e-5: FP32 blocks of about 2e2 x 6e-8.
 
@@ -14,7 +15,7 @@ import pytest
 import scipy.sparse as sp
 import torch
 
-from calculixpp_b200 import Material, Model, Plan, ThermalPlan
+from calculixpp_b200 import Material, Model, Plan, ThermalPlan, _lib
 from calculixpp_b200 import meshgen as mg
 from oracle.oracle import make_material
 from tests.helpers import ISO_TABLE, box_model, per_element_materials, rel_fro, to_np
@@ -105,3 +106,31 @@ def test_plastic_elements_that_name_a_node_twice(cuda, port):
         assert (to_np(plan.state(committed=False))[:, 6] > 0).any()
         assert rel_fro(to_np(vals), v) <= 1e-12
         assert rel_fro(to_np(f_int), fi) <= 1e-12
+
+
+def between_doubles(values):
+    """A device copy of the values four bytes off their alignment: (buffer, address)."""
+    raw = torch.zeros(8 * values.size + 8, dtype=torch.uint8, device="cuda")
+    raw[4:-4] = torch.as_tensor(np.ascontiguousarray(values).reshape(-1).view(np.uint8), device="cuda")
+    return raw, raw.data_ptr() + 4
+
+
+def test_buffers_between_two_doubles(cuda):
+    model = box_model(mg.C3D8, 2, 2, 2)
+    with Plan(model) as plan:
+        want = np.random.default_rng(0).normal(size=(plan.n_gauss, 13))
+        for slot in (0, 1):
+            raw, at = between_doubles(want)
+            _lib.check(plan.lib.cxg_state_set(plan.h, slot, at))
+            back, at = between_doubles(np.zeros_like(want))
+            _lib.check(plan.lib.cxg_state_get(plan.h, slot, at))
+            assert np.array_equal(to_np(back)[4:-4].view(np.float64).reshape(want.shape), want)
+    q = np.random.default_rng(1).normal(size=model.mesh.n_nodes)
+    k = torch.ones(model.mesh.n_elems, dtype=torch.float64, device=cuda)
+    with ThermalPlan(model.mesh, [0], [300.0]) as plan:
+        vals, rhs = plan.assemble_conduction(k, q)
+        raw, at = between_doubles(q)
+        v, r = torch.empty_like(vals), torch.empty_like(rhs)
+        _lib.check(plan.lib.cxg_assemble_conduction(plan.h, k.data_ptr(), at, v.data_ptr(), r.data_ptr(), None))
+        plan.check()
+        assert torch.equal(v, vals) and torch.equal(r, rhs)

@@ -1,5 +1,6 @@
 """The library's host-only runtime files against a stand-in for the CUDA runtime
-(tests/fake_cudart.cpp): which device is waited for before memory is freed. No GPU."""
+(tests/fake_cudart.cpp): which device is waited for before memory is freed, and which buffers of a
+caller a kernel may take in place. No GPU."""
 import ctypes as C
 import os
 import subprocess
@@ -28,6 +29,7 @@ def fake(built, tmp_path):
     lib.fake_log.restype = C.c_char_p
     lib.t_alloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
     lib.t_free.argtypes = [C.c_void_p]
+    lib.t_kernel_reads.argtypes = [C.c_int, C.c_void_p]
     lib.t_free_all.argtypes = [C.c_int, C.POINTER(C.c_void_p), C.c_int]
     return lib
 
@@ -54,3 +56,13 @@ def test_free_waits_for_the_device_of_the_blocks(fake, current):
     fake.t_free_all(1, (C.c_void_p * 3)(*[p for _, p in blocks], None), 3)
     back = ["set@0"] if current == 0 else []
     assert calls(fake) == (["set@1"] if back else []) + ["wait@1", "give@1", "free@1"] + back
+
+
+def test_only_aligned_memory_of_the_device_is_read_in_place(fake):
+    fake.cudaSetDevice(1)
+    _, p = alloc(fake, MB)
+    assert fake.t_kernel_reads(1, p)
+    assert not fake.t_kernel_reads(0, p)             # another device's memory
+    assert not fake.t_kernel_reads(1, p.value + 4)   # not a place for doubles
+    assert not fake.t_kernel_reads(1, None)
+    assert not fake.t_kernel_reads(1, C.cast(C.create_string_buffer(64), C.c_void_p))  # host memory
