@@ -312,6 +312,8 @@ cudaError_t ensure_tables();
 // Resident blocks per SM of a kernel and the SM count of the current device, asked of the
 // runtime once per thread, kernel and shape (cxg_launch.cu); sets the kernel's shared memory.
 cudaError_t kernel_shape(const void* kern, int threads, size_t smem, int* per_sm, int* sms);
+// Lets kern be launched with that much dynamic shared memory on the current device.
+cudaError_t allow_smem(const void* kern, size_t smem);
 // Launches kern. Unless s is being captured, it may start while the kernel before it on s
 // drains (programmatic stream serialisation): kernels launched this way wait_for_kernel_before()
 // ahead of anything an earlier kernel may have written, or may still read.

@@ -5,6 +5,7 @@
 // start-up followed the first one's end.
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <unordered_map>
 
 #include "cxg_internal.cuh"
@@ -32,11 +33,32 @@ struct Shape {
 };
 thread_local std::unordered_map<Key, Shape, Hash> g_shapes;
 
-cudaError_t allow_smem(const void* kern, size_t smem) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-}
+struct Limit {
+  const void* kern;
+  int device;
+  bool operator==(const Limit& o) const { return kern == o.kern && device == o.device; }
+};
+struct LimitHash {
+  size_t operator()(const Limit& k) const { return reinterpret_cast<size_t>(k.kern) ^ static_cast<size_t>(k.device) << 1; }
+};
+std::mutex g_limits_mu;
+std::unordered_map<Limit, size_t, LimitHash> g_limits;
 
 }  // namespace
+
+// The limit belongs to the kernel, not to a launch or a thread: lowered for one launch it would
+// fail another thread's, or a later one whose shape is already known. So it only ever rises.
+cudaError_t allow_smem(const void* kern, size_t smem) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(g_limits_mu);
+  size_t& limit = g_limits[Limit{kern, dev}];
+  if (smem <= limit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (e == cudaSuccess) limit = smem;
+  return e;
+}
 
 cudaError_t kernel_shape(const void* kern, int threads, size_t smem, int* per_sm, int* sms) {
   int dev = 0;
@@ -73,14 +95,7 @@ cudaError_t launch_kernel(const void* kern, int64_t grid, int threads, size_t sm
   cfg.stream = s;
   cfg.attrs = &at;
   cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
-  e = cudaLaunchKernelExC(&cfg, kern, args);
-  if (e == cudaErrorInvalidValue && smem > 0) {
-    // the shared-memory limit set when the shape was asked for is gone (a device reset)
-    cudaGetLastError();
-    g_shapes.clear();
-    if ((e = allow_smem(kern, smem)) == cudaSuccess) e = cudaLaunchKernelExC(&cfg, kern, args);
-  }
-  return e;
+  return cudaLaunchKernelExC(&cfg, kern, args);
 }
 
 }  // namespace cxg

@@ -445,8 +445,8 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
       sweep_smem = 0;
       CXG_TRY(device_alloc(&big, sizeof(Cand) * static_cast<size_t>(cap) * kWarps * sweep_grid));
     } else {
-      CXG_TRY(cudaFuncSetAttribute(count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sweep_smem)));
-      CXG_TRY(cudaFuncSetAttribute(write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sweep_smem)));
+      CXG_TRY(allow_smem(reinterpret_cast<const void*>(count_kernel), sweep_smem));
+      CXG_TRY(allow_smem(reinterpret_cast<const void*>(write_kernel), sweep_smem));
     }
     S = Sweep{d_conn, out->inc_ptr, out->inc_code, npe, blocks_padded(npe)};
     int64_t *lens[3], *offs[3];

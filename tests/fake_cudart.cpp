@@ -14,6 +14,8 @@ cudaError_t device_alloc(void** out, size_t bytes);
 void device_free(void* ptr);
 void device_free_all(int device, void* const* blocks, int n);
 bool kernel_reads(int device, const void* ptr);
+cudaError_t kernel_shape(const void* kern, int threads, size_t smem, int* per_sm, int* sms);
+cudaError_t launch_kernel(const void* kern, int64_t grid, int threads, size_t smem, cudaStream_t s, void** args);
 }  // namespace cxg
 
 namespace {
@@ -28,6 +30,7 @@ struct Block {
 int g_device = 0;
 size_t g_used[2] = {0, 0}, g_idle[2] = {0, 0};  // in use, and kept by the device's pool
 std::map<void*, Block> g_blocks;
+std::map<std::pair<const void*, int>, int> g_limit;
 std::string g_log;
 
 void note(const std::string& s) { g_log += s + "@" + std::to_string(g_device) + " "; }
@@ -89,6 +92,18 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* at, const void* p) {
   at->device = b->second.device;
   return cudaSuccess;
 }
+cudaError_t cudaFuncSetAttribute(const void* kern, cudaFuncAttribute, int n) {
+  note("limit" + std::to_string(n));
+  g_limit[{kern, g_device}] = n;
+  return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t) { return *n = 1, cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 148, cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) { return *s = cudaStreamCaptureStatusNone, cudaSuccess; }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* kern, void**) {
+  if (c->dynamicSmemBytes <= static_cast<size_t>(g_limit[{kern, g_device}])) return note("launch"), cudaSuccess;
+  return note("refused"), cudaErrorInvalidValue;
+}
 
 // ---- what the tests call
 const char* fake_log() { return g_log.c_str(); }
@@ -97,5 +112,10 @@ int t_alloc(void** p, size_t n) { return cxg::device_alloc(p, n); }
 void t_free(void* p) { cxg::device_free(p); }
 void t_free_all(int device, void* const* p, int n) { cxg::device_free_all(device, p, n); }
 int t_kernel_reads(int device, const void* p) { return cxg::kernel_reads(device, p); }
+int t_shape(const void* kern, size_t smem) {
+  int per_sm, sms;
+  return cxg::kernel_shape(kern, 128, smem, &per_sm, &sms);
+}
+int t_launch(const void* kern, size_t smem) { return cxg::launch_kernel(kern, 1, 128, smem, nullptr, nullptr); }
 
 }  // extern "C"

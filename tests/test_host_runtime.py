@@ -1,6 +1,6 @@
 """The library's host-only runtime files against a stand-in for the CUDA runtime
-(tests/fake_cudart.cpp): which device is waited for before memory is freed, and which buffers of a
-caller a kernel may take in place. No GPU."""
+(tests/fake_cudart.cpp): which device is waited for before memory is freed, which buffers of a
+caller a kernel may take in place, and that a kernel's shared-memory limit never falls. No GPU."""
 import ctypes as C
 import os
 import subprocess
@@ -17,7 +17,7 @@ def built(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
     include = next(p for p in (os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include"),) if os.path.isdir(p))
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-w", "-Wl,-Bsymbolic", "-I", include, "-x", "c++",
-                    os.path.join(HERE, "fake_cudart.cpp"), os.path.join(CSRC, "cxg_pool.cu"), "-o", out], check=True)
+                    os.path.join(HERE, "fake_cudart.cpp"), os.path.join(CSRC, "cxg_pool.cu"), os.path.join(CSRC, "cxg_launch.cu"), "-o", out], check=True)
     return out
 
 
@@ -29,6 +29,8 @@ def fake(built, tmp_path):
     lib.fake_log.restype = C.c_char_p
     lib.t_alloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
     lib.t_free.argtypes = [C.c_void_p]
+    for f in (lib.t_shape, lib.t_launch):
+        f.argtypes = [C.c_void_p, C.c_size_t]
     lib.t_kernel_reads.argtypes = [C.c_int, C.c_void_p]
     lib.t_free_all.argtypes = [C.c_int, C.POINTER(C.c_void_p), C.c_int]
     return lib
@@ -66,3 +68,22 @@ def test_only_aligned_memory_of_the_device_is_read_in_place(fake):
     assert not fake.t_kernel_reads(1, p.value + 4)   # not a place for doubles
     assert not fake.t_kernel_reads(1, None)
     assert not fake.t_kernel_reads(1, C.cast(C.create_string_buffer(64), C.c_void_p))  # host memory
+
+
+def test_shared_memory_limit_never_falls(fake):
+    """Shapes of one kernel known in any order, and on another thread: every launch goes at once."""
+    import threading
+    kern = 0x1000
+    for smem in (60000, 20000, 100000):
+        assert fake.t_shape(kern, smem) == 0
+    other = threading.Thread(target=fake.t_shape, args=(kern, 8192))
+    other.start()
+    other.join()
+    assert fake.t_shape(kern, 60000) == 0
+    assert calls(fake) == ["limit60000@0", "limit100000@0"]
+    for smem in (60000, 100000, 8192):
+        assert fake.t_launch(kern, smem) == 0
+    assert calls(fake) == ["launch@0"] * 3
+    fake.cudaSetDevice(1)  # a limit of its own on every device
+    assert fake.t_shape(kern, 20000) == 0 and fake.t_launch(kern, 20000) == 0
+    assert calls(fake) == ["set@1", "limit20000@1", "launch@1"]
