@@ -61,9 +61,24 @@ namespace {
 template <typename T>
 cudaError_t alloc_copy(T** dst, const T* src, size_t count, cudaStream_t s, int64_t* bytes) {
   *bytes += static_cast<int64_t>(count * sizeof(T));
-  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(dst), std::max<size_t>(count, 1) * sizeof(T));
+  cudaError_t e = device_malloc(dst, std::max<size_t>(count, 1) * sizeof(T));
   if (e != cudaSuccess || !src || count == 0) return e;
   return cudaMemcpyAsync(*dst, src, count * sizeof(T), cudaMemcpyDefault, s);
+}
+
+// alloc(), and where it finds no memory once more without the plan's idle scratch.
+template <class F>
+cudaError_t or_drop_work(cxg_plan* p, F alloc) {
+  const cudaError_t e = alloc();
+  const std::unique_lock<std::mutex> lock(p->work_mu, std::try_to_lock);
+  if (e != cudaErrorMemoryAllocation || !lock.owns_lock() || !p->work) return e;
+  cudaGetLastError();
+  void* const work[] = {p->work};
+  device_free_all(p->device, work, 1);
+  p->device_bytes -= static_cast<int64_t>(p->work_bytes);
+  p->work = nullptr;
+  p->work_bytes = 0;
+  return alloc();
 }
 
 // Device view of a caller buffer: the pointer itself when it is device memory, else a
@@ -82,7 +97,7 @@ int staged(cxg_plan* p, int slot, const void* ptr, size_t bytes, bool upload, cu
     cudaFree(p->stage[slot]);
     p->stage[slot] = nullptr;
     p->stage_bytes[slot] = 0;
-    CHECK_CUDA(cudaMalloc(&p->stage[slot], bytes), "staging allocation");
+    CHECK_CUDA(or_drop_work(p, [&] { return device_malloc(&p->stage[slot], bytes); }), "staging allocation");
     p->stage_bytes[slot] = bytes;
   }
   if (upload) CHECK_CUDA(cudaMemcpyAsync(p->stage[slot], ptr, bytes, cudaMemcpyHostToDevice, s), "upload");
@@ -220,7 +235,7 @@ WorkLease::WorkLease(cxg_plan* p, size_t bytes, cudaStream_t s) : p_(p), s_(s) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if ((error = cudaStreamIsCapturing(s, &cap)) != cudaSuccess) return;
   if (cap != cudaStreamCaptureStatusNone) {
-    error = cudaMallocAsync(reinterpret_cast<void**>(&ptr), bytes, s);
+    error = device_malloc_async(reinterpret_cast<void**>(&ptr), bytes, s);
     return;
   }
   lock_ = std::unique_lock<std::mutex>(p->work_mu);
@@ -258,7 +273,7 @@ int ensure_state(cxg_plan* p, cudaStream_t s) {
   if (p->state[0]) return CXG_OK;
   const size_t bytes = sizeof(double) * kStateDoubles * static_cast<size_t>(std::max<int64_t>(p->n_gauss, 1));
   for (int i = 0; i < 2; ++i) {
-    CHECK_CUDA(cudaMalloc(&p->state[i], bytes), "state allocation");
+    CHECK_CUDA(or_drop_work(p, [&] { return device_malloc(&p->state[i], bytes); }), "state allocation");
     CHECK_CUDA(cudaMemsetAsync(p->state[i], 0, bytes, s), "state init");
   }
   p->device_bytes += 2 * static_cast<int64_t>(bytes);
@@ -300,7 +315,7 @@ int build_schedule(cxg_plan* p, size_t bpe, WinSched& w) {
   if (p->ring_bytes <= 0 || p->n_elems < 2 * min_w) return CXG_OK;
   if (p->node_first.empty()) {
     int32_t* d = nullptr;
-    CHECK_CUDA(cudaMalloc(&d, sizeof(int32_t) * 2 * static_cast<size_t>(p->n_nodes)), "node spans");
+    CHECK_CUDA(device_malloc(&d, sizeof(int32_t) * 2 * static_cast<size_t>(p->n_nodes)), "node spans");
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>((p->n_nodes + 255) / 256, 4096));
     node_span_kernel<<<grid, 256>>>(p->pat.inc_ptr, p->pat.inc_code, nodes_of(p->type), p->n_nodes, d,
                                     d + p->n_nodes);
@@ -331,7 +346,7 @@ int build_schedule(cxg_plan* p, size_t bpe, WinSched& w) {
   for (int64_t a = 0; a < p->n_nodes; ++a)
     order[static_cast<size_t>(pos[static_cast<size_t>(std::max(p->node_last[a], 0) / W)]++)] = static_cast<int32_t>(a);
   if (!w.node_order) {
-    CHECK_CUDA(cudaMalloc(&w.node_order, sizeof(int32_t) * static_cast<size_t>(p->n_nodes)), "node order");
+    CHECK_CUDA(device_malloc(&w.node_order, sizeof(int32_t) * static_cast<size_t>(p->n_nodes)), "node order");
     p->device_bytes += static_cast<int64_t>(sizeof(int32_t) * p->n_nodes);
   }
   CHECK_CUDA(cudaMemcpy(w.node_order, order.data(), sizeof(int32_t) * p->n_nodes, cudaMemcpyHostToDevice),
@@ -357,7 +372,7 @@ int ensure_v2(cxg_plan* p, bool tangent) {
     p->edata = nullptr;
     p->device_bytes -= static_cast<int64_t>(p->edata_bytes);
     p->edata_bytes = 0;
-    CHECK_CUDA(device_alloc(&p->edata, need), "element buffer");
+    CHECK_CUDA(or_drop_work(p, [&] { return device_alloc(&p->edata, need); }), "element buffer");
     p->edata_bytes = need;
     p->device_bytes += static_cast<int64_t>(need);
   }
@@ -368,7 +383,7 @@ int ensure_v2(cxg_plan* p, bool tangent) {
     p->fdata = nullptr;
     p->device_bytes -= static_cast<int64_t>(p->fdata_bytes);
     p->fdata_bytes = 0;
-    CHECK_CUDA(device_alloc(reinterpret_cast<void**>(&p->fdata), fb), "force buffer");
+    CHECK_CUDA(or_drop_work(p, [&] { return device_alloc(reinterpret_cast<void**>(&p->fdata), fb); }), "force buffer");
     p->fdata_bytes = fb;
     p->device_bytes += static_cast<int64_t>(fb);
   }
@@ -635,7 +650,7 @@ int cxg_plan_create_mpc(const cxg_mesh_desc* m, const cxg_dofmap_desc* d, const 
   if (rc) return rc;
   MpcPlan& mp = p->mpc;
   auto up = [&](void** dst, const void* src, size_t bytes) {
-    cudaError_t e = cudaMalloc(dst, std::max<size_t>(bytes, 16));
+    cudaError_t e = device_malloc(dst, std::max<size_t>(bytes, 16));
     if (e == cudaSuccess && bytes) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
     return e;
   };
@@ -644,10 +659,10 @@ int cxg_plan_create_mpc(const cxg_mesh_desc* m, const cxg_dofmap_desc* d, const 
   if (e == cudaSuccess) e = up(reinterpret_cast<void**>(&mp.term_eq), teq.data(), 4 * teq.size());
   if (e == cudaSuccess) e = up(reinterpret_cast<void**>(&mp.term_coeff), tco.data(), 8 * tco.size());
   if (e == cudaSuccess && any_c) e = up(reinterpret_cast<void**>(&mp.c_x), cx.data(), 8 * cx.size());
-  if (e == cudaSuccess && any_c) e = cudaMalloc(&mp.kc_x, 8 * static_cast<size_t>(std::max(nx, 1)));
-  if (e == cudaSuccess) e = cudaMalloc(&mp.vals_x, 8 * static_cast<size_t>(std::max<int64_t>(p->pat.nnz, 1)));
-  if (e == cudaSuccess) e = cudaMalloc(&mp.rhs_x, 8 * static_cast<size_t>(std::max(nx, 1)));
-  if (e == cudaSuccess) e = cudaMalloc(&mp.tmp_x, 8 * static_cast<size_t>(std::max(nx, 1)));
+  if (e == cudaSuccess && any_c) e = device_malloc(&mp.kc_x, 8 * static_cast<size_t>(std::max(nx, 1)));
+  if (e == cudaSuccess) e = device_malloc(&mp.vals_x, 8 * static_cast<size_t>(std::max<int64_t>(p->pat.nnz, 1)));
+  if (e == cudaSuccess) e = device_malloc(&mp.rhs_x, 8 * static_cast<size_t>(std::max(nx, 1)));
+  if (e == cudaSuccess) e = device_malloc(&mp.tmp_x, 8 * static_cast<size_t>(std::max(nx, 1)));
   cudaStream_t s = nullptr;
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
   if (e == cudaSuccess)
@@ -800,8 +815,8 @@ int cxg_plan_use_reference_pattern(cxg_plan* p, int32_t enable) {
   CHECK_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
   double *flags = nullptr, *counts = nullptr;
   RefPattern nr;
-  cudaError_t e = cudaMalloc(&flags, std::max<size_t>(v2_edata_bytes(p->type, p->n_elems, CXG_FP64), 16));
-  if (e == cudaSuccess) e = cudaMalloc(&counts, sizeof(double) * static_cast<size_t>(std::max<int64_t>(p->pat.nnz, 1)));
+  cudaError_t e = device_malloc(&flags, std::max<size_t>(v2_edata_bytes(p->type, p->n_elems, CXG_FP64), 16));
+  if (e == cudaSuccess) e = device_malloc(&counts, sizeof(double) * static_cast<size_t>(std::max<int64_t>(p->pat.nnz, 1)));
   ElemArgs a = base_args(p);
   // 1.0 / 0.0 per element-matrix entry: nonzero in the reference's arithmetic or not
   if (e == cudaSuccess) e = launch_refmask(p->type, a, flags, s);
@@ -817,7 +832,7 @@ int cxg_plan_use_reference_pattern(cxg_plan* p, int32_t enable) {
     e = compact_pattern(p->pat.row_ptr, p->pat.col_idx, p->n_free, p->pat.nnz, counts, &nr.row_ptr, &nr.col_idx,
                         &nr.src, &nr.nnz, s);
   if (e == cudaSuccess)
-    e = cudaMalloc(&nr.topo_vals, sizeof(double) * static_cast<size_t>(std::max<int64_t>(p->pat.nnz, 1)));
+    e = device_malloc(&nr.topo_vals, sizeof(double) * static_cast<size_t>(std::max<int64_t>(p->pat.nnz, 1)));
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   cudaFree(flags);
   cudaFree(counts);
@@ -891,11 +906,11 @@ int cxg_plan_set_thermal_strain(cxg_plan* p, const double* node_temp, const uint
   if (!elem_alpha || !elem_tref) return set_err(CXG_ERR_INVALID_ARGUMENT, "elem_alpha and elem_tref are required");
   if (p->thermal) return set_err(CXG_ERR_UNSUPPORTED, "thermal strain applies to displacement plans");
   const size_t N = static_cast<size_t>(std::max<int64_t>(p->n_nodes, 1)), E = static_cast<size_t>(std::max<int64_t>(p->n_elems, 1));
-  cudaError_t e = cudaMalloc(&p->th_temp, sizeof(double) * N);
-  if (e == cudaSuccess && node_applied) e = cudaMalloc(&p->th_applied, N);
-  if (e == cudaSuccess) e = cudaMalloc(&p->th_alpha, sizeof(double) * E);
-  if (e == cudaSuccess) e = cudaMalloc(&p->th_tref, sizeof(double) * E);
-  if (e == cudaSuccess) e = cudaMalloc(&p->th_load, sizeof(double) * 3 * N);
+  cudaError_t e = device_malloc(&p->th_temp, sizeof(double) * N);
+  if (e == cudaSuccess && node_applied) e = device_malloc(&p->th_applied, N);
+  if (e == cudaSuccess) e = device_malloc(&p->th_alpha, sizeof(double) * E);
+  if (e == cudaSuccess) e = device_malloc(&p->th_tref, sizeof(double) * E);
+  if (e == cudaSuccess) e = device_malloc(&p->th_load, sizeof(double) * 3 * N);
   const size_t nn = static_cast<size_t>(p->n_nodes), ne = static_cast<size_t>(p->n_elems);
   if (e == cudaSuccess && nn) e = cudaMemcpy(p->th_temp, node_temp, sizeof(double) * nn, cudaMemcpyDefault);
   if (e == cudaSuccess && nn && node_applied) e = cudaMemcpy(p->th_applied, node_applied, nn, cudaMemcpyDefault);
@@ -1025,7 +1040,7 @@ int ensure_scalar(cxg_plan* p) {
   p->edata = nullptr;
   p->device_bytes -= static_cast<int64_t>(p->edata_bytes);
   p->edata_bytes = 0;
-  CHECK_CUDA(device_alloc(&p->edata, need), "element buffer");
+  CHECK_CUDA(or_drop_work(p, [&] { return device_alloc(&p->edata, need); }), "element buffer");
   p->edata_bytes = need;
   p->device_bytes += static_cast<int64_t>(need);
   return CXG_OK;
@@ -1161,7 +1176,7 @@ int cxg_thermal_plan_set_films(cxg_plan* p, int64_t n_films, const int64_t* elem
   const size_t bytes = 8 * (felem.size() + fnode.size() + 3 * nF + 8 * nF) +
                        4 * (fptr.size() + order.size() + nF + fnptr.size() + fnlist.size()) + 64;
   char* mem = nullptr;
-  CHECK_CUDA(cudaMalloc(&mem, bytes), "film arrays");
+  CHECK_CUDA(device_malloc(&mem, bytes), "film arrays");
   p->film_mem = mem;
   size_t off = 0;
   auto put = [&](const void* src, size_t b) {
@@ -1220,7 +1235,7 @@ int cxg_assemble_conduction(cxg_plan* p, const double* conductivity, const doubl
       cudaFree(p->stage[2]);
       p->stage[2] = nullptr;
       p->stage_bytes[2] = 0;
-      CHECK_CUDA(cudaMalloc(&p->stage[2], 8 * N), "flux staging");
+      CHECK_CUDA(or_drop_work(p, [&] { return device_malloc(&p->stage[2], 8 * N); }), "flux staging");
       p->stage_bytes[2] = 8 * N;
     }
     df = p->stage[2];
@@ -1320,7 +1335,7 @@ int cxg_state_get(const cxg_plan* cp, int32_t slot, double* out) {
     return CXG_OK;
   }
   void* tmp = nullptr;
-  CHECK_CUDA(cudaMalloc(&tmp, std::max<size_t>(bytes, 8)), "state staging");
+  CHECK_CUDA(or_drop_work(p, [&] { return device_malloc(&tmp, std::max<size_t>(bytes, 8)); }), "state staging");
   cudaError_t e = launch_state_transpose(p->state[slot], static_cast<double*>(tmp), p->n_gauss, false, nullptr);
   if (e == cudaSuccess) e = cudaMemcpy(out, tmp, bytes, cudaMemcpyDefault);
   cudaFree(tmp);
@@ -1341,7 +1356,7 @@ int cxg_state_set(cxg_plan* p, int32_t slot, const double* in) {
     return CXG_OK;
   }
   void* tmp = nullptr;
-  CHECK_CUDA(cudaMalloc(&tmp, std::max<size_t>(bytes, 8)), "state staging");
+  CHECK_CUDA(or_drop_work(p, [&] { return device_malloc(&tmp, std::max<size_t>(bytes, 8)); }), "state staging");
   cudaError_t e = cudaMemcpy(tmp, in, bytes, cudaMemcpyDefault);
   if (e == cudaSuccess) e = launch_state_transpose(static_cast<double*>(tmp), p->state[slot], p->n_gauss, true, nullptr);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -1389,7 +1404,7 @@ int element_level(int32_t t, int64_t n_elems, const double* coords, const double
       *outp = const_cast<void*>(ptr);
       return cudaSuccess;
     }
-    cudaError_t e = cudaMalloc(outp, std::max<size_t>(bytes, 8));
+    cudaError_t e = device_malloc(outp, std::max<size_t>(bytes, 8));
     if (e != cudaSuccess) return e;
     owned.push_back(*outp);
     return cudaMemcpyAsync(*outp, ptr, bytes, cudaMemcpyHostToDevice, s);
@@ -1403,7 +1418,7 @@ int element_level(int32_t t, int64_t n_elems, const double* coords, const double
       *outp = ptr;
       return cudaSuccess;
     }
-    cudaError_t e = cudaMalloc(outp, std::max<size_t>(bytes, 8));
+    cudaError_t e = device_malloc(outp, std::max<size_t>(bytes, 8));
     if (e == cudaSuccess) owned.push_back(*outp);
     return e;
   };
@@ -1439,7 +1454,7 @@ int element_level(int32_t t, int64_t n_elems, const double* coords, const double
   double *dsc = nullptr, *dst_t = nullptr, *aos = nullptr;
   const int64_t G = n_elems * nq;
   const size_t sbytes = sizeof(double) * kStateDoubles * static_cast<size_t>(std::max<int64_t>(G, 1));
-  e = cudaMalloc(&dst, sizeof(DevStatus));
+  e = device_malloc(&dst, sizeof(DevStatus));
   if (e == cudaSuccess) owned.push_back(dst);
   DevStatus z{0, 0, ~0ull};
   if (e == cudaSuccess) e = cudaMemcpyAsync(dst, &z, sizeof z, cudaMemcpyHostToDevice, s);
@@ -1454,11 +1469,11 @@ int element_level(int32_t t, int64_t n_elems, const double* coords, const double
     int64_t counted = 0;
     e = alloc_copy(&dmat, mats.data(), 1, s, &counted);
     if (e == cudaSuccess) owned.push_back(dmat);
-    if (e == cudaSuccess) e = cudaMalloc(&dsc, sbytes);
+    if (e == cudaSuccess) e = device_malloc(&dsc, sbytes);
     if (e == cudaSuccess) owned.push_back(dsc);
-    if (e == cudaSuccess) e = cudaMalloc(&dst_t, sbytes);
+    if (e == cudaSuccess) e = device_malloc(&dst_t, sbytes);
     if (e == cudaSuccess) owned.push_back(dst_t);
-    if (e == cudaSuccess) e = cudaMalloc(&aos, sbytes);
+    if (e == cudaSuccess) e = device_malloc(&aos, sbytes);
     if (e == cudaSuccess) owned.push_back(aos);
     if (e == cudaSuccess) {
       if (sc)
@@ -1580,7 +1595,7 @@ int cxg_solve_cg(cxg_plan* p, const double* vals, const double* rhs, double* x, 
     cudaFree(p->stage[5]);
     p->stage[5] = nullptr;
     p->stage_bytes[5] = 0;
-    CHECK_CUDA(cudaMalloc(&p->stage[5], wb), "solver work");
+    CHECK_CUDA(or_drop_work(p, [&] { return device_malloc(&p->stage[5], wb); }), "solver work");
     p->stage_bytes[5] = wb;
   }
   int it = 0;

@@ -444,7 +444,7 @@ int cxg_batch_create(int32_t n_models, const cxg_mesh_desc* meshes, const cxg_do
   int rc = CXG_OK;
   std::vector<void*> tmp;
   auto dalloc = [&](void** p, size_t bytes) -> bool {
-    if (cudaMalloc(p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+    if (device_malloc(p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
       rc = cuda_err(cudaErrorMemoryAllocation, "batch staging");
       return false;
     }
@@ -674,10 +674,10 @@ int cxg_batch_assemble(cxg_batch* b, double* vals, double* rhs, const double* f_
   if (rc) return rc;
   const bool hv = !on_device(vals), hr = rhs && !on_device(rhs), hf = f_ext && !on_device(f_ext);
   double *dv = vals, *dr = rhs, *df = const_cast<double*>(f_ext);
-  if (hv) CHECK_CUDA(cudaMallocAsync(&dv, 8 * std::max<int64_t>(b->nnz, 1), s), "vals staging");
-  if (hr) CHECK_CUDA(cudaMallocAsync(&dr, 8 * std::max<int64_t>(b->n_free, 1), s), "rhs staging");
+  if (hv) CHECK_CUDA(device_malloc_async(&dv, 8 * std::max<int64_t>(b->nnz, 1), s), "vals staging");
+  if (hr) CHECK_CUDA(device_malloc_async(&dr, 8 * std::max<int64_t>(b->n_free, 1), s), "rhs staging");
   if (hf) {
-    CHECK_CUDA(cudaMallocAsync(&df, 24 * b->n_nodes, s), "load staging");
+    CHECK_CUDA(device_malloc_async(&df, 24 * b->n_nodes, s), "load staging");
     CHECK_CUDA(cudaMemcpyAsync(df, f_ext, 24 * b->n_nodes, cudaMemcpyHostToDevice, s), "load upload");
   }
   if (b->launch == CXG_BATCH_ONE_LAUNCH) {
@@ -957,7 +957,7 @@ int cxg_batch_get_state(const cxg_batch* b, int32_t k, int32_t slot, double* out
   const size_t nq = static_cast<size_t>(gauss_of(p->type));
   const size_t all = static_cast<size_t>(kStateDoubles) * static_cast<size_t>(p->n_gauss);
   double* tmp = nullptr;
-  CHECK_CUDA(cudaMalloc(&tmp, std::max<size_t>(all, 1) * sizeof(double)), "state staging");
+  CHECK_CUDA(device_malloc(&tmp, std::max<size_t>(all, 1) * sizeof(double)), "state staging");
   int rc = cxg_state_get(p, slot, tmp);
   if (!rc) {
     const cudaError_t e = cudaMemcpy(out, tmp + kStateDoubles * nq * static_cast<size_t>(md.e0),

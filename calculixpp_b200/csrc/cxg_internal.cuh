@@ -327,8 +327,20 @@ __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepc
 // 512 MB of what is freed. device_free expects that no work on the block is pending.
 // device_free_all waits for all work of `device` (as cudaFree would, once), whichever device
 // is current, frees its blocks and returns what is above the 512 MB to the device.
+// device_malloc and device_malloc_async are cudaMalloc and cudaMallocAsync. Each tries again with
+// the pool emptied where the device has no memory left.
 cudaError_t device_alloc(void** out, size_t bytes);
+cudaError_t device_malloc(void** out, size_t bytes);
+cudaError_t device_malloc_async(void** out, size_t bytes, cudaStream_t s);
 void device_free(void* ptr);
+template <typename T>
+cudaError_t device_malloc(T** out, size_t bytes) {
+  return device_malloc(reinterpret_cast<void**>(out), bytes);
+}
+template <typename T>
+cudaError_t device_malloc_async(T** out, size_t bytes, cudaStream_t s) {
+  return device_malloc_async(reinterpret_cast<void**>(out), bytes, s);
+}
 void device_free_all(int device, void* const* blocks, int n);
 // Whether a kernel on `device` can take the caller's doubles at ptr where they are: managed, or
 // in that device's own memory, and aligned. Anything else cudaMemcpy takes is copied first.

@@ -179,12 +179,12 @@ cudaError_t sort_lists(uint64_t* key, int64_t* order, int64_t* src, double* w, i
   int64_t* o2 = nullptr;
   void* temp = nullptr;
   size_t tb = 0;
-  cudaError_t e = cudaMalloc(&k2, sizeof(uint64_t) * std::max<int64_t>(n, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&o2, sizeof(int64_t) * std::max<int64_t>(n, 1));
-  if (e == cudaSuccess) e = cudaMalloc(src_sorted, sizeof(int64_t) * std::max<int64_t>(n, 1));
-  if (e == cudaSuccess) e = cudaMalloc(w_sorted, sizeof(double) * std::max<int64_t>(n, 1));
+  cudaError_t e = device_malloc(&k2, sizeof(uint64_t) * std::max<int64_t>(n, 1));
+  if (e == cudaSuccess) e = device_malloc(&o2, sizeof(int64_t) * std::max<int64_t>(n, 1));
+  if (e == cudaSuccess) e = device_malloc(src_sorted, sizeof(int64_t) * std::max<int64_t>(n, 1));
+  if (e == cudaSuccess) e = device_malloc(w_sorted, sizeof(double) * std::max<int64_t>(n, 1));
   if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(nullptr, tb, key, k2, order, o2, n, 0, end_bit, s);
-  if (e == cudaSuccess) e = cudaMalloc(&temp, std::max<size_t>(tb, 16));
+  if (e == cudaSuccess) e = device_malloc(&temp, std::max<size_t>(tb, 16));
   if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(temp, tb, key, k2, order, o2, n, 0, end_bit, s);
   if (e == cudaSuccess) {
     permute_kernel<<<grid_n(n), 256, 0, s>>>(o2, src, w, n, *src_sorted, *w_sorted);
@@ -211,7 +211,7 @@ cudaError_t build_mpc_reduce(const int64_t* x_row_ptr, const int32_t* x_col, int
   Expansion T{ext_map, term_ptr, term_eq, term_coeff};
   std::vector<void*> tmp;
   auto alloc = [&](void** p, size_t bytes) {
-    const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+    const cudaError_t e = device_malloc(p, std::max<size_t>(bytes, 16));
     if (e == cudaSuccess) tmp.push_back(*p);
     return e;
   };
@@ -261,15 +261,15 @@ cudaError_t build_mpc_reduce(const int64_t* x_row_ptr, const int32_t* x_col, int
   int64_t nu = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&nu, n_u, 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) e = cudaMalloc(&out->tgt_ptr, 8 * (nu + 1));
+  if (e == cudaSuccess) e = device_malloc(&out->tgt_ptr, 8 * (nu + 1));
   if (e == cudaSuccess) e = cudaMemsetAsync(runs + nu, 0, 8, s);
   size_t tb3 = 0;
   void* temp3 = nullptr;
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tb3, runs, out->tgt_ptr, nu + 1, s);
   if (e == cudaSuccess) e = alloc(&temp3, tb3);
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(temp3, tb3, runs, out->tgt_ptr, nu + 1, s);
-  if (e == cudaSuccess) e = cudaMalloc(&out->row_ptr, 8 * (static_cast<size_t>(n_free) + 1));
-  if (e == cudaSuccess) e = cudaMalloc(&out->col_idx, 4 * std::max<int64_t>(nu, 1));
+  if (e == cudaSuccess) e = device_malloc(&out->row_ptr, 8 * (static_cast<size_t>(n_free) + 1));
+  if (e == cudaSuccess) e = device_malloc(&out->col_idx, 4 * std::max<int64_t>(nu, 1));
   if (e == cudaSuccess) {
     rows_from_keys_kernel<<<grid_n(std::max<int64_t>(nu, n_free + 1)), 256, 0, s>>>(ukey, nu, n_free, nf, out->row_ptr,
                                                                                     out->col_idx);
@@ -305,7 +305,7 @@ cudaError_t build_mpc_reduce(const int64_t* x_row_ptr, const int32_t* x_col, int
   if (e == cudaSuccess)
     e = sort_lists(rkey, rorder, rsrc, rw, xtotal, end_bit_for(nf), &rks, &out->rhs_src, &out->rhs_w, s);
   if (rks) tmp.push_back(rks);
-  if (e == cudaSuccess) e = cudaMalloc(&out->rhs_ptr, 8 * (static_cast<size_t>(n_free) + 1));
+  if (e == cudaSuccess) e = device_malloc(&out->rhs_ptr, 8 * (static_cast<size_t>(n_free) + 1));
   if (e == cudaSuccess) {
     ptr_from_keys_kernel<<<grid_n(n_free + 1), 256, 0, s>>>(rks, xtotal, n_free, out->rhs_ptr);
     e = cudaGetLastError();

@@ -62,12 +62,34 @@ cudaError_t pool_of(Pool* out) {
   return cudaSuccess;
 }
 
+// alloc(), and where it finds no memory once more with what the pool keeps returned.
+template <class F>
+cudaError_t or_trim(F alloc) {
+  cudaError_t e = alloc();
+  Pool p;
+  if (e != cudaErrorMemoryAllocation || pool_of(&p) != cudaSuccess) return e;
+  cudaGetLastError();
+  cudaStreamSynchronize(p.stream);  // the frees before it
+  if (cudaMemPoolTrimTo(p.pool, 0) != cudaSuccess) return e;
+  return alloc();
+}
+
 }  // namespace
+
+cudaError_t device_malloc(void** out, size_t bytes) {
+  *out = nullptr;
+  return or_trim([&] { return cudaMalloc(out, bytes); });
+}
+
+cudaError_t device_malloc_async(void** out, size_t bytes, cudaStream_t s) {
+  *out = nullptr;
+  return or_trim([&] { return cudaMallocAsync(out, bytes, s); });
+}
 
 cudaError_t device_alloc(void** out, size_t bytes) {
   *out = nullptr;
   if (bytes > kPooled) {
-    const cudaError_t e = cudaMalloc(out, bytes);
+    const cudaError_t e = device_malloc(out, bytes);
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lock(g_mu);
     g_large.insert(*out);
@@ -76,7 +98,7 @@ cudaError_t device_alloc(void** out, size_t bytes) {
   Pool p;
   cudaError_t e = pool_of(&p);
   if (e != cudaSuccess) return e;
-  e = cudaMallocFromPoolAsync(out, std::max<size_t>(bytes, 16), p.pool, p.stream);
+  e = or_trim([&] { return cudaMallocFromPoolAsync(out, std::max<size_t>(bytes, 16), p.pool, p.stream); });
   if (e == cudaSuccess) e = cudaStreamSynchronize(p.stream);
   return e;
 }

@@ -405,10 +405,10 @@ cudaError_t compact_pattern(const int64_t* row_ptr, const int32_t* col_idx, int3
   int64_t *row_len = nullptr, *d_count = nullptr;
   void* temp = nullptr;
   size_t temp_bytes = 0, t2 = 0;
-  cudaError_t e = cudaMalloc(&keep, std::max<int64_t>(nnz, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&row_len, sizeof(int64_t) * (static_cast<size_t>(n_rows) + 1));
-  if (e == cudaSuccess) e = cudaMalloc(&d_count, sizeof(int64_t));
-  if (e == cudaSuccess) e = cudaMalloc(row_ptr_c, sizeof(int64_t) * (static_cast<size_t>(n_rows) + 1));
+  cudaError_t e = device_malloc(&keep, std::max<int64_t>(nnz, 1));
+  if (e == cudaSuccess) e = device_malloc(&row_len, sizeof(int64_t) * (static_cast<size_t>(n_rows) + 1));
+  if (e == cudaSuccess) e = device_malloc(&d_count, sizeof(int64_t));
+  if (e == cudaSuccess) e = device_malloc(row_ptr_c, sizeof(int64_t) * (static_cast<size_t>(n_rows) + 1));
   if (e == cudaSuccess) {
     keep_kernel<<<grid_of(nnz), 256, 0, s>>>(counts, keep, nnz);
     row_len_kernel<<<grid_of(n_rows), 256, 0, s>>>(row_ptr, keep, n_rows, row_len);
@@ -418,12 +418,12 @@ cudaError_t compact_pattern(const int64_t* row_ptr, const int32_t* col_idx, int3
   cub::CountingInputIterator<int64_t> idx(0);
   if (e == cudaSuccess) e = cub::DeviceSelect::Flagged(nullptr, t2, idx, keep, static_cast<int64_t*>(nullptr), d_count, nnz, s);
   temp_bytes = std::max(temp_bytes, t2);
-  if (e == cudaSuccess) e = cudaMalloc(&temp, std::max<size_t>(temp_bytes, 16));
+  if (e == cudaSuccess) e = device_malloc(&temp, std::max<size_t>(temp_bytes, 16));
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(temp, temp_bytes, row_len, *row_ptr_c, n_rows + 1, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(nnz_c, *row_ptr_c + n_rows, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) e = cudaMalloc(src, sizeof(int64_t) * static_cast<size_t>(std::max<int64_t>(*nnz_c, 1)));
-  if (e == cudaSuccess) e = cudaMalloc(col_idx_c, sizeof(int32_t) * static_cast<size_t>(std::max<int64_t>(*nnz_c, 1)));
+  if (e == cudaSuccess) e = device_malloc(src, sizeof(int64_t) * static_cast<size_t>(std::max<int64_t>(*nnz_c, 1)));
+  if (e == cudaSuccess) e = device_malloc(col_idx_c, sizeof(int32_t) * static_cast<size_t>(std::max<int64_t>(*nnz_c, 1)));
   if (e == cudaSuccess) e = cub::DeviceSelect::Flagged(temp, temp_bytes, idx, keep, *src, d_count, nnz, s);
   if (e == cudaSuccess) {
     gather_cols_kernel<<<grid_of(*nnz_c), 256, 0, s>>>(*src, col_idx, *nnz_c, *col_idx_c);

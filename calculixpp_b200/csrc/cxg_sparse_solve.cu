@@ -132,9 +132,9 @@ struct Ic0 {
 int ic0_build(Ic0& P, int32_t n, int32_t nnz, const int32_t* rp, const int32_t* ci, const double* A, double* r,
               double* z, cudaStream_t s) {
   P.s = s;
-  CHECK_CUDA(cudaMalloc(&P.L, sizeof(double) * std::max<int32_t>(nnz, 1)), "IC0 factor");
-  CHECK_CUDA(cudaMalloc(&P.y, sizeof(double) * std::max<int32_t>(n, 1)), "IC0 vector");
-  CHECK_CUDA(cudaMalloc(&P.bad, sizeof(int)), "IC0 flag");
+  CHECK_CUDA(device_malloc(&P.L, sizeof(double) * std::max<int32_t>(nnz, 1)), "IC0 factor");
+  CHECK_CUDA(device_malloc(&P.y, sizeof(double) * std::max<int32_t>(n, 1)), "IC0 vector");
+  CHECK_CUDA(device_malloc(&P.bad, sizeof(int)), "IC0 flag");
   IC0_SP(cusparseCreate(&P.h), "handle");
   IC0_SP(cusparseSetStream(P.h, s), "stream");
   IC0_SP(cusparseCreateMatDescr(&P.descr), "descriptor");
@@ -143,7 +143,7 @@ int ic0_build(Ic0& P, int32_t n, int32_t nnz, const int32_t* rp, const int32_t* 
   IC0_SP(cusparseCreateCsric02Info(&P.info), "info");
   int bytes = 0;
   IC0_SP(cusparseDcsric02_bufferSize(P.h, n, nnz, P.descr, P.L, rp, ci, P.info, &bytes), "buffer size");
-  CHECK_CUDA(cudaMalloc(&P.buf, std::max(bytes, 16)), "IC0 buffer");
+  CHECK_CUDA(device_malloc(&P.buf, std::max(bytes, 16)), "IC0 buffer");
   IC0_SP(cusparseDcsric02_analysis(P.h, n, nnz, P.descr, P.L, rp, ci, P.info, CUSPARSE_SOLVE_POLICY_USE_LEVEL, P.buf),
          "analysis");
   int pos = -1;
@@ -189,8 +189,8 @@ int ic0_build(Ic0& P, int32_t n, int32_t nnz, const int32_t* rp, const int32_t* 
   IC0_SP(cusparseSpSV_bufferSize(P.h, CUSPARSE_OPERATION_TRANSPOSE, &one, P.mat, P.vy, P.vz, CUDA_R_64F,
                                  CUSPARSE_SPSV_ALG_DEFAULT, P.slt, &b2),
          "solve buffer");
-  CHECK_CUDA(cudaMalloc(&P.bl, std::max<size_t>(b1, 16)), "IC0 solve buffer");
-  CHECK_CUDA(cudaMalloc(&P.blt, std::max<size_t>(b2, 16)), "IC0 solve buffer");
+  CHECK_CUDA(device_malloc(&P.bl, std::max<size_t>(b1, 16)), "IC0 solve buffer");
+  CHECK_CUDA(device_malloc(&P.blt, std::max<size_t>(b2, 16)), "IC0 solve buffer");
   IC0_SP(cusparseSpSV_analysis(P.h, CUSPARSE_OPERATION_NON_TRANSPOSE, &one, P.mat, P.vr, P.vy, CUDA_R_64F,
                                CUSPARSE_SPSV_ALG_DEFAULT, P.sl, P.bl),
          "solve analysis");
@@ -217,7 +217,7 @@ cudaError_t ic0_apply(Ic0& P, const double* r, double* z) {
 struct Scratch {
   std::vector<void*> p;
   cudaError_t alloc(void** q, size_t bytes) {
-    const cudaError_t e = cudaMalloc(q, std::max<size_t>(bytes, 16));
+    const cudaError_t e = device_malloc(q, std::max<size_t>(bytes, 16));
     if (e == cudaSuccess) p.push_back(*q);
     return e;
   }

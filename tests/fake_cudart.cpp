@@ -11,6 +11,7 @@
 
 namespace cxg {
 cudaError_t device_alloc(void** out, size_t bytes);
+cudaError_t device_malloc(void** out, size_t bytes);
 void device_free(void* ptr);
 void device_free_all(int device, void* const* blocks, int n);
 bool kernel_reads(int device, const void* ptr);
@@ -75,6 +76,12 @@ cudaError_t cudaMemPoolCreate(cudaMemPool_t* m, const cudaMemPoolProps* p) {
 cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { return cudaSuccess; }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) { return note("pool"), take(p, n, true); }
+cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return note("async"), take(p, n, false); }
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) {
+  note("trim");
+  g_idle[g_device] = 0;
+  return cudaSuccess;
+}
 cudaError_t cudaFreeAsync(void* p, cudaStream_t s) {
   note("give");
   const Block b = g_blocks[p];
@@ -109,6 +116,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* kern, v
 const char* fake_log() { return g_log.c_str(); }
 void fake_clear() { g_log.clear(); }
 int t_alloc(void** p, size_t n) { return cxg::device_alloc(p, n); }
+int t_malloc(void** p, size_t n) { return cxg::device_malloc(p, n); }
 void t_free(void* p) { cxg::device_free(p); }
 void t_free_all(int device, void* const* p, int n) { cxg::device_free_all(device, p, n); }
 int t_kernel_reads(int device, const void* p) { return cxg::kernel_reads(device, p); }

@@ -1,6 +1,7 @@
 """The library's host-only runtime files against a stand-in for the CUDA runtime
 (tests/fake_cudart.cpp): which device is waited for before memory is freed, which buffers of a
-caller a kernel may take in place, and that a kernel's shared-memory limit never falls. No GPU."""
+caller a kernel may take in place, that a kernel's shared-memory limit
+never falls, and that memory the pool keeps fails no allocation. No GPU."""
 import ctypes as C
 import os
 import subprocess
@@ -27,7 +28,7 @@ def fake(built, tmp_path):
     import shutil
     lib = C.CDLL(shutil.copy(built, tmp_path / "libfake.so"))
     lib.fake_log.restype = C.c_char_p
-    lib.t_alloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
+    lib.t_alloc.argtypes = lib.t_malloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
     lib.t_free.argtypes = [C.c_void_p]
     for f in (lib.t_shape, lib.t_launch):
         f.argtypes = [C.c_void_p, C.c_size_t]
@@ -42,9 +43,9 @@ def calls(lib):
     return got
 
 
-def alloc(lib, nbytes):
+def alloc(lib, nbytes, call="t_alloc"):
     p = C.c_void_p()
-    rc = lib.t_alloc(C.byref(p), nbytes)
+    rc = getattr(lib, call)(C.byref(p), nbytes)
     return rc, p
 
 
@@ -87,3 +88,15 @@ def test_shared_memory_limit_never_falls(fake):
     fake.cudaSetDevice(1)  # a limit of its own on every device
     assert fake.t_shape(kern, 20000) == 0 and fake.t_launch(kern, 20000) == 0
     assert calls(fake) == ["set@1", "limit20000@1", "launch@1"]
+
+
+@pytest.mark.parametrize("call", ["t_alloc", "t_malloc"])
+def test_memory_the_pool_keeps_fails_no_allocation(fake, call):
+    for _, p in [alloc(fake, 200 * MB) for _ in range(2)]:
+        fake.t_free(p)  # 400 of the device's 1024 MB idle in the pool
+    calls(fake)
+    rc, p = alloc(fake, 900 * MB, call)
+    assert rc == 0 and calls(fake) == ["malloc@0", "trim@0", "malloc@0"]
+    rc, _ = alloc(fake, 200 * MB, call)
+    assert rc != 0  # there is no more: an error, not a second trim
+    assert [c.split("@")[0] for c in calls(fake)] == (["pool", "trim", "pool"] if call == "t_alloc" else ["malloc", "trim", "malloc"])
