@@ -58,14 +58,6 @@ bool on_device(const void* p) {
 
 namespace {
 
-template <typename T>
-cudaError_t alloc_copy(T** dst, const T* src, size_t count, cudaStream_t s, int64_t* bytes) {
-  *bytes += static_cast<int64_t>(count * sizeof(T));
-  cudaError_t e = device_malloc(dst, std::max<size_t>(count, 1) * sizeof(T));
-  if (e != cudaSuccess || !src || count == 0) return e;
-  return cudaMemcpyAsync(*dst, src, count * sizeof(T), cudaMemcpyDefault, s);
-}
-
 // alloc(), and where it finds no memory once more without the plan's idle scratch.
 template <class F>
 cudaError_t or_drop_work(cxg_plan* p, F alloc) {
@@ -1391,9 +1383,17 @@ int element_level(int32_t t, int64_t n_elems, const double* coords, const double
   CHECK_CUDA(ensure_tables(), "constant tables");
   const int n = nodes_of(t), nq = gauss_of(t), nd = 3 * n;
   const size_t E = static_cast<size_t>(n_elems);
+  // Pool blocks: a cudaMalloc and a cudaFree of the error word alone took most of a call once no
+  // other small cudaMalloc kept their page mapped (20,000 C3D8 elements 950 us, this way 170).
   std::vector<void*> owned;
+  auto own = [&](auto** out, size_t bytes) {
+    const cudaError_t e = device_alloc(reinterpret_cast<void**>(out), bytes);
+    if (e == cudaSuccess) owned.push_back(*out);
+    return e;
+  };
   auto cleanup = [&]() {
-    for (void* b : owned) cudaFree(b);
+    cudaStreamSynchronize(s);  // (an error may have left work on them)
+    for (void* b : owned) device_free(b);
   };
   auto dev_in = [&](const void* ptr, size_t bytes, void** outp) -> cudaError_t {
     if (!ptr) {
@@ -1404,9 +1404,8 @@ int element_level(int32_t t, int64_t n_elems, const double* coords, const double
       *outp = const_cast<void*>(ptr);
       return cudaSuccess;
     }
-    cudaError_t e = device_malloc(outp, std::max<size_t>(bytes, 8));
+    const cudaError_t e = own(outp, bytes);
     if (e != cudaSuccess) return e;
-    owned.push_back(*outp);
     return cudaMemcpyAsync(*outp, ptr, bytes, cudaMemcpyHostToDevice, s);
   };
   auto dev_out = [&](void* ptr, size_t bytes, void** outp) -> cudaError_t {
@@ -1418,9 +1417,7 @@ int element_level(int32_t t, int64_t n_elems, const double* coords, const double
       *outp = ptr;
       return cudaSuccess;
     }
-    cudaError_t e = device_malloc(outp, std::max<size_t>(bytes, 8));
-    if (e == cudaSuccess) owned.push_back(*outp);
-    return e;
+    return own(outp, bytes);
   };
   ElemArgs a{};
   a.n_elems = n_elems;
@@ -1454,8 +1451,7 @@ int element_level(int32_t t, int64_t n_elems, const double* coords, const double
   double *dsc = nullptr, *dst_t = nullptr, *aos = nullptr;
   const int64_t G = n_elems * nq;
   const size_t sbytes = sizeof(double) * kStateDoubles * static_cast<size_t>(std::max<int64_t>(G, 1));
-  e = device_malloc(&dst, sizeof(DevStatus));
-  if (e == cudaSuccess) owned.push_back(dst);
+  e = own(&dst, sizeof(DevStatus));
   DevStatus z{0, 0, ~0ull};
   if (e == cudaSuccess) e = cudaMemcpyAsync(dst, &z, sizeof z, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && tangent) {
@@ -1466,15 +1462,11 @@ int element_level(int32_t t, int64_t n_elems, const double* coords, const double
       cleanup();
       return rc;
     }
-    int64_t counted = 0;
-    e = alloc_copy(&dmat, mats.data(), 1, s, &counted);
-    if (e == cudaSuccess) owned.push_back(dmat);
-    if (e == cudaSuccess) e = device_malloc(&dsc, sbytes);
-    if (e == cudaSuccess) owned.push_back(dsc);
-    if (e == cudaSuccess) e = device_malloc(&dst_t, sbytes);
-    if (e == cudaSuccess) owned.push_back(dst_t);
-    if (e == cudaSuccess) e = device_malloc(&aos, sbytes);
-    if (e == cudaSuccess) owned.push_back(aos);
+    e = own(&dmat, sizeof(J2Mat));
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dmat, mats.data(), sizeof(J2Mat), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = own(&dsc, sbytes);
+    if (e == cudaSuccess) e = own(&dst_t, sbytes);
+    if (e == cudaSuccess) e = own(&aos, sbytes);
     if (e == cudaSuccess) {
       if (sc)
         e = cudaMemcpyAsync(aos, sc, sizeof(double) * kStateDoubles * G, cudaMemcpyDefault, s);
