@@ -427,8 +427,7 @@ ElemArgs base_args(cxg_plan* p) {
   a.node_mask = p->pat.node_mask;
   a.prescribed = p->prescribed;
   a.pairs = p->pat.pairs;
-  a.bnd_node = p->pat.bnd_node;
-  a.bnd_col = p->pat.bnd_col;
+  a.bnd = p->pat.bnd;
   a.n_gauss = p->n_gauss;
   a.status = p->status;
   a.th_temp = p->th_temp;
@@ -569,7 +568,7 @@ int cxg_plan_create(const cxg_mesh_desc* m, const cxg_dofmap_desc* d, int32_t pr
     }
   }
   const char* msg = nullptr;
-  rc = build_pattern(m->elem_type, m->n_nodes, m->n_elems, p->conn, p->dof_eq, d->n_free, &p->pat, &msg, s);
+  rc = build_pattern(m->elem_type, m->n_nodes, m->n_elems, p->conn, p->dof_eq, p->prescribed, d->n_free, &p->pat, &msg, s);
   if (rc) return fail(set_err(rc, std::string("pattern: ") + (msg ? msg : "")));
   p->device_bytes += p->pat.device_bytes;
   TRYC(cudaStreamSynchronize(s), "plan build");

@@ -62,6 +62,11 @@ __device__ __forceinline__ PairRec load_pairs(const PairRec* p) {
   return u.r;
 }
 
+__device__ __forceinline__ BndRec load_bnd(const BndRec* p) {
+  const int2 q = __ldg(reinterpret_cast<const int2*>(p));
+  return {static_cast<uint32_t>(q.x), q.y};
+}
+
 // Index of a stored block in the element buffer. With windows the buffer is a ring of
 // `ring` elements; every element of a window lies in [ring_base, ring_base + 2 ring), so
 // one conditional subtraction gives the slot.
@@ -119,98 +124,144 @@ __device__ __forceinline__ void gather_node(const ElemArgs& A, const V2Args& V, 
   wait_for_kernel_before();
   if (gridDim.x <= kOneWave) let_next_kernel_start();
   double* const rows = A.vals + nd.base;
-  // what prescribed columns move to the rhs: of row ki (own pair and later ones), of
-  // row kj (earlier ones)
+  // Where the lane's entry of a pair goes: entry (ki, kj) of the block from the own pair on,
+  // entry (kj, ki) before it. At full rows the place moves three columns a pair; at compressed
+  // ones it is the row's start and the pair's column and free components (BndRec): the lane's
+  // column is free, or its prescribed value is not zero, or nothing is to do, as on every lane
+  // whose row is not free.
+  double* row = rows;
+  uint32_t free = 0, moves = 0, below = 0;
+  auto side = [&](bool early) {
+    const int i = early ? kj : ki, j = early ? ki : kj;
+    const bool on = (ma >> i) & 1;
+    free = on ? 1u << (28 + j) : 0u;
+    moves = on ? 0x80000000u : 0u;
+    below = ((1u << j) - 1) << 28;
+    row = rows + static_cast<int64_t>(__popc(ma & ((1 << i) - 1))) * L;
+  };
+  // what prescribed columns move to the rhs: of row ki, and (rt) of row kj before the own pair
   double rd = 0.0, rt = 0.0;
-  // the lane's entry of the block of pair p, wherever it goes
-  auto put = [&](int p, double v) {
-    const int i = p < self ? kj : ki, j = p < self ? ki : kj;
-    if (full) {
-      double* o = rows + i * L + 3 * p + j;
+  auto put = [&](BndRec b, double v) {
+    if (b.at & free) {
+      double* o = row + (b.at & 0xfffffff) + __popc(b.at & below);
       *o = V.accumulate ? *o + v : v;
-      return;
-    }
-    if (!((ma >> i) & 1)) return;
-    const uint32_t at = static_cast<uint32_t>(__ldg(A.bnd_col + nd.bnd0 + p));
-    const int mb = at >> 28;
-    if ((mb >> j) & 1) {
-      double* o = rows + static_cast<int64_t>(__popc(ma & ((1 << i) - 1))) * L + (at & 0xfffffff) +
-                  __popc(mb & ((1 << j) - 1));
-      *o = V.accumulate ? *o + v : v;
-    } else {
-      // (a zero value moves nothing, not even from an infinite entry, src/fem/assembly.cpp:95)
-      const double u = A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p)) + j];
-      const double c = u != 0.0 ? v * u : 0.0;
-      if (p < self)
-        rt -= c;
-      else
-        rd -= c;
+    } else if (b.at & moves) {
+      // (a value of zero moves nothing, not even from an infinite entry, src/fem/assembly.cpp:95)
+      const double u = A.prescribed[3 * static_cast<int64_t>(b.node) + __popc(below)];
+      if (u != 0.0) rd -= v * u;
     }
   };
   if (ma) {
-    int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
+    const int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
+    // a run that ends before the own pair holds earlier pairs only
+    const bool early = (q == 0 ? nd.pair1 : q == 1 ? nd.pair2 : K) <= self;
     // the off-diagonal blocks' sums (DIAG): entry (ki, kj) of the blocks from the own
     // pair on, entry (kj, ki) of those before it
     double own = 0.0, before = 0.0;
     double v = 0.0;
-    // before the own pair a lane writes entry (kj, ki), from there on (ki, kj)
-    double* o = rows + 3 * p + (p < self ? kj * L + ki : ki * L + kj);
-    const int64_t turn = static_cast<int64_t>(ki - kj) * (L - 1);
-    for (uint32_t r = 0; r < nd.rounds; ++r) {
-      R x[UN];
-#pragma unroll
-      for (int i = 0; i < UN; ++i) {
-        x[i] = R(0);
-        if (mine) x[i] = ed[(SCALAR ? 1 : 9) * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks)];
-      }
-      const bool turns = rec.flags >> 31;
-      const unsigned ends = lane < 27 ? rec.flags : 0u;
-      list += 3;
-      if (r + 1 < nd.rounds) rec = load_pairs(list);
-      if (plain && !turns) {
+    // step(x, ends, turns) for every round: its contributions, and where pairs end among them
+    auto rounds = [&](auto step) {
+      for (uint32_t r = 0; r < nd.rounds; ++r) {
+        R x[UN];
 #pragma unroll
         for (int i = 0; i < UN; ++i) {
-          v += static_cast<double>(x[i]);
-          end_pair<DIAG>(ends & (1u << i), o, v, own);
+          x[i] = R(0);
+          if (mine) x[i] = ed[(SCALAR ? 1 : 9) * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks)];
         }
-      } else if (plain) {
+        const bool turns = rec.flags >> 31;
+        const unsigned ends = lane < 27 ? rec.flags : 0u;
+        list += 3;
+        if (r + 1 < nd.rounds) rec = load_pairs(list);
+        step(x, ends, turns);
+      }
+    };
+    if (full) {
+      // before the own pair a lane writes entry (kj, ki), from there on (ki, kj)
+      double* o = rows + 3 * p + (p < self ? kj * L + ki : ki * L + kj);
+      const int64_t turn = static_cast<int64_t>(ki - kj) * (L - 1);
+      rounds([&](const R(&x)[UN], unsigned ends, bool turns) {
+        if (plain && !turns) {
 #pragma unroll
-        for (int i = 0; i < UN; ++i) {
-          v += static_cast<double>(x[i]);
-          end_pair<DIAG>(ends & (1u << i), o, v, own);
-          if (ends & (0x10000u << i)) {
-            o += turn;
-            if (DIAG) before = own;
-            own = DIAG ? 0.0 : own;
+          for (int i = 0; i < UN; ++i) {
+            v += static_cast<double>(x[i]);
+            end_pair<DIAG>(ends & (1u << i), o, v, own);
+          }
+        } else if (plain) {
+#pragma unroll
+          for (int i = 0; i < UN; ++i) {
+            v += static_cast<double>(x[i]);
+            end_pair<DIAG>(ends & (1u << i), o, v, own);
+            if (ends & (0x10000u << i)) {
+              o += turn;
+              if (DIAG) before = own;
+              own = DIAG ? 0.0 : own;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < UN; ++i) {
+            v += static_cast<double>(x[i]);
+            if (ends & (1u << i)) {
+              *o += v;
+              own += v;
+              v = 0.0;
+              o += 3;
+              if (ends & (0x10000u << i)) {
+                o += turn;
+                if (DIAG) before = own;
+                own = DIAG ? 0.0 : own;
+              }
+            }
           }
         }
-      } else {
+      });
+    } else {
+      side(p < self);
+      const BndRec* list_b = A.bnd + nd.bnd0 + p;
+      BndRec b = load_bnd(list_b);
+      rounds([&](const R(&x)[UN], unsigned ends, bool) {
+        // the next pair's column is on its way while the pair is summed
 #pragma unroll
         for (int i = 0; i < UN; ++i) {
           v += static_cast<double>(x[i]);
           if (ends & (1u << i)) {
-            if (!DIAG || p != self) put(p, v);
+            put(b, v);
             own += v;
             v = 0.0;
-            ++p;
-            if (DIAG && (ends & (0x10000u << i))) {
-              before = own;
-              own = 0.0;
+            b = load_bnd(++list_b);
+            if (ends & (0x10000u << i)) {
+              rt = rd;
+              rd = 0.0;
+              side(false);
+              if (DIAG) before = own;
+              own = DIAG ? 0.0 : own;
             }
           }
         }
+      });
+      if (early) {
+        rt = rd;
+        rd = 0.0;
       }
     }
     if constexpr (DIAG) {
-      // a run that ends before the own pair holds earlier pairs only
-      if ((q == 0 ? nd.pair1 : q == 1 ? nd.pair2 : K) <= self) {
+      if (early) {
         before = own;
         own = 0.0;
       }
       __syncwarp();  // orders the block below after the loop's write of the same place
       const double t = own + __shfl_sync(kAll, before, min(9 * (lane / 9) + 3 * kj + ki, 31));
       const double t1 = __shfl_sync(kAll, t, (lane + 9) & 31), t2 = __shfl_sync(kAll, t, (lane + 18) & 31);
-      if (lane < 9 && K > 0) put(self, -((t + t1) + t2));
+      if (lane < 9 && K > 0) {
+        const double d = -((t + t1) + t2);
+        if (full) {
+          double* o = rows + ki * L + 3 * self + kj;
+          *o = V.accumulate ? *o + d : d;
+        } else {
+          side(false);
+          put(load_bnd(A.bnd + nd.bnd0 + self), d);
+        }
+      }
     }
     if (A.rhs) {
       double v = 0.0;
@@ -264,11 +315,11 @@ __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& 
           if (full) {
             o[p] = v;
           } else {
-            const uint32_t at = static_cast<uint32_t>(__ldg(A.bnd_col + nd.bnd0 + p));
-            if (at >> 28) {
-              o[at & 0xfffffff] = v;
-            } else {
-              const double u = A.prescribed[3 * static_cast<int64_t>(__ldg(A.bnd_node + nd.bnd0 + p))];
+            const BndRec b = load_bnd(A.bnd + nd.bnd0 + p);
+            if ((b.at >> 28) & 1) {
+              o[b.at & 0xfffffff] = v;
+            } else if (b.at >> 31) {
+              const double u = A.prescribed[3 * static_cast<int64_t>(b.node)];
               if (u != 0.0) rr -= v * u;
             }
           }

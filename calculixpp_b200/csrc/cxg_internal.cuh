@@ -66,7 +66,7 @@ struct __align__(16) NodeRec {
   int32_t eq0;       // first free equation (or -1)
   uint32_t list0;
   uint32_t rounds;
-  uint32_t bnd0;     // first of the node's entries in bnd_node / bnd_col
+  uint32_t bnd0;     // first of the node's BndRecs
   uint16_t npair;
   uint16_t diag;     // the node's own position among its pairs
   uint16_t pair1, pair2;
@@ -85,6 +85,12 @@ struct __align__(16) PairRec {
   uint32_t block[kPairRec];
 };
 static_assert(sizeof(PairRec) == 48, "PairRec is three 16-byte loads");
+
+// A pair of a node whose rows are compressed (some neighbour is not fully free).
+struct __align__(8) BndRec {
+  uint32_t at;   // first column | free components << 28 | (some prescribed value is not zero) << 31
+  int32_t node;  // the neighbour
+};
 
 // 3x3 blocks of an element in the element buffer: one per local node pair (a, b), a <= b,
 // 9 consecutive values at 9 * blk_index. The stored block is that of the two nodes in
@@ -117,8 +123,7 @@ struct ElemArgs {
   const uint8_t* node_mask;   // [N] bit i: component i free
   const double* prescribed;   // [3N]
   const PairRec* pairs;
-  const int32_t* bnd_node;
-  const int32_t* bnd_col;
+  const BndRec* bnd;
   // state (tangent mode), SoA [13][G]
   const double* state_c;
   double* state_t;
@@ -355,10 +360,7 @@ struct PatternOut {
   NodeRec* node = nullptr;      // [N]
   uint8_t* node_mask = nullptr; // [N]
   PairRec* pairs = nullptr;     // contributions of the element blocks, see NodeRec
-  // neighbour, and compressed column | free components << 28, of every pair of the nodes
-  // with a neighbour that is not fully free (NodeRec::bnd0)
-  int32_t* bnd_node = nullptr;
-  int32_t* bnd_col = nullptr;
+  BndRec* bnd = nullptr;        // of every pair of the nodes with a neighbour that is not fully free
   // node -> incident elements, ascending element order: codes e*n + local node index
   int64_t* inc_ptr = nullptr;   // [N+1]
   int32_t* inc_code = nullptr;  // [E*n]
@@ -366,7 +368,7 @@ struct PatternOut {
 };
 // Returns a cxg_status code; on error *msg is set.
 int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t* d_conn,
-                  const int32_t* d_dof_eq, int32_t n_free, PatternOut* out, const char** msg,
+                  const int32_t* d_dof_eq, const double* d_prescribed, int32_t n_free, PatternOut* out, const char** msg,
                   cudaStream_t s);
 
 }  // namespace cxg

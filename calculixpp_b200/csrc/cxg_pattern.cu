@@ -15,7 +15,7 @@
 //   4. a second sweep orders the candidates again and writes row_ptr, col_idx, the
 //      records that the row gather reads (NodeRec, PairRec) and, for the nodes with a
 //      neighbour that is not fully free (their rows are compressed), the neighbours and
-//      their columns (bnd_node, bnd_col).
+//      their columns (BndRec).
 // A global sort of all element node pairs would carry 24 bytes of scratch per pair through
 // six passes, and its allocations alone took longer than both sweeps together.
 // The pattern is topological: an entry whose every element contribution is exactly
@@ -231,11 +231,11 @@ __global__ void __launch_bounds__(kWarps * 32) count_kernel(Sweep S, int64_t n_n
 
 // Second sweep: the CSR rows, the records and the lists of the compressed-row nodes.
 __global__ void __launch_bounds__(kWarps * 32) write_kernel(Sweep S, int64_t n_nodes, const uint8_t* mask,
-                                                            const int32_t* eq0, const int64_t* node_base,
+                                                            const int32_t* eq0, const double* prescribed,
+                                                            const int64_t* node_base,
                                                             const int64_t* bnd_ptr, const int64_t* rec_ptr, int cap,
                                                             Cand* big, NodeRec* node, int64_t* row_ptr,
-                                                            int32_t* col_idx, PairRec* pairs, int32_t* bnd_node,
-                                                            int32_t* bnd_col) {
+                                                            int32_t* col_idx, PairRec* pairs, BndRec* bnd) {
   extern __shared__ Cand sh[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t gw = static_cast<int64_t>(blockIdx.x) * kWarps + warp, nw = static_cast<int64_t>(gridDim.x) * kWarps;
@@ -273,8 +273,9 @@ __global__ void __launch_bounds__(kWarps * 32) write_kernel(Sweep S, int64_t n_n
       for (int i = 0; i < nfa; ++i)
         for (int j = 0; j < pc; ++j) col_idx[nd.base + static_cast<int64_t>(i) * L + col + j] = e + j;
       if (L != 3 * K) {
-        bnd_node[nd.bnd0 + p] = b;
-        bnd_col[nd.bnd0 + p] = col | mb << 28;
+        bool moves = false;
+        for (int d = 0; d < 3; ++d) moves = moves || (!((mb >> d) & 1) && prescribed[3 * static_cast<int64_t>(b) + d] != 0.0);
+        bnd[nd.bnd0 + p] = BndRec{static_cast<uint32_t>(col) | static_cast<uint32_t>(mb) << 28 | (moves ? 0x80000000u : 0u), b};
       }
     });
     own = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(own + 1)) - 1;
@@ -341,7 +342,7 @@ T* part(void* base, size_t at) {
   } while (0)
 
 int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t* d_conn,
-                  const int32_t* d_dof_eq, int32_t n_free, PatternOut* out, const char** msg,
+                  const int32_t* d_dof_eq, const double* d_prescribed, int32_t n_free, PatternOut* out, const char** msg,
                   cudaStream_t s) {
   const int npe = nodes_of(elem_type);
   const int64_t P = n_elems * npe * npe, m = n_elems * npe;
@@ -473,21 +474,20 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
       goto done;
     }
     out->nnz = last[0] + len[0];
-    const size_t nbnd = static_cast<size_t>(last[1] + len[1]);
+    // (one more: the gather reads the record after a list's last)
+    const size_t nbnd = static_cast<size_t>(last[1] + len[1]) + 1;
     Parts rest;
     const size_t r_col = rest.add<int32_t>(static_cast<size_t>(out->nnz)),
-                 r_pairs = rest.add<PairRec>(static_cast<size_t>(last[2] + len[2])), r_bn = rest.add<int32_t>(nbnd),
-                 r_bc = rest.add<int32_t>(nbnd);
+                 r_pairs = rest.add<PairRec>(static_cast<size_t>(last[2] + len[2])), r_bnd = rest.add<BndRec>(nbnd);
     CXG_TRY(device_alloc(&out->mem[1], rest.bytes));
     out->device_bytes += static_cast<int64_t>(rest.bytes);
     out->col_idx = part<int32_t>(out->mem[1], r_col);
     out->pairs = part<PairRec>(out->mem[1], r_pairs);
-    out->bnd_node = part<int32_t>(out->mem[1], r_bn);
-    out->bnd_col = part<int32_t>(out->mem[1], r_bc);
+    out->bnd = part<BndRec>(out->mem[1], r_bnd);
     CXG_TRY(cudaMemcpyAsync(out->row_ptr + n_free, &out->nnz, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    write_kernel<<<sweep_grid, kWarps * 32, sweep_smem, s>>>(S, n_nodes, out->node_mask, eq0, offs[0], offs[1], offs[2],
-                                                             cap, static_cast<Cand*>(big), out->node, out->row_ptr,
-                                                             out->col_idx, out->pairs, out->bnd_node, out->bnd_col);
+    write_kernel<<<sweep_grid, kWarps * 32, sweep_smem, s>>>(S, n_nodes, out->node_mask, eq0, d_prescribed, offs[0],
+                                                             offs[1], offs[2], cap, static_cast<Cand*>(big), out->node, out->row_ptr,
+                                                             out->col_idx, out->pairs, out->bnd);
     CXG_TRY(cudaGetLastError());
     CXG_TRY(cudaStreamSynchronize(s));
   }
