@@ -401,6 +401,7 @@ V2Args v2_args(cxg_plan* p, const double* f_ext, bool accumulate) {
   v.f_ext = f_ext;
   v.npe = nodes_of(p->type);
   v.nbp = blocks_padded(v.npe);
+  v.named_twice = p->pat.named_twice;
   v.accumulate = accumulate ? 1 : 0;
   v.e_begin = 0;
   v.e_end = p->n_elems;

@@ -96,7 +96,7 @@ struct __align__(8) BndRec {
 // 9 consecutive values at 9 * blk_index. The stored block is that of the two nodes in
 // ascending mesh order (K_ba where node b precedes node a), so all elements that share a
 // pair store it the same way round; a node with itself, where an element names a node twice,
-// as the symmetric part, since (a, b) and (b, a) are the same pair then. An element's block count is padded so that every
+// as the symmetric part (zeros in FP32), since (a, b) and (b, a) are the same pair then. An element's block count is padded so that every
 // element starts 16-byte aligned in both precisions, which bulk copies need (8-byte
 // aligned in FP32 for the families of 4 and 6 nodes, which copy with plain stores).
 __host__ __device__ constexpr int blk_index(int n, int a, int b) { return a * n - a * (a - 1) / 2 + (b - a); }
@@ -159,6 +159,7 @@ struct V2Args {
   const int32_t* inc_code;
   const double* f_ext;      // [3N] load vector for the rhs, or null
   int npe, nbp;             // nodes and (padded) blocks per element
+  int named_twice;          // some element names a node at two places
   int accumulate;           // add into vals / rhs / f_int instead of overwriting
   // The window of one element-pass + row-gather pair: the element pass integrates
   // elements [e_begin, e_end), the row gather the nodes node_order[n_begin..n_end)
@@ -355,6 +356,7 @@ bool kernel_reads(int device, const void* ptr);
 struct PatternOut {
   void* mem[2] = {nullptr, nullptr};  // the device blocks that hold all of these
   int64_t nnz = 0;
+  bool named_twice = false;     // some element names a node at two places
   int64_t* row_ptr = nullptr;   // [n_free+1]
   int32_t* col_idx = nullptr;   // [nnz]
   NodeRec* node = nullptr;      // [N]

@@ -32,7 +32,7 @@ namespace cxg {
 namespace {
 
 struct BuildFlags {
-  int bad_conn, bad_numbering, too_many, pad;
+  int bad_conn, bad_numbering, too_many, named_twice;
   unsigned long long bad_elem;
 };
 
@@ -176,11 +176,12 @@ __global__ void __launch_bounds__(kWarps * 32) count_kernel(Sweep S, int64_t n_n
   Cand* k = big ? big + gw * cap : sh + warp * cap;
   for (int64_t a = gw; a < n_nodes; a += nw) {
     const int cnt = order_candidates(S, a, k);
-    int len = 0, K = 0, self = 0;
+    int len = 0, K = 0, self = 0, own = 0;
     // the neighbour starts nearest to one and two thirds of the contributions
     int cut[2] = {cnt, cnt}, pos[2] = {0, 0}, err[2] = {3 * cnt + 1, 3 * cnt + 1};
     each_candidate(k, cnt, [&](int r, int p, bool first) {
       if (r >= cnt) return;
+      own += k[r].node == a;
       if (first) {
         len += __popc(mask[k[r].node]);
         if (k[r].node == a) self = p;
@@ -198,6 +199,7 @@ __global__ void __launch_bounds__(kWarps * 32) count_kernel(Sweep S, int64_t n_n
     len = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(len));
     K = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(K));
     self = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(self));
+    own = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(own));
     for (int g = 0; g < 2; ++g) {
       // (the end of the list is a cut too, for nodes with one or two neighbours)
       const unsigned e = __reduce_min_sync(0xffffffffu, static_cast<unsigned>(err[g]));
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(kWarps * 32) count_kernel(Sweep S, int64_t n_n
       r.pad[0] = static_cast<uint32_t>(cut[0]);
       r.pad[1] = static_cast<uint32_t>(cut[1]);
       if (K > 65535) atomicExch(&f->too_many, 1);  // list positions are uint16
+      if (own * S.npe != cnt) atomicExch(&f->named_twice, 1);  // not once per incident element
       node[a] = r;
       node_nnz[a] = static_cast<int64_t>(__popc(mask[a])) * len;
       bnd_len[a] = len == 3 * K ? 0 : K;
@@ -473,6 +476,7 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
       rc = 5;
       goto done;
     }
+    out->named_twice = hf.named_twice != 0;
     out->nnz = last[0] + len[0];
     // (one more: the gather reads the record after a list's last)
     const size_t nbnd = static_cast<size_t>(last[1] + len[1]) + 1;

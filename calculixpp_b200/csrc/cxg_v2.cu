@@ -844,7 +844,9 @@ cudaError_t launch_p1_batch(int mode, int precision, bool j2f32, const BatchSlot
   }
   P.n = n;
   void* args[] = {&P};
-  return launch_kernel(kern, blk, kT1, smem, s, args);
+  cudaError_t e = launch_kernel(kern, blk, kT1, smem, s, args);
+  for (int k = 0; k < n && e == cudaSuccess && !precision; ++k) e = launch_named_twice(in[k].a, in[k].v, s);
+  return e;
 }
 
 cudaError_t launch_v2_batch(int mode, int precision, const BatchSlotIn* in, int n, int passes, cudaStream_t s) {

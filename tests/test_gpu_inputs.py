@@ -15,7 +15,7 @@ import pytest
 import scipy.sparse as sp
 import torch
 
-from calculixpp_b200 import Material, Model, Plan, ThermalPlan, _lib
+from calculixpp_b200 import Batch, Material, Model, Plan, ThermalPlan, _lib
 from calculixpp_b200 import meshgen as mg
 from oracle.oracle import make_material
 from tests.helpers import ISO_TABLE, box_model, per_element_materials, rel_fro, to_np
@@ -59,10 +59,10 @@ def test_flux_in_the_memory_of_the_rhs(cuda):
         assert torch.equal(v, vals) and torch.equal(r, rhs)
 
 
-def collapsed(etype, jitter=0.05):
+def collapsed(etype, jitter=0.05, cells=(2, 2, 3)):
     """Wedges written as hexahedra whose fourth edge has collapsed onto the third."""
     quadratic = etype in (mg.C3D20, mg.C3D20R)
-    w = mg.box_mesh(mg.C3D15 if quadratic else mg.C3D6, 2, 2, 3, jitter=jitter, seed=1, straight_edges=True)
+    w = mg.box_mesh(mg.C3D15 if quadratic else mg.C3D6, *cells, jitter=jitter, seed=1, straight_edges=True)
     local = [0, 1, 2, 2, 3, 4, 5, 5] + ([6, 7, 2, 8, 9, 10, 5, 11, 12, 13, 14, 14] if quadratic else [])
     m = mg.Mesh(w.coords, np.ascontiguousarray(w.conn[:, local]), etype)
     m.young = np.random.default_rng(2).uniform(70e3, 210e3, m.n_elems)
@@ -90,6 +90,22 @@ def test_elements_that_name_a_node_twice(cuda, port, etype, jitter, precision, b
         assert rel_fro(to_np(r), rhs) <= bar
         plan.use_reference_pattern()
         assert all(np.array_equal(to_np(a), b) for a, b in zip(plan.pattern(), (rp, ci)))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_elements_that_name_a_node_twice_in_windows_and_batches(cuda, precision):
+    models = [collapsed(mg.C3D8, cells=(2, 2, 24)), box_model(mg.C3D20, 2, 2, 2)]
+    with Plan(models[0], precision) as plan:
+        want = plan.assemble_linear()
+        plan.set_ring_bytes(72 * 36 * (72 if precision == "fp64" else 36))
+        got = plan.assemble_linear()
+        assert plan.windows()[0] > 1
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    batch = Batch(models, precision)
+    for mode in ("per_group", "one_launch"):
+        batch.set_launch(mode)
+        got = batch.slices(0, *batch.assemble())
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
 def test_plastic_elements_that_name_a_node_twice(cuda, port):
