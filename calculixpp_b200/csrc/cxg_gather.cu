@@ -39,8 +39,8 @@ constexpr unsigned kAll = 0xffffffffu;
 constexpr int kWarps = 4;
 // Grids that are resident at once on a B200 let the next kernel on the stream start early.
 constexpr unsigned kOneWave = 148 * 6;
-// (Registers: 64 a thread where the blocks are FP32, 80 where they are FP64: 64 spill there
-// and lose, C3D8 128^3 2908 -> 3239 us; with FP32 they win, C3D20 64^3 2190 -> 2007 us.)
+// (Registers: 64 a thread where the blocks are FP32, bound by the launch bounds: C3D20 64^3
+// 2190 us without, 2007 with; 68 where they are FP64, 64 spill there.)
 
 __device__ __forceinline__ NodeRec load_node(const NodeRec* p) {
   union {
@@ -49,6 +49,20 @@ __device__ __forceinline__ NodeRec load_node(const NodeRec* p) {
   } u;
 #pragma unroll
   for (int i = 0; i < 3; ++i) u.q[i] = __ldg(reinterpret_cast<const int4*>(p) + i);
+  return u.r;
+}
+
+// The same, not merged with an earlier load.
+__device__ __forceinline__ NodeRec fresh_node(const NodeRec* p) {
+  union {
+    int4 q[3];
+    NodeRec r;
+  } u;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    asm volatile("ld.global.nc.v4.s32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(u.q[i].x), "=r"(u.q[i].y), "=r"(u.q[i].z), "=r"(u.q[i].w)
+                 : "l"(reinterpret_cast<const int4*>(p) + i));
   return u.r;
 }
 
@@ -69,219 +83,257 @@ __device__ __forceinline__ BndRec load_bnd(const BndRec* p) {
 
 // Index of a stored block in the element buffer. With windows the buffer is a ring of
 // `ring` elements; every element of a window lies in [ring_base, ring_base + 2 ring), so
-// one conditional subtraction gives the slot.
+// one conditional subtraction gives the slot. (A plan has fewer than 2^31 blocks.)
 template <bool WIN>
-__device__ __forceinline__ int64_t block_slot(uint32_t block, int64_t ring_blocks, int64_t base_blocks) {
+__device__ __forceinline__ int64_t block_slot(uint32_t block, uint32_t ring_blocks, uint32_t base_blocks) {
   if constexpr (WIN) {
-    const int64_t d = static_cast<int64_t>(block) - base_blocks;
+    const uint32_t d = block - base_blocks;
     return d < ring_blocks ? d : d - ring_blocks;
   }
   return block;
 }
 
 // Where a pair ends: write the entry, start the next pair three columns on. Predicated
-// rather than branched: some group ends a pair at most steps.
-template <bool SUM>
+// rather than branched: some group ends a pair at most steps. ADD: onto what is there, as a
+// reduction in L2 (each entry has one lane, so the sum is the same as read, added and
+// written, and nothing waits for the read: 110,592 C3D8 FP64 405 -> 252 us an assembly).
+template <bool SUM, bool ADD>
 __device__ __forceinline__ void end_pair(unsigned last, double*& o, double& v, double& sum) {
-  if constexpr (SUM)
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.u32 p, %3, 0;\n@p st.global.f64 [%0], %1;\n@p add.f64 %2, %2, %1;\n"
-        "@p mov.f64 %1, 0d0000000000000000;\n@p add.s64 %0, %0, 24;\n}"
-        : "+l"(o), "+d"(v), "+d"(sum)
-        : "r"(last)
-        : "memory");
-  else
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.global.f64 [%0], %1;\n"
-        "@p mov.f64 %1, 0d0000000000000000;\n@p add.s64 %0, %0, 24;\n}"
-        : "+l"(o), "+d"(v)
-        : "r"(last)
-        : "memory");
+#define CXG_SUMMED(WRITE)                                                                                  \
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %3, 0;\n@p " WRITE " [%0], %1;\n@p add.f64 %2, %2, %1;\n" \
+               "@p mov.f64 %1, 0d0000000000000000;\n@p add.s64 %0, %0, 24;\n}"                             \
+               : "+l"(o), "+d"(v), "+d"(sum)                                                               \
+               : "r"(last)                                                                                 \
+               : "memory")
+#define CXG_WRITTEN(WRITE)                                                      \
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p " WRITE " [%0], %1;\n" \
+               "@p mov.f64 %1, 0d0000000000000000;\n@p add.s64 %0, %0, 24;\n}"  \
+               : "+l"(o), "+d"(v)                                               \
+               : "r"(last)                                                      \
+               : "memory")
+  if constexpr (SUM && ADD) CXG_SUMMED("red.global.add.f64");
+  if constexpr (SUM && !ADD) CXG_SUMMED("st.global.f64");
+  if constexpr (!SUM && ADD) CXG_WRITTEN("red.global.add.f64");
+  if constexpr (!SUM && !ADD) CXG_WRITTEN("st.global.f64");
+#undef CXG_SUMMED
+#undef CXG_WRITTEN
 }
 
-template <typename R, int KIND, bool WIN>
-__device__ __forceinline__ void gather_node(const ElemArgs& A, const V2Args& V, unsigned bid) {
-  constexpr bool DIAG = KIND == GATHER_DIAG, SCALAR = KIND == GATHER_SCALAR;
+// One entry outside such a run.
+template <bool ADD>
+__device__ __forceinline__ void write_entry(double* o, double v) {
+  if constexpr (ADD)
+    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(o), "d"(v) : "memory");
+  else
+    *o = v;
+}
+
+// The place of a lane in a node's gather: lanes 27 .. 31 follow the third group without writing.
+struct Lane {
+  int lane, q, ki, kj;
+  __device__ __forceinline__ Lane() {
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));  // (made again rather than kept)
+    q = min(lane / 9, 2);
+    const int k = lane < 27 ? lane - 9 * q : 0;
+    ki = k / 3;
+    kj = k - 3 * ki;
+  }
+};
+
+// step(x, ends, turns) for every round of the lane's run: its contributions, and where pairs
+// end among them. rec: the run's first record.
+template <typename R, bool SCALAR, bool WIN, class F>
+__device__ __forceinline__ void each_round(const ElemArgs& A, const V2Args& V, const NodeRec& nd, const Lane& l,
+                                           PairRec rec, F step) {
   constexpr int UN = kPairRec;
-  const int lane = threadIdx.x & 31;
-  const int64_t n_begin = WIN ? V.n_begin : 0, n_end = WIN ? V.n_end : A.n_nodes;
-  const int64_t idx = n_begin + static_cast<int64_t>(bid) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (idx >= n_end) return;
-  // lanes 27 .. 31 follow the third group without writing
-  const int q = min(lane / 9, 2), k = lane < 27 ? lane - 9 * q : 0, ki = k / 3, kj = k - 3 * ki;
-  const R* ed = reinterpret_cast<const R*>(V.edata) + (SCALAR ? 0 : k);
-  const bool mine = !SCALAR || ki == kj;  // the other entries of a multiple of I are zero
-  const int64_t ring_blocks = V.ring * V.nbp, base_blocks = V.ring_base * V.nbp;
-  const int64_t a = WIN ? static_cast<int64_t>(V.node_order[idx]) : n_end - 1 - idx;
-  const NodeRec nd = load_node(A.node + a);
-  const int K = nd.npair, L = nd.len_mask & 0xfffffff, ma = nd.len_mask >> 28, self = nd.diag;
-  const bool full = L == 3 * K, plain = full && !V.accumulate;
-  const PairRec* list = A.pairs + nd.list0 + q;
-  PairRec rec{};
-  if (ma && nd.rounds) rec = load_pairs(list);
-  // (the records are the plan's own; blocks and outputs are other kernels' too, and are
-  // read with plain loads, since the element pass may still be writing when this starts)
-  wait_for_kernel_before();
-  if (gridDim.x <= kOneWave) let_next_kernel_start();
-  double* const rows = A.vals + nd.base;
+  const R* ed = reinterpret_cast<const R*>(V.edata) + (SCALAR ? 0 : 3 * l.ki + l.kj);
+  const bool mine = !SCALAR || l.ki == l.kj;  // the other entries of a multiple of I are zero
+  const uint32_t ring_blocks = static_cast<uint32_t>(V.ring * V.nbp), base_blocks = static_cast<uint32_t>(V.ring_base * V.nbp);
+  const PairRec* list = A.pairs + nd.list0 + l.q;
+  for (uint32_t r = 0; r < nd.rounds; ++r) {
+    R x[UN];
+#pragma unroll
+    for (int i = 0; i < UN; ++i) {
+      x[i] = R(0);
+      if (mine) x[i] = ed[(SCALAR ? 1 : 9) * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks)];
+    }
+    const bool turns = rec.flags >> 31;
+    const unsigned ends = l.lane < 27 ? rec.flags : 0u;
+    list += 3;
+    if (r + 1 < nd.rounds) rec = load_pairs(list);
+    step(x, ends, turns);
+  }
+}
+
+// The diagonal block's entry of lanes 0 .. 8 (DIAG) from the lanes' sums of entry (ki, kj) of
+// the blocks from the own pair on and of entry (kj, ki) of those before it.
+__device__ __forceinline__ double diagonal(const Lane& l, double own, double before) {
+  const double t = own + __shfl_sync(kAll, before, min(9 * (l.lane / 9) + 3 * l.kj + l.ki, 31));
+  const double t1 = __shfl_sync(kAll, t, (l.lane + 9) & 31), t2 = __shfl_sync(kAll, t, (l.lane + 18) & 31);
+  return -((t + t1) + t2);
+}
+
+// Row r of the rhs on lane 3 r: the load (or what is there, ADD) and v.
+template <bool ADD>
+__device__ __forceinline__ void write_rhs(const ElemArgs& A, const V2Args& V, const NodeRec& nd, int64_t a, int lane,
+                                          double v) {
+  const int ma = nd.len_mask >> 28, r = lane / 3;
+  if ((lane == 0 || lane == 3 || lane == 6) && ((ma >> r) & 1)) {
+    const int64_t eq = nd.eq0 + __popc(ma & ((1 << r) - 1));
+    const double prev = ADD ? A.rhs[eq] : (V.f_ext ? V.f_ext[3 * a + r] : 0.0);
+    A.rhs[eq] = prev + v;
+  }
+}
+
+// A node with a neighbour that is not fully free. The node's record is read again where it is
+// needed (fresh_node) instead of kept through the walk, which has 64 registers a thread with
+// FP32 blocks (kept, the walk of the full rows spilled too: C3D8 64^3 293 -> 327 us).
+template <typename R, int KIND, bool WIN, bool ADD>
+__device__ __forceinline__ void gather_compressed(const ElemArgs& A, const V2Args& V, int64_t a) {
+  constexpr bool DIAG = KIND == GATHER_DIAG;
+  constexpr int UN = kPairRec;
   // Where the lane's entry of a pair goes: entry (ki, kj) of the block from the own pair on,
-  // entry (kj, ki) before it. At full rows the place moves three columns a pair; at compressed
-  // ones it is the row's start and the pair's column and free components (BndRec): the lane's
-  // column is free, or its prescribed value is not zero, or nothing is to do, as on every lane
-  // whose row is not free.
-  double* row = rows;
+  // entry (kj, ki) before it; the row's start and the pair's column and free components
+  // (BndRec): the lane's column is free, or its prescribed value is not zero, or nothing is to
+  // do, as on every lane whose row is not free.
+  double* row = nullptr;
   uint32_t free = 0, moves = 0, below = 0;
-  auto side = [&](bool early) {
-    const int i = early ? kj : ki, j = early ? ki : kj;
+  auto side = [&](const NodeRec& nd, const Lane& l, bool early) {
+    const int i = early ? l.kj : l.ki, j = early ? l.ki : l.kj, ma = nd.len_mask >> 28;
     const bool on = (ma >> i) & 1;
     free = on ? 1u << (28 + j) : 0u;
     moves = on ? 0x80000000u : 0u;
     below = ((1u << j) - 1) << 28;
-    row = rows + static_cast<int64_t>(__popc(ma & ((1 << i) - 1))) * L;
+    row = A.vals + nd.base + static_cast<int64_t>(__popc(ma & ((1 << i) - 1))) * (nd.len_mask & 0xfffffff);
   };
   // what prescribed columns move to the rhs: of row ki, and (rt) of row kj before the own pair
   double rd = 0.0, rt = 0.0;
   auto put = [&](BndRec b, double v) {
     if (b.at & free) {
-      double* o = row + (b.at & 0xfffffff) + __popc(b.at & below);
-      *o = V.accumulate ? *o + v : v;
+      write_entry<ADD>(row + (b.at & 0xfffffff) + __popc(b.at & below), v);
     } else if (b.at & moves) {
       // (a value of zero moves nothing, not even from an infinite entry, src/fem/assembly.cpp:95)
       const double u = A.prescribed[3 * static_cast<int64_t>(b.node) + __popc(below)];
       if (u != 0.0) rd -= v * u;
     }
   };
-  if (ma) {
-    const int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
-    // a run that ends before the own pair holds earlier pairs only
-    const bool early = (q == 0 ? nd.pair1 : q == 1 ? nd.pair2 : K) <= self;
-    // the off-diagonal blocks' sums (DIAG): entry (ki, kj) of the blocks from the own
-    // pair on, entry (kj, ki) of those before it
-    double own = 0.0, before = 0.0;
-    double v = 0.0;
-    // step(x, ends, turns) for every round: its contributions, and where pairs end among them
-    auto rounds = [&](auto step) {
-      for (uint32_t r = 0; r < nd.rounds; ++r) {
-        R x[UN];
-#pragma unroll
-        for (int i = 0; i < UN; ++i) {
-          x[i] = R(0);
-          if (mine) x[i] = ed[(SCALAR ? 1 : 9) * block_slot<WIN>(rec.block[i], ring_blocks, base_blocks)];
-        }
-        const bool turns = rec.flags >> 31;
-        const unsigned ends = lane < 27 ? rec.flags : 0u;
-        list += 3;
-        if (r + 1 < nd.rounds) rec = load_pairs(list);
-        step(x, ends, turns);
-      }
-    };
-    if (full) {
-      // before the own pair a lane writes entry (kj, ki), from there on (ki, kj)
-      double* o = rows + 3 * p + (p < self ? kj * L + ki : ki * L + kj);
-      const int64_t turn = static_cast<int64_t>(ki - kj) * (L - 1);
-      rounds([&](const R(&x)[UN], unsigned ends, bool turns) {
-        if (plain && !turns) {
-#pragma unroll
-          for (int i = 0; i < UN; ++i) {
-            v += static_cast<double>(x[i]);
-            end_pair<DIAG>(ends & (1u << i), o, v, own);
-          }
-        } else if (plain) {
-#pragma unroll
-          for (int i = 0; i < UN; ++i) {
-            v += static_cast<double>(x[i]);
-            end_pair<DIAG>(ends & (1u << i), o, v, own);
-            if (ends & (0x10000u << i)) {
-              o += turn;
-              if (DIAG) before = own;
-              own = DIAG ? 0.0 : own;
-            }
-          }
-        } else {
+  double own = 0.0, before = 0.0, v = 0.0;
+  {
+    const Lane l;
+    const NodeRec nd = load_node(A.node + a);
+    const int p = l.q == 0 ? 0 : l.q == 1 ? nd.pair1 : nd.pair2;
+    side(nd, l, p < nd.diag);
+    const BndRec* list = A.bnd + nd.bnd0 + p;
+    BndRec b = load_bnd(list);
+    each_round<R, KIND == GATHER_SCALAR, WIN>(
+        A, V, nd, l, load_pairs(A.pairs + nd.list0 + l.q), [&](const R(&x)[UN], unsigned ends, bool) {
+          // the next pair's column is on its way while the pair is summed
 #pragma unroll
           for (int i = 0; i < UN; ++i) {
             v += static_cast<double>(x[i]);
             if (ends & (1u << i)) {
-              *o += v;
-              own += v;
+              put(b, v);
+              if (DIAG) own += v;
               v = 0.0;
-              o += 3;
+              b = load_bnd(++list);
               if (ends & (0x10000u << i)) {
-                o += turn;
-                if (DIAG) before = own;
-                own = DIAG ? 0.0 : own;
+                side(fresh_node(A.node + a), Lane(), false);
+                rt = rd;
+                rd = 0.0;
+                before = own;
+                own = 0.0;
               }
             }
           }
-        }
-      });
-    } else {
-      side(p < self);
-      const BndRec* list_b = A.bnd + nd.bnd0 + p;
-      BndRec b = load_bnd(list_b);
-      rounds([&](const R(&x)[UN], unsigned ends, bool) {
-        // the next pair's column is on its way while the pair is summed
-#pragma unroll
-        for (int i = 0; i < UN; ++i) {
-          v += static_cast<double>(x[i]);
-          if (ends & (1u << i)) {
-            put(b, v);
-            own += v;
-            v = 0.0;
-            b = load_bnd(++list_b);
-            if (ends & (0x10000u << i)) {
-              rt = rd;
-              rd = 0.0;
-              side(false);
-              if (DIAG) before = own;
-              own = DIAG ? 0.0 : own;
-            }
-          }
-        }
-      });
-      if (early) {
-        rt = rd;
-        rd = 0.0;
-      }
-    }
-    if constexpr (DIAG) {
-      if (early) {
-        before = own;
-        own = 0.0;
-      }
-      __syncwarp();  // orders the block below after the loop's write of the same place
-      const double t = own + __shfl_sync(kAll, before, min(9 * (lane / 9) + 3 * kj + ki, 31));
-      const double t1 = __shfl_sync(kAll, t, (lane + 9) & 31), t2 = __shfl_sync(kAll, t, (lane + 18) & 31);
-      if (lane < 9 && K > 0) {
-        const double d = -((t + t1) + t2);
-        if (full) {
-          double* o = rows + ki * L + 3 * self + kj;
-          *o = V.accumulate ? *o + d : d;
-        } else {
-          side(false);
-          put(load_bnd(A.bnd + nd.bnd0 + self), d);
-        }
-      }
-    }
-    if (A.rhs) {
-      double v = 0.0;
-      if (!full) {  // (full rows have no prescribed column)
-        rd += __shfl_down_sync(kAll, rd, 9) + __shfl_down_sync(kAll, rd, 18);
-        rt += __shfl_down_sync(kAll, rt, 9) + __shfl_down_sync(kAll, rt, 18);
-        rd += __shfl_down_sync(kAll, rd, 1) + __shfl_down_sync(kAll, rd, 2);  // lane 3 i: row i
-        rt += __shfl_down_sync(kAll, rt, 3) + __shfl_down_sync(kAll, rt, 6);  // lane i: row i
-        v = rd + __shfl_sync(kAll, rt, lane / 3);
-      }
-      if (lane == 0 || lane == 3 || lane == 6) {
-        const int r = lane / 3;
-        if ((ma >> r) & 1) {
-          const int64_t eq = nd.eq0 + __popc(ma & ((1 << r) - 1));
-          const double prev = V.accumulate ? A.rhs[eq] : (V.f_ext ? V.f_ext[3 * a + r] : 0.0);
-          A.rhs[eq] = prev + v;
-        }
-      }
+        });
+  }
+  const Lane l;
+  const NodeRec nd = fresh_node(A.node + a);
+  // a run that ends before the own pair holds earlier pairs only
+  if ((l.q == 0 ? nd.pair1 : l.q == 1 ? nd.pair2 : nd.npair) <= nd.diag) {
+    rt = rd;
+    rd = 0.0;
+    before = own;
+    own = 0.0;
+  }
+  if constexpr (DIAG) {
+    __syncwarp();  // orders the block below after the loop's write of the same place
+    const double d = diagonal(l, own, before);
+    if (l.lane < 9) {
+      side(nd, l, false);
+      put(load_bnd(A.bnd + nd.bnd0 + nd.diag), d);
     }
   }
+  if (A.rhs) {
+    rd += __shfl_down_sync(kAll, rd, 9) + __shfl_down_sync(kAll, rd, 18);
+    rt += __shfl_down_sync(kAll, rt, 9) + __shfl_down_sync(kAll, rt, 18);
+    rd += __shfl_down_sync(kAll, rd, 1) + __shfl_down_sync(kAll, rd, 2);  // lane 3 i: row i
+    rt += __shfl_down_sync(kAll, rt, 3) + __shfl_down_sync(kAll, rt, 6);  // lane i: row i
+    write_rhs<ADD>(A, V, nd, a, l.lane, rd + __shfl_sync(kAll, rt, l.lane / 3));
+  }
+}
+
+// ADD: onto vals and rhs (V.accumulate).
+template <typename R, int KIND, bool WIN, bool ADD>
+__device__ __forceinline__ void gather_node(const ElemArgs& A, const V2Args& V, unsigned bid) {
+  constexpr bool DIAG = KIND == GATHER_DIAG;
+  constexpr int UN = kPairRec;
+  const int64_t n_begin = WIN ? V.n_begin : 0, n_end = WIN ? V.n_end : A.n_nodes;
+  const int64_t idx = n_begin + static_cast<int64_t>(bid) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (idx >= n_end) return;
+  const Lane l;
+  const int64_t a = WIN ? static_cast<int64_t>(V.node_order[idx]) : n_end - 1 - idx;
+  const NodeRec nd = load_node(A.node + a);
+  const int K = nd.npair, L = nd.len_mask & 0xfffffff, ma = nd.len_mask >> 28, self = nd.diag;
+  PairRec rec{};
+  if (ma && nd.rounds) rec = load_pairs(A.pairs + nd.list0 + l.q);
+  // (the records are the plan's own; blocks and outputs are other kernels' too, and are
+  // read with plain loads, since the element pass may still be writing when this starts)
+  wait_for_kernel_before();
+  if (gridDim.x <= kOneWave) let_next_kernel_start();
+  if (!ma) return;
+  if (L != 3 * K) {
+    gather_compressed<R, KIND, WIN, ADD>(A, V, a);
+    return;
+  }
+  double* const rows = A.vals + nd.base;
+  const int p = l.q == 0 ? 0 : l.q == 1 ? nd.pair1 : nd.pair2;
+  // before the own pair a lane writes entry (kj, ki), from there on (ki, kj)
+  double* o = rows + 3 * p + (p < self ? l.kj * L + l.ki : l.ki * L + l.kj);
+  const int64_t turn = static_cast<int64_t>(l.ki - l.kj) * (L - 1);
+  // the off-diagonal blocks' sums (DIAG), see diagonal
+  double own = 0.0, before = 0.0, v = 0.0;
+  each_round<R, KIND == GATHER_SCALAR, WIN>(A, V, nd, l, rec, [&](const R(&x)[UN], unsigned ends, bool turns) {
+    if (!turns) {
+#pragma unroll
+      for (int i = 0; i < UN; ++i) {
+        v += static_cast<double>(x[i]);
+        end_pair<DIAG, ADD>(ends & (1u << i), o, v, own);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < UN; ++i) {
+        v += static_cast<double>(x[i]);
+        end_pair<DIAG, ADD>(ends & (1u << i), o, v, own);
+        if (ends & (0x10000u << i)) {
+          o += turn;
+          if (DIAG) before = own;
+          own = DIAG ? 0.0 : own;
+        }
+      }
+    }
+  });
+  if constexpr (DIAG) {
+    // a run that ends before the own pair holds earlier pairs only
+    if ((l.q == 0 ? nd.pair1 : l.q == 1 ? nd.pair2 : K) <= self) {
+      before = own;
+      own = 0.0;
+    }
+    __syncwarp();  // orders the block below after the loop's write of the same place
+    const double d = diagonal(l, own, before);
+    if (l.lane < 9 && K > 0) write_entry<ADD>(rows + l.ki * L + 3 * self + l.kj, d);
+  }
+  if (A.rhs) write_rhs<ADD>(A, V, nd, a, l.lane, 0.0);  // (full rows have no prescribed column)
 }
 
 // One temperature per node: a lane walks one of the three runs of a node, ten nodes to a
@@ -333,12 +385,13 @@ __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& 
   if (A.rhs && free && q == 0) A.rhs[nd.eq0] = (V.f_ext ? V.f_ext[a] : 0.0) + ((rr + r1) + r2);
 }
 
-template <typename R, int KIND, bool WIN>
-__global__ void __launch_bounds__(256, KIND == GATHER_DIAG ? 4 : 3) gather_kernel(ElemArgs A, V2Args V) {
+template <typename R, int KIND, bool WIN, bool ADD>
+__global__ void __launch_bounds__(256, KIND == GATHER_DIAG ? 4 : 3) gather_kernel(const __grid_constant__ ElemArgs A,
+                                                                                          const __grid_constant__ V2Args V) {
   if constexpr (KIND == GATHER_ONE_DOF)
     gather_one_dof(A, V);
   else
-    gather_node<R, KIND, WIN>(A, V, blockIdx.x);
+    gather_node<R, KIND, WIN, ADD>(A, V, blockIdx.x);
 }
 
 // Internal force of every node: one thread per component, the element forces in element
@@ -376,9 +429,10 @@ cudaError_t launch_forces(const ElemArgs& a, const V2Args& v, cudaStream_t s) {
 
 template <typename R, int KIND>
 cudaError_t launch_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, cudaStream_t s) {
-  auto kern = gather_kernel<R, KIND, false>;
+  auto kern = gather_kernel<R, KIND, false, false>;
   if constexpr (KIND == GATHER_FULL || KIND == GATHER_DIAG) {
-    if (v.node_order) kern = gather_kernel<R, KIND, true>;
+    kern = v.node_order ? (v.accumulate ? gather_kernel<R, KIND, true, true> : gather_kernel<R, KIND, true, false>)
+                        : (v.accumulate ? gather_kernel<R, KIND, false, true> : kern);
   }
   const int warps = cfg.p2_warps > 0 ? std::min(cfg.p2_warps, 8) : kWarps;
   const int64_t count = v.n_end - v.n_begin;
@@ -427,7 +481,7 @@ __global__ void __launch_bounds__(256) gather_batch_kernel(const __grid_constant
   int k = 0;
   while (k + 1 < P.n && static_cast<int64_t>(blockIdx.x) >= P.s[k + 1].blk0) ++k;
   const GatherSlot& S = P.s[k];
-  gather_node<R, KIND, false>(S.a, S.v, blockIdx.x - static_cast<unsigned>(S.blk0));
+  gather_node<R, KIND, false, false>(S.a, S.v, blockIdx.x - static_cast<unsigned>(S.blk0));
 }
 
 template <typename R, int KIND>

@@ -5,6 +5,8 @@
   the rhs exactly the load where all prescribed values are zero;
 * a nodal flux and a rhs in the same memory;
 * device buffers that start between two doubles, for the history and the nodal flux;
+* accumulation onto any values: each entry the rounded sum of what was there and what an
+  assembly alone gives, in rows with and without prescribed columns;
 * elements that name a node two or three times: hexahedra collapsed to wedges, against the
   oracle. In mixed precision 1e-5: FP32 blocks of about 2e2 x 6e-8.
 
@@ -150,3 +152,17 @@ def test_buffers_between_two_doubles(cuda):
         _lib.check(plan.lib.cxg_assemble_conduction(plan.h, k.data_ptr(), at, v.data_ptr(), r.data_ptr(), None))
         plan.check()
         assert torch.equal(v, vals) and torch.equal(r, rhs)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("etype", [mg.C3D8, mg.C3D10, mg.C3D20])
+def test_accumulation_is_the_sum(cuda, etype, precision):
+    model = box_model(etype, 5, 3, 3, prescribe=1e-3)
+    rng = np.random.default_rng(etype)
+    with Plan(model, precision) as plan:
+        vals, rhs = plan.assemble_linear()
+        v0 = torch.as_tensor(rng.normal(size=plan.nnz) * float(vals.abs().max()), device=cuda)
+        r0 = torch.as_tensor(rng.normal(size=plan.n_free) * float(rhs.abs().max()), device=cuda)
+        v, r = v0.clone(), r0.clone()
+        plan.accumulate_linear(v, r)
+        assert torch.equal(v, v0 + vals) and torch.equal(r, r0 + rhs)
