@@ -385,62 +385,92 @@ __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& 
   if (A.rhs && free && q == 0) A.rhs[nd.eq0] = (V.f_ext ? V.f_ext[a] : 0.0) + ((rr + r1) + r2);
 }
 
-template <typename R, int KIND, bool WIN, bool ADD>
-__global__ void __launch_bounds__(256, KIND == GATHER_DIAG ? 4 : 3) gather_kernel(const __grid_constant__ ElemArgs A,
-                                                                                          const __grid_constant__ V2Args V) {
+// Internal force of every node (material-point assembly): one thread per component, the
+// element forces in element order. In blocks of their own among the gather's: beside a node's
+// walk the three dependent loads of this sum cost every node their latency, and a kernel of its
+// own costs a launch for every group of a batch (nine small models, FP64: 348 -> 299 us). Spread
+// over the grid, they run while other blocks of the SM walk (C3D8 J2 128^3: 98 us as a kernel).
+template <bool WIN>
+__device__ __forceinline__ void node_forces(const ElemArgs& A, const V2Args& V, unsigned bid) {
+  const int64_t first = 3 * (WIN ? V.n_begin : 0), last = 3 * (WIN ? V.n_end : A.n_nodes);
+  const int64_t t = first + static_cast<int64_t>(bid) * blockDim.x + threadIdx.x;
+  wait_for_kernel_before();
+  if (gridDim.x <= kOneWave) let_next_kernel_start();
+  if (t >= last) return;
+  const int64_t a = WIN ? static_cast<int64_t>(V.node_order[t / 3]) : t / 3;
+  const int d = static_cast<int>(t % 3);
+  const int64_t i1 = V.inc_ptr[a + 1];
+  double f = 0.0;
+#pragma unroll 4
+  for (int64_t i = V.inc_ptr[a]; i < i1; ++i) {
+    int64_t s = __ldg(V.inc_code + i);
+    if constexpr (WIN) {
+      s -= V.ring_base * V.npe;
+      if (s >= V.ring * V.npe) s -= V.ring * V.npe;
+    }
+    f += V.fdata[3 * s + d];
+  }
+  A.f_int[3 * a + d] = f;
+}
+
+// Blocks of `threads` for n nodes: the gather's, and those of the forces, one after every
+// `force_every` of them (the rest of the gather's at the end).
+int64_t gather_grid(V2Args& v, bool forces, int64_t n, int block_nodes, int threads) {
+  const int64_t walk = (n + block_nodes - 1) / block_nodes;
+  v.force_blocks = forces ? static_cast<uint32_t>((3 * n + threads - 1) / threads) : 0;
+  v.force_every = v.force_blocks ? static_cast<uint32_t>(std::max<int64_t>(1, walk / v.force_blocks)) : 0;
+  return walk + v.force_blocks;
+}
+
+// Whether block bid sums forces; bid becomes its number among its own kind.
+__device__ __forceinline__ bool force_block(const V2Args& V, unsigned& bid) {
+  const unsigned g = bid / (V.force_every + 1), r = bid - g * (V.force_every + 1);
+  const bool forces = g < V.force_blocks && r == V.force_every;
+  bid = forces ? g : bid - min(g, V.force_blocks);
+  return forces;
+}
+
+// What a gather does beside the walk: OVER writes vals and rhs, ADD adds onto them
+// (V.accumulate), FORCES writes them and sums the internal forces.
+enum GatherMode : int { OVER = 0, ADD = 1, FORCES = 2 };
+
+template <typename R, int KIND, bool WIN, int MODE>
+__device__ __forceinline__ void gather_block(const ElemArgs& A, const V2Args& V, unsigned bid) {
+  if constexpr (MODE == FORCES) {
+    if (force_block(V, bid)) {
+      node_forces<WIN>(A, V, bid);
+      return;
+    }
+  }
   if constexpr (KIND == GATHER_ONE_DOF)
     gather_one_dof(A, V);
   else
-    gather_node<R, KIND, WIN, ADD>(A, V, blockIdx.x);
+    gather_node<R, KIND, WIN, MODE == ADD>(A, V, bid);
 }
 
-// Internal force of every node: one thread per component, the element forces in element
-// order. Beside the row gather the three dependent loads of this sum cost every node
-// their latency; here they overlap across threads.
-template <bool WIN>
-__global__ void __launch_bounds__(256) force_kernel(ElemArgs A, V2Args V) {
-  const int64_t first = 3 * (WIN ? V.n_begin : 0), last = 3 * (WIN ? V.n_end : A.n_nodes);
-  for (int64_t t = first + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < last;
-       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t a = WIN ? static_cast<int64_t>(V.node_order[t / 3]) : t / 3;
-    const int d = static_cast<int>(t % 3);
-    const int64_t i1 = V.inc_ptr[a + 1];
-    double f = 0.0;
-#pragma unroll 4
-    for (int64_t i = V.inc_ptr[a]; i < i1; ++i) {
-      int64_t s = __ldg(V.inc_code + i);
-      if constexpr (WIN) {
-        s -= V.ring_base * V.npe;
-        if (s >= V.ring * V.npe) s -= V.ring * V.npe;
-      }
-      f += V.fdata[3 * s + d];
-    }
-    A.f_int[3 * a + d] = (V.accumulate ? A.f_int[3 * a + d] : 0.0) + f;
-  }
-}
-
-cudaError_t launch_forces(const ElemArgs& a, const V2Args& v, cudaStream_t s) {
-  const int64_t count = 3 * (v.n_end - v.n_begin);
-  if (!a.f_int || count <= 0) return cudaSuccess;
-  const int64_t grid = std::min<int64_t>((count + 255) / 256, 148 * 8);
-  (v.node_order ? force_kernel<true> : force_kernel<false>)<<<static_cast<unsigned>(grid), 256, 0, s>>>(a, v);
-  return cudaGetLastError();
+template <typename R, int KIND, bool WIN, int MODE>
+__global__ void __launch_bounds__(256, KIND == GATHER_DIAG ? 4 : 3)
+    gather_kernel(const __grid_constant__ ElemArgs A, const __grid_constant__ V2Args V) {
+  gather_block<R, KIND, WIN, MODE>(A, V, blockIdx.x);
 }
 
 template <typename R, int KIND>
-cudaError_t launch_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, cudaStream_t s) {
-  auto kern = gather_kernel<R, KIND, false, false>;
+cudaError_t launch_t(bool forces, const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, cudaStream_t s) {
+  auto kern = gather_kernel<R, KIND, false, OVER>;
   if constexpr (KIND == GATHER_FULL || KIND == GATHER_DIAG) {
-    kern = v.node_order ? (v.accumulate ? gather_kernel<R, KIND, true, true> : gather_kernel<R, KIND, true, false>)
-                        : (v.accumulate ? gather_kernel<R, KIND, false, true> : kern);
+    if (forces)
+      kern = v.node_order ? gather_kernel<R, KIND, true, FORCES> : gather_kernel<R, KIND, false, FORCES>;
+    else if (v.accumulate)
+      kern = v.node_order ? gather_kernel<R, KIND, true, ADD> : gather_kernel<R, KIND, false, ADD>;
+    else if (v.node_order)
+      kern = gather_kernel<R, KIND, true, OVER>;
   }
   const int warps = cfg.p2_warps > 0 ? std::min(cfg.p2_warps, 8) : kWarps;
   const int64_t count = v.n_end - v.n_begin;
   if (count <= 0) return cudaSuccess;
-  const int64_t block_nodes = static_cast<int64_t>(warps) * (KIND == GATHER_ONE_DOF ? 10 : 1);
-  const int64_t grid = (count + block_nodes - 1) / block_nodes;
   ElemArgs A = a;
   V2Args V = v;
+  const int64_t grid = gather_grid(V, forces, count, warps * (KIND == GATHER_ONE_DOF ? 10 : 1), warps * 32);
   void* args[] = {&A, &V};
   return launch_kernel(reinterpret_cast<const void*>(kern), grid, warps * 32, 0, s, args);
 }
@@ -449,15 +479,14 @@ cudaError_t launch_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, c
 
 cudaError_t launch_gather(int kind, bool tangent, const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg,
                           cudaStream_t s) {
-  cudaError_t e;
+  const bool forces = tangent && a.f_int;
   switch (kind) {
-    case GATHER_FULL: e = launch_t<double, GATHER_FULL>(a, v, cfg, s); break;
-    case GATHER_DIAG: e = launch_t<float, GATHER_DIAG>(a, v, cfg, s); break;
-    case GATHER_SCALAR: e = launch_t<double, GATHER_SCALAR>(a, v, cfg, s); break;
-    case GATHER_ONE_DOF: e = launch_t<double, GATHER_ONE_DOF>(a, v, cfg, s); break;
+    case GATHER_FULL: return launch_t<double, GATHER_FULL>(forces, a, v, cfg, s);
+    case GATHER_DIAG: return launch_t<float, GATHER_DIAG>(forces, a, v, cfg, s);
+    case GATHER_SCALAR: return launch_t<double, GATHER_SCALAR>(false, a, v, cfg, s);
+    case GATHER_ONE_DOF: return launch_t<double, GATHER_ONE_DOF>(false, a, v, cfg, s);
     default: return cudaErrorInvalidValue;
   }
-  return e == cudaSuccess && tangent ? launch_forces(a, v, s) : e;
 }
 
 // ---- one gather for a batch of element-type groups ------------------------------------
@@ -476,17 +505,19 @@ static_assert(sizeof(GatherPass) <= 4096, "batch pass arguments exceed the kerne
 
 // Slot k owns blocks [blk0_k, blk0_{k+1}) of the grid; the arguments are read in place
 // from the parameter space.
-template <typename R, int KIND>
-__global__ void __launch_bounds__(256) gather_batch_kernel(const __grid_constant__ GatherPass P) {
+template <typename R, int KIND, int MODE>
+__global__ void __launch_bounds__(256, KIND == GATHER_DIAG ? 4 : 3)
+    gather_batch_kernel(const __grid_constant__ GatherPass P) {
   int k = 0;
   while (k + 1 < P.n && static_cast<int64_t>(blockIdx.x) >= P.s[k + 1].blk0) ++k;
   const GatherSlot& S = P.s[k];
-  gather_node<R, KIND, false, false>(S.a, S.v, blockIdx.x - static_cast<unsigned>(S.blk0));
+  gather_block<R, KIND, false, MODE>(S.a, S.v, blockIdx.x - static_cast<unsigned>(S.blk0));
 }
 
 template <typename R, int KIND>
-cudaError_t launch_batch_t(const BatchSlotIn* in, int n, cudaStream_t s) {
-  auto kern = gather_batch_kernel<R, KIND>;
+cudaError_t launch_batch_t(bool tangent, const BatchSlotIn* in, int n, cudaStream_t s) {
+  const bool forces = tangent && in[0].a.f_int;
+  auto kern = forces ? gather_batch_kernel<R, KIND, FORCES> : gather_batch_kernel<R, KIND, OVER>;
   GatherPass P{};
   int warps = 0;  // one block shape for every slot: the smallest that was asked for
   for (int k = 0; k < n; ++k)
@@ -497,7 +528,7 @@ cudaError_t launch_batch_t(const BatchSlotIn* in, int n, cudaStream_t s) {
     P.s[k].a = in[k].a;
     P.s[k].v = in[k].v;
     P.s[k].blk0 = blk;
-    blk += (in[k].v.n_end - in[k].v.n_begin + warps - 1) / warps;
+    blk += gather_grid(P.s[k].v, forces, in[k].v.n_end - in[k].v.n_begin, warps, warps * 32);
   }
   if (blk <= 0) return cudaSuccess;
   P.n = n;
@@ -508,13 +539,8 @@ cudaError_t launch_batch_t(const BatchSlotIn* in, int n, cudaStream_t s) {
 }  // namespace
 
 cudaError_t launch_gather_batch(int kind, bool tangent, const BatchSlotIn* in, int n, cudaStream_t s) {
-  if (tangent)
-    for (int k = 0; k < n; ++k) {
-      const cudaError_t e = launch_forces(in[k].a, in[k].v, s);
-      if (e != cudaSuccess) return e;
-    }
-  if (kind == GATHER_DIAG) return launch_batch_t<float, GATHER_DIAG>(in, n, s);
-  if (kind == GATHER_FULL) return launch_batch_t<double, GATHER_FULL>(in, n, s);
+  if (kind == GATHER_DIAG) return launch_batch_t<float, GATHER_DIAG>(tangent, in, n, s);
+  if (kind == GATHER_FULL) return launch_batch_t<double, GATHER_FULL>(tangent, in, n, s);
   return cudaErrorInvalidValue;
 }
 

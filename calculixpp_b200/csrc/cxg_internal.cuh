@@ -160,7 +160,7 @@ struct V2Args {
   const double* f_ext;      // [3N] load vector for the rhs, or null
   int npe, nbp;             // nodes and (padded) blocks per element
   int named_twice;          // some element names a node at two places
-  int accumulate;           // add into vals / rhs / f_int instead of overwriting
+  int accumulate;           // add into vals / rhs instead of overwriting
   // The window of one element-pass + row-gather pair: the element pass integrates
   // elements [e_begin, e_end), the row gather the nodes node_order[n_begin..n_end)
   // (node_order null: nodes n_begin..n_end in mesh order). The element buffers hold
@@ -174,6 +174,7 @@ struct V2Args {
   int32_t n_win;
   const int64_t* win_e;
   const int64_t* win_n;
+  uint32_t force_blocks, force_every;  // set by the gather's launcher
 };
 // Launch shape of the two passes. tile: node-pair tile of the mixed-precision linear element
 // pass (0 = 2x4, 1 = 2x2, 2 = 4x4; the others have one shape); p1_blocks_per_sm: persistent
