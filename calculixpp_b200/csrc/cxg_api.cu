@@ -425,7 +425,6 @@ ElemArgs base_args(cxg_plan* p) {
   a.elem_mat = p->elem_mat;
   a.mats = p->mats;
   a.node = p->pat.node;
-  a.node_mask = p->pat.node_mask;
   a.prescribed = p->prescribed;
   a.pairs = p->pat.pairs;
   a.bnd = p->pat.bnd;

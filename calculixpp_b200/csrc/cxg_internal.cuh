@@ -120,7 +120,6 @@ struct ElemArgs {
   const J2Mat* mats;        // [n_mats]
   // DOF map / CSR addressing (row gather), see PatternOut
   const NodeRec* node;        // [N]
-  const uint8_t* node_mask;   // [N] bit i: component i free
   const double* prescribed;   // [3N]
   const PairRec* pairs;
   const BndRec* bnd;
