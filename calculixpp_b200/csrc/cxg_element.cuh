@@ -221,8 +221,8 @@ struct P1Shape {
 // FP64 element pass (cxg_fp64.cu): one launch, and the batch kernel with its figures.
 cudaError_t launch_p1_fp64(int t, int mode, const ElemArgs& a, const V2Args& v, const LaunchCfg& c, cudaStream_t s);
 const void* p1_fp64_batch(int mode);
-// After an FP64 element pass of a plan whose elements name nodes twice (launch_p1_fp64 does it).
-cudaError_t launch_named_twice(const ElemArgs& a, const V2Args& v, cudaStream_t s);
+// After an element pass: nothing to do unless some element names a node twice.
+cudaError_t launch_named_twice(int precision, const ElemArgs& a, const V2Args& v, cudaStream_t s);
 P1Shape p1_fp64_shape(int t, int mode);
 
 }  // namespace cxg

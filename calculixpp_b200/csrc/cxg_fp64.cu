@@ -467,20 +467,23 @@ cudaError_t launch_t(const ElemArgs& a, const V2Args& v, const LaunchCfg& cfg, c
 }
 
 // Elements that name a mesh node at two places a < b: the gather adds block (a, b) for the
-// pair and again for (b, a), K_ab + K_ab^T in all, so it is given the symmetric part. A pass of
-// its own, for the meshes that have such elements: a comparison where the blocks are staged cost
-// every mesh 2 to 7 % of the element pass (C3D20 41x37x33 529 -> 543 us, C3D4 87 -> 93).
+// pair and again for (b, a), K_ab + K_ab^T in all, so it is given the symmetric part; zeros in
+// FP32, where the gather forms all of a node's own block. A pass of its own, for the meshes that
+// have such elements: a comparison where the blocks are staged cost every mesh 1 to 7 % of the
+// element pass (C3D20 41x37x33 FP64 529 -> 543 us, C3D4 87 -> 93, C3D8 J2 mixed 292 -> 297).
+template <typename R>
 __global__ void __launch_bounds__(256) named_twice_kernel(ElemArgs A, V2Args V) {
   for (int64_t e = V.e_begin + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < V.e_end;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    double* blocks = reinterpret_cast<double*>(V.edata) + ring_slot(e, V) * (V.nbp * 9);
+    R* blocks = reinterpret_cast<R*>(V.edata) + ring_slot(e, V) * (V.nbp * 9);
     const int32_t* id = A.conn + e * V.npe;
     for (int a = 0; a < V.npe; ++a)
       for (int b = a + 1; b < V.npe; ++b) {
         if (id[a] != id[b]) continue;
-        double* k = blocks + blk_index(V.npe, a, b) * 9;
+        R* k = blocks + blk_index(V.npe, a, b) * 9;
         for (int x = 0; x < 3; ++x)
-          for (int y = x + 1; y < 3; ++y) k[3 * x + y] = k[3 * y + x] = 0.5 * (k[3 * x + y] + k[3 * y + x]);
+          for (int y = x; y < 3; ++y)
+            k[3 * x + y] = k[3 * y + x] = sizeof(R) == 4 ? R(0) : R(0.5) * (k[3 * x + y] + k[3 * y + x]);
       }
   }
 }
@@ -711,10 +714,14 @@ cudaError_t launch_scalar_pass(int t, int kind, const ElemArgs& a, const V2Args&
   }
 }
 
-cudaError_t launch_named_twice(const ElemArgs& a, const V2Args& v, cudaStream_t s) {
+cudaError_t launch_named_twice(int precision, const ElemArgs& a, const V2Args& v, cudaStream_t s) {
   const int64_t count = v.e_end - v.e_begin;
   if (!v.named_twice || count <= 0) return cudaSuccess;
-  named_twice_kernel<<<static_cast<unsigned>(std::min<int64_t>((count + 255) / 256, 148 * 8)), 256, 0, s>>>(a, v);
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((count + 255) / 256, 148 * 8));
+  if (precision)
+    named_twice_kernel<float><<<grid, 256, 0, s>>>(a, v);
+  else
+    named_twice_kernel<double><<<grid, 256, 0, s>>>(a, v);
   return cudaGetLastError();
 }
 
@@ -737,7 +744,7 @@ cudaError_t launch_p1_fp64(int t, int mode, const ElemArgs& a, const V2Args& v, 
 #undef CXG_P1
     default: break;
   }
-  return e == cudaSuccess ? launch_named_twice(a, v, s) : e;
+  return e == cudaSuccess ? launch_named_twice(0, a, v, s) : e;
 }
 
 const void* p1_fp64_batch(int mode) {

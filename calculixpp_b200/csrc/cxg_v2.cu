@@ -485,11 +485,11 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
               for (int al = 0; al < 4; ++al) hd = fma(W.gam[ei][al * 8 + a], W.gam[ei][al * 8 + b], hd);
               h = static_cast<R>(hd * W.kappa[ei]);
             }
+            // FP32 diagonal blocks are not used: the gather forms them (GATHER_DIAG)
+            const bool drop = a == b;
             R* d = stg + ei * WS::kElem + blk_index(n, a, b) * 9;
             // in mesh order of the two nodes: transposed when b precedes a
             const int na = W.id[ei][a], nb = W.id[ei][b], sx = na > nb ? 1 : 3, sy = 4 - sx;
-            // FP32 blocks of a mesh node with itself are not used: the gather forms them (GATHER_DIAG)
-            const bool drop = na == nb;
 #pragma unroll
             for (int x = 0; x < 3; ++x)
 #pragma unroll
@@ -646,8 +646,9 @@ cudaError_t launch_p1_tile(const ElemArgs& a, const V2Args& v, const LaunchCfg& 
   ElemArgs A = a;
   V2Args V = v;
   void* args[] = {&A, &V};
-  return launch_persistent(reinterpret_cast<const void*>(kern), smem, (count + per_block - 1) / per_block,
-                           cfg.p1_blocks_per_sm, s, args);
+  const cudaError_t e = launch_persistent(reinterpret_cast<const void*>(kern), smem, (count + per_block - 1) / per_block,
+                                          cfg.p1_blocks_per_sm, s, args);
+  return e == cudaSuccess ? launch_named_twice(1, a, v, s) : e;
 }
 
 // Tile shapes of the FP32 pass: 2x4, 2x2 and 4x4 in linear mode. The material-point pass
@@ -845,7 +846,7 @@ cudaError_t launch_p1_batch(int mode, int precision, bool j2f32, const BatchSlot
   P.n = n;
   void* args[] = {&P};
   cudaError_t e = launch_kernel(kern, blk, kT1, smem, s, args);
-  for (int k = 0; k < n && e == cudaSuccess && !precision; ++k) e = launch_named_twice(in[k].a, in[k].v, s);
+  for (int k = 0; k < n && e == cudaSuccess; ++k) e = launch_named_twice(precision, in[k].a, in[k].v, s);
   return e;
 }
 
