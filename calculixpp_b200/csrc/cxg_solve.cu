@@ -48,12 +48,36 @@ __device__ __forceinline__ double2 sum_parts(const double* p, int np, const doub
   return block_sum(u, v);
 }
 
+// Sum over the lane's entries of a row of len entries, W loads of each kind in flight: a loop
+// that the compiler unrolls takes the last of them one by one, and most rows are shorter than
+// one round of it.
+template <int W>
+__device__ __forceinline__ double row_sum(const double* v, const int32_t* cols, int len, const double* x, int lane) {
+  double s = 0.0;
+  for (int c0 = lane; c0 < len; c0 += 32 * W) {
+    double xc[W], a[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const int c = c0 + 32 * i;
+      xc[i] = a[i] = 0.0;
+      if (c < len) {
+        xc[i] = __ldg(x + __ldg(cols + c));
+        a[i] = __ldg(v + c);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < W; ++i) s = fma(a[i], xc[i], s);
+  }
+  return s;
+}
+
 // y = A x, and with parts the block's share of x . y. NODES: a plan's own pattern, whose
 // nodes' rows share one column structure: a warp per node reads each column index and
 // each entry of x once for up to three rows, which are three independent streams of
-// values (a warp per row, 8-byte values with 4-byte columns and one load in flight per
-// lane, read 203,400 rows of 79 entries in 53 us on a B200; this way 41 us, and 39 in
-// alternate directions). Otherwise a warp per row. back: from the last row to the first;
+// values (us, one warp a row / one load in flight / two: C3D8 48^3 92 / 70 / 55, C3D20 22^3
+// 55 / 68 / 47, C3D10 18^3 42 / 48 / 33). Otherwise a warp per row: rows of up to 96 entries in
+// one round of three loads, longer ones eight at a time (the reference pattern's rows, C3D8 48^3
+// 94 us one at a time, 77 so; C3D20 40^3 314 and 304). back: from the last row to the first;
 // products one after the other that change direction find in L2 what the last one read
 // last (a matrix a little larger than L2 is otherwise evicted just before its next use).
 template <bool NODES>
@@ -74,12 +98,26 @@ __global__ void __launch_bounds__(kSpmvThreads, 4) spmv_kernel(int32_t nrows, co
       const double *v0 = v + base, *v1 = nf > 1 ? v0 + L : v0, *v2 = nf > 2 ? v1 + L : v1;
       const int32_t* cols = ci + base;
       double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-#pragma unroll 1  // 64 warps a SM with 32 registers each beat more loads per warp
-      for (int c = lane; c < L; c += 32) {
-        const double xc = __ldg(x + __ldg(cols + c));
-        s0 = fma(__ldg(v0 + c), xc, s0);
-        s1 = fma(__ldg(v1 + c), xc, s1);
-        s2 = fma(__ldg(v2 + c), xc, s2);
+      constexpr int W = 2;  // (as in row_sum; 32 registers, 64 warps a SM: three spill and lose)
+      for (int c0 = lane; c0 < L; c0 += 32 * W) {
+        double xc[W], a0[W], a1[W], a2[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const int c = c0 + 32 * i;
+          xc[i] = a0[i] = a1[i] = a2[i] = 0.0;
+          if (c < L) {
+            xc[i] = __ldg(x + __ldg(cols + c));
+            a0[i] = __ldg(v0 + c);
+            a1[i] = __ldg(v1 + c);
+            a2[i] = __ldg(v2 + c);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          s0 = fma(a0[i], xc[i], s0);
+          s1 = fma(a1[i], xc[i], s1);
+          s2 = fma(a2[i], xc[i], s2);
+        }
       }
       for (int off = 16; off > 0; off >>= 1) {
         s0 += __shfl_xor_sync(0xffffffffu, s0, off);
@@ -96,10 +134,9 @@ __global__ void __launch_bounds__(kSpmvThreads, 4) spmv_kernel(int32_t nrows, co
   } else {
     for (int64_t w = w0; w < nrows; w += nw) {
       const int64_t r = back ? nrows - 1 - w : w;
-      const int64_t end = rp[r + 1];
-      double s = 0.0;
-#pragma unroll 4
-      for (int64_t k = rp[r] + lane; k < end; k += 32) s = fma(v[k], x[ci[k]], s);
+      const int64_t begin = rp[r];
+      const int len = static_cast<int>(rp[r + 1] - begin);
+      double s = len <= 96 ? row_sum<3>(v + begin, ci + begin, len, x, lane) : row_sum<8>(v + begin, ci + begin, len, x, lane);
       for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
       if (lane == 0) {
         y[r] = s;
