@@ -66,9 +66,11 @@ struct DGeo {
   static constexpr int EPB = n > 8 ? (nq == 27 ? 1 : nq == 4 ? 4 : 2) : (nq == 8 ? 4 : 8);
   static constexpr int ES = EPB == 1 ? kRaw : (kRaw + 15) / 16 * 16 + 8;
   static constexpr int kElem = blocks_padded(n) * 9;
-  // Staged blocks: one element, leaving as one bulk copy, or one tile pair.
-  static constexpr bool BULK = NTL == 1;
-  static constexpr int kStage = BULK ? kElem : 578;
+  // Staged blocks: one element, leaving as one bulk copy, or one tile pair. C3D4, with four
+  // nodes and one point, would fill a sixteenth of a product: its lanes take a block each
+  // (PAIRS), and a batch's elements are staged together.
+  static constexpr bool BULK = NTL == 1, PAIRS = n == 4 && nq == 1;
+  static constexpr int kStage = PAIRS ? EPB * kElem : BULK ? kElem : 578;
   // (rows of 8 blocks, one value further from row 2 and two from row 6 on: a half warp's
   // stores then lie in different banks; C3D20 536 -> 529 us)
   static __host__ __device__ constexpr int stage_row(int r) { return r * 72 + (r + 2) / 4; }
@@ -291,6 +293,61 @@ __device__ __forceinline__ void p1d_body(const ElemArgs& A, const V2Args& V, uns
         for (int d = 0; d < 3; ++d) V.fdata[ring_slot(e, V) * (3 * n) + 3 * a + d] = f[d];
       }
     }
+    if constexpr (G::PAIRS) {
+      // ---- blocks, one node pair a lane (196,608 C3D4, J2: element pass 182 us by products, 101 so)
+      bulk_wait_read();  // the last batch's copies have left
+      __syncwarp();
+      for (int t = lane; t < EPB * (n * (n + 1) / 2); t += 32) {
+        const int ei = t / (n * (n + 1) / 2), blk = t - ei * (n * (n + 1) / 2);
+        if (e0 + ei >= e_end) break;
+        int a = 0;
+        while (blk >= blk_index(n, a + 1, a + 1)) ++a;
+        const int b = blk - blk_index(n, a, a) + a;
+        double ga[3], gb[3], k[3][3];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+          ga[x] = W.g[ei * ES + x * P + a * QS];
+          gb[x] = W.g[ei * ES + x * P + b * QS];
+        }
+        const double sl = TAN ? W.dp[ei][0][0] : W.s[ei][0] * W.lam[ei], sm = TAN ? W.dp[ei][1][0] : W.s[ei][0] * W.mu[ei];
+        const double tr = sm * (ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2]);
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+#pragma unroll
+          for (int y = 0; y < 3; ++y)
+            k[x][y] = fma(sl, mul(ga[x], gb[y]), mul(sm, mul(ga[y], gb[x]))) + (x == y ? tr : 0.0);
+        if (TAN && W.plastic[ei]) {
+          const double sc = W.dp[ei][2][0];
+          auto turned = [&](const double (&v)[3], double (&m)[3]) {  // m = N g
+            const auto& N = W.N[ei];
+            m[0] = fma(N[0][0], v[0], fma(N[3][0], v[1], mul(N[4][0], v[2])));
+            m[1] = fma(N[3][0], v[0], fma(N[1][0], v[1], mul(N[5][0], v[2])));
+            m[2] = fma(N[4][0], v[0], fma(N[5][0], v[1], mul(N[2][0], v[2])));
+          };
+          double ma[3], mb[3];
+          turned(ga, ma);
+          turned(gb, mb);
+#pragma unroll
+          for (int x = 0; x < 3; ++x)
+#pragma unroll
+            for (int y = 0; y < 3; ++y) k[x][y] = fma(-sc, mul(ma[x], mb[y]), k[x][y]);
+        }
+        const int sx = W.id[ei][a] > W.id[ei][b] ? 1 : 3, sy = 4 - sx;
+        double* d = W.stg + ei * G::kElem + blk * 9;
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+#pragma unroll
+          for (int y = 0; y < 3; ++y) d[x * sx + y * sy] = k[x][y];
+      }
+      fence_async_shared();
+      __syncwarp();
+      if (lane < EPB && e0 + lane < e_end) {
+        bulk_store(reinterpret_cast<double*>(V.edata) + ring_slot(e0 + lane, V) * G::kElem, W.stg + lane * G::kElem,
+                   G::kElem * sizeof(double));
+        bulk_commit();
+      }
+      continue;
+    }
     // ---- blocks, one element after the other, one pair of node tiles at a time
     const int row = lane >> 2, col = lane & 3, turn = G::turn(row);
 #pragma unroll 1
@@ -444,7 +501,7 @@ __device__ __forceinline__ void p1d_body(const ElemArgs& A, const V2Args& V, uns
     }
     __syncwarp();
   }
-  if (G::BULK && lane == 0) bulk_wait();
+  if (G::PAIRS || (G::BULK && lane == 0)) bulk_wait();
 }
 
 template <int ET, bool TAN>
