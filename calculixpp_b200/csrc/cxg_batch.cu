@@ -137,16 +137,19 @@ cudaError_t launch_group(cxg_batch* b, Group& g, double* vals, double* rhs, cons
   return launch_v2(p->type, MODE_LINEAR, b->precision, a, v, s, override_cfg ? *override_cfg : p->cfg[b->precision]);
 }
 
-// Element-pass time of a group when the tuner has not measured it, in units that all groups
-// share: node pairs x (Gauss points + block stores).
-double p1_estimate(int t, int64_t ne) {
-  const double n = nodes_of(t), nq = gauss_of(t);
-  return static_cast<double>(ne) * n * n * (nq + 4.0);
-}
+// Element-pass time of one element in ns, FP64 and mixed, linear and material-point, by family:
+// measured on blocks of 87,000 to 280,000 elements (a B200 at 1965 MHz).
+constexpr double kPassNs[2][2][8] = {
+    {{0.21, 1.80, 0.70, 0.80, 11.1, 5.05, 0.52, 2.79}, {0.43, 2.99, 1.42, 1.59, 21.0, 10.6, 1.05, 5.02}},
+    {{0.21, 1.10, 0.74, 0.79, 6.44, 3.54, 0.48, 2.26}, {0.36, 2.05, 1.90, 1.52, 16.7, 8.20, 0.82, 7.06}}};
+static_assert(C3D4 == 0 && C3D10 == 1 && C3D8 == 2 && C3D8R == 3 && C3D20 == 4 && C3D20R == 5 && C3D6 == 6 && C3D15 == 7,
+              "order of kPassNs");
 
 // Every group as one slot of the one-launch kernels. Linear mode when u is null, else
-// the material-point (tangent) assembly. Weights are the tuned times when every group
-// has one, else the estimates.
+// the material-point (tangent) assembly. Weights are the tuned times of the linear pass when
+// every group has one (for the material-point pass in the ratio of kPassNs), else kPassNs. (Nine
+// small models, eight families, us of the element pass with node pairs x points as weight and
+// with these: FP64 linear 70 and 41, mixed material-point 204 and 136.)
 int fill_slots(cxg_batch* b, const double* u, double* vals, double* f_int, double* rhs, const double* f_ext,
                cudaStream_t s, std::vector<BatchSlotIn>& slots) {
   const int pr = b->precision ? 1 : 0;
@@ -178,7 +181,9 @@ int fill_slots(cxg_batch* b, const double* u, double* vals, double* f_int, doubl
     in.cfg = tan ? p->tcfg[pr] : p->cfg[pr];
     in.cfg.tile = tan ? 1 : g.ftile[pr];
     in.cfg.p2_warps = b->fwarps[pr];
-    in.p1_weight = tuned ? g.fms1[pr] : p1_estimate(g.type, p->n_elems);
+    const double* ns = kPassNs[pr][0];
+    in.p1_weight = tuned ? g.fms1[pr] : static_cast<double>(p->n_elems) * ns[g.type];
+    if (tan) in.p1_weight *= kPassNs[pr][1][g.type] / ns[g.type];
     slots.push_back(in);
   }
   return CXG_OK;
