@@ -34,10 +34,10 @@ namespace {
 struct Group {
   int32_t type = 0;
   cxg_plan* plan = nullptr;
-  // one-launch mode, per precision: element-pass tile and the slot's pass times in ms
+  // one-launch mode, per precision: element-pass tile and the slot's element-pass time in ms
   // from the tuner (0: estimated from the element count and family)
   int ftile[2] = {1, 1};
-  double fms1[2] = {0.0, 0.0}, fms2[2] = {0.0, 0.0};
+  double fms1[2] = {0.0, 0.0};
   int64_t node0 = 0, vals0 = 0, rhs0 = 0;  // offsets in the batch's node / vals / rhs order
   cudaStream_t side = nullptr;               // branch stream of the graph
   cudaEvent_t join = nullptr;
@@ -91,7 +91,7 @@ struct cxg_batch {
   int32_t key_precision = -1;
   uint64_t key_cfg = 0;
   int32_t launch = CXG_BATCH_PER_GROUP;
-  int fwarps[2] = {0, 0};  // one-launch row gather: warps per block (0: as many as fit, <= 8)
+  int fwarps[2] = {0, 0};  // one-launch row gather: warps per block (0: 4)
 };
 
 namespace {
@@ -102,10 +102,9 @@ uint64_t cfg_hash(const cxg_batch* b) {
     for (int pr = 0; pr < 2; ++pr) {
       const LaunchCfg& c = g.plan->cfg[pr];
       for (int v : {c.tile, c.p1_blocks_per_sm, c.p2_warps}) h = (h ^ static_cast<uint64_t>(v + 7)) * 1099511628211ull;
-      uint64_t w1 = 0, w2 = 0;
+      uint64_t w1 = 0;
       std::memcpy(&w1, &g.fms1[pr], 8);
-      std::memcpy(&w2, &g.fms2[pr], 8);
-      for (uint64_t v : {static_cast<uint64_t>(g.ftile[pr]), w1, w2}) h = (h ^ v) * 1099511628211ull;
+      for (uint64_t v : {static_cast<uint64_t>(g.ftile[pr]), w1}) h = (h ^ v) * 1099511628211ull;
     }
   for (int v : {b->launch, b->fwarps[0], b->fwarps[1]}) h = (h ^ static_cast<uint64_t>(v + 7)) * 1099511628211ull;
   return h;
@@ -157,7 +156,7 @@ int fill_slots(cxg_batch* b, const double* u, double* vals, double* f_int, doubl
   if (b->groups.size() > static_cast<size_t>(kMaxBatchSlots))
     return set_err(CXG_ERR_UNSUPPORTED, "one-launch batch holds at most 8 element-type groups");
   bool tuned = true;
-  for (const Group& g : b->groups) tuned = tuned && g.fms1[pr] > 0.0 && g.fms2[pr] > 0.0;
+  for (const Group& g : b->groups) tuned = tuned && g.fms1[pr] > 0.0;
   slots.clear();
   for (Group& g : b->groups) {
     cxg_plan* p = g.plan;
@@ -336,7 +335,6 @@ int tune_one_launch(cxg_batch* b, double* vals, double* rhs, const double* f_ext
       const CacheEntry& c = cache[cache_key(b, g) + "/one-launch"];
       g.ftile[pr] = c.tile;
       g.fms1[pr] = c.p1_ms;
-      g.fms2[pr] = c.p2_ms;
       b->fwarps[pr] = c.warps;
     }
   } else {
@@ -376,22 +374,24 @@ int tune_one_launch(cxg_batch* b, double* vals, double* rhs, const double* f_ext
       }
     }
     b->fwarps[pr] = best_warps;
+    std::vector<double> gather_ms(b->groups.size(), 0.0);  // for the cache's readers
     for (size_t gi = 0; gi < b->groups.size() && !rc; ++gi) {
       std::vector<BatchSlotIn> one(1, all[gi]);
       one[0].cfg.p2_warps = best_warps;
       double ms = 0.0;
       if ((rc = time_one(b, one, 2, s, e0, e1, &ms))) break;
-      b->groups[gi].fms2[pr] = ms > 0.0 ? ms : 0.0;
+      gather_ms[gi] = ms > 0.0 ? ms : 0.0;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc) return rc;
-    for (Group& g : b->groups) {
+    for (size_t gi = 0; gi < b->groups.size(); ++gi) {
+      const Group& g = b->groups[gi];
       CacheEntry c;
       c.tile = g.ftile[pr];
       c.warps = b->fwarps[pr];
       c.p1_ms = g.fms1[pr];
-      c.p2_ms = g.fms2[pr];
+      c.p2_ms = gather_ms[gi];
       cache[cache_key(b, g) + "/one-launch"] = c;
     }
     *changed = true;

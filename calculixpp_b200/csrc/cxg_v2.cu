@@ -392,9 +392,9 @@ __device__ __forceinline__ void p1_body(const ElemArgs& A, const V2Args& V, unsi
         }
         double lt, mt, ct, mhg;
         // FP64 return, or with J2F32 the FP32 return (with the FP64 band near yield)
-        const int r = (sizeof(R) == 8 || !J2F32) ? kJ2Fp64
-                                     : j2_point_mixed(A.mats[mat], W.lam[ei], W.mu[ei], W.mu_j2[ei], eps, cs, ts, sig,
-                                                      lt, mt, ct, nv, mhg);
+        const int r = !J2F32 ? kJ2Fp64
+                             : j2_point_mixed(A.mats[mat], W.lam[ei], W.mu[ei], W.mu_j2[ei], eps, cs, ts, sig, lt, mt, ct,
+                                              nv, mhg);
         const bool pl = r == kJ2Fp64
                             ? j2_point(A.mats[mat], W.lam[ei], W.mu[ei], W.mu_j2[ei], eps, cs, ts, sig, lt, mt, ct, nv, mhg)
                             : r != 0;
@@ -742,11 +742,6 @@ cudaError_t launch_v2(int t, int mode, int precision, const ElemArgs& a, const V
 }
 
 // ---- one launch per pass for a batch of element-type groups ---------------------------
-template <int ET, int MODE, typename R, int TILE, bool J2F32>
-__device__ __forceinline__ void p1_slot(const ElemArgs& A, const V2Args& V, unsigned bid, unsigned nblk) {
-  p1_body<ET, MODE, R, TILE, J2F32>(A, V, bid, nblk);
-}
-
 // The batch kernels carry the tiles whose accumulators fit 168 registers, so that 3
 // blocks of 4 warps stay resident per SM whatever families share the launch: 2x2
 // everywhere and 2x4 in the mixed-precision linear pass.
@@ -758,11 +753,11 @@ template <int ET, int MODE, typename R, bool J2F32>
 __device__ __forceinline__ void p1_slot_tile(int tile, const ElemArgs& A, const V2Args& V, unsigned bid, unsigned nblk) {
   if constexpr (MODE == MODE_LINEAR && sizeof(R) == 4) {
     if (tile == 0) {
-      p1_slot<ET, MODE, R, 0, J2F32>(A, V, bid, nblk);
+      p1_body<ET, MODE, R, 0, J2F32>(A, V, bid, nblk);
       return;
     }
   }
-  p1_slot<ET, MODE, R, 1, J2F32>(A, V, bid, nblk);
+  p1_body<ET, MODE, R, 1, J2F32>(A, V, bid, nblk);
 }
 
 template <int MODE, typename R, bool J2F32>
