@@ -37,8 +37,9 @@ constexpr unsigned kAll = 0xffffffffu;
 // even out (a grid of resident blocks striding over the nodes: C3D20 64^3 mixed 2885 us,
 // this way 2218; blocks of 8 warps 2330).
 constexpr int kWarps = 4;
-// Grids that are resident at once on a B200 let the next kernel on the stream start early.
-constexpr unsigned kOneWave = 148 * 6;
+// Grids that are resident at once on a B200, 24 warps a SM whatever the block, let the next
+// kernel on the stream start early.
+__device__ __forceinline__ bool one_wave() { return gridDim.x * (blockDim.x >> 5) <= 148 * 24; }
 // (Registers: 64 a thread where the blocks are FP32, bound by the launch bounds: C3D20 64^3
 // 2190 us without, 2007 with; 68 where they are FP64, 64 spill there.)
 
@@ -290,7 +291,7 @@ __device__ __forceinline__ void gather_node(const ElemArgs& A, const V2Args& V, 
   // (the records are the plan's own; blocks and outputs are other kernels' too, and are
   // read with plain loads, since the element pass may still be writing when this starts)
   wait_for_kernel_before();
-  if (gridDim.x <= kOneWave) let_next_kernel_start();
+  if (one_wave()) let_next_kernel_start();
   if (!ma) return;
   if (L != 3 * K) {
     gather_compressed<R, KIND, WIN, ADD>(A, V, a);
@@ -348,7 +349,7 @@ __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& 
   if (on) nd = load_node(A.node + a);
   const bool free = (nd.len_mask >> 28) & 1, full = (nd.len_mask & 0xfffffff) == nd.npair;
   wait_for_kernel_before();
-  if (gridDim.x <= kOneWave) let_next_kernel_start();
+  if (one_wave()) let_next_kernel_start();
   double rr = 0.0;
   if (free) {
     int p = q == 0 ? 0 : q == 1 ? nd.pair1 : nd.pair2;
@@ -395,7 +396,7 @@ __device__ __forceinline__ void node_forces(const ElemArgs& A, const V2Args& V, 
   const int64_t first = 3 * (WIN ? V.n_begin : 0), last = 3 * (WIN ? V.n_end : A.n_nodes);
   const int64_t t = first + static_cast<int64_t>(bid) * blockDim.x + threadIdx.x;
   wait_for_kernel_before();
-  if (gridDim.x <= kOneWave) let_next_kernel_start();
+  if (one_wave()) let_next_kernel_start();
   if (t >= last) return;
   const int64_t a = WIN ? static_cast<int64_t>(V.node_order[t / 3]) : t / 3;
   const int d = static_cast<int>(t % 3);
