@@ -5,8 +5,9 @@
 // pattern is built once per mesh and DOF map, in canonical sorted CSR form, node by node:
 //   1. the node -> element incidence comes from one stable sort of the connectivity;
 //   2. one warp per node gathers the nodes of its incident elements (its candidates, in
-//      element order), and orders them by (node, position) in shared memory: equal nodes
-//      are then one neighbour of the node and its contributions in element order;
+//      element order), and orders them by (node, position) in shared memory (lists of more
+//      than 2048 by a block each beforehand): equal nodes are then one neighbour of the node
+//      and its contributions in element order;
 //   3. a first sweep counts: neighbours, the row length (all rows of a node share one
 //      column structure, the free components of its neighbours, ascending), the cuts of
 //      the contribution list; scans over the nodes give every node its place in the CSR
@@ -150,6 +151,73 @@ __device__ int order_candidates(const Sweep& S, int64_t a, Cand* k) {
   return cnt;
 }
 
+// Nodes with more candidates than a warp's list in shared memory holds (kList): a block each
+// orders them, in shared memory up to kBlockList of them, and both sweeps read the result.
+// (In the sweeps themselves, one warp and every node's list in global memory, a fan of 360
+// wedges took 3.0 ms for a plan, 1.0 so; with a sort of all pairs 2.2.)
+constexpr int kList = 2048, kBlockList = 16384, kHubThreads = 1024;
+struct Hub {
+  int64_t at;  // its list's place
+  int32_t node;
+};
+struct HubTotals {
+  unsigned long long count, cands;
+};
+
+__device__ __forceinline__ int64_t power_of_two(int64_t n) {
+  int64_t m = 2;
+  while (m < n) m *= 2;
+  return m;
+}
+
+// hubs null: their number and their lists' total length.
+__global__ void hubs_kernel(Sweep S, int64_t n_nodes, HubTotals* t, Hub* hubs) {
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n_nodes;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t cnt = (S.inc_ptr[a + 1] - S.inc_ptr[a]) * S.npe;
+    if (cnt <= kList) continue;
+    const unsigned long long i = atomicAdd(&t->count, 1ull), at = atomicAdd(&t->cands, static_cast<unsigned long long>(power_of_two(cnt)));
+    if (hubs) hubs[i] = Hub{static_cast<int64_t>(at), static_cast<int32_t>(a)};
+  }
+}
+
+__global__ void __launch_bounds__(kHubThreads) sort_hubs_kernel(Sweep S, const Hub* hubs, int64_t n_hubs, Cand* lists) {
+  extern __shared__ Cand sh[];
+  for (int64_t h = blockIdx.x; h < n_hubs; h += gridDim.x) {
+    const int64_t a = hubs[h].node, i0 = S.inc_ptr[a], cnt = (S.inc_ptr[a + 1] - i0) * S.npe, m = power_of_two(cnt);
+    Cand* out = lists + hubs[h].at;
+    Cand* k = m <= kBlockList ? sh : out;
+    for (int64_t c = threadIdx.x; c < m; c += kHubThreads)
+      k[c] = Cand{static_cast<int32_t>(c),
+                  c < cnt ? S.conn[static_cast<int64_t>(S.inc_code[i0 + c / S.npe] / S.npe) * S.npe + c % S.npe] : 0x7fffffff};
+    __syncthreads();
+    for (int64_t len = 2; len <= m; len *= 2)
+      for (int64_t d = len / 2; d > 0; d /= 2) {
+        for (int64_t t = threadIdx.x; t < m / 2; t += kHubThreads) {
+          const int64_t lo = 2 * t - (t & (d - 1)), hi = lo + d;
+          const Cand x = k[lo], y = k[hi];
+          if ((y < x) == ((lo & len) == 0)) {
+            k[lo] = y;
+            k[hi] = x;
+          }
+        }
+        __syncthreads();
+      }
+    if (k != out)
+      for (int64_t c = threadIdx.x; c < cnt; c += kHubThreads) out[c] = k[c];
+    __syncthreads();
+  }
+}
+
+// The nodes of a sweep: those with lists of at most kList candidates, ordered in the warp's
+// part of shared memory, or the hubs, whose lists are ordered (HUBS).
+template <bool HUBS>
+struct Nodes {
+  int64_t n;         // nodes, or hubs
+  const Hub* hubs;
+  Cand* lists;
+};
+
 // Neighbours before and contribution runs: calls at(r, p, first) for every candidate rank
 // r on its lane, p its neighbour's position and first whether it opens that neighbour.
 template <class F>
@@ -166,16 +234,32 @@ __device__ void each_candidate(const Cand* k, int cnt, F at) {
   }
 }
 
+// Node a and its ordered candidates k for number a of the sweep; returns how many, or less than
+// none for a hub, which has a sweep of its own.
+__device__ __forceinline__ int candidates(const Sweep& S, const Nodes<false>&, int64_t& a, Cand*& k) {
+  if ((S.inc_ptr[a + 1] - S.inc_ptr[a]) * S.npe > kList) return -1;
+  return order_candidates(S, a, k);
+}
+__device__ __forceinline__ int candidates(const Sweep& S, const Nodes<true>& N, int64_t& a, Cand*& k) {
+  const Hub h = N.hubs[a];
+  a = h.node;
+  k = N.lists + h.at;
+  return static_cast<int>(S.inc_ptr[a + 1] - S.inc_ptr[a]) * S.npe;
+}
+
 // First sweep: counts, row length, cuts.
-__global__ void __launch_bounds__(kWarps * 32) count_kernel(Sweep S, int64_t n_nodes, const uint8_t* mask, int cap,
-                                                            Cand* big, NodeRec* node, int64_t* node_nnz,
-                                                            int64_t* bnd_len, int64_t* n_rec, BuildFlags* f) {
+template <bool HUBS>
+__global__ void __launch_bounds__(kWarps * 32) count_kernel(Sweep S, Nodes<HUBS> N, const uint8_t* mask, int cap,
+                                                            NodeRec* node, int64_t* node_nnz, int64_t* bnd_len,
+                                                            int64_t* n_rec, BuildFlags* f) {
   extern __shared__ Cand sh[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t gw = static_cast<int64_t>(blockIdx.x) * kWarps + warp, nw = static_cast<int64_t>(gridDim.x) * kWarps;
-  Cand* k = big ? big + gw * cap : sh + warp * cap;
-  for (int64_t a = gw; a < n_nodes; a += nw) {
-    const int cnt = order_candidates(S, a, k);
+  for (int64_t w = gw; w < N.n; w += nw) {
+    Cand* k = sh + warp * cap;
+    int64_t a = w;
+    const int cnt = candidates(S, N, a, k);
+    if (cnt < 0) continue;
     int len = 0, K = 0, self = 0, own = 0;
     // the neighbour starts nearest to one and two thirds of the contributions
     int cut[2] = {cnt, cnt}, pos[2] = {0, 0}, err[2] = {3 * cnt + 1, 3 * cnt + 1};
@@ -233,18 +317,21 @@ __global__ void __launch_bounds__(kWarps * 32) count_kernel(Sweep S, int64_t n_n
 }
 
 // Second sweep: the CSR rows, the records and the lists of the compressed-row nodes.
-__global__ void __launch_bounds__(kWarps * 32) write_kernel(Sweep S, int64_t n_nodes, const uint8_t* mask,
+template <bool HUBS>
+__global__ void __launch_bounds__(kWarps * 32) write_kernel(Sweep S, Nodes<HUBS> N, const uint8_t* mask,
                                                             const int32_t* eq0, const double* prescribed,
-                                                            const int64_t* node_base,
-                                                            const int64_t* bnd_ptr, const int64_t* rec_ptr, int cap,
-                                                            Cand* big, NodeRec* node, int64_t* row_ptr,
-                                                            int32_t* col_idx, PairRec* pairs, BndRec* bnd) {
+                                                            const int64_t* node_base, const int64_t* bnd_ptr,
+                                                            const int64_t* rec_ptr, int cap, NodeRec* node,
+                                                            int64_t* row_ptr, int32_t* col_idx, PairRec* pairs,
+                                                            BndRec* bnd) {
   extern __shared__ Cand sh[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t gw = static_cast<int64_t>(blockIdx.x) * kWarps + warp, nw = static_cast<int64_t>(gridDim.x) * kWarps;
-  Cand* k = big ? big + gw * cap : sh + warp * cap;
-  for (int64_t a = gw; a < n_nodes; a += nw) {
-    const int cnt = order_candidates(S, a, k);
+  for (int64_t w = gw; w < N.n; w += nw) {
+    Cand* k = sh + warp * cap;
+    int64_t a = w;
+    const int cnt = candidates(S, N, a, k);
+    if (cnt < 0) continue;
     NodeRec nd = node[a];
     const int cut1 = static_cast<int>(nd.pad[0]), cut2 = static_cast<int>(nd.pad[1]);
     const int L = static_cast<int>(nd.len_mask), ma = mask[a], nfa = __popc(ma), K = nd.npair;
@@ -364,7 +451,7 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
 
   // What stays with the plan and has a known size, and the build's scratch: one block each.
   void* scratch = nullptr;
-  void* big = nullptr;
+  void* hub_mem = nullptr;
   Parts keep, tmp;
   const size_t k_mask = keep.add<uint8_t>(n_nodes), k_node = keep.add<NodeRec>(n_nodes),
                k_row = keep.add<int64_t>(static_cast<size_t>(n_free) + 1), k_inc = keep.add<int64_t>(n_nodes + 1),
@@ -376,7 +463,7 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
   cub::DeviceScan::ExclusiveSum(nullptr, scan32, static_cast<int32_t*>(nullptr), static_cast<int32_t*>(nullptr), in, s);
   cub::DeviceScan::ExclusiveSum(nullptr, scan64, static_cast<int64_t*>(nullptr), static_cast<int64_t*>(nullptr), in, s);
   const size_t cub_bytes = std::max(sort_bytes, std::max(scan32, scan64));
-  const size_t t_flags = tmp.add<BuildFlags>(1), t_max = tmp.add<int>(1), t_cub = tmp.add<char>(cub_bytes),
+  const size_t t_flags = tmp.add<BuildFlags>(1), t_max = tmp.add<int>(1), t_hubs = tmp.add<HubTotals>(2), t_cub = tmp.add<char>(cub_bytes),
                t_eq0 = tmp.add<int32_t>(n_nodes), t_free = tmp.add<int32_t>(n_nodes), t_scan = tmp.add<int32_t>(n_nodes),
                t_sorted = tmp.add<int32_t>(m), t_codes = tmp.add<int32_t>(m);
   size_t t_len[3], t_off[3];  // node_nnz, bnd_len, n_rec and their scans
@@ -388,7 +475,9 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
   int max_inc = 0, cap = 0;
   int64_t last[3] = {0, 0, 0}, len[3] = {0, 0, 0};
   Sweep S{};
-  unsigned sweep_grid = 0;
+  Nodes<false> nodes{n_nodes, nullptr, nullptr};
+  Nodes<true> hubs{0, nullptr, nullptr};
+  unsigned sweep_grid = 0, hub_grid = 0;
   size_t sweep_smem = 0;
   {
     CXG_TRY(device_alloc(&out->mem[0], keep.bytes));
@@ -439,27 +528,41 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
       rc = 5;
       goto done;
     }
-    // The sweeps' candidate lists: shared memory up to 2048 per warp (64 KB a block), one
-    // slice of global memory per warp beyond.
-    for (cap = 2; cap < max_inc * npe && cap < 1 << 30;) cap *= 2;
+    S = Sweep{d_conn, out->inc_ptr, out->inc_code, npe, blocks_padded(npe)};
+    for (cap = 2; cap < max_inc * npe && cap < kList;) cap *= 2;
     sweep_smem = sizeof(Cand) * kWarps * static_cast<size_t>(cap);
     sweep_grid = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((n_nodes + kWarps - 1) / kWarps, 65536)));
-    if (cap > 2048) {
-      sweep_grid = std::min(sweep_grid, 256u);
-      sweep_smem = 0;
-      CXG_TRY(device_alloc(&big, sizeof(Cand) * static_cast<size_t>(cap) * kWarps * sweep_grid));
-    } else {
-      CXG_TRY(allow_smem(reinterpret_cast<const void*>(count_kernel), sweep_smem));
-      CXG_TRY(allow_smem(reinterpret_cast<const void*>(write_kernel), sweep_smem));
+    CXG_TRY(allow_smem(reinterpret_cast<const void*>(count_kernel<false>), sweep_smem));
+    CXG_TRY(allow_smem(reinterpret_cast<const void*>(write_kernel<false>), sweep_smem));
+    if (static_cast<int64_t>(max_inc) * npe > kList) {
+      HubTotals* totals = part<HubTotals>(scratch, t_hubs);  // counted, then taken up again while the lists are placed
+      HubTotals h{};
+      CXG_TRY(cudaMemsetAsync(totals, 0, 2 * sizeof(HubTotals), s));
+      hubs_kernel<<<grid_for(n_nodes), 256, 0, s>>>(S, n_nodes, totals, nullptr);
+      CXG_TRY(cudaMemcpyAsync(&h, totals, sizeof h, cudaMemcpyDeviceToHost, s));
+      CXG_TRY(cudaStreamSynchronize(s));
+      Parts hp;
+      const size_t h_hub = hp.add<Hub>(h.count), h_list = hp.add<Cand>(h.cands);
+      CXG_TRY(device_alloc(&hub_mem, hp.bytes));
+      hubs = Nodes<true>{static_cast<int64_t>(h.count), part<Hub>(hub_mem, h_hub), part<Cand>(hub_mem, h_list)};
+      hub_grid = static_cast<unsigned>(std::min<int64_t>((hubs.n + kWarps - 1) / kWarps, 65536));
+      hubs_kernel<<<grid_for(n_nodes), 256, 0, s>>>(S, n_nodes, totals + 1, part<Hub>(hub_mem, h_hub));
+      CXG_TRY(cudaGetLastError());
+      CXG_TRY(allow_smem(reinterpret_cast<const void*>(sort_hubs_kernel), sizeof(Cand) * kBlockList));
+      sort_hubs_kernel<<<static_cast<unsigned>(std::min<int64_t>(hubs.n, 65536)), kHubThreads, sizeof(Cand) * kBlockList, s>>>(
+          S, hubs.hubs, hubs.n, hubs.lists);
+      CXG_TRY(cudaGetLastError());
     }
-    S = Sweep{d_conn, out->inc_ptr, out->inc_code, npe, blocks_padded(npe)};
     int64_t *lens[3], *offs[3];
     for (int i = 0; i < 3; ++i) {
       lens[i] = part<int64_t>(scratch, t_len[i]);
       offs[i] = part<int64_t>(scratch, t_off[i]);
     }
-    count_kernel<<<sweep_grid, kWarps * 32, sweep_smem, s>>>(S, n_nodes, out->node_mask, cap, static_cast<Cand*>(big),
-                                                             out->node, lens[0], lens[1], lens[2], f);
+    count_kernel<false><<<sweep_grid, kWarps * 32, sweep_smem, s>>>(S, nodes, out->node_mask, cap, out->node, lens[0],
+                                                                    lens[1], lens[2], f);
+    if (hub_grid)
+      count_kernel<true><<<hub_grid, kWarps * 32, 0, s>>>(S, hubs, out->node_mask, 0, out->node, lens[0], lens[1],
+                                                          lens[2], f);
     CXG_TRY(cudaGetLastError());
     for (int i = 0; i < 3; ++i) {
       cb = cub_bytes;
@@ -489,16 +592,20 @@ int build_pattern(int elem_type, int64_t n_nodes, int64_t n_elems, const int32_t
     out->pairs = part<PairRec>(out->mem[1], r_pairs);
     out->bnd = part<BndRec>(out->mem[1], r_bnd);
     CXG_TRY(cudaMemcpyAsync(out->row_ptr + n_free, &out->nnz, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    write_kernel<<<sweep_grid, kWarps * 32, sweep_smem, s>>>(S, n_nodes, out->node_mask, eq0, d_prescribed, offs[0],
-                                                             offs[1], offs[2], cap, static_cast<Cand*>(big), out->node, out->row_ptr,
-                                                             out->col_idx, out->pairs, out->bnd);
+    write_kernel<false><<<sweep_grid, kWarps * 32, sweep_smem, s>>>(S, nodes, out->node_mask, eq0, d_prescribed, offs[0],
+                                                                    offs[1], offs[2], cap, out->node, out->row_ptr,
+                                                                    out->col_idx, out->pairs, out->bnd);
+    if (hub_grid)
+      write_kernel<true><<<hub_grid, kWarps * 32, 0, s>>>(S, hubs, out->node_mask, eq0, d_prescribed, offs[0], offs[1],
+                                                          offs[2], 0, out->node, out->row_ptr, out->col_idx, out->pairs,
+                                                          out->bnd);
     CXG_TRY(cudaGetLastError());
     CXG_TRY(cudaStreamSynchronize(s));
   }
 
 done:
   cudaStreamSynchronize(s);  // (an error may have left work on the scratch)
-  device_free(big);
+  device_free(hub_mem);
   device_free(scratch);
   return rc;
 }

@@ -7,6 +7,8 @@
 * device buffers that start between two doubles, for the history and the nodal flux;
 * accumulation onto any values: each entry the rounded sum of what was there and what an
   assembly alone gives, in rows with and without prescribed columns;
+* an edge with 4096 and 4200 elements around it: candidate lists that fill the shared memory of
+  a block, and longer ones;
 * elements that name a node two or three times: hexahedra collapsed to wedges, against the
   oracle. In mixed precision 1e-5: FP32 blocks of about 2e2 x 6e-8.
 
@@ -20,6 +22,7 @@ import torch
 from calculixpp_b200 import Batch, Material, Model, Plan, ThermalPlan, _lib
 from calculixpp_b200 import meshgen as mg
 from oracle.oracle import make_material
+from tests.test_gpu_edges import check_linear, constrained, shuffled
 from tests.helpers import ISO_TABLE, box_model, per_element_materials, rel_fro, to_np
 
 pytestmark = pytest.mark.gpu
@@ -166,3 +169,14 @@ def test_accumulation_is_the_sum(cuda, etype, precision):
         v, r = v0.clone(), r0.clone()
         plan.accumulate_linear(v, r)
         assert torch.equal(v, v0 + vals) and torch.equal(r, r0 + rhs)
+
+
+@pytest.mark.parametrize("count", [4096, 4200])
+def test_large_fan_around_an_edge(cuda, port, count):
+    rng = np.random.default_rng(count)
+    a = 2.0 * np.pi * np.arange(count) / count
+    ring = np.stack([np.cos(a), np.sin(a), np.zeros(count)], axis=1)
+    i = np.arange(count)
+    conn = np.stack([np.zeros_like(i), 2 + i, 2 + (i + 1) % count, np.ones_like(i)], axis=1).astype(np.int32)
+    fan = mg.Mesh(np.concatenate([[[0.0, 0.0, -0.5], [0.0, 0.0, 0.5]], ring]), conn, mg.C3D4)
+    check_linear(port, constrained(shuffled(fan, rng), rng, 0.1))
