@@ -1,4 +1,5 @@
-// P2, the row gather: every CSR value written exactly once, no atomics, no shared memory.
+// P2, the row gather: every CSR value written exactly once, no atomics, no shared memory (an
+// accumulating assembly adds each value once, as a reduction in L2).
 //
 // One warp per node a. The plan lists the element blocks that contribute to a's node pairs
 // (a, b), pair by pair and in element order, in records of 11 (NodeRec, PairRec). Three
@@ -9,17 +10,17 @@
 // number of records, so a round is straight-line code: 11 block reads in flight per lane,
 // the next record fetched meanwhile.
 //
-// What bounds it: the L1's wavefronts (66 % of its rate) and issue slots. The element
+// What bounds it: the L1's wavefronts (%L1% of its rate) and issue slots. The element
 // blocks come in from HBM once and the values go out once; in between the L1 serves every
 // block twice (rows of a and of b), one contribution to a read of nine lanes. Against the
-// rows summed in shared memory: C3D8 J2 128^3 3852 -> 2815 us, C3D20 64^3 mixed 3141 ->
-// 2005.
+// rows summed in shared memory: C3D8 J2 128^3 3852 -> 2798 us, forces included, C3D20 64^3
+// mixed 3141 -> 1899.
 //
 // Mixed precision (DIAG) forms the diagonal block as minus the FP64 sum of the row's
 // other entries (per group, then the three groups in order; the element pass stores the
 // blocks (a, a) as zeros), so rigid translations stay in the null space to FP64 accuracy.
-// Interior nodes (every neighbour fully free) write full-width rows; at the others the list
-// of neighbours gives each pair's compressed column, and prescribed columns go to the rhs
+// Interior nodes (every neighbour fully free) write full-width rows; at the others each
+// pair's record (BndRec) gives its compressed column, and prescribed columns go to the rhs
 // (-K_fc u_c, src/fem/assembly.cpp:95-96).
 #include <cuda_runtime.h>
 
@@ -356,6 +357,9 @@ __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& 
     const PairRec* list = A.pairs + nd.list0 + q;
     double* o = A.vals + nd.base;
     double v = 0.0;
+    const BndRec* list_b = A.bnd + nd.bnd0 + p;
+    BndRec b{};
+    if (!full) b = load_bnd(list_b);
     for (uint32_t r = 0; r < nd.rounds; ++r, list += 3) {
       const PairRec rec = load_pairs(list);
       double x[UN];
@@ -368,13 +372,13 @@ __device__ __forceinline__ void gather_one_dof(const ElemArgs& A, const V2Args& 
           if (full) {
             o[p] = v;
           } else {
-            const BndRec b = load_bnd(A.bnd + nd.bnd0 + p);
             if ((b.at >> 28) & 1) {
               o[b.at & 0xfffffff] = v;
             } else if (b.at >> 31) {
               const double u = A.prescribed[3 * static_cast<int64_t>(b.node)];
               if (u != 0.0) rr -= v * u;
             }
+            b = load_bnd(++list_b);
           }
           v = 0.0;
           ++p;
