@@ -19,7 +19,7 @@
 // What bounds it: latency of the phases a warp goes through in turn, with the matrix unit
 // 46 % and the shared-memory pipe 56 % busy on C3D20 (8 or 12 warps per SM ran alike).
 // C3D8 J2 128^3 4605 us with tiles of FMAs, 3087 so; C3D20 41x37x33
-// linear 510 -> 529 us, for a gather that takes 438 us instead of 574 from the blocks' order.
+// linear 510 -> 529 us, for a gather that takes 408 us instead of 574 from the blocks' order.
 //
 // Lanes first take (element, Gauss point) tasks: Jacobian, inverse, gradients, and in
 // material-point mode the strain and the J2 return, as in the FP32 pass.

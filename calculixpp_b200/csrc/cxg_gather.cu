@@ -10,7 +10,7 @@
 // number of records, so a round is straight-line code: 11 block reads in flight per lane,
 // the next record fetched meanwhile.
 //
-// What bounds it: the L1's wavefronts (%L1% of its rate) and issue slots. The element
+// What bounds it: the L1's wavefronts (66 to 69 % of its rate) and issue slots. The element
 // blocks come in from HBM once and the values go out once; in between the L1 serves every
 // block twice (rows of a and of b), one contribution to a read of nine lanes. Against the
 // rows summed in shared memory: C3D8 J2 128^3 3852 -> 2798 us, forces included, C3D20 64^3
