@@ -171,6 +171,18 @@ def test_accumulation_is_the_sum(cuda, etype, precision):
         assert torch.equal(v, v0 + vals) and torch.equal(r, r0 + rhs)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_accumulation_in_windows(cuda, precision):
+    model = box_model(mg.C3D8, 32, 2, 3, prescribe=1e-3)
+    with Plan(model, precision) as plan:
+        vals, rhs = plan.assemble_linear()
+        plan.set_ring_bytes(192 * 36 * (72 if precision == "fp64" else 36))
+        v, r = vals.clone(), rhs.clone()
+        plan.accumulate_linear(v, r)
+        assert plan.windows()[0] > 1
+        assert torch.equal(v, vals + vals) and torch.equal(r, rhs + rhs)
+
+
 @pytest.mark.parametrize("count", [4096, 4200])
 def test_large_fan_around_an_edge(cuda, port, count):
     rng = np.random.default_rng(count)
